@@ -218,8 +218,8 @@ class _OnTape:
         return out
 
     def begin(self):
-        for name in self.bufs:
-            self.tape.zero_accumulated_gradient(self.ids[name])
+        for nid in self.ids.values():
+            self.tape.zero_accumulated_gradient(nid)
 
 
 def prepare(case, seed):
