@@ -132,6 +132,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// The same wait made by a whole converged warp, with one answer for the warp.  The roles that issue TMA copies and MMAs use
+// it together with warp_index(): their control flow is then uniform for the compiler, loop state and descriptors live in
+// uniform registers, and an elect_one() region issues its instructions back to back.  With `threadIdx.x >> 5`, per-lane
+// waits and `lane == 0` regions the same four MMAs and a commit took 418 cycles (256 x 128 pair tile: 256 cycles of work).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const WaitCtx& c, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const bool ok = mbar_wait(bar, parity, c, code);
+  return __all_sync(0xffffffffu, ok);
+}
+// Set-up barrier among `threads` threads (hardware barrier 1; nothing can have aborted yet where it is used).
+__device__ __forceinline__ void setup_barrier(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Barrier among the warps that share `bar` (initialised with one arrival per warp), with the
 // same bounded wait as everything else: a warp that left through an abort never arrives, and the
 // others give up when they see the abort flag or run out of budget, where a named hardware
@@ -284,6 +297,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
 // addresses of the two CTAs differ in bit 24 of the shared::cluster window, so clearing that
 // bit in a barrier address names the leader's barrier.  No copy here is multicast.
 // ----------------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 constexpr uint32_t FT_PEER_BIT_MASK = 0xFEFFFFFFu;
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -413,6 +432,52 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, int a_mn, i
 // ----------------------------------------------------------------------------
 // small math helpers
 // ----------------------------------------------------------------------------
+// Two fp32 lanes per instruction (each lane rounded as its scalar form).
+struct f32x2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 up2(f32x2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+// Unsigned division by a run-time constant prepared on the host: n / d for n < 2^31 (Granlund and Montgomery's
+// round-up multiplier).  A work item is decoded by every role of every CTA; a 32-bit divide is ~150 cycles.
+struct FastDiv {
+  uint32_t d, mul, shift;
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  FastDiv() : d(1), mul(1), shift(0) {}
+#ifdef __CUDACC__
+  __host__ __device__
+#endif
+  explicit FastDiv(uint32_t div) : d(div), shift(0) {
+    while ((1ull << shift) < div) ++shift;
+    mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - div)) / div + 1);
+  }
+  __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);

@@ -43,7 +43,7 @@ typedef struct FtkGemmDesc {
   int epi;
   int out_fp32;
   int accumulate;        // D += result
-  int force_bn;          // 0 = heuristic, else 128 or 256
+  int force_bn;          // 0 = heuristic, 128 / 192 / 256 = single-CTA tile, 256 + 128 / 192 / 256 = CTA-pair tile
   int max_ctas;          // 0 = all SMs
   // Deterministic split-K (plain fp32/bf16 store epilogues only): partial tiles go to
   // `workspace` (fp32, split_count*M*N*4 bytes needed) and are summed in ascending split order.

@@ -15,8 +15,7 @@
 //                         accumulate.  The order is fixed, so the sum is reproducible.
 // Every wait on a flag that another CTA or rank sets is bounded and ends in the status word.
 #pragma once
-#include "ft_sm100.cuh"
-#include "ftk_api.h"
+#include "gemm_epilogue.cuh"
 
 namespace ftk {
 
@@ -30,29 +29,6 @@ constexpr int G_COPY_SLOT = 32768;   // bytes per bulk copy of the gather ring
 constexpr int G_COPY_SLOTS = 6;
 constexpr int G_SCATTER_BATCH = 8;   // reduce-scatter tiles per system-scope fence
 constexpr long long G_PEER_WAIT_CYCLES = 4000000000ll;
-
-struct GemmArgs {
-  int M, N, K, L0, L1;
-  int a_mn, b_mn;
-  void* D;
-  long long ldd, d_s0, d_s1;
-  const __nv_bfloat16* bias;
-  const __nv_bfloat16* resid;
-  long long ldr, r_s0, r_s1;
-  __nv_bfloat16* aux;  // optional bf16 copy of the pre-activation (same layout as D)
-  float alpha;
-  int epi;
-  int out_fp32;
-  int accumulate;
-  int splits;          // >1: split-K, partial tiles go to `ws` as fp32 [split][M][N]
-  float* ws;
-  int* status;
-  // Ragged rows (expert batches): the M rows of batch l are segments of `seg_rows` rows of which
-  // only the first seg_counts[l * segs + s] are in use; a 128-row tile without a used row is
-  // skipped by every role (no loads, no MMAs, no stores).  NULL = all rows in use.
-  const int* seg_counts;
-  int seg_rows;
-};
 
 // True when rows [m_t * 128, m_t * 128 + 128) of batch l hold at least one row in use.  Every role of a
 // CTA evaluates this for the same items, so the pipelines stay in step.
@@ -92,113 +68,10 @@ struct GemmCfg {
   static constexpr int STAGES = (BN == 128) ? 6 : 4;
   static constexpr int ACC_STRIDE = (BN == 192) ? 256 : BN;  // TMEM columns between accumulators
   static constexpr int TMEM_COLS = (BN == 128) ? 256 : 512;  // power of two
-  static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + 1024 /*align*/ + 256 /*barriers*/ +
-                              G_EPI_WARPS * 4096 /*output staging tiles*/;
-};
-
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// Epilogue activations use the hardware tanh (relative error ~2^-11, below bf16 rounding).
-__device__ __forceinline__ float gelu_tanh_fast(float x) {
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.f + tanh_fast(u));
-}
-__device__ __forceinline__ float gelu_tanh_grad_fast(float x) {
-  const float x2 = x * x;
-  const float t = tanh_fast(0.7978845608028654f * (x + 0.044715f * x * x2));
-  const float du = 0.7978845608028654f * (1.f + 3.f * 0.044715f * x2);
-  return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
-}
-
-// v[i] = f(v[i], rr[i]) for the 32 values of one row chunk; the switch is outside the loop.
-__device__ __forceinline__ void apply_epi32(float* v, const float* rr, int epi) {
-  switch (epi) {
-    case FTK_EPI_GELU_TANH:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = gelu_tanh_fast(v[i]);
-      break;
-    case FTK_EPI_GELU_ERF:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = gelu_erf_f(v[i]);
-      break;
-    case FTK_EPI_RELU:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = v[i] > 0.f ? v[i] : 0.f;
-      break;
-    case FTK_EPI_MUL_DGELU_TANH:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] *= gelu_tanh_grad_fast(rr[i]);
-      break;
-    case FTK_EPI_MUL_DGELU_ERF:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] *= gelu_erf_grad_f(rr[i]);
-      break;
-    case FTK_EPI_MUL_DRELU:
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = rr[i] > 0.f ? v[i] : 0.f;
-      break;
-    default:
-      break;
-  }
-}
-
-// ------------------------------------------------------------------ coalescing bf16 output stores
-// One warp's staging tile: 32 rows x 128 B in shared memory, 16-byte segments XOR-swizzled by
-// the row.  A thread `put`s the packed bf16 of its row for one 32-column chunk; after two chunks
-// (or at the end of the tile) `flush` reads the tile transposed so that 8 consecutive lanes
-// write 128 contiguous bytes (4 lanes / 64 bytes when only one chunk is staged) of one row.
-struct OutStager {
-  uint8_t* tile;
-  __nv_bfloat16* d_base;       // row 0 of the output (of this batch entry)
-  long long row0, ldd;         // first output row of this warp's slab, leading dimension
-  int M, lane, staged, n_start;
-  bool usable;
-  __device__ __forceinline__ OutStager(uint8_t* t, const GemmArgs& p, __nv_bfloat16* d, long long r0, int ln)
-      : tile(t), d_base(d), row0(r0), ldd(p.ldd), M(p.M), lane(ln), staged(0), n_start(0) {
-    usable = !p.out_fp32 && !p.accumulate && p.splits == 1 && (p.ldd % 8 == 0) &&
-             ((reinterpret_cast<uintptr_t>(d) & 15) == 0);
-  }
-  __device__ __forceinline__ void put(const float* v) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint4 o;
-      o.x = pack_bf16(v[8 * i + 0], v[8 * i + 1]);
-      o.y = pack_bf16(v[8 * i + 2], v[8 * i + 3]);
-      o.z = pack_bf16(v[8 * i + 4], v[8 * i + 5]);
-      o.w = pack_bf16(v[8 * i + 6], v[8 * i + 7]);
-      *reinterpret_cast<uint4*>(tile + lane * 128 + (((staged * 4 + i) ^ (lane & 7)) << 4)) = o;
-    }
-  }
-  __device__ __forceinline__ void chunk_done(int n0) {
-    if (staged == 0) n_start = n0;
-    if (++staged == 2) flush();
-  }
-  __device__ __forceinline__ void flush() {
-    if (staged == 0) return;
-    __syncwarp();
-    if (staged == 2) {
-      const int seg = lane & 7;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int rr = 4 * i + (lane >> 3);
-        const uint4 o = *reinterpret_cast<const uint4*>(tile + rr * 128 + ((seg ^ (rr & 7)) << 4));
-        if (row0 + rr < M) *reinterpret_cast<uint4*>(d_base + (row0 + rr) * ldd + n_start + seg * 8) = o;
-      }
-    } else {
-      const int seg = lane & 3;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int rr = 8 * i + (lane >> 2);
-        const uint4 o = *reinterpret_cast<const uint4*>(tile + rr * 128 + ((seg ^ (rr & 7)) << 4));
-        if (row0 + rr < M) *reinterpret_cast<uint4*>(d_base + (row0 + rr) * ldd + n_start + seg * 8) = o;
-      }
-    }
-    __syncwarp();
-    staged = 0;
-  }
+  static constexpr int OFF_BARS = STAGES * (A_BYTES + B_BYTES);
+  static constexpr int OFF_STAGE = OFF_BARS + 256;                          // epilogue tiles, one per warp
+  static constexpr int OFF_BIAS = OFF_STAGE + G_EPI_WARPS * EPI_STAGE_BYTES;
+  static constexpr int SMEM = OFF_BIAS + G_EPI_WARPS * EPI_BIAS_BYTES;
 };
 
 // ------------------------------------------------------------------ flags between CTAs / ranks
@@ -273,13 +146,11 @@ __device__ __forceinline__ TileCoord decode_item(int item, const GemmArgs& p, co
                                                  int tiles_m, int tiles_n, int nbatch) {
   TileCoord t;
   if (!COMM || c.mode == FTK_COMM_NONE || (c.mode == FTK_COMM_GATHER_B && p.b_mn)) {
-    const int tiles_mn = tiles_m * tiles_n;
-    t.sp = item / (tiles_mn * nbatch);
-    const int rem = item - t.sp * (tiles_mn * nbatch);
-    t.l = rem / tiles_mn;
-    const int tt = rem - t.l * tiles_mn;
-    t.m_t = tt % tiles_m;
-    t.n_t = tt / tiles_m;
+    const int sl = p.by_tiles_mn.div(item), tt = item - sl * tiles_m * tiles_n;
+    t.sp = p.by_batches.div(sl);
+    t.l = sl - t.sp * nbatch;
+    t.n_t = p.by_tiles_m.div(tt);
+    t.m_t = tt - t.n_t * tiles_m;
     return t;
   }
   t.sp = 0;
@@ -665,7 +536,7 @@ struct EpiPusher {
 };
 
 // ------------------------------------------------------------------ the kernel
-template <int BN, int COMM>
+template <int BN, int COMM, int KIND>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
                        const __grid_constant__ CUtensorMap tmB,
@@ -674,12 +545,10 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
   static_assert(!COMM || G_COPY_SLOTS * G_COPY_SLOT <= Cfg::STAGES * (Cfg::A_BYTES + Cfg::B_BYTES),
                 "gather ring must fit the operand ring");
   static_assert(!COMM || 2 * G_COPY_SLOTS <= 2 * Cfg::STAGES + 4, "barrier space");
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sA = smem;
   uint8_t* sB = smem + Cfg::STAGES * Cfg::A_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::STAGES * (Cfg::A_BYTES + Cfg::B_BYTES));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BARS);
   uint64_t* full = bars;
   uint64_t* empty = bars + Cfg::STAGES;
   uint64_t* tfull = bars + 2 * Cfg::STAGES;
@@ -690,9 +559,13 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
   static_assert((2 * Cfg::STAGES + 6) * 8 <= 256, "barrier space");
   uint32_t wbar_ph = 0;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
+  if ((smem_u32(smem) & 1023u) != 0u) {      // swizzled tiles need 1024-byte aligned bases
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
+    return;
+  }
 
   const int n_compute = COMM ? (int)gridDim.x - c.comm_ctas : (int)gridDim.x;
   const bool comm_cta = COMM && (int)blockIdx.x >= n_compute;
@@ -719,13 +592,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     *abort_f = 0;
     fence_mbar_init();
   }
-  if (warp == 1 && !comm_cta) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
-    tmem_relinquish();
+  if (warp == 0 && elect_one()) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
   }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
 
   if (comm_cta) {
     if (COMM) {
@@ -740,22 +611,29 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     __syncthreads();
     return;
   }
-  const uint32_t tmem_base = *tmem_slot;
+  // The producer warp leaves for its loop here; tensor memory is allocated behind its first loads.
+  uint32_t tmem_base = 0;
+  if (warp != 0) {
+    if (warp == 1) {
+      tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+      tmem_relinquish();
+    }
+    tc_fence_before();
+    setup_barrier(G_THREADS - 32);
+    tc_fence_after();
+    tmem_base = *tmem_slot;
+  }
 
-  const int tiles_m = (p.M + G_BM - 1) / G_BM;
+  const int tiles_m = (int)p.by_tiles_m.d;
   const int tiles_n = (p.N + BN - 1) / BN;
-  const int tiles_mn = tiles_m * tiles_n;
-  const int nbatch = p.L0 * p.L1;
+  const int tiles_mn = (int)p.by_tiles_mn.d;
+  const int nbatch = (int)p.by_batches.d;
   const int total = tiles_mn * nbatch * p.splits;  // work item = (split, batch, n tile, m tile)
   const int kblocks_all = (p.K + G_BK - 1) / G_BK;
-  const int kb_per_split = (kblocks_all + p.splits - 1) / p.splits;
+  const int kb_per_split = p.splits > 1 ? (kblocks_all + p.splits - 1) / p.splits : kblocks_all;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
-    }
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
@@ -768,7 +646,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
       const TileCoord t = decode_item<BN, COMM>(item, p, c, tiles_m, tiles_n, nbatch);
       if (!tile_has_rows(p, t.l, t.m_t)) continue;
       const int m_t = t.m_t, n_t = t.n_t;
-      const int l0 = t.l % p.L0, l1 = t.l / p.L0;
+      const int l1 = p.by_l0.div(t.l), l0 = t.l - l1 * p.L0;
       const int kb0 = t.sp * kb_per_split;
       const int kb1 = min(kblocks_all, kb0 + kb_per_split);
       const bool k_sharded = COMM && c.mode == FTK_COMM_GATHER_B && p.b_mn;
@@ -823,11 +701,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           if (!ok) break;
         }
-        if (!mbar_wait(&empty[s], ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) {
+        if (!mbar_wait_warp(&empty[s], ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) {
           ok = false;
           break;
         }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_arrive_expect_tx(&full[s], Cfg::A_BYTES + Cfg::B_BYTES);
           uint8_t* a_dst = sA + s * Cfg::A_BYTES;
           uint8_t* b_dst = sB + s * Cfg::B_BYTES;
@@ -872,19 +750,19 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
         const TileCoord tc = decode_item<BN, COMM>(item, p, c, tiles_m, tiles_n, nbatch);
         if (!tile_has_rows(p, tc.l, tc.m_t)) continue;
       }
-      const int sp = (COMM && c.mode != FTK_COMM_NONE) ? 0 : item / (tiles_mn * nbatch);
+      const int sp = (COMM && c.mode != FTK_COMM_NONE) ? 0 : p.by_batches.div(p.by_tiles_mn.div(item));
       const int kb0 = sp * kb_per_split;
       const int kb1 = min(kblocks_all, kb0 + kb_per_split);
-      if (!mbar_wait(&tempty[acc], ((acc_ph >> acc) & 1u) ^ 1u, ctx, FT_ERR_WAIT_TMEM_EMPTY)) break;
+      if (!mbar_wait_warp(&tempty[acc], ((acc_ph >> acc) & 1u) ^ 1u, ctx, FT_ERR_WAIT_TMEM_EMPTY)) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full[s], ph, ctx, FT_ERR_WAIT_FULL)) {
+        if (!mbar_wait_warp(&full[s], ph, ctx, FT_ERR_WAIT_FULL)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           // descriptor low words of this stage, stepped by (bytes >> 4) per k-step
           const uint32_t a_lo = a_lo0 + (uint32_t)s * (Cfg::A_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + (uint32_t)s * (Cfg::B_BYTES >> 4);
@@ -901,7 +779,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
           ph ^= 1u;
         }
       }
-      if (kb1 <= kb0 && lane == 0) umma_commit(&tfull[acc]);  // empty split: nothing to wait for
+      if (kb1 <= kb0 && elect_one()) umma_commit(&tfull[acc]);  // empty split: nothing to wait for
       __syncwarp();
       acc_ph ^= (1u << acc);
       acc ^= 1;
@@ -911,7 +789,6 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     const int ew = warp - 2;
     const int q = warp & 3;               // TMEM lane quarter this warp may read
     const int half = ew >> 2;             // which half of the tile's columns
-    const int row_in_tile = q * 32 + lane;
     constexpr int CHUNKS = BN / 32;
     constexpr int C_HALF = (CHUNKS + 1) / 2;
     const int c_begin = half == 0 ? 0 : C_HALF;
@@ -921,14 +798,17 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     int pend_owner[G_SCATTER_BATCH], pend_tile[G_SCATTER_BATCH], n_pend = 0;   // scatter: unpublished tiles
     bool epi_ok = true;   // false once this warp gave up a wait: it then skips every later barrier
     const bool ew_push = COMM && c.push == 3 && (c.mode == FTK_COMM_GATHER_A || c.mode == FTK_COMM_GATHER_B);
+    TileEpilogue<KIND> epi(p, smem + Cfg::OFF_STAGE + ew * EPI_STAGE_BYTES,
+                     reinterpret_cast<__nv_bfloat16*>(smem + Cfg::OFF_BIAS + ew * EPI_BIAS_BYTES), lane);
     EpiPusher pusher(c, ew_push, (int)blockIdx.x * G_EPI_WARPS + ew, n_compute * G_EPI_WARPS, lane,
                      c.mode == FTK_COMM_GATHER_A);
     for (int item = blockIdx.x; item < total; item += n_compute) {
       const TileCoord t = decode_item<BN, COMM>(item, p, c, tiles_m, tiles_n, nbatch);
       if (!tile_has_rows(p, t.l, t.m_t)) continue;
       const int sp = t.sp, l = t.l, m_t = t.m_t, n_t = t.n_t;
-      const int l0 = l % p.L0, l1 = l / p.L0;
-      const bool empty_split = (sp * kb_per_split >= kblocks_all);
+      if (!COMM || c.mode != FTK_COMM_SCATTER_D)
+        epi.begin(sp, l, m_t * G_BM + q * 32, n_t * BN + c_begin * 32, c_end - c_begin,
+                  sp * kb_per_split >= kblocks_all);
       if (COMM && ew_push) {
         // push 4 KB of the shard per poll while the accumulator is not ready
         while (pusher.busy()) {
@@ -943,7 +823,6 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
         break;
       }
       tc_fence_after();
-      const long long row = (long long)m_t * G_BM + row_in_tile;
       if (COMM && c.mode == FTK_COMM_SCATTER_D) {
         // partial tile -> inbox of the owning rank, slot of this rank; then one flag per tile
         const int tpc = c.chunk_rows / G_BM;
@@ -954,7 +833,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
         // Peer stores want long contiguous runs: two 32-column chunks are packed to bf16,
         // transposed through a per-warp smem tile (32 rows x 128 B, XOR-swizzled 16-byte
         // segments) and written so that 8 consecutive lanes cover 128 contiguous bytes of a row.
-        uint8_t* stage = smem + Cfg::STAGES * (Cfg::A_BYTES + Cfg::B_BYTES) + 256 + ew * 4096;
+        uint8_t* stage = smem + Cfg::OFF_STAGE + ew * EPI_STAGE_BYTES;
 #pragma unroll 1
         for (int ci = c_begin; ci < c_end; ci += 2) {
           const int c0 = ci * 32;
@@ -1007,144 +886,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
         acc ^= 1;
         continue;
       }
-      const long long d_off = l0 * p.d_s0 + l1 * p.d_s1 + row * p.ldd;
-      const long long r_off = l0 * p.r_s0 + l1 * p.r_s1 + row * p.ldr;
-      const bool need_r = p.resid != nullptr;
-      // bf16 outputs leave through a per-warp smem tile (32 rows x 128 B, XOR-swizzled 16-byte
-      // segments): a thread owns one row of the accumulator, so direct stores would touch 32
-      // rows per instruction with 16 bytes each; after the transpose 8 consecutive lanes write
-      // 128 contiguous bytes of one row.
-      OutStager stager(smem + Cfg::STAGES * (Cfg::A_BYTES + Cfg::B_BYTES) + 256 + ew * 4096, p,
-                       reinterpret_cast<__nv_bfloat16*>(p.D) + l0 * p.d_s0 + l1 * p.d_s1,
-                       (long long)m_t * G_BM + q * 32, lane);
-#pragma unroll 1
-      for (int ci = c_begin; ci < c_end; ++ci) {
-        const int c0 = ci * 32;
-        uint32_t r[32];
-        tmem_ld32(tmem_base + acc * Cfg::ACC_STRIDE + c0 + ((uint32_t)(q * 32) << 16), r);
-        tmem_ld_wait();
-        const int n0 = n_t * BN + c0;
-        const bool stage_this = stager.usable && n0 + 32 <= p.N;     // warp-uniform
-        if (!stage_this) stager.flush();
-        if (row < p.M && n0 < p.N) {
-          float v[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = empty_split ? 0.f : __uint_as_float(r[i]) * p.alpha;
-          const bool full_chunk = (n0 + 32 <= p.N);
-          if (p.splits > 1) {
-            // raw partial tile -> workspace [split][batch][M][N] (fp32)
-            float* wp = p.ws + (((long long)sp * nbatch + l) * p.M + row) * p.N + n0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(wp) & 15) == 0)) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                reinterpret_cast<float4*>(wp)[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (n0 + i < p.N) wp[i] = v[i];
-            }
-            continue;
-          }
-          if (p.bias) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (full_chunk || n0 + i < p.N) v[i] += __bfloat162float(__ldg(p.bias + n0 + i));
-          }
-          if (p.aux) {
-            __nv_bfloat16* ap = p.aux + d_off + n0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(ap) & 15) == 0)) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                uint4 o;
-                o.x = pack_bf16(v[8 * i + 0], v[8 * i + 1]);
-                o.y = pack_bf16(v[8 * i + 2], v[8 * i + 3]);
-                o.z = pack_bf16(v[8 * i + 4], v[8 * i + 5]);
-                o.w = pack_bf16(v[8 * i + 6], v[8 * i + 7]);
-                reinterpret_cast<uint4*>(ap)[i] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (n0 + i < p.N) ap[i] = __float2bfloat16(v[i]);
-            }
-          }
-          float rr[32];
-          if (need_r) {
-            const __nv_bfloat16* rp = p.resid + r_off + n0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(rp) & 15) == 0)) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                uint4 u = __ldg(reinterpret_cast<const uint4*>(rp) + i);
-                float2 f0 = unpack_bf16(u.x), f1 = unpack_bf16(u.y), f2 = unpack_bf16(u.z),
-                       f3 = unpack_bf16(u.w);
-                rr[8 * i + 0] = f0.x; rr[8 * i + 1] = f0.y; rr[8 * i + 2] = f1.x;
-                rr[8 * i + 3] = f1.y; rr[8 * i + 4] = f2.x; rr[8 * i + 5] = f2.y;
-                rr[8 * i + 6] = f3.x; rr[8 * i + 7] = f3.y;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                rr[i] = (n0 + i < p.N) ? __bfloat162float(rp[i]) : 0.f;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) rr[i] = 0.f;
-          }
-          const bool r_is_operand = (p.epi >= FTK_EPI_MUL_DGELU_TANH);
-          if (p.epi != FTK_EPI_NONE) apply_epi32(v, rr, p.epi);
-          if (need_r && !r_is_operand) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] += rr[i];
-          }
-          if (p.out_fp32) {
-            float* dp = reinterpret_cast<float*>(p.D) + d_off + n0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(dp) & 15) == 0)) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                float4 o = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                if (p.accumulate) {
-                  float4 old = reinterpret_cast<float4*>(dp)[i];
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                reinterpret_cast<float4*>(dp)[i] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (n0 + i < p.N) dp[i] = p.accumulate ? dp[i] + v[i] : v[i];
-            }
-          } else if (stage_this) {
-            stager.put(v);
-          } else {
-            __nv_bfloat16* dp = reinterpret_cast<__nv_bfloat16*>(p.D) + d_off + n0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(dp) & 15) == 0)) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                if (p.accumulate) {
-                  uint4 u = reinterpret_cast<uint4*>(dp)[i];
-                  float2 f0 = unpack_bf16(u.x), f1 = unpack_bf16(u.y), f2 = unpack_bf16(u.z),
-                         f3 = unpack_bf16(u.w);
-                  v[8 * i + 0] += f0.x; v[8 * i + 1] += f0.y; v[8 * i + 2] += f1.x;
-                  v[8 * i + 3] += f1.y; v[8 * i + 4] += f2.x; v[8 * i + 5] += f2.y;
-                  v[8 * i + 6] += f3.x; v[8 * i + 7] += f3.y;
-                }
-                uint4 o;
-                o.x = pack_bf16(v[8 * i + 0], v[8 * i + 1]);
-                o.y = pack_bf16(v[8 * i + 2], v[8 * i + 3]);
-                o.z = pack_bf16(v[8 * i + 4], v[8 * i + 5]);
-                o.w = pack_bf16(v[8 * i + 6], v[8 * i + 7]);
-                reinterpret_cast<uint4*>(dp)[i] = o;
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (n0 + i < p.N)
-                  dp[i] = __float2bfloat16(p.accumulate ? __bfloat162float(dp[i]) + v[i] : v[i]);
-            }
-          }
-        }
-        if (stage_this) stager.chunk_done(n0);     // every lane of the warp, also rows past M
-      }
-      stager.flush();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
+      epi.run(tmem_base + acc * Cfg::ACC_STRIDE + c_begin * 32 + ((uint32_t)(q * 32) << 16), c_end - c_begin, [&] {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[acc]);
+      });
       acc_ph ^= (1u << acc);
       acc ^= 1;
     }

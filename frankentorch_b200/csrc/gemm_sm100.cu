@@ -141,55 +141,110 @@ struct PerDeviceOnce {
   }
 };
 
-template <int BN>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a,
-                       int max_ctas, cudaStream_t stream) {
+// Divisors of the work-item decode for tiles of bm x bn.
+static void set_divisors(GemmArgs& a, int bm, int bn) {
+  const uint32_t tm = (uint32_t)((a.M + bm - 1) / bm), tn = (uint32_t)((a.N + bn - 1) / bn);
+  a.by_tiles_m = FastDiv(tm);
+  a.by_tiles_mn = FastDiv(tm * tn);
+  a.by_batches = FastDiv((uint32_t)(a.L0 * a.L1));
+  a.by_l0 = FastDiv((uint32_t)a.L0);
+}
+
+// The epilogue instantiation of a problem: a special kind where its parts are exactly those of the kind and every row is
+// made of 16-byte segments, else the general one.
+static int epilogue_kind(const GemmArgs& a) {
+  const bool any_batch = a.L0 * a.L1 > 1;
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (a.splits > 1)
+    return (a.N % 4 == 0 && al(a.ws)) ? EPI_KIND_F32 : EPI_KIND_ANY;
+  if (!al(a.D) || any_batch) return EPI_KIND_ANY;
+  if (a.out_fp32)
+    return (a.epi == FTK_EPI_NONE && !a.bias && !a.resid && !a.aux && a.ldd % 4 == 0 && a.N % 4 == 0) ? EPI_KIND_F32
+                                                                                                    : EPI_KIND_ANY;
+  if (a.accumulate || a.ldd % 8 || a.N % 8) return EPI_KIND_ANY;
+  if (a.resid && (!al(a.resid) || a.ldr % 8)) return EPI_KIND_ANY;
+  if (a.aux && !al(a.aux)) return EPI_KIND_ANY;
+  if (a.epi == FTK_EPI_NONE && !a.aux) return a.resid ? EPI_KIND_RESID : EPI_KIND_PLAIN;
+  if (a.epi == FTK_EPI_GELU_TANH && !a.resid) return a.aux ? EPI_KIND_GELU_AUX : EPI_KIND_GELU;
+  if (a.epi == FTK_EPI_MUL_DGELU_TANH && a.resid && !a.aux && !a.bias) return EPI_KIND_DGELU;
+  return EPI_KIND_ANY;
+}
+
+template <int BN, int KIND>
+static int launch_gemm_kind(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmArgs a, int max_ctas,
+                            cudaStream_t stream) {
   using Cfg = GemmCfg<BN>;
   static PerDeviceOnce once;
   bool* attr_set_p = once.slot();
   if (!*attr_set_p) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_sm100_kernel<BN, 0>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_sm100_kernel<BN, 0, KIND>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
     *attr_set_p = true;
   }
+  set_divisors(a, G_BM, BN);
   long long items = (long long)((a.M + G_BM - 1) / G_BM) * ((a.N + BN - 1) / BN) * a.L0 * a.L1 * a.splits;
+  if (items > 0x7fffffffll) return -2;
   int grid = (int)(items < max_ctas ? items : max_ctas);
   if (grid <= 0) return 0;
   CommArgs none;
   memset(&none, 0, sizeof(none));
-  gemm_bf16_sm100_kernel<BN, 0><<<grid, G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, tmA, a, none);
+  gemm_bf16_sm100_kernel<BN, 0, KIND><<<grid, G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, tmA, a, none);
   return (int)cudaGetLastError();
 }
 
 // CTA-pair kernel: grid = 2 CTAs per cluster, at most sms / 2 clusters.
-// Relative cost of a pair tile in the tile-choice model (a lone 128 x 256 tile = 1.0); the
-// environment variable FT_GEMM_PAIR_COST overrides it (a large value disables the pair kernel).
-static double pair_tile_cost() {
+// Weight of the pair tiles in the tile-choice model, 0.92 = as measured; the environment variable FT_GEMM_PAIR_COST
+// overrides it (a large value disables the pair kernel).
+static double pair_cost_scale() {
   static double c = -1.0;
   if (c < 0.0) {
     const char* e = getenv("FT_GEMM_PAIR_COST");
-    c = (e && atof(e) > 0.0) ? atof(e) : 0.92;
+    c = (e && atof(e) > 0.0) ? atof(e) / 0.92 : 1.0;
   }
   return c;
 }
-static int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, int max_ctas,
-                            cudaStream_t stream) {
-  using Cfg = Gemm2Cfg;
+template <int BN, int KIND>
+static int launch_gemm_pair_kind(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmArgs a, int max_ctas,
+                                 cudaStream_t stream) {
+  using Cfg = PairCfg<BN>;
   static PerDeviceOnce once;
   bool* attr_set_p = once.slot();
   if (!*attr_set_p) {
-    cudaError_t e = cudaFuncSetAttribute(gemm2_bf16_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm2_bf16_sm100_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::SMEM);
     if (e != cudaSuccess) return (int)e;
     *attr_set_p = true;
   }
-  const long long items = (long long)((a.M + 255) / 256) * ((a.N + 255) / 256) * a.L0 * a.L1 * a.splits;
+  set_divisors(a, 2 * G_BM, BN);
+  const long long items = (long long)((a.M + 255) / 256) * ((a.N + BN - 1) / BN) * a.L0 * a.L1 * a.splits;
+  if (items > 0x7fffffffll) return -2;
   long long pairs = max_ctas / 2;
   if (items < pairs) pairs = items;
   if (pairs <= 0) return 0;
-  gemm2_bf16_sm100_kernel<<<(unsigned)(2 * pairs), G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, a);
+  gemm2_bf16_sm100_kernel<BN, KIND><<<(unsigned)(2 * pairs), G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, a);
   return (int)cudaGetLastError();
+}
+
+template <int BN, bool PAIR>
+static int launch_gemm(int kind, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, int max_ctas,
+                       cudaStream_t stream) {
+#define FT_LAUNCH_KIND(K)                                                                  \
+  case K:                                                                                  \
+    return PAIR ? launch_gemm_pair_kind<BN, K>(tmA, tmB, a, max_ctas, stream)              \
+                : launch_gemm_kind<BN, K>(tmA, tmB, a, max_ctas, stream);
+  switch (kind) {
+    FT_LAUNCH_KIND(EPI_KIND_PLAIN)
+    FT_LAUNCH_KIND(EPI_KIND_RESID)
+    FT_LAUNCH_KIND(EPI_KIND_GELU)
+    FT_LAUNCH_KIND(EPI_KIND_GELU_AUX)
+    FT_LAUNCH_KIND(EPI_KIND_DGELU)
+    FT_LAUNCH_KIND(EPI_KIND_F32)
+    default:
+      return PAIR ? launch_gemm_pair_kind<BN, EPI_KIND_ANY>(tmA, tmB, a, max_ctas, stream)
+                  : launch_gemm_kind<BN, EPI_KIND_ANY>(tmA, tmB, a, max_ctas, stream);
+  }
+#undef FT_LAUNCH_KIND
 }
 
 static int make_operand_maps(const FtkGemmDesc* g, int L0, int L1, int bn, CUtensorMap* tmA,
@@ -267,58 +322,54 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     return -4;
 
   const int sms = g->max_ctas > 0 ? g->max_ctas : num_sms();
-  const long long tiles_m = (g->M + G_BM - 1) / G_BM;
-  // Tile choice: time ~ waves x per-tile cost.  Narrow tiles move more operand bytes per MMA
-  // cycle (measured: a 128-wide tile costs ~0.86 of a 256-wide one for half the work).
+  // Tile choice by modelled time: waves x (fixed cost of a tile + its k-blocks).  A k-block of 64 takes the tensor pipe
+  // 2 BN cycles on one SM or on a pair; with every SM loading, operand delivery from L2 makes that longer by the
+  // measured amounts below, in proportion to the SMs in use.  Measured against the model (us, 256 x 256 / 256 x 192 /
+  // 256 x 128 pairs, then 128 x 256 / 192 / 128; all L2-resident): 8192 x 768 x 3072 36.7 / 31.3 / 34.5, 40.6 / 37.6 / 38.9;
+  // 1500 x 1280 x 5120 29.6 / 23.7 / 19.3, 29.2 / 23.4 / 21.6; 1500 x 3840 x 1280 17.8 / 14.7 / 16.0, 18.6 / 15.5 / 17.9;
+  // 8192 x 2304 x 768 21.9 / 23.0 / 25.0, 24.4 / 26.6 / 27.7.
   // Split-K (weight-gradient shapes: few output tiles, long reduction) is considered when the
   // epilogue is a plain store and the caller supplied a workspace.
   const int kblocks = (g->K + G_BK - 1) / G_BK;
   if (g->seg_counts && g->seg_rows <= 0) return -2;
   const bool splittable = g->epi == FTK_EPI_NONE && !g->bias && !g->resid && !g->aux && g->workspace &&
                           (g->N % 4 == 0) && (g->ldd % 4 == 0) && L0 * L1 == 1 && !g->seg_counts;
-  // Option 512 is the CTA-pair kernel: 256 x 256 tiles on sms / 2 clusters; per SM it does the
-  // work of a 128 x 256 tile with a third less operand traffic.
-  // The unit is the time of one 128 x 256 tile over all of K on one SM at the sustained rate (~6.9 ns per
-  // unit of K).  A split costs the reduction kernel: s fp32 partials read, the output written (and read when
+  // A split costs the reduction kernel: s fp32 partials read, the output written (and read when
   // it accumulates) at ~4 TB/s plus a launch - 17 us for an [8192, 768] bf16 output with two splits, which is
   // why an activation-sized output is hardly ever worth splitting while a weight gradient is.
-  const double unit_us = 6.93e-3 * (double)g->K;
   auto split_penalty = [&](int s) {
     if (s <= 1) return 0.0;
     const double mn = (double)g->M * (double)g->N;
     const double bytes = mn * 4.0 * s + mn * (g->out_fp32 ? 4.0 : 2.0) * (g->accumulate ? 2.0 : 1.0);
-    return (bytes / 4.0e6 + 3.0) / unit_us;
+    return bytes / 4.0e6 + 3.0;
   };
   auto cost = [&](int bn, int s) {
-    if (bn == 512) {
-      const long long tiles = ((g->M + 255) / 256) * ((g->N + 255) / 256) * L0 * L1;
-      const long long waves = (tiles * s + sms / 2 - 1) / (sms / 2);
-      // A pair tile has twice the epilogue of a single one and a longer pipeline fill, which a long K
-      // amortises: measured against 128 x 192 tiles it costs ~1.0 at K = 768 and ~0.72 at K = 3072
-      // (8192 x 768 x 2304: 37.5 vs 45.8 us, x 3072: 47.5 vs 53.0 us), and about a tenth more when B is given
-      // [K, N] (8192 x 3072 x 768: 65.2 vs 54.3 us).  The base value is the K = 768 calibration.
-      double kr = 768.0 * s / (double)g->K;
-      if (kr > 1.5) kr = 1.5;
-      static const bool k_scaled = !(getenv("FT_GEMM_PAIR_KSCALE") && atoi(getenv("FT_GEMM_PAIR_KSCALE")) == 0);
-      const double c = k_scaled ? pair_tile_cost() * (0.608 + 0.392 * kr) * (g->b_mn ? 1.08 : 1.0) : pair_tile_cost();
-      return (double)waves * c / s + split_penalty(s);
-    }
-    const long long tiles = tiles_m * ((g->N + bn - 1) / bn) * L0 * L1;
-    const long long waves = (tiles * s + sms - 1) / sms;
-    const double w = bn == 256 ? 1.0 : (bn == 192 ? 0.80 : 0.86);
-    return (double)waves * w / s + split_penalty(s);
+    const bool pair = bn > 256;
+    const int w = pair ? bn - 256 : bn;
+    const double tile = w == 256 ? 0.4 : (w == 192 ? 0.1 : 0.3);
+    const double mma = w == 256 ? 0.278 : (w == 192 ? 0.21 : 0.143);
+    const double full = pair ? (w == 256 ? 0.375 : (w == 192 ? 0.32 : 0.235)) : (w == 256 ? 0.42 : (w == 192 ? 0.385 : 0.27));
+    const long long items = ((g->M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * (long long)((g->N + w - 1) / w) * L0 * L1 * s;
+    const long long units = pair ? sms / 2 : sms;
+    const long long waves = (items + units - 1) / units;
+    const double busy = items < units ? (double)items / (double)units : 1.0;
+    // the last tile's epilogue and a pair's hand-shakes are not hidden: 128 x 192 x 64 takes 4.1 / 4.7 / 4.8 us on one
+    // SM and 4.6 / 5.1 / 5.3 us on a pair
+    const double exposed = (w == 256 ? 0.75 : (w == 192 ? 0.55 : 0.0)) + (pair ? 0.5 : 0.0);
+    return ((double)waves * (tile + (double)kblocks / s * (mma + (full - mma) * busy)) + exposed) *
+               (pair ? pair_cost_scale() : 1.0) + split_penalty(s);
   };
   auto split_ok = [&](int s) {
     if (s == 1) return true;
     if (!splittable || g->split_k == 1 || kblocks / s < 8) return false;
     return (long long)s * g->M * g->N * 4 <= g->workspace_bytes;
   };
-  static const int bn_opts[4] = {512, 256, 192, 128};
+  static const int bn_opts[6] = {512, 448, 384, 256, 192, 128};
   static const int s_opts[8] = {1, 2, 3, 4, 6, 8, 12, 16};
   int bn = g->force_bn, splits = 1;
   double best = 1e30;
-  for (int bi = 0; bi < 4; ++bi) {
-    if (bn_opts[bi] == 512 && (sms < 2 || g->M < 256 || g->seg_counts)) continue;
+  for (int bi = 0; bi < 6; ++bi) {
+    if (bn_opts[bi] > 256 && (sms < 2 || g->M < 256 || g->seg_counts)) continue;
     if (g->force_bn && bn_opts[bi] != g->force_bn) continue;
     for (int si = 0; si < 8; ++si) {
       const int s = s_opts[si];
@@ -333,20 +384,34 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     }
   }
   if (g->split_k > 1 && split_ok(g->split_k)) splits = g->split_k;
-  if (bn != 128 && bn != 192 && bn != 256 && bn != 512) return -5;
+  if (bn != 128 && bn != 192 && bn != 256 && bn != 384 && bn != 448 && bn != 512) return -5;
   *bn_out = bn;
   *splits_out = splits;
   return 0;
 }
 
+template <int KIND>
+static int launch_group(const GroupMaps& maps, const GroupArgs& ga, int pairs, cudaStream_t stream) {
+  constexpr int SMEM = PairCfg<GG_BN>::SMEM;
+  static PerDeviceOnce once;
+  bool* attr_set_p = once.slot();
+  if (!*attr_set_p) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_group_bf16_sm100_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SMEM);
+    if (e != cudaSuccess) return (int)e;
+    *attr_set_p = true;
+  }
+  gemm_group_bf16_sm100_kernel<KIND><<<2 * pairs, G_THREADS, SMEM, stream>>>(maps, ga);
+  return (int)cudaGetLastError();
+}
+
 // Grouped launch: `n` (1..8) independent products with the same K and operand layouts, fp32 outputs with a plain
-// store or accumulate epilogue, in one persistent kernel of 128 x 192 tiles (see gemm_group_kernel.cuh).
+// store or accumulate epilogue, in one persistent kernel of 256 x 192 pair tiles (see gemm_group_kernel.cuh).
 extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   if (!descs || n < 1 || n > GG_MAX) return -2;
-  GroupArgs ga;
+  GroupArgs ga = {};
   GroupMaps maps;
-  memset(&ga, 0, sizeof(ga));
   memset(&maps, 0, sizeof(maps));
   const FtkGemmDesc& g0 = descs[0];
   ga.n = n; ga.K = g0.K; ga.a_mn = g0.a_mn ? 1 : 0; ga.b_mn = g0.b_mn ? 1 : 0; ga.alpha = g0.alpha;
@@ -363,29 +428,24 @@ extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream
       return -7;
     if ((reinterpret_cast<uintptr_t>(g->A) & 15) || (reinterpret_cast<uintptr_t>(g->B) & 15)) return -3;
     if ((g->lda % 8) || (g->ldb % 8)) return -4;
-    int rc = make_operand_maps(g, 1, 1, GG_BN, &maps.a[p], &maps.b[p]);
+    int rc = make_operand_maps(g, 1, 1, PairCfg<GG_BN>::HALF, &maps.a[p], &maps.b[p]);
     if (rc) return rc;
     ga.M[p] = g->M; ga.N[p] = g->N;
     ga.D[p] = reinterpret_cast<float*>(g->D);
     ga.ldd[p] = g->ldd;
     ga.accumulate[p] = g->accumulate ? 1 : 0;
-    total += ((g->M + G_BM - 1) / G_BM) * ((g->N + GG_BN - 1) / GG_BN);
+    ga.by_tiles_m[p] = FastDiv((uint32_t)((g->M + 2 * G_BM - 1) / (2 * G_BM)));
+    total += ((g->M + 2 * G_BM - 1) / (2 * G_BM)) * ((g->N + GG_BN - 1) / GG_BN);
     ga.tile_end[p] = total;
   }
   for (int p = n; p < GG_MAX; ++p) ga.tile_end[p] = total;
-  using Cfg = GemmCfg<GG_BN>;
-  static PerDeviceOnce once;
-  bool* attr_set_p = once.slot();
-  if (!*attr_set_p) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_group_bf16_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         GG_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    *attr_set_p = true;
-  }
+  bool aligned = true;
+  for (int p = 0; p < n; ++p)
+    aligned = aligned && ga.N[p] % 4 == 0 && ga.ldd[p] % 4 == 0 && (reinterpret_cast<uintptr_t>(ga.D[p]) & 15) == 0;
   const int sms = g0.max_ctas > 0 ? g0.max_ctas : num_sms();
-  const int grid = total < sms ? total : sms;
-  gemm_group_bf16_sm100_kernel<<<grid, G_THREADS, GG_SMEM, stream>>>(maps, ga);
-  return (int)cudaGetLastError();
+  int pairs = sms / 2 > 0 ? sms / 2 : 1;
+  if (total < pairs) pairs = total;
+  return aligned ? launch_group<EPI_KIND_F32>(maps, ga, pairs, stream) : launch_group<EPI_KIND_ANY>(maps, ga, pairs, stream);
 }
 
 // Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile
@@ -404,17 +464,20 @@ extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
   const int sms = g->max_ctas > 0 ? g->max_ctas : num_sms();
 
   CUtensorMap tmA, tmB;
-  int rc = make_operand_maps(g, L0, L1, bn == 512 ? 128 : bn, &tmA, &tmB);   // a pair stages 128 B rows per CTA
+  int rc = make_operand_maps(g, L0, L1, bn > 256 ? (bn - 256) / 2 : bn, &tmA, &tmB);   // a pair stages half of B per CTA
   if (rc) return rc;
 
   GemmArgs a;
   fill_gemm_args(a, g, L0, L1);
   a.splits = splits;
   if (!a.status) return -6;
-  rc = bn == 512 ? launch_gemm_pair(tmA, tmB, a, sms, stream)
-       : bn == 256 ? launch_gemm<256>(tmA, tmB, a, sms, stream)
-                   : (bn == 192 ? launch_gemm<192>(tmA, tmB, a, sms, stream)
-                                : launch_gemm<128>(tmA, tmB, a, sms, stream));
+  const int kind = epilogue_kind(a);
+  rc = bn == 512   ? launch_gemm<256, true>(kind, tmA, tmB, a, sms, stream)
+       : bn == 448 ? launch_gemm<192, true>(kind, tmA, tmB, a, sms, stream)
+       : bn == 384 ? launch_gemm<128, true>(kind, tmA, tmB, a, sms, stream)
+       : bn == 256 ? launch_gemm<256, false>(kind, tmA, tmB, a, sms, stream)
+       : bn == 192 ? launch_gemm<192, false>(kind, tmA, tmB, a, sms, stream)
+                   : launch_gemm<128, false>(kind, tmA, tmB, a, sms, stream);
   if (rc || splits == 1) return rc;
   const long long total4 = ((long long)g->M * g->N) >> 2;
   long long blocks = (total4 + 255) / 256;
@@ -531,11 +594,12 @@ extern "C" int ftk_gemm_comm_bf16(const FtkGemmDesc* g, const FtkCommDesc* cd, v
   static PerDeviceOnce once;
   bool* attr_set_p = once.slot();
   if (!*attr_set_p) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_sm100_kernel<BN, 1>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_sm100_kernel<BN, 1, EPI_KIND_ANY>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, COMM_SMEM);
     if (e != cudaSuccess) return (int)e;
     *attr_set_p = true;
   }
+  set_divisors(a, G_BM, BN);
   const long long items = (long long)((a.M + G_BM - 1) / G_BM) * ((a.N + BN - 1) / BN);
   long long n_compute = sms - c.comm_ctas;
   if (items < n_compute) n_compute = items;
@@ -547,6 +611,6 @@ extern "C" int ftk_gemm_comm_bf16(const FtkGemmDesc* g, const FtkCommDesc* cd, v
   else if (cd->mode == FTK_COMM_GATHER_B && !g->b_mn && cd->chunk_rows >= BN)
     rc = ftk_make_tmap_bf16(&tmOwn, cd->src[cd->rank], g->K, cd->chunk_rows, 1, 1, g->K, 0, 0, G_BK, BN);
   if (rc) return 3000 + rc;
-  gemm_bf16_sm100_kernel<BN, 1><<<grid, G_THREADS, COMM_SMEM, stream>>>(tmA, tmB, tmOwn, a, c);
+  gemm_bf16_sm100_kernel<BN, 1, EPI_KIND_ANY><<<grid, G_THREADS, COMM_SMEM, stream>>>(tmA, tmB, tmOwn, a, c);
   return (int)cudaGetLastError();
 }

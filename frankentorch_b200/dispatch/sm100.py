@@ -94,8 +94,8 @@ def gemm_kernel_name(M: int, N: int, Kd: int, *, a_mn: bool = False, b_mn: bool 
     rc = lib.ftk_gemm_plan(C.byref(g), C.byref(bn), C.byref(sp))
     if rc != 0:
         return "ftk::gemm_bf16_sm100<unplanned>"
-    if bn.value == 512:
-        return f"ftk::gemm2_bf16_sm100<256x256,cta_group2,splitK={sp.value}>"
+    if bn.value > 256:
+        return f"ftk::gemm2_bf16_sm100<256x{bn.value - 256},cta_group2,splitK={sp.value}>"
     return f"ftk::gemm_bf16_sm100<128x{bn.value},splitK={sp.value}>"
 
 

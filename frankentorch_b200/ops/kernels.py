@@ -176,7 +176,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if _TRACE is not None:          # name the tile the planner picks for this problem
         bn, sp = C.c_int(0), C.c_int(1)
         if lib.ftk_gemm_plan(C.byref(g), C.byref(bn), C.byref(sp)) == 0:
-            what = ("ftk::gemm2_bf16_sm100<256x256,cta_group2,splitK=%d>" % sp.value) if bn.value == 512 else \
+            what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn.value - 256, sp.value)) if bn.value > 256 else \
                 ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn.value, sp.value))
     _chk(lib.ftk_gemm_bf16(C.byref(g), _stream()), what)
     if reduce_stream is not None and g.workspace:

@@ -1,0 +1,113 @@
+"""Every tile width of the GEMM (single CTA 128 / 192 / 256, CTA pair 256 x 128 / 192 / 256) with every epilogue
+instantiation, at the edges of its tiles, and the row-by-row path of outputs without aligned 16-byte segments."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+WIDTHS = [128, 192, 256, 256 + 128, 256 + 192, 256 + 256]
+
+
+def _rand(shape, seed, dev, scale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=g) * scale).to(torch.bfloat16).to(dev)
+
+
+def _gelu(x):
+    return torch.nn.functional.gelu(x, approximate="tanh")
+
+
+def _dgelu(x):
+    x = x.clone().requires_grad_(True)
+    return torch.autograd.grad(_gelu(x).sum(), x)[0]
+
+
+def _close(out, ref, act=False):
+    # the output's rounding (at most 2^-9 relative for bf16, twice that here), the error of fp32 sums of at most 1096
+    # products whose squares add up to about one (1096 * 2^-24 = 7e-5), and 2^-10 |x| of the hardware tanh
+    bound = (2.0 ** -8 if out.dtype == torch.bfloat16 else 2.0 ** -20) * ref.abs() + 1e-4
+    if act:
+        bound = bound + 2.0 ** -9 * ref.abs().max()
+    assert out.double().isfinite().all()
+    err = (out.double() - ref).abs()
+    assert bool((err <= bound).all()), float((err - bound).max())
+
+
+@pytest.mark.parametrize("bn", WIDTHS)
+@pytest.mark.parametrize("M,N,K", [
+    (256, 64, 64),          # one tile, one k-block, columns end inside the tile
+    (1, 8, 8),              # the smallest extents
+    (257, 200, 136),        # one row into the second pair tile, ragged N and K
+    (384, 584, 1096),       # several tiles, more k-blocks than stages
+])
+@pytest.mark.parametrize("kind", ["plain", "bias", "bias_resid", "gelu", "gelu_aux", "dgelu", "relu_resid", "f32", "f32_acc"])
+def test_tiles_and_epilogues(cuda_device, bn, M, N, K, kind):
+    from frankentorch_b200.ops import kernels as k
+    b_mn = kind in ("dgelu", "plain")            # the layouts that training uses: dgrad reads the weight as [K, N]
+    if b_mn and N % 8:
+        pytest.skip("an MN-major operand has rows of whole 16-byte segments")
+    a, w = _rand((M, K), 1, cuda_device), _rand((K, N) if b_mn else (N, K), 2, cuda_device, K ** -0.5)
+    bias, r = _rand((N,), 3, cuda_device), _rand((M, N), 4, cuda_device)
+    ref = a.double() @ (w.double() if b_mn else w.double().t())
+    kw, aux = {}, None
+    if kind in ("bias", "bias_resid", "gelu", "gelu_aux", "relu_resid"):
+        kw["bias"], ref = bias, ref + bias.double()
+    if kind.startswith("gelu"):
+        pre, ref = ref, _gelu(ref)
+        kw["epi"] = k.EPI_GELU_TANH
+        if kind == "gelu_aux":
+            kw["aux"] = aux = torch.empty((M, N), dtype=torch.bfloat16, device=cuda_device)
+    if kind == "dgelu":
+        ref = ref * _dgelu(r.double())
+        kw.update(epi=k.EPI_MUL_DGELU_TANH, resid=r)
+    if kind == "relu_resid":
+        kw["epi"], ref = k.EPI_RELU, torch.relu(ref)
+    if kind in ("bias_resid", "relu_resid"):
+        kw["resid"], ref = r, ref + r.double()
+    if kind.startswith("f32"):
+        kw.update(out_dtype=torch.float32, split_k=1)
+        if kind == "f32_acc":
+            out0 = torch.full((M, N), 0.5, device=cuda_device)
+            kw.update(out=out0, accumulate=True)
+            ref = ref + 0.5
+    out = k.gemm(a, w, b_mn=b_mn, force_bn=bn, **kw)
+    k.check_status()
+    _close(out, ref, act="gelu" in kind)
+    if aux is not None:
+        _close(aux, pre)
+
+
+@pytest.mark.parametrize("bn", WIDTHS)
+@pytest.mark.parametrize("N,ldd,off", [(37, 37, 0), (40, 41, 0), (40, 40, 1), (72, 80, 3)])
+def test_rows_without_aligned_segments(cuda_device, bn, N, ldd, off):
+    """Odd widths, leading dimensions and bases, bf16 accumulation: the general epilogue, nothing written beside it."""
+    from frankentorch_b200.ops import kernels as k
+    M, K = 200, 72
+    a, w = _rand((M, K), 5, cuda_device), _rand((N, K), 6, cuda_device, K ** -0.5)
+    bias = _rand((N,), 7, cuda_device)
+    store = torch.full((M * ldd + off + 8,), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    out = store[off:off + M * ldd].view(M, ldd)[:, :N]
+    k.gemm(a, w, bias=bias, out=out, force_bn=bn)
+    ref = a.double() @ w.double().t() + bias.double()
+    _close(out, ref)
+    k.gemm(a, w, out=out, accumulate=True, force_bn=bn)
+    k.check_status()
+    assert float((out.double() - (2 * ref - bias.double())).abs().max()) <= 2.0 ** -7 * float(ref.abs().max()) + 1e-3
+    mask = torch.ones_like(store, dtype=torch.bool)
+    mask[off:off + M * ldd].view(M, ldd)[:, :N] = False
+    assert bool((store[mask] == 7.0).all())
+
+
+def test_grouped_products_with_unaligned_outputs(cuda_device):
+    from frankentorch_b200.ops import kernels as k
+    K, shapes = 264, [(264, 200), (16, 8), (520, 40)]
+    probs, refs = [], []
+    for i, (M, N) in enumerate(shapes):
+        a, b = _rand((K, M), 10 + i, cuda_device), _rand((K, N), 20 + i, cuda_device, K ** -0.5)
+        out = torch.full((M, N + 1), 0.25, device=cuda_device)[:, :N]
+        probs.append((a, b, out, True))
+        refs.append(a.double().t() @ b.double() + 0.25)
+    k.gemm_grouped(probs)
+    k.check_status()
+    for (_, _, out, _), ref in zip(probs, refs):
+        _close(out, ref)
