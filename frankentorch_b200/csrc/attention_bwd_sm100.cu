@@ -88,19 +88,6 @@ __device__ __forceinline__ void store_out32(__nv_bfloat16* dst, const uint32_t* 
 }
 
 // =============================================================================== backward: dK, dV
-#ifdef FT_ATTN_TRACE
-// Optional timeline of CTA 0 of each backward kernel (development builds only):
-// [kernel][role][iteration][point] clock64 values.
-__device__ long long g_attn_bwd_trace[2 * 3 * 16 * 8];
-#define FT_BTRACE(kern, role, it, pt)                                                              \
-  do {                                                                                             \
-    if (blockIdx.x == 0 && lane == 0 && (it) < 16)                                                 \
-      g_attn_bwd_trace[(((kern) * 3 + (role)) * 16 + (it)) * 8 + (pt)] = clock64();                \
-  } while (0)
-#else
-#define FT_BTRACE(kern, role, it, pt) do { } while (0)
-#endif
-
 template <int HD>
 struct DkvCfg {
   static constexpr int TILE = (HD / 64) * AT_REGION;
@@ -108,24 +95,28 @@ struct DkvCfg {
   // written there by the threads that own their rows, and the dV / dK products read their A
   // operand from tensor memory, so neither tile crosses shared memory (which a 128-row CTA tile
   // already saturates with its B operands).  head_dim 128 fills all 512 columns with
-  // accumulators and stages both tiles in shared memory.
+  // accumulators: P^T takes the place of the scores it was made from, dS^T is staged in shared
+  // memory, and the two Q / dO stages that this leaves room for keep a load ahead of every block (with one stage and both
+  // tiles in shared memory a block took ~6000 cycles, 2500 of them waiting for that load).
   static constexpr bool TS = (HD == 64);
-  static constexpr int STAGES = (HD == 64) ? 4 : 1;          // Q / dO ring
-  static constexpr int NBUF = 1;                             // P^T / dS^T buffers
-  static constexpr int OFF_K = 0;
-  static constexpr int OFF_V = TILE;
-  static constexpr int OFF_Q = 2 * TILE;                     // [STAGES]
+  static constexpr int STAGES = (HD == 64) ? 4 : 2;          // Q / dO ring
+  static constexpr int KVB = (HD == 64) ? 2 : 1;             // K / V buffers (one per work item)
+  static constexpr int OFF_KV = 0;                           // [KVB] K, V
+  static constexpr int OFF_Q = KVB * 2 * TILE;               // [STAGES]
   static constexpr int OFF_DO = OFF_Q + STAGES * TILE;       // [STAGES]
-  static constexpr int OFF_PT = OFF_DO + STAGES * TILE;      // [NBUF] P^T  [keys x queries]
-  static constexpr int OFF_DST = OFF_PT + (TS ? 0 : NBUF * 2 * AT_REGION);   // [NBUF] dS^T
-  static constexpr int OFF_STAT = OFF_DST + (TS ? 0 : NBUF * 2 * AT_REGION); // [STAGES][2][128] floats
+  static constexpr int OFF_DST = OFF_DO + STAGES * TILE;     // dS^T [keys x queries] (not TS)
+  static constexpr int OFF_STAT = OFF_DST + (TS ? 0 : 2 * AT_REGION);   // [STAGES][2][128] floats
   static constexpr int OFF_BAR = OFF_STAT + STAGES * 2 * 128 * 4;
-  static constexpr int SMEM = OFF_BAR + 512;
+  static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_ST = 0, TM_DPT = 128, TM_DV = 256, TM_DK = 256 + HD;
-  static constexpr int TM_PT = 256 + 2 * HD, TM_DST = 256 + 2 * HD + 64;   // TS only
+  static constexpr int TM_PT = TS ? 256 + 2 * HD : TM_ST, TM_DST = 256 + 2 * HD + 64;   // TM_DST: TS only
+  static_assert(SMEM <= 232448, "shared memory");
 };
 
+// One persistent CTA per SM walks (key block, head, batch) items; every ring and every barrier runs on across items, so the
+// loads and the first score products of an item are issued under the last block and the output of the one before.  With one
+// CTA per item, set-up, first loads and output were ~15000 cycles per item against 1800 per block.
 template <int HD>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -134,16 +125,22 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   using C = DkvCfg<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
-  uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;    // [4]
-  uint64_t* qdo_empty = bars + 5;   // [4]
-  uint64_t* st_full = bars + 9;     // S^T and dP^T in TMEM
-  uint64_t* st_free = bars + 10;    // both copied to registers (one arrival per warp)
-  uint64_t* pds_ready = bars + 11;  // [2] P^T and dS^T handed to the tensor core (one arrival per warp)
-  uint64_t* acc_done = bars + 13;   // [2] dV/dK MMAs that read the buffer finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* kv_full = bars;         // [2]
+  uint64_t* kv_empty = bars + 2;    // [2] the item's score products are done
+  uint64_t* q_full = bars + 4;      // [4] Q tile and the block's statistics
+  uint64_t* q_empty = bars + 8;     // [4]
+  uint64_t* do_full = bars + 12;    // [4]
+  uint64_t* do_empty = bars + 16;   // [4] head_dim 128: dO is done with after dV, half a block before Q
+  uint64_t* st_full = bars + 20;    // S^T and dP^T in TMEM
+  uint64_t* st_free = bars + 21;    // both copied to registers (one arrival per warp)
+  uint64_t* pt_ready = bars + 22;   // P^T handed to the tensor core (one arrival per warp); TS: P^T and dS^T
+  uint64_t* ds_ready = bars + 23;   // dS^T in shared memory (not TS)
+  uint64_t* dv_done = bars + 24;    // dV product of the block done (not TS)
+  uint64_t* acc_done = bars + 25;   // dV and dK products of the block done
+  uint64_t* acc_free = bars + 26;   // the item's dV / dK copied to registers (one arrival per warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   int* abort_f = reinterpret_cast<int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
 
   if ((smem_u32(smem) & 1023u) != 0u) {
@@ -151,19 +148,31 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     return;
   }
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
-    }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&pds_ready[i], BW_MATH);
-      mbar_init(&acc_done[i], 1);
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&do_full[i], 1);
+      mbar_init(&do_empty[i], 1);
     }
     mbar_init(st_full, 1);
     mbar_init(st_free, BW_MATH);
+    mbar_init(pt_ready, BW_MATH);
+    mbar_init(ds_ready, BW_MATH);
+    mbar_init(dv_done, 1);
+    mbar_init(acc_done, 1);
+    mbar_init(acc_free, BW_MATH);
     *abort_f = 0;
     fence_mbar_init();
+  }
+  if (warp == BW_WARP_TMA && elect_one()) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmDO);
   }
   if (warp == BW_WARP_MMA) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -174,213 +183,320 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // linear grid, key blocks with the most query blocks (the early ones under a causal mask) first
   const int n_hb = p.H * p.B;
-  const int kb = (int)blockIdx.x / n_hb;
-  const int hb = (int)blockIdx.x % n_hb;
-  const int h = hb % p.H, b = hb / p.H;
-  const int k0 = kb * AT_T;
   const int nq_all = (p.S + AT_T - 1) / AT_T;
-  const int qb_first = p.causal ? kb : 0;
-  const int nit = nq_all - qb_first;
   float* stat = reinterpret_cast<float*>(smem + C::OFF_STAT);
+  TileWalk walk(p.n_tiles);
 
   if (warp == BW_WARP_TMA) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmDO);
-      mbar_arrive_expect_tx(kv_full, 2 * C::TILE);
-      load_tile<HD>(smem + C::OFF_K, &tmK, kv_full, k0, h, b);
-      load_tile<HD>(smem + C::OFF_V, &tmV, kv_full, k0, h, b);
-    }
-    // Per-query statistics (-lse and delta) of a block travel with its Q / dO tiles: they are
-    // fetched into registers one iteration ahead, so their global-memory latency is spent while
-    // this warp waits for the stage, not between the stage becoming free and its TMA loads.
-    const long long sbase = ((long long)b * p.H + h) * p.S;
-    float nl_r[4], dl_r[4];
-    auto fetch_stats = [&](int it) {
-      const int q0 = (qb_first + it) * AT_T;
+    Ring<C::STAGES> rq;
+    Ring<C::KVB> rk;
+    bool ok = true;
+#pragma unroll 1
+    for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+      const int kb = p.by_hb.div(item), hb = item - kb * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int qb_first = p.causal ? kb : 0, nit = nq_all - qb_first;
+      // Per-query statistics (-lse and -delta) of a block travel with its Q / dO tiles: they are
+      // fetched into registers one iteration ahead, so their global-memory latency is spent while
+      // this warp waits for the stage, not between the stage becoming free and its TMA loads.
+      const long long sbase = ((long long)b * p.H + h) * p.S;
+      float nl_r[4], dl_r[4];
+      auto fetch_stats = [&](int it) {
+        const int q0 = (qb_first + it) * AT_T;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int gq = q0 + lane + 32 * u;
-        nl_r[u] = gq < p.S ? -p.lse[sbase + gq] : -INFINITY;
-        dl_r[u] = gq < p.S ? p.delta[sbase + gq] : 0.f;
-      }
-    };
-    if (nit > 0) fetch_stats(0);
-    for (int it = 0; it < nit; ++it) {
-      const int st = it % C::STAGES;
-      const uint32_t ph = (it / C::STAGES) & 1;
-      if (!mbar_wait(&qdo_empty[st], ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) break;
-      const int q0 = (qb_first + it) * AT_T;
-      float* sl = stat + st * 256;          // published by the arrive below
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        sl[lane + 32 * u] = nl_r[u];
-        sl[128 + lane + 32 * u] = dl_r[u];
+        for (int u = 0; u < 4; ++u) {
+          const int gq = q0 + lane + 32 * u;
+          nl_r[u] = gq < p.S ? -p.lse[sbase + gq] : -INFINITY;
+          dl_r[u] = gq < p.S ? -p.delta[sbase + gq] : 0.f;
+        }
+      };
+      fetch_stats(0);
+      if (!mbar_wait_warp(&kv_empty[rk.s], rk.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) break;
+      if (elect_one()) {
+        uint8_t* kv = smem + C::OFF_KV + rk.s * 2 * C::TILE;
+        mbar_arrive_expect_tx(&kv_full[rk.s], 2 * C::TILE);
+        load_tile<HD>(kv, &tmK, &kv_full[rk.s], kb * AT_T, h, b);
+        load_tile<HD>(kv + C::TILE, &tmV, &kv_full[rk.s], kb * AT_T, h, b);
       }
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&qdo_full[st], 2 * C::TILE);
-        load_tile<HD>(smem + C::OFF_Q + st * C::TILE, &tmQ, &qdo_full[st], q0, h, b);
-        load_tile<HD>(smem + C::OFF_DO + st * C::TILE, &tmDO, &qdo_full[st], q0, h, b);
+      rk.step();
+#pragma unroll 1
+      for (int it = 0; it < nit; ++it) {
+        const int st = rq.s;
+        const int q0 = (qb_first + it) * AT_T;
+        if (!mbar_wait_warp(&do_empty[st], rq.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&do_full[st], C::TILE);
+          load_tile<HD>(smem + C::OFF_DO + st * C::TILE, &tmDO, &do_full[st], q0, h, b);
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(&q_empty[st], rq.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+        float* sl = stat + st * 256;          // published by the arrive below
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          sl[lane + 32 * u] = nl_r[u];
+          sl[128 + lane + 32 * u] = dl_r[u];
+        }
+        __syncwarp();
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&q_full[st], C::TILE);
+          load_tile<HD>(smem + C::OFF_Q + st * C::TILE, &tmQ, &q_full[st], q0, h, b);
+        }
+        __syncwarp();
+        rq.step();
+        if (it + 1 < nit) fetch_stats(it + 1);
       }
-      __syncwarp();
-      if (it + 1 < nit) fetch_stats(it + 1);
     }
   } else if (warp == BW_WARP_MMA) {
     // ---------------------------------------------------------- issuer 1: S^T = K Q^T, dP^T = V dO^T
-    // (two issuing warps: the issuing thread runs in step with the tensor pipe, so the waits and
+    // (two issuing warps with head_dim 64: the issuing thread runs in step with the tensor pipe, so the waits and
     // descriptor steps of one product would otherwise idle the pipe for the other)
     const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-    const uint32_t k_addr = smem_u32(smem + C::OFF_K), v_addr = smem_u32(smem + C::OFF_V);
+    const uint32_t kv_addr = smem_u32(smem + C::OFF_KV);
     const uint32_t q_addr = smem_u32(smem + C::OFF_Q), do_addr = smem_u32(smem + C::OFF_DO);
-    bool ok = mbar_wait(kv_full, 0, ctx, FT_ERR_WAIT_FULL);
-    for (int i = 0; ok && i < nit; ++i) {
-      const int st = i % C::STAGES;
-      FT_BTRACE(0, 2, i, 0);
-      // needs Q_i / dO_i and the score tiles of iteration i - 1 copied to registers
-      if (!mbar_wait(&qdo_full[st], (i / C::STAGES) & 1, ctx, FT_ERR_WAIT_FULL)) break;
-      if (i > 0 && !mbar_wait(st_free, (i - 1) & 1, ctx, FT_ERR_WAIT_TMEM_EMPTY)) break;
-      FT_BTRACE(0, 2, i, 1);
-      tc_fence_after();
-      if (lane == 0) {
-        mma_kmajor<HD>(tmem_base + C::TM_ST, k_addr, q_addr + st * C::TILE, idesc_s);
-        mma_kmajor<HD>(tmem_base + C::TM_DPT, v_addr, do_addr + st * C::TILE, idesc_s);
-        umma_commit(st_full);
+    if constexpr (C::TS) {
+      Ring<C::STAGES> rq;
+      Ring<C::KVB> rk;
+      uint32_t ph = 0;             // parity of the previous block
+      bool ok = true, first = true;
+#pragma unroll 1
+      for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+        const int nit = nq_all - (p.causal ? p.by_hb.div(item) : 0);
+        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL)) break;
+        const uint32_t k_addr = kv_addr + rk.s * 2 * C::TILE, v_addr = k_addr + C::TILE;
+#pragma unroll 1
+        for (int i = 0; i < nit; ++i) {
+          // needs Q_i / dO_i and the score tiles of the previous block copied to registers
+          if (!mbar_wait_warp(&do_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL) ||
+              !mbar_wait_warp(&q_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL) ||
+              (!first && !mbar_wait_warp(st_free, ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
+          if (!first) ph ^= 1u;
+          first = false;
+          tc_fence_after();
+          if (elect_one()) {
+            mma_kmajor<HD>(tmem_base + C::TM_ST, k_addr, q_addr + rq.s * C::TILE, idesc_s);
+            mma_kmajor<HD>(tmem_base + C::TM_DPT, v_addr, do_addr + rq.s * C::TILE, idesc_s);
+            umma_commit(st_full);
+            if (i == nit - 1) umma_commit(&kv_empty[rk.s]);
+          }
+          __syncwarp();
+          rq.step();
+        }
+        rk.step();
       }
-      __syncwarp();
-      FT_BTRACE(0, 2, i, 2);
+    } else {
+      // One issuer for all four products of head_dim 128.  In the steady state block g + 1's dP^T runs under block g's
+      // exponentials, then dV += P^T dO as soon as P^T is there, the next scores as soon as dV has read P^T (which lies
+      // in their columns), and dK last, under the next exponentials.
+      const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);
+      const uint32_t dst_addr = smem_u32(smem + C::OFF_DST);
+      const uint32_t k_addr = kv_addr, v_addr = kv_addr + C::TILE;
+      Ring<C::STAGES> rn, rc;      // stage of the next block's scores, of the current block
+      uint32_t kv_ph = 0, blk = 0, tile_ph = 0;      // parity of the item, of the block, of the finished item
+      bool ok = true;
+      auto dp_next = [&]() -> bool {
+        if (!mbar_wait_warp(&do_full[rn.s], rn.ph, ctx, FT_ERR_WAIT_FULL)) return false;
+        tc_fence_after();
+        if (elect_one()) mma_kmajor<HD>(tmem_base + C::TM_DPT, v_addr, do_addr + rn.s * C::TILE, idesc_s);
+        __syncwarp();
+        return true;
+      };
+      auto s_next = [&](bool last) -> bool {
+        if (!mbar_wait_warp(&q_full[rn.s], rn.ph, ctx, FT_ERR_WAIT_FULL)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          mma_kmajor<HD>(tmem_base + C::TM_ST, k_addr, q_addr + rn.s * C::TILE, idesc_s);
+          umma_commit(st_full);
+          if (last) umma_commit(&kv_empty[0]);
+        }
+        __syncwarp();
+        rn.step();
+        return true;
+      };
+      bool first_item = true;
+#pragma unroll 1
+      for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+        const int nit = nq_all - (p.causal ? p.by_hb.div(item) : 0);
+        // the item's first scores (the score columns are free: its predecessor's last dV has finished)
+        ok = mbar_wait_warp(&kv_full[0], kv_ph, ctx, FT_ERR_WAIT_FULL) && dp_next() && s_next(nit == 1);
+        if (!ok) break;
+        kv_ph ^= 1u;
+#pragma unroll 1
+        for (int i = 0; i < nit; ++i) {
+          const bool more = i + 1 < nit;
+          if (more && (!mbar_wait_warp(st_free, blk, ctx, FT_ERR_WAIT_TMEM_EMPTY) || !dp_next())) { ok = false; break; }
+          if (!mbar_wait_warp(pt_ready, blk, ctx, FT_ERR_WAIT_SOFTMAX) ||
+              (i == 0 && !first_item && !mbar_wait_warp(acc_free, tile_ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            mma_ptmem_times_rows(tmem_base + C::TM_DV, tmem_base + C::TM_PT, do_addr + rc.s * C::TILE, idesc_acc, i > 0);
+            umma_commit(dv_done);
+            umma_commit(&do_empty[rc.s]);
+          }
+          __syncwarp();
+          if (!mbar_wait_warp(dv_done, blk, ctx, FT_ERR_WAIT_TMEM_FULL) || (more && !s_next(i + 2 == nit)) ||
+              !mbar_wait_warp(ds_ready, blk, ctx, FT_ERR_WAIT_SOFTMAX)) { ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            mma_p_times_rows(tmem_base + C::TM_DK, dst_addr, q_addr + rc.s * C::TILE, idesc_acc, i > 0);
+            umma_commit(acc_done);
+            umma_commit(&q_empty[rc.s]);
+          }
+          __syncwarp();
+          rc.step();
+          blk ^= 1u;
+        }
+        if (!first_item) tile_ph ^= 1u;
+        first_item = false;
+      }
     }
   } else if (warp == BW_WARP_MMA2) {
-    // ---------------------------------------------------------- issuer 2: dV += P^T dO, dK += dS^T Q
-    const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);
-    const uint32_t q_addr = smem_u32(smem + C::OFF_Q), do_addr = smem_u32(smem + C::OFF_DO);
-    const uint32_t pt_addr = smem_u32(smem + C::OFF_PT), dst_addr = smem_u32(smem + C::OFF_DST);
-    for (int it = 0; it < nit; ++it) {
-      const int st = it % C::STAGES, buf = it % C::NBUF;
-      if (!mbar_wait(&qdo_full[st], (it / C::STAGES) & 1, ctx, FT_ERR_WAIT_FULL)) break;
-      FT_BTRACE(0, 2, it, 3);
-      if (!mbar_wait(&pds_ready[buf], (it / C::NBUF) & 1, ctx, FT_ERR_WAIT_SOFTMAX)) break;
-      FT_BTRACE(0, 2, it, 4);
-      tc_fence_after();
-      if (lane == 0) {
-        if constexpr (C::TS) {
-          mma_ptmem_times_rows(tmem_base + C::TM_DV, tmem_base + C::TM_PT, do_addr + st * C::TILE,
-                               idesc_acc, it > 0);
-          mma_ptmem_times_rows(tmem_base + C::TM_DK, tmem_base + C::TM_DST, q_addr + st * C::TILE,
-                               idesc_acc, it > 0);
-        } else {
-          mma_p_times_rows(tmem_base + C::TM_DV, pt_addr + buf * 2 * AT_REGION, do_addr + st * C::TILE,
-                           idesc_acc, it > 0);
-          mma_p_times_rows(tmem_base + C::TM_DK, dst_addr + buf * 2 * AT_REGION, q_addr + st * C::TILE,
-                           idesc_acc, it > 0);
+    if constexpr (C::TS) {
+      // ---------------------------------------------------------- issuer 2: dV += P^T dO, dK += dS^T Q
+      const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);
+      const uint32_t q_addr = smem_u32(smem + C::OFF_Q), do_addr = smem_u32(smem + C::OFF_DO);
+      Ring<C::STAGES> rq;
+      uint32_t blk = 0, tile_ph = 0;
+      bool ok = true, first_item = true;
+#pragma unroll 1
+      for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+        const int nit = nq_all - (p.causal ? p.by_hb.div(item) : 0);
+#pragma unroll 1
+        for (int it = 0; it < nit; ++it) {
+          if (!mbar_wait_warp(pt_ready, blk, ctx, FT_ERR_WAIT_SOFTMAX) ||
+              (it == 0 && !first_item && !mbar_wait_warp(acc_free, tile_ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            mma_ptmem_times_rows(tmem_base + C::TM_DV, tmem_base + C::TM_PT, do_addr + rq.s * C::TILE, idesc_acc, it > 0);
+            mma_ptmem_times_rows(tmem_base + C::TM_DK, tmem_base + C::TM_DST, q_addr + rq.s * C::TILE, idesc_acc, it > 0);
+            umma_commit(acc_done);
+            umma_commit(&do_empty[rq.s]);      // S^T / dP^T of this stage finished before the math ran
+            umma_commit(&q_empty[rq.s]);
+          }
+          __syncwarp();
+          rq.step();
+          blk ^= 1u;
         }
-        umma_commit(&acc_done[buf]);
-        umma_commit(&qdo_empty[st]);     // S^T / dP^T of this stage finished before the math ran
+        if (!first_item) tile_ph ^= 1u;
+        first_item = false;
       }
-      __syncwarp();
-      FT_BTRACE(0, 2, it, 5);
     }
   } else if (warp < BW_MATH) {
     const int g = warp >> 2;               // column group: queries [32 g, 32 g + 32) of the block
     const int qd = warp & 3;
     const int row = qd * 32 + lane;        // key row of this thread
-    const int gk = k0 + row;
     const int c0 = 32 * g;
     const uint32_t lane_sel = (uint32_t)(qd * 32) << 16;
-    bool ok = true;
-    for (int it = 0; it < nit; ++it) {
-      const int st = it % C::STAGES, buf = it % C::NBUF;
-      const int q0 = (qb_first + it) * AT_T;
-      // statistics were written by the producer before its arrive on qdo_full
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 0);
-      if (!mbar_wait(&qdo_full[st], (it / C::STAGES) & 1, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
-      if (!mbar_wait(st_full, it & 1, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 1);
-      tc_fence_after();
-      uint32_t rs[32], rd[32];
-      tmem_ld32(tmem_base + C::TM_ST + c0 + lane_sel, rs);
-      tmem_ld32(tmem_base + C::TM_DPT + c0 + lane_sel, rd);
-      tmem_ld_wait();
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 2);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(st_free);      // one arrival per warp
-      const float4* sl4 = reinterpret_cast<const float4*>(stat + st * 256 + c0);
-      const float4* dl4 = reinterpret_cast<const float4*>(stat + st * 256 + 128 + c0);
-      const bool need_mask = (q0 + AT_T > p.S) || (k0 + AT_T > p.S) || (p.causal && q0 < k0 + AT_T - 1);
-      uint32_t pw[16], dw[16];
-      // masked scores become -inf in a pass of their own (diagonal and ragged blocks only), so
-      // the main loop carries no per-element predicates
-      if (need_mask) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int gq = q0 + c0 + i;
-          if (gq >= p.S || gk >= p.S || (p.causal && gk > gq)) rs[i] = __float_as_uint(-INFINITY);
-        }
-      }
-#pragma unroll
-      for (int i4 = 0; i4 < 8; ++i4) {
-        const float4 nl = sl4[i4], dl = dl4[i4];
-        const float nls[4] = {nl.x, nl.y, nl.z, nl.w}, dls[4] = {dl.x, dl.y, dl.z, dl.w};
-        float e[4], d[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = 4 * i4 + u;
-          e[u] = fast_exp2(fmaf(__uint_as_float(rs[i]), p.sl2, nls[u]));
-          d[u] = e[u] * (__uint_as_float(rd[i]) - dls[u]);
-        }
-        pw[2 * i4] = pack_bf16(e[0], e[1]);
-        pw[2 * i4 + 1] = pack_bf16(e[2], e[3]);
-        dw[2 * i4] = pack_bf16(d[0], d[1]);
-        dw[2 * i4 + 1] = pack_bf16(d[2], d[3]);
-      }
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 3);
-      // the buffer's previous reader (dV/dK of iteration it - NBUF) must have finished
-      if (it >= C::NBUF &&
-          !mbar_wait(&acc_done[buf], ((it / C::NBUF) - 1) & 1, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 4);
-      if constexpr (C::TS) {
-        // this thread's 32 queries of its key row: 16 packed columns of each operand tile
+    const f32x2 sl2 = pk2(p.sl2, p.sl2);
+    Ring<C::STAGES> rq;
+    uint32_t blk = 0;                      // parity of the block
+    bool ok = true, first = true;
+#pragma unroll 1
+    for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+      const int kb = p.by_hb.div(item), hb = item - kb * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int k0 = kb * AT_T, gk = k0 + row;
+      const int qb_first = p.causal ? kb : 0, nit = nq_all - qb_first;
+#pragma unroll 1
+      for (int it = 0; it < nit; ++it) {
+        const int st = rq.s;
+        const int q0 = (qb_first + it) * AT_T;
+        // statistics were written by the producer before its arrive on q_full
+        if (!mbar_wait_warp(&q_full[st], rq.ph, ctx, FT_ERR_WAIT_FULL) ||
+            !mbar_wait_warp(st_full, blk, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-        tmem_st16(tmem_base + C::TM_PT + 16 * g + lane_sel, pw);
-        tmem_st16(tmem_base + C::TM_DST + 16 * g + lane_sel, dw);
-        tmem_st_wait();
+        uint32_t rs[32], rd[32];
+        tmem_ld32(tmem_base + C::TM_ST + c0 + lane_sel, rs);
+        tmem_ld32(tmem_base + C::TM_DPT + c0 + lane_sel, rd);
+        tmem_ld_wait();
         tc_fence_before();
-      } else {
-        store_row32_packed(smem + C::OFF_PT + buf * 2 * AT_REGION, row, c0, pw);
-        store_row32_packed(smem + C::OFF_DST + buf * 2 * AT_REGION, row, c0, dw);
-        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(st_free);      // one arrival per warp
+        const float4* sl4 = reinterpret_cast<const float4*>(stat + st * 256 + c0);
+        const float4* dl4 = reinterpret_cast<const float4*>(stat + st * 256 + 128 + c0);
+        // Queries before the key become -inf, in the diagonal block and the warps that hold such pairs only.  Queries past
+        // the end have -lse = -inf; key rows past the end are never stored and touch no other row.
+        if (p.causal && q0 + c0 < k0 + qd * 32 + 31) {
+          const int lo = gk - q0 - c0;            // first valid column of this thread
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i < lo) rs[i] = __float_as_uint(-INFINITY);
+        }
+        uint32_t pw[16], dw[16];
+        if constexpr (C::TS) {
+#pragma unroll
+          for (int i4 = 0; i4 < 8; ++i4) {
+            const float4 nl = sl4[i4], dl = dl4[i4];
+            const f32x2 e0 = exp2_pair(fma2(acc2(rs, 4 * i4), sl2, pk2(nl.x, nl.y)));
+            const f32x2 e1 = exp2_pair(fma2(acc2(rs, 4 * i4 + 2), sl2, pk2(nl.z, nl.w)));
+            pw[2 * i4] = pack2(e0);
+            pw[2 * i4 + 1] = pack2(e1);
+            dw[2 * i4] = pack2(mul2(e0, add2(acc2(rd, 4 * i4), pk2(dl.x, dl.y))));
+            dw[2 * i4 + 1] = pack2(mul2(e1, add2(acc2(rd, 4 * i4 + 2), pk2(dl.z, dl.w))));
+          }
+          // the operand tiles' previous readers (dV / dK of the block before) must have finished
+          if (!first && !mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+          // this thread's 32 queries of its key row: 16 packed columns of each operand tile
+          tc_fence_after();
+          tmem_st16(tmem_base + C::TM_PT + 16 * g + lane_sel, pw);
+          tmem_st16(tmem_base + C::TM_DST + 16 * g + lane_sel, dw);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(pt_ready);      // one arrival per warp
+        } else {
+          f32x2 e[16];
+#pragma unroll
+          for (int i4 = 0; i4 < 8; ++i4) {
+            const float4 nl = sl4[i4];
+            e[2 * i4] = exp2_pair(fma2(acc2(rs, 4 * i4), sl2, pk2(nl.x, nl.y)));
+            e[2 * i4 + 1] = exp2_pair(fma2(acc2(rs, 4 * i4 + 2), sl2, pk2(nl.z, nl.w)));
+            pw[2 * i4] = pack2(e[2 * i4]);
+            pw[2 * i4 + 1] = pack2(e[2 * i4 + 1]);
+          }
+          // P^T goes where the scores were, once every warp has copied its part of them
+          if (!mbar_wait_warp(st_free, blk, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
+          tc_fence_after();
+          tmem_st16(tmem_base + C::TM_PT + 16 * g + lane_sel, pw);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(pt_ready);
+#pragma unroll
+          for (int i4 = 0; i4 < 8; ++i4) {
+            const float4 dl = dl4[i4];
+            dw[2 * i4] = pack2(mul2(e[2 * i4], add2(acc2(rd, 4 * i4), pk2(dl.x, dl.y))));
+            dw[2 * i4 + 1] = pack2(mul2(e[2 * i4 + 1], add2(acc2(rd, 4 * i4 + 2), pk2(dl.z, dl.w))));
+          }
+          if (!first && !mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+          store_row32_packed(smem + C::OFF_DST, row, c0, dw);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ds_ready);
+        }
+        first = false;
+        rq.step();
+        blk ^= 1u;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&pds_ready[buf]);      // one arrival per warp
-      FT_BTRACE(0, warp == 0 ? 0 : 1, it, 5);
-    }
-    if (ok && nit > 0)
-      ok = mbar_wait(&acc_done[(nit - 1) % C::NBUF], ((nit - 1) / C::NBUF) & 1, ctx, FT_ERR_WAIT_TMEM_FULL);
-    if (ok) {
+      if (!ok || !mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       __nv_bfloat16* dvp = p.dv + (long long)b * p.dv_bs + (long long)gk * p.dv_ss + (long long)h * p.dv_hs;
       __nv_bfloat16* dkp = p.dk + (long long)b * p.dk_bs + (long long)gk * p.dk_ss + (long long)h * p.dk_hs;
       // 2 HD / 32 column chunks (dV first, then dK) spread over the four groups
+      constexpr int NCH = 2 * HD / 32 / 4;
+      uint32_t r[NCH][32];
 #pragma unroll
-      for (int ch = g; ch < 2 * HD / 32; ch += 4) {
+      for (int u = 0; u < NCH; ++u) tmem_ld32(tmem_base + C::TM_DV + (g + 4 * u) * 32 + lane_sel, r[u]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
+#pragma unroll
+      for (int u = 0; u < NCH; ++u) {
+        const int ch = g + 4 * u;
         const bool is_dk = ch >= HD / 32;
         const int c = (is_dk ? ch - HD / 32 : ch) * 32;
-        uint32_t r[32];
-        if (nit > 0) {
-          tmem_ld32(tmem_base + (is_dk ? C::TM_DK : C::TM_DV) + c + lane_sel, r);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = 0u;
-        }
-        if (gk < p.S) store_out32((is_dk ? dkp : dvp) + c, r, is_dk ? p.scale : 1.f);
+        if (gk < p.S) store_out32((is_dk ? dkp : dvp) + c, r[u], is_dk ? p.scale : 1.f);
       }
-      tc_fence_before();
     }
   }
 
@@ -396,21 +512,19 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 template <int HD>
 struct DqCfg {
   static constexpr int TILE = (HD / 64) * AT_REGION;
-  static constexpr bool TS = (HD == 64);                 // dS in tensor memory (see DkvCfg)
-  static constexpr int STAGES = (HD == 64) ? 4 : 2;      // K / V ring
-  static constexpr int NBUF = (HD == 64) ? 2 : 1;        // dS buffers
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_DO = TILE;
-  static constexpr int OFF_K = 2 * TILE;                 // [STAGES]
-  static constexpr int OFF_V = OFF_K + STAGES * TILE;    // [STAGES]
-  static constexpr int OFF_DS = OFF_V + STAGES * TILE;   // [NBUF] dS [queries x keys]
-  static constexpr int OFF_BAR = OFF_DS + (TS ? 0 : NBUF * 2 * AT_REGION);
+  static constexpr int QB = (HD == 64) ? 2 : 1;          // Q / dO buffers (one per work item)
+  static constexpr int NSLOT = (HD == 64) ? 8 : 5;       // ring of single K / V tiles: a V slot is free after dP, a K slot after dQ
+  static constexpr int OFF_QDO = 0;                      // [QB] Q, dO
+  static constexpr int OFF_KV = QB * 2 * TILE;           // [NSLOT]
+  static constexpr int OFF_BAR = OFF_KV + NSLOT * TILE;
   static constexpr int SMEM = OFF_BAR + 512;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256;
-  static constexpr int TM_DS = 384;                      // TS: dS buffer i at TM_DS + 64 i
+  static constexpr int TM_DS = 384;                      // dS buffer i (packed bf16) at TM_DS + 64 i
+  static_assert(SMEM <= 232448, "shared memory");
 };
 
+// Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.
 template <int HD>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -419,16 +533,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   using C = DqCfg<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
-  uint64_t* qdo_full = bars;
-  uint64_t* kv_full = bars + 1;    // [4]
-  uint64_t* kv_empty = bars + 5;   // [4]
-  uint64_t* s_full = bars + 9;     // S and dP in TMEM
-  uint64_t* s_free = bars + 10;    // both copied to registers (one arrival per warp)
-  uint64_t* ds_ready = bars + 11;  // [2] dS handed to the tensor core (one arrival per warp)
-  uint64_t* acc_done = bars + 13;  // [2] dQ MMA that read the buffer finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* qdo_full = bars;        // [2]
+  uint64_t* qdo_empty = bars + 2;   // [2] the item's score products are done
+  uint64_t* kv_full = bars + 4;     // [8]
+  uint64_t* kv_empty = bars + 12;   // [8]
+  uint64_t* s_full = bars + 20;     // S and dP in TMEM
+  uint64_t* s_free = bars + 21;     // both copied to registers (one arrival per warp)
+  uint64_t* ds_ready = bars + 22;   // [2] dS handed to the tensor core (one arrival per warp)
+  uint64_t* acc_done = bars + 24;   // [2] dQ product that read the buffer done
+  uint64_t* acc_free = bars + 26;   // the item's dQ copied to registers (one arrival per warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   int* abort_f = reinterpret_cast<int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
 
   if ((smem_u32(smem) & 1023u) != 0u) {
@@ -436,19 +552,27 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     return;
   }
   if (threadIdx.x == 0) {
-    mbar_init(qdo_full, 1);
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-    }
     for (int i = 0; i < 2; ++i) {
+      mbar_init(&qdo_full[i], 1);
+      mbar_init(&qdo_empty[i], 1);
       mbar_init(&ds_ready[i], BW_MATH);
       mbar_init(&acc_done[i], 1);
     }
+    for (int i = 0; i < 8; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+    }
     mbar_init(s_full, 1);
     mbar_init(s_free, BW_MATH);
+    mbar_init(acc_free, BW_MATH);
     *abort_f = 0;
     fence_mbar_init();
+  }
+  if (warp == BW_WARP_TMA && elect_one()) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    tma_prefetch_desc(&tmDO);
   }
   if (warp == BW_WARP_MMA) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -459,153 +583,192 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // linear grid, query blocks with the most key blocks (the late ones under a causal mask) first
+  // items are numbered with the most key blocks (the late query blocks under a causal mask) first
   const int n_hb = p.H * p.B;
-  const int qb = (int)gridDim.x / n_hb - 1 - (int)blockIdx.x / n_hb;
-  const int hb = (int)blockIdx.x % n_hb;
-  const int h = hb % p.H, b = hb / p.H;
-  const int q0 = qb * AT_T;
   const int nkv_all = (p.S + AT_T - 1) / AT_T;
-  const int nkv = p.causal ? min(qb + 1, nkv_all) : nkv_all;
+  auto query_block = [&](int item) { return nkv_all - 1 - p.by_hb.div(item); };
+  auto key_blocks = [&](int qb) { return p.causal ? qb + 1 : nkv_all; };
+  TileWalk walk(p.n_tiles);
 
   if (warp == BW_WARP_TMA) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmDO);
-      mbar_arrive_expect_tx(qdo_full, 2 * C::TILE);
-      load_tile<HD>(smem + C::OFF_Q, &tmQ, qdo_full, q0, h, b);
-      load_tile<HD>(smem + C::OFF_DO, &tmDO, qdo_full, q0, h, b);
-    }
-    for (int j = 0; j < nkv; ++j) {
-      const int st = j % C::STAGES;
-      const uint32_t ph = (j / C::STAGES) & 1;
-      if (!mbar_wait(&kv_empty[st], ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) break;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&kv_full[st], 2 * C::TILE);
-        load_tile<HD>(smem + C::OFF_K + st * C::TILE, &tmK, &kv_full[st], j * AT_T, h, b);
-        load_tile<HD>(smem + C::OFF_V + st * C::TILE, &tmV, &kv_full[st], j * AT_T, h, b);
+    Ring<C::QB> rq;
+    Ring<C::NSLOT> rk;
+    bool ok = true;
+#pragma unroll 1
+    for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int nkv = key_blocks(qb);
+      if (!mbar_wait_warp(&qdo_empty[rq.s], rq.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) break;
+      if (elect_one()) {
+        uint8_t* qd = smem + C::OFF_QDO + rq.s * 2 * C::TILE;
+        mbar_arrive_expect_tx(&qdo_full[rq.s], 2 * C::TILE);
+        load_tile<HD>(qd, &tmQ, &qdo_full[rq.s], qb * AT_T, h, b);
+        load_tile<HD>(qd + C::TILE, &tmDO, &qdo_full[rq.s], qb * AT_T, h, b);
       }
       __syncwarp();
+      rq.step();
+#pragma unroll 1
+      for (int n = 0; n < 2 * nkv; ++n) {      // K_0, V_0, K_1, V_1, ...
+        if (!mbar_wait_warp(&kv_empty[rk.s], rk.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&kv_full[rk.s], C::TILE);
+          load_tile<HD>(smem + C::OFF_KV + rk.s * C::TILE, (n & 1) ? &tmV : &tmK, &kv_full[rk.s], (n >> 1) * AT_T, h, b);
+        }
+        __syncwarp();
+        rk.step();
+      }
     }
   } else if (warp == BW_WARP_MMA) {
     // ---------------------------------------------------------- issuer 1: S = Q K^T, dP = dO V^T
     const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-    const uint32_t q_addr = smem_u32(smem + C::OFF_Q), do_addr = smem_u32(smem + C::OFF_DO);
-    const uint32_t k_addr = smem_u32(smem + C::OFF_K), v_addr = smem_u32(smem + C::OFF_V);
-    bool ok = mbar_wait(qdo_full, 0, ctx, FT_ERR_WAIT_FULL);
-    for (int jj = 0; ok && jj < nkv; ++jj) {
-      const int st = jj % C::STAGES;
-      FT_BTRACE(1, 2, jj, 0);
-      if (!mbar_wait(&kv_full[st], (jj / C::STAGES) & 1, ctx, FT_ERR_WAIT_FULL)) break;
-      if (jj > 0 && !mbar_wait(s_free, (jj - 1) & 1, ctx, FT_ERR_WAIT_TMEM_EMPTY)) break;
-      FT_BTRACE(1, 2, jj, 1);
-      tc_fence_after();
-      if (lane == 0) {
-        mma_kmajor<HD>(tmem_base + C::TM_S, q_addr, k_addr + st * C::TILE, idesc_s);
-        mma_kmajor<HD>(tmem_base + C::TM_DP, do_addr, v_addr + st * C::TILE, idesc_s);
-        umma_commit(s_full);
+    const uint32_t qdo_addr = smem_u32(smem + C::OFF_QDO), kv_addr = smem_u32(smem + C::OFF_KV);
+    Ring<C::QB> rq;
+    Ring<C::NSLOT> rk;
+    uint32_t ph = 0;
+    bool ok = true, first = true;
+#pragma unroll 1
+    for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+      const int nkv = key_blocks(query_block(item));
+      if (!mbar_wait_warp(&qdo_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL)) break;
+      const uint32_t q_addr = qdo_addr + rq.s * 2 * C::TILE, do_addr = q_addr + C::TILE;
+#pragma unroll 1
+      for (int j = 0; j < nkv; ++j) {
+        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL) ||
+            (!first && !mbar_wait_warp(s_free, ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
+        if (!first) ph ^= 1u;
+        first = false;
+        tc_fence_after();
+        if (elect_one()) mma_kmajor<HD>(tmem_base + C::TM_S, q_addr, kv_addr + rk.s * C::TILE, idesc_s);
+        __syncwarp();
+        rk.step();
+        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          mma_kmajor<HD>(tmem_base + C::TM_DP, do_addr, kv_addr + rk.s * C::TILE, idesc_s);
+          umma_commit(s_full);
+          umma_commit(&kv_empty[rk.s]);
+          if (j == nkv - 1) umma_commit(&qdo_empty[rq.s]);
+        }
+        __syncwarp();
+        rk.step();
       }
-      __syncwarp();
-      FT_BTRACE(1, 2, jj, 2);
+      rq.step();
     }
   } else if (warp == BW_WARP_MMA2) {
     // ---------------------------------------------------------- issuer 2: dQ += dS K
     const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);
-    const uint32_t k_addr = smem_u32(smem + C::OFF_K);
-    const uint32_t ds_addr = smem_u32(smem + C::OFF_DS);
-    for (int j = 0; j < nkv; ++j) {
-      const int st = j % C::STAGES, buf = j % C::NBUF;
-      if (!mbar_wait(&kv_full[st], (j / C::STAGES) & 1, ctx, FT_ERR_WAIT_FULL)) break;
-      FT_BTRACE(1, 2, j, 3);
-      if (!mbar_wait(&ds_ready[buf], (j / C::NBUF) & 1, ctx, FT_ERR_WAIT_SOFTMAX)) break;
-      FT_BTRACE(1, 2, j, 4);
-      tc_fence_after();
-      if (lane == 0) {
-        if constexpr (C::TS)
-          mma_ptmem_times_rows(tmem_base + C::TM_DQ, tmem_base + C::TM_DS + 64 * buf, k_addr + st * C::TILE,
+    const uint32_t kv_addr = smem_u32(smem + C::OFF_KV);
+    Ring<C::NSLOT> rk;
+    Ring<2> rd;
+    uint32_t tile_ph = 0;
+    bool ok = true, first_item = true;
+#pragma unroll 1
+    for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
+      const int nkv = key_blocks(query_block(item));
+#pragma unroll 1
+      for (int j = 0; j < nkv; ++j) {
+        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL) ||
+            !mbar_wait_warp(&ds_ready[rd.s], rd.ph, ctx, FT_ERR_WAIT_SOFTMAX) ||
+            (j == 0 && !first_item && !mbar_wait_warp(acc_free, tile_ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          mma_ptmem_times_rows(tmem_base + C::TM_DQ, tmem_base + C::TM_DS + 64 * rd.s, kv_addr + rk.s * C::TILE,
                                idesc_acc, j > 0);
-        else
-          mma_p_times_rows(tmem_base + C::TM_DQ, ds_addr + buf * 2 * AT_REGION, k_addr + st * C::TILE,
-                           idesc_acc, j > 0);
-        umma_commit(&acc_done[buf]);
-        umma_commit(&kv_empty[st]);      // S / dP of this stage finished before the math ran
+          umma_commit(&acc_done[rd.s]);
+          umma_commit(&kv_empty[rk.s]);      // S of this tile finished before the math ran
+        }
+        __syncwarp();
+        rk.step();
+        rk.step();
+        rd.step();
       }
-      __syncwarp();
-      FT_BTRACE(1, 2, j, 5);
+      if (!first_item) tile_ph ^= 1u;
+      first_item = false;
     }
   } else if (warp < BW_MATH) {
     const int g = warp >> 2;               // column group: keys [32 g, 32 g + 32) of the block
     const int qd = warp & 3;
     const int row = qd * 32 + lane;
-    const int grow = q0 + row;
     const int c0 = 32 * g;
     const uint32_t lane_sel = (uint32_t)(qd * 32) << 16;
-    const long long sbase = ((long long)b * p.H + h) * p.S;
-    const float nlse = grow < p.S ? -p.lse[sbase + grow] : -INFINITY;
-    const float dl = grow < p.S ? p.delta[sbase + grow] : 0.f;
+    const f32x2 sl2 = pk2(p.sl2, p.sl2);
+    Ring<2> rd;
+    uint32_t blk = 0;                      // parity of the block
+    int filled = 0;                        // dS buffers written so far (2 = both have had a reader)
     bool ok = true;
-    for (int j = 0; j < nkv; ++j) {
-      const int buf = j % C::NBUF;
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 0);
-      if (!mbar_wait(s_full, j & 1, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 1);
-      tc_fence_after();
-      uint32_t rs[32], rd[32];
-      tmem_ld32(tmem_base + C::TM_S + c0 + lane_sel, rs);
-      tmem_ld32(tmem_base + C::TM_DP + c0 + lane_sel, rd);
-      tmem_ld_wait();
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 2);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(s_free);      // one arrival per warp
-      const int k0 = j * AT_T;
-      const bool need_mask = (k0 + AT_T > p.S) || (q0 + AT_T > p.S) || (p.causal && k0 + AT_T - 1 > q0);
-      uint32_t dw[16];
-      if (need_mask) {      // masked scores become -inf in a pass of their own
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int kc = k0 + c0 + i;
-          if (kc >= p.S || grow >= p.S || (p.causal && kc > grow)) rs[i] = __float_as_uint(-INFINITY);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        const float e0 = fast_exp2(fmaf(__uint_as_float(rs[i]), p.sl2, nlse));
-        const float e1 = fast_exp2(fmaf(__uint_as_float(rs[i + 1]), p.sl2, nlse));
-        dw[i >> 1] = pack_bf16(e0 * (__uint_as_float(rd[i]) - dl), e1 * (__uint_as_float(rd[i + 1]) - dl));
-      }
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 3);
-      if (j >= C::NBUF &&
-          !mbar_wait(&acc_done[buf], ((j / C::NBUF) - 1) & 1, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 4);
-      if constexpr (C::TS) {
+    // statistics of this thread's row, fetched one item ahead
+    float nl_n = 0.f, dl_n = 0.f;
+    auto fetch_stats = [&](int item) {
+      if (item < 0) return;
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb;
+      const int grow = qb * AT_T + row;
+      const long long s = (long long)hb * p.S + grow;      // lse and delta are [B, H, S]
+      nl_n = grow < p.S ? -p.lse[s] : -INFINITY;
+      dl_n = grow < p.S ? -p.delta[s] : 0.f;
+    };
+    int item = walk.next();
+    fetch_stats(item);
+    while (ok && item >= 0) {
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
+      const f32x2 nl = pk2(nl_n, nl_n), dl = pk2(dl_n, dl_n);
+      item = walk.next();
+      fetch_stats(item);
+      const int last_col = p.causal ? min(grow, p.S - 1) : p.S - 1;                 // last valid key of this row
+      const int warp_last = p.causal ? min(q0 + qd * 32, p.S - 1) : p.S - 1;       // of the warp's first row
+#pragma unroll 1
+      for (int j = 0; j < nkv; ++j) {
+        if (!mbar_wait_warp(s_full, blk, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
         tc_fence_after();
-        tmem_st16(tmem_base + C::TM_DS + 64 * buf + 16 * g + lane_sel, dw);
+        uint32_t rs[32], rdp[32];
+        tmem_ld32(tmem_base + C::TM_S + c0 + lane_sel, rs);
+        tmem_ld32(tmem_base + C::TM_DP + c0 + lane_sel, rdp);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);      // one arrival per warp
+        const int k0 = j * AT_T + c0;
+        uint32_t dw[16];
+        if (k0 + 31 > warp_last) {      // masked scores become -inf in a pass of their own
+          const int lim = last_col - k0;
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (i > lim) rs[i] = __float_as_uint(-INFINITY);
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          const f32x2 e = exp2_pair(fma2(acc2(rs, i), sl2, nl));
+          dw[i >> 1] = pack2(mul2(e, add2(acc2(rdp, i), dl)));
+        }
+        if (filled == 2 && !mbar_wait_warp(&acc_done[rd.s], rd.ph ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        if (filled < 2) ++filled;
+        tc_fence_after();
+        tmem_st16(tmem_base + C::TM_DS + 64 * rd.s + 16 * g + lane_sel, dw);
         tmem_st_wait();
         tc_fence_before();
-      } else {
-        store_row32_packed(smem + C::OFF_DS + buf * 2 * AT_REGION, row, c0, dw);
-        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ds_ready[rd.s]);      // one arrival per warp
+        rd.step();
+        blk ^= 1u;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_ready[buf]);      // one arrival per warp
-      FT_BTRACE(1, warp == 0 ? 0 : 1, j, 5);
-    }
-    if (ok && nkv > 0)
-      ok = mbar_wait(&acc_done[(nkv - 1) % C::NBUF], ((nkv - 1) / C::NBUF) & 1, ctx, FT_ERR_WAIT_TMEM_FULL);
-    if (ok && nkv > 0) {
+      // the buffer of the last block is the one before rd
+      if (!ok || !mbar_wait_warp(&acc_done[rd.s ^ 1], rd.s == 0 ? rd.ph ^ 1u : rd.ph, ctx, FT_ERR_WAIT_TMEM_FULL)) {
+        ok = false;
+        break;
+      }
       tc_fence_after();
       __nv_bfloat16* dqp = p.dq + (long long)b * p.dq_bs + (long long)grow * p.dq_ss + (long long)h * p.dq_hs;
-#pragma unroll
-      for (int ch = g; ch < HD / 32; ch += 4) {
+      if (g < HD / 32) {
         uint32_t r[32];
-        tmem_ld32(tmem_base + C::TM_DQ + ch * 32 + lane_sel, r);
+        tmem_ld32(tmem_base + C::TM_DQ + g * 32 + lane_sel, r);
         tmem_ld_wait();
-        if (grow < p.S) store_out32(dqp + ch * 32, r, p.scale);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_free);
+        if (grow < p.S) store_out32(dqp + g * 32, r, p.scale);
+      } else if (lane == 0) {
+        mbar_arrive(acc_free);
       }
-      tc_fence_before();
     }
   }
 
@@ -639,7 +802,8 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   attn_delta_kernel<LPR><<<(unsigned)((nrows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(a->o), reinterpret_cast<const __nv_bfloat16*>(a->d_o),
       a->delta, a->B, a->H, a->S, a->o_bs, a->o_ss, a->o_hs);
-  dim3 grid((unsigned)(((a->S + AT_T - 1) / AT_T) * a->H * a->B));
+  unsigned grid = 0;
+  if ((rc = set_items(p, a, AT_T, &grid))) return rc;
   attn_bwd_dkv_kernel<HD><<<grid, BW_THREADS, DkvCfg<HD>::SMEM, s>>>(tq, tk, tv, tdo, p);
   attn_bwd_dq_kernel<HD><<<grid, BW_THREADS, DqCfg<HD>::SMEM, s>>>(tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
@@ -648,12 +812,6 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
 }  // namespace ftk
 
 using namespace ftk;
-
-#ifdef FT_ATTN_TRACE
-extern "C" int ftk_attn_bwd_trace_read(long long* host, int n) {
-  return (int)cudaMemcpyFromSymbol(host, g_attn_bwd_trace, sizeof(long long) * n);
-}
-#endif
 
 extern "C" int ftk_attn_bwd(const FtkAttnDesc* a, void* stream) {
   if (!a || a->B <= 0 || a->H <= 0 || a->S <= 0 || !a->delta || !a->lse) return -2;

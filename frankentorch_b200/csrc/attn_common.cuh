@@ -12,7 +12,6 @@ int ftk_make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint6
                        uint64_t s1_elems, uint32_t box_inner, uint32_t box_outer);
 
 constexpr int AT_T = 128;           // tile rows (queries) == tile keys
-constexpr int AT_THREADS = 192;
 constexpr int AT_REGION = 16384;    // one [128 rows x 64 bf16] swizzled region
 
 struct AttnArgs {
@@ -27,12 +26,54 @@ struct AttnArgs {
   __nv_bfloat16 *dq, *dk, *dv;
   long long dq_bs, dq_ss, dq_hs, dk_bs, dk_ss, dk_hs, dv_bs, dv_ss, dv_hs;
   int* status;
+  int n_tiles;             // work items of the persistent kernels: blocks of rows x heads x batch
+  FastDiv by_hb, by_h;     // / (H * B), / H
+};
+
+// Work items of one persistent CTA.  Items are numbered heaviest first (most blocks to visit under a causal mask); round r
+// of the walk hands out gridDim.x of them, forwards in even rounds and backwards in odd ones, so that the CTA with the
+// heaviest item of one round gets the lightest of the next.  Fixed by the grid: no counters, the same on every run.
+struct TileWalk {
+  int r, n;
+  __device__ __forceinline__ explicit TileWalk(int n_items) : r(0), n(n_items) {}
+  __device__ __forceinline__ int next() {
+    const int G = (int)gridDim.x, c = (int)blockIdx.x;
+    const int idx = r * G + ((r & 1) ? G - 1 - c : c);
+    ++r;
+    return idx < n ? idx : -1;
+  }
+};
+// Ring position: slot and phase parity of the n-th use.
+template <int N>
+struct Ring {
+  int s;
+  uint32_t ph;
+  __device__ __forceinline__ Ring() : s(0), ph(0) {}
+  __device__ __forceinline__ void step() {
+    if (++s == N) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two fp32 lanes of exp2.
+__device__ __forceinline__ f32x2 exp2_pair(f32x2 x) {
+  const float2 f = up2(x);
+  return pk2(fast_exp2(f.x), fast_exp2(f.y));
+}
+__device__ __forceinline__ uint32_t pack2(f32x2 a) {
+  const float2 f = up2(a);
+  return pack_bf16(f.x, f.y);
+}
+__device__ __forceinline__ f32x2 acc2(const uint32_t* r, int i) {
+  return pk2(__uint_as_float(r[i]), __uint_as_float(r[i + 1]));
 }
 
 // A (K-major) x B (K-major)^T with K = HD, operands stored as HD/64 regions.  The descriptors'
@@ -60,28 +101,15 @@ __device__ __forceinline__ void mma_p_times_rows(uint32_t d_tmem, uint32_t p_bas
 }
 // Same product with A = probabilities held in tensor memory: 128 lanes (rows) x 64 columns of
 // packed bf16 pairs (K = 128), written by the row-owning threads with tcgen05.st.
+// K steps [K0, K1) of 16.
+template <int K0 = 0, int K1 = AT_T / 16>
 __device__ __forceinline__ void mma_ptmem_times_rows(uint32_t d_tmem, uint32_t p_tmem, uint32_t b_base,
                                                      uint32_t idesc, bool accumulate) {
   const uint32_t b_lo = desc_lo(b_base, AT_REGION);
 #pragma unroll
-  for (int kk = 0; kk < AT_T / 16; ++kk) {
+  for (int kk = K0; kk < K1; ++kk) {
     umma_bf16_ts_lo(d_tmem, p_tmem + kk * 8, b_lo + (uint32_t)(kk * 128), idesc,
                     (accumulate || kk != 0) ? 1u : 0u);
-  }
-}
-// Write 32 fp32 values of one tile row as bf16 into the swizzled K-major tile.
-__device__ __forceinline__ void store_row32_swizzled(uint8_t* tile, int row, int col0,
-                                                     const float* v) {
-  uint8_t* base = tile + (col0 >> 6) * AT_REGION + row * 128;
-  const int j0 = (col0 & 63) >> 3;
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    uint4 u;
-    u.x = pack_bf16(v[8 * t + 0], v[8 * t + 1]);
-    u.y = pack_bf16(v[8 * t + 2], v[8 * t + 3]);
-    u.z = pack_bf16(v[8 * t + 4], v[8 * t + 5]);
-    u.w = pack_bf16(v[8 * t + 6], v[8 * t + 7]);
-    *reinterpret_cast<uint4*>(base + (((j0 + t) ^ (row & 7)) << 4)) = u;
   }
 }
 template <int HD>
@@ -135,6 +163,30 @@ static inline void fill_args(AttnArgs& p, const FtkAttnDesc* a) {
   p.dk_bs = a->k_bs; p.dk_ss = a->k_ss; p.dk_hs = a->k_hs;
   p.dv_bs = a->v_bs; p.dv_ss = a->v_ss; p.dv_hs = a->v_hs;
   p.status = ftk_status_word();
+}
+
+static inline int device_sms() {
+  static int cache[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (!cache[dev]) {
+    int n = 0;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    cache[dev] = n > 0 ? n : 148;
+  }
+  return cache[dev];
+}
+
+// Work items of `rows` rows each and the grid that walks them.
+static inline int set_items(AttnArgs& p, const FtkAttnDesc* a, int rows, unsigned* grid) {
+  const long long items = ((long long)a->S + rows - 1) / rows * a->H * a->B;
+  if (items > 0x3fffffffll) return -2;
+  p.n_tiles = (int)items;
+  p.by_hb = FastDiv((uint32_t)(a->H * a->B));
+  p.by_h = FastDiv((uint32_t)a->H);
+  const int sms = device_sms();
+  *grid = (unsigned)(items < sms ? items : sms);
+  return 0;
 }
 
 template <typename K>

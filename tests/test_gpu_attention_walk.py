@@ -1,0 +1,50 @@
+"""Attention kernels with fewer and with more work items than SMs, at the edges of their 128-row blocks: gradients and
+outputs against 64-bit arithmetic, and the same bits again on a second run."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, go, causal):
+    q, k, v = (t.double().detach().requires_grad_(True) for t in (q, k, v))
+    S = q.shape[1]
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k) / math.sqrt(q.shape[-1])
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=q.device).triu(1), -math.inf)
+    o = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v)
+    return (o.detach(),) + torch.autograd.grad(o, (q, k, v), go.double())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,S,H", [
+    (1, 1, 1), (1, 127, 1), (2, 128, 3), (1, 129, 2), (1, 257, 1),
+    (3, 383, 5),        # three blocks, ragged
+    (2, 640, 16),       # 160 items: a second round with a few items only
+    (5, 264, 40),       # 600 items, several rounds, one or two blocks each
+    (1, 1500, 3),       # twelve blocks, ragged
+])
+def test_walk_over_items(cuda_device, B, S, H, hd, causal):
+    from frankentorch_b200.ops import kernels as K
+    g = torch.Generator().manual_seed(B * 1000 + S)
+    qkv = torch.randn(B, S, 3, H, hd, generator=g).to(torch.bfloat16).to(cuda_device)
+    q, k, v = (qkv[:, :, i] for i in range(3))
+    go = torch.randn(B, S, H, hd, generator=g).to(torch.bfloat16).to(cuda_device)
+    runs = []
+    for _ in range(2):
+        o, lse = K.attention_fwd(q, k, v, causal=causal)
+        d = torch.full_like(qkv, float("nan"))
+        K.attention_bwd(q, k, v, o, lse, go, causal=causal, dq=d[:, :, 0], dk=d[:, :, 1], dv=d[:, :, 2])
+        runs.append((o, d))
+    K.check_status()
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+    o, d = runs[0]
+    ro, rq, rk, rv = _reference(q, k, v, go, causal)
+    # P, dS and the outputs are rounded to bf16 (2^-9 each, independent over the sums): under 1 % of the 2-norm
+    for name, got, ref in (("o", o, ro), ("dq", d[:, :, 0], rq), ("dk", d[:, :, 1], rk), ("dv", d[:, :, 2], rv)):
+        assert got.isfinite().all(), name
+        err = float((got.double() - ref).norm() / ref.norm().clamp_min(1e-3 * go.double().norm()))
+        assert err < 1e-2, (name, err)
