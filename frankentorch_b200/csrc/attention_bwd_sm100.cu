@@ -38,30 +38,38 @@ template <int LPR>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   float* __restrict__ delta, int B, int H, int S, long long bs, long long ss,
-                  long long hs) {
-  constexpr int RPW = 32 / LPR;                       // rows per warp
+                  long long hs, FastDiv by_h, FastDiv by_s) {
+  constexpr int RPW = 32 / LPR;                       // rows per warp and step
+  constexpr int U = 4;                                // steps: four rows' loads in flight per thread
   const int lane = threadIdx.x & 31;
-  const long long w = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * RPW + lane / LPR;
   const int sub = lane % LPR;
-  float acc = 0.f;
-  const bool live = w < (long long)B * S * H;
-  int h = 0, s = 0, b = 0;
-  if (live) {
-    h = (int)(w % H);
-    const long long t = w / H;
-    s = (int)(t % S);
-    b = (int)(t / S);
-    const long long off = (long long)b * bs + (long long)s * ss + (long long)h * hs + sub * 8;
-    const uint4 a = *reinterpret_cast<const uint4*>(o + off);
-    const uint4 g = *reinterpret_cast<const uint4*>(d_o + off);
-    float2 a0 = unpack_bf16(a.x), a1 = unpack_bf16(a.y), a2 = unpack_bf16(a.z), a3 = unpack_bf16(a.w);
-    float2 g0 = unpack_bf16(g.x), g1 = unpack_bf16(g.y), g2 = unpack_bf16(g.z), g3 = unpack_bf16(g.w);
-    acc = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y + a2.x * g2.x + a2.y * g2.y +
-          a3.x * g3.x + a3.y * g3.y;
+  const long long total = (long long)B * S * H;
+  const long long w0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (RPW * U) + lane / LPR;
+  uint4 a[U], g[U];
+  long long dst[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long w = w0 + u * RPW;
+    dst[u] = -1;
+    a[u] = g[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (w < total) {
+      const int t = by_h.div((int)w), h = (int)w - t * H, b = by_s.div(t), s = t - b * S;
+      const long long off = (long long)b * bs + (long long)s * ss + (long long)h * hs + sub * 8;
+      a[u] = *reinterpret_cast<const uint4*>(o + off);
+      g[u] = *reinterpret_cast<const uint4*>(d_o + off);
+      dst[u] = ((long long)b * H + h) * S + s;
+    }
   }
 #pragma unroll
-  for (int d = LPR / 2; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-  if (live && sub == 0) delta[((long long)b * H + h) * S + s] = acc;
+  for (int u = 0; u < U; ++u) {
+    float2 a0 = unpack_bf16(a[u].x), a1 = unpack_bf16(a[u].y), a2 = unpack_bf16(a[u].z), a3 = unpack_bf16(a[u].w);
+    float2 g0 = unpack_bf16(g[u].x), g1 = unpack_bf16(g[u].y), g2 = unpack_bf16(g[u].z), g3 = unpack_bf16(g[u].w);
+    float acc = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y + a2.x * g2.x + a2.y * g2.y +
+                a3.x * g3.x + a3.y * g3.y;
+#pragma unroll
+    for (int d = LPR / 2; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (dst[u] >= 0 && sub == 0) delta[dst[u]] = acc;
+  }
 }
 
 // Store 32 packed-bf16 columns (16 words) of one tile row into the swizzled K-major tile.
@@ -74,17 +82,26 @@ __device__ __forceinline__ void store_row32_packed(uint8_t* tile, int row, int c
     *reinterpret_cast<uint4*>(base + (((j0 + t) ^ (row & 7)) << 4)) =
         make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
 }
-// Scale 32 fp32 accumulator values and store them as 32 contiguous bf16.
-__device__ __forceinline__ void store_out32(__nv_bfloat16* dst, const uint32_t* r, float scale) {
+// One warp's 32 rows x 32 columns of an output: scaled fp32 accumulator rows (a thread owns one) through the warp's part of
+// a swizzled [128 x 128] bf16 tile in shared memory, so that four lanes write 64 contiguous bytes of a row.  Stored straight
+// from its thread, a row 12 KB from the next costs 32 line accesses per instruction: ~9000 cycles per item of 128 x 2 x 128.
+__device__ __forceinline__ void store_out32(uint8_t* tile, int qd, int c0, int lane, const uint32_t* r, float scale,
+                                            __nv_bfloat16* row0, long long ss, int rows) {
+  uint32_t w[16];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    uint4 u;
-    u.x = pack_bf16(__uint_as_float(r[8 * t + 0]) * scale, __uint_as_float(r[8 * t + 1]) * scale);
-    u.y = pack_bf16(__uint_as_float(r[8 * t + 2]) * scale, __uint_as_float(r[8 * t + 3]) * scale);
-    u.z = pack_bf16(__uint_as_float(r[8 * t + 4]) * scale, __uint_as_float(r[8 * t + 5]) * scale);
-    u.w = pack_bf16(__uint_as_float(r[8 * t + 6]) * scale, __uint_as_float(r[8 * t + 7]) * scale);
-    *reinterpret_cast<uint4*>(dst + 8 * t) = u;
+  for (int i = 0; i < 16; ++i)
+    w[i] = pack_bf16(__uint_as_float(r[2 * i]) * scale, __uint_as_float(r[2 * i + 1]) * scale);
+  store_row32_packed(tile, qd * 32 + lane, c0, w);
+  __syncwarp();
+  const uint8_t* base = tile + (c0 >> 6) * AT_REGION;
+  const int seg = ((c0 & 63) >> 3) + (lane & 3);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int rr = 8 * i + (lane >> 2), row = qd * 32 + rr;
+    const uint4 u = *reinterpret_cast<const uint4*>(base + row * 128 + ((seg ^ (row & 7)) << 4));
+    if (rr < rows) *reinterpret_cast<uint4*>(row0 + (long long)rr * ss + (lane & 3) * 8) = u;
   }
+  __syncwarp();
 }
 
 // =============================================================================== backward: dK, dV
@@ -99,13 +116,13 @@ struct DkvCfg {
   // memory, and the two Q / dO stages that this leaves room for keep a load ahead of every block (with one stage and both
   // tiles in shared memory a block took ~6000 cycles, 2500 of them waiting for that load).
   static constexpr bool TS = (HD == 64);
-  static constexpr int STAGES = (HD == 64) ? 4 : 2;          // Q / dO ring
+  static constexpr int STAGES = (HD == 64) ? 3 : 2;          // Q / dO ring
   static constexpr int KVB = (HD == 64) ? 2 : 1;             // K / V buffers (one per work item)
   static constexpr int OFF_KV = 0;                           // [KVB] K, V
   static constexpr int OFF_Q = KVB * 2 * TILE;               // [STAGES]
   static constexpr int OFF_DO = OFF_Q + STAGES * TILE;       // [STAGES]
-  static constexpr int OFF_DST = OFF_DO + STAGES * TILE;     // dS^T [keys x queries] (not TS)
-  static constexpr int OFF_STAT = OFF_DST + (TS ? 0 : 2 * AT_REGION);   // [STAGES][2][128] floats
+  static constexpr int OFF_DST = OFF_DO + STAGES * TILE;     // dS^T [keys x queries] (not TS), output staging
+  static constexpr int OFF_STAT = OFF_DST + 2 * AT_REGION;   // [STAGES][2][128] floats
   static constexpr int OFF_BAR = OFF_STAT + STAGES * 2 * 128 * 4;
   static constexpr int SMEM = OFF_BAR + 256;
   static constexpr int TMEM_COLS = 512;
@@ -479,8 +496,6 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       if (!ok || !mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      __nv_bfloat16* dvp = p.dv + (long long)b * p.dv_bs + (long long)gk * p.dv_ss + (long long)h * p.dv_hs;
-      __nv_bfloat16* dkp = p.dk + (long long)b * p.dk_bs + (long long)gk * p.dk_ss + (long long)h * p.dk_hs;
       // 2 HD / 32 column chunks (dV first, then dK) spread over the four groups
       constexpr int NCH = 2 * HD / 32 / 4;
       uint32_t r[NCH][32];
@@ -495,7 +510,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const int ch = g + 4 * u;
         const bool is_dk = ch >= HD / 32;
         const int c = (is_dk ? ch - HD / 32 : ch) * 32;
-        if (gk < p.S) store_out32((is_dk ? dkp : dvp) + c, r[u], is_dk ? p.scale : 1.f);
+        const long long bs = is_dk ? p.dk_bs : p.dv_bs, ss = is_dk ? p.dk_ss : p.dv_ss, hs = is_dk ? p.dk_hs : p.dv_hs;
+        const int r0 = k0 + qd * 32;
+        store_out32(smem + C::OFF_DST, qd, c0, lane, r[u], is_dk ? p.scale : 1.f,
+                    (is_dk ? p.dk : p.dv) + b * bs + r0 * ss + h * hs + c, ss, p.S - r0);
       }
     }
   }
@@ -513,10 +531,11 @@ template <int HD>
 struct DqCfg {
   static constexpr int TILE = (HD / 64) * AT_REGION;
   static constexpr int QB = (HD == 64) ? 2 : 1;          // Q / dO buffers (one per work item)
-  static constexpr int NSLOT = (HD == 64) ? 8 : 5;       // ring of single K / V tiles: a V slot is free after dP, a K slot after dQ
+  static constexpr int NSLOT = (HD == 64) ? 8 : 4;       // ring of single K / V tiles: a V slot is free after dP, a K slot after dQ
   static constexpr int OFF_QDO = 0;                      // [QB] Q, dO
   static constexpr int OFF_KV = QB * 2 * TILE;           // [NSLOT]
-  static constexpr int OFF_BAR = OFF_KV + NSLOT * TILE;
+  static constexpr int OFF_OUT = OFF_KV + NSLOT * TILE;  // output staging
+  static constexpr int OFF_BAR = OFF_OUT + 2 * AT_REGION;
   static constexpr int SMEM = OFF_BAR + 512;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256;
@@ -757,7 +776,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         break;
       }
       tc_fence_after();
-      __nv_bfloat16* dqp = p.dq + (long long)b * p.dq_bs + (long long)grow * p.dq_ss + (long long)h * p.dq_hs;
       if (g < HD / 32) {
         uint32_t r[32];
         tmem_ld32(tmem_base + C::TM_DQ + g * 32 + lane_sel, r);
@@ -765,7 +783,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_free);
-        if (grow < p.S) store_out32(dqp + g * 32, r, p.scale);
+        const int r0 = q0 + qd * 32;
+        store_out32(smem + C::OFF_OUT, qd, c0, lane, r, p.scale,
+                    p.dq + b * p.dq_bs + r0 * p.dq_ss + h * p.dq_hs + c0, p.dq_ss, p.S - r0);
       } else if (lane == 0) {
         mbar_arrive(acc_free);
       }
@@ -798,10 +818,11 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
     attr = true;
   }
   const long long nrows = (long long)a->B * a->S * a->H;
-  constexpr int LPR = HD / 8, ROWS_PER_CTA = 8 * (32 / LPR);
+  if (nrows > 0x7fffffffll) return -2;
+  constexpr int LPR = HD / 8, ROWS_PER_CTA = 8 * (32 / LPR) * 4;
   attn_delta_kernel<LPR><<<(unsigned)((nrows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(a->o), reinterpret_cast<const __nv_bfloat16*>(a->d_o),
-      a->delta, a->B, a->H, a->S, a->o_bs, a->o_ss, a->o_hs);
+      a->delta, a->B, a->H, a->S, a->o_bs, a->o_ss, a->o_hs, FastDiv((uint32_t)a->H), FastDiv((uint32_t)a->S));
   unsigned grid = 0;
   if ((rc = set_items(p, a, AT_T, &grid))) return rc;
   attn_bwd_dkv_kernel<HD><<<grid, BW_THREADS, DkvCfg<HD>::SMEM, s>>>(tq, tk, tv, tdo, p);

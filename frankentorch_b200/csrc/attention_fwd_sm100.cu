@@ -32,6 +32,7 @@ template <int HD>
 struct Fwd2Cfg {
   static constexpr int TILE = (HD / 64) * AT_REGION;        // one [128 x HD] bf16 tile
   static constexpr bool ALIAS = (HD == 128);                // P in the columns of S
+  static constexpr bool TURNS = !ALIAS;                     // the groups' exponentials alternate
   static constexpr int QS = (HD == 64) ? 4 : 3;             // Q tiles
   static constexpr int KS = (HD == 64) ? 4 : 2;             // K ring
   static constexpr int VS = (HD == 64) ? 4 : 2;             // V ring
@@ -88,7 +89,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* q_full = bars;             // [4]
-  uint64_t* q_empty = bars + 4;        // [4]
+  uint64_t* q_empty = bars + 4;        // [4] the item's output has left through the tile (one arrival per warp)
   uint64_t* k_full = bars + 8;         // [4]
   uint64_t* k_empty = bars + 12;       // [4]
   uint64_t* v_full = bars + 16;        // [4]
@@ -109,7 +110,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     return;
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 24; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 24; ++i) mbar_init(&bars[i], i >= 4 && i < 8 ? 4 : 1);    // q_empty: one arrival per warp
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&s_free[i], 4);      // one arrival per warp of the group
@@ -215,7 +216,6 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (elect_one()) {
               mma_kmajor<HD>(tmem_base + C::TM_S + 128 * t, q_addr + q_slot[t] * C::TILE, k_addr + rk.s * C::TILE, idesc_s);
               umma_commit(&s_full[t]);
-              if (j == it.nb[t] - 1) umma_commit(&q_empty[q_slot[t]]);
             }
             __syncwarp();
           }
@@ -285,6 +285,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t p_tmem = tmem_base + C::TM_P + C::P_STRIDE * t + lane_sel;
     const f32x2 sl2 = pk2(p.sl2, p.sl2);
     uint32_t blk = 0;                        // parity of the tile's block
+    Ring<C::QS> rq;                          // the Q tile of the group's next item
     uint32_t other = 0;                      // blocks of the other group in the items before this one
     bool ok = true;
 #pragma unroll 1
@@ -293,6 +294,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int n_my = t == 0 ? it.nb[0] : it.nb[1], n_other = t == 0 ? it.nb[1] : it.nb[0];
       const uint32_t other0 = other;
       other += (uint32_t)n_other;
+      if (t == 1 && n_other > 0) rq.step();         // tile 0's Q comes first
+      const int q_slot = rq.s;
+      if (n_my > 0) rq.step();
+      if (t == 0 && n_other > 0) rq.step();
       if (n_my == 0) continue;
       const int grow = it.q0 + t * AT_T + row;
       const int last_col = p.causal ? min(grow, p.S - 1) : p.S - 1;                            // last valid key of this row
@@ -370,8 +375,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
         // The groups take turns: A's exponentials of block j, B's of block j, A's of block j + 1.  Side by side they halve
-        // each other's rate on the one unit that evaluates them, and both groups' other work then leaves it idle.
-        if (t == 0 ? (j > 0 && n_other > 0) : j < n_other) {
+        // each other's rate on the one unit that evaluates them, and both groups' other work then leaves it idle
+        // (1 x 1500 x 20 heads of 64: 26.0 us side by side, 23.5 us in turns).  With head_dim 128 the score products keep the
+        // groups apart by themselves (4 x 2048 x 16, causal: 77.5 us in turns, 75.3 us without).
+        if (C::TURNS && (t == 0 ? (j > 0 && n_other > 0) : j < n_other)) {
           const uint32_t want = other0 + (uint32_t)(t == 0 ? j - 1 : j);      // index of the other group's block
           if (!mbar_wait_warp(&e_done[t ^ 1], want & 1u, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
         }
@@ -383,7 +390,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[t]);
         exp_half(64);
-        if (lane == 0) mbar_arrive(&e_done[t]);
+        if (C::TURNS && lane == 0) mbar_arrive(&e_done[t]);
         tmem_st32(p_tmem + 32, r + 32);
         const float2 s0 = up2(add2(rs0, rs1));
         l = l * alpha + (s0.x + s0.y);
@@ -396,7 +403,6 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (!ok || !mbar_wait_warp(&pv_done[t], blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* op = p.o + (long long)it.b * p.o_bs + (long long)grow * p.o_ss + (long long)it.h * p.o_hs;
       uint32_t v[HD];
 #pragma unroll
       for (int c = 0; c < HD; c += 32) tmem_ld32(o_tmem + c, v + c);
@@ -404,19 +410,38 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&o_free[t]);
-      if (grow < p.S) {
+      // The output leaves through the warp's 32 rows of the Q tile, which the scores no longer need: eight lanes write 128
+      // contiguous bytes of a row.
+      const int r0 = it.q0 + t * AT_T + qd * 32;
+      __nv_bfloat16* op = p.o + it.b * p.o_bs + r0 * p.o_ss + it.h * p.o_hs;
+      uint8_t* stage = smem + C::OFF_Q + q_slot * C::TILE + qd * 32 * 128;
 #pragma unroll
-        for (int i = 0; i < HD; i += 8) {
+      for (int c = 0; c < HD; c += 64) {
+#pragma unroll
+        for (int i = 0; i < 64; i += 8) {
           uint4 u;
-          u.x = pack_bf16(__uint_as_float(v[i + 0]) * inv, __uint_as_float(v[i + 1]) * inv);
-          u.y = pack_bf16(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
-          u.z = pack_bf16(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv);
-          u.w = pack_bf16(__uint_as_float(v[i + 6]) * inv, __uint_as_float(v[i + 7]) * inv);
-          *reinterpret_cast<uint4*>(op + i) = u;
+          u.x = pack_bf16(__uint_as_float(v[c + i + 0]) * inv, __uint_as_float(v[c + i + 1]) * inv);
+          u.y = pack_bf16(__uint_as_float(v[c + i + 2]) * inv, __uint_as_float(v[c + i + 3]) * inv);
+          u.z = pack_bf16(__uint_as_float(v[c + i + 4]) * inv, __uint_as_float(v[c + i + 5]) * inv);
+          u.w = pack_bf16(__uint_as_float(v[c + i + 6]) * inv, __uint_as_float(v[c + i + 7]) * inv);
+          *reinterpret_cast<uint4*>(stage + (c / 64) * AT_REGION + lane * 128 + (((i >> 3) ^ (lane & 7)) << 4)) = u;
         }
-        if (p.lse)
-          p.lse[((long long)it.b * p.H + it.h) * p.S + grow] = (l > 0.f) ? m2 + log2f(l) : -INFINITY;
       }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < HD; c += 64) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = 4 * i + (lane >> 3), seg = lane & 7;
+          const uint4 u = *reinterpret_cast<const uint4*>(stage + (c / 64) * AT_REGION + rr * 128 + ((seg ^ (rr & 7)) << 4));
+          if (r0 + rr < p.S) *reinterpret_cast<uint4*>(op + rr * p.o_ss + c + seg * 8) = u;
+        }
+      }
+      fence_proxy_async_smem();        // the tile goes back to the loader
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&q_empty[q_slot]);
+      if (p.lse && grow < p.S)
+        p.lse[((long long)it.b * p.H + it.h) * p.S + grow] = (l > 0.f) ? m2 + log2f(l) : -INFINITY;
     }
   }
 

@@ -63,7 +63,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Two fp32 lanes of exp2.
+// Two fp32 lanes of exp2, on the special-function unit.
 __device__ __forceinline__ f32x2 exp2_pair(f32x2 x) {
   const float2 f = up2(x);
   return pk2(fast_exp2(f.x), fast_exp2(f.y));
