@@ -461,6 +461,9 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
   return r;
 }
+__device__ __forceinline__ f32x2 unpack_bf16_2(uint32_t u) {
+  return pk2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
 // Unsigned division by a run-time constant prepared on the host: n / d for n < 2^31 (Granlund and Montgomery's
 // round-up multiplier).  A work item is decoded by every role of every CTA; a 32-bit divide is ~150 cycles.
 struct FastDiv {

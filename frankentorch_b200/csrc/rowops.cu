@@ -34,18 +34,149 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return u;
 }
 
+// The same as pairs, two values per instruction from here on.
+__device__ __forceinline__ void unpack4x2(const uint4& u, f32x2* f) {
+  f[0] = unpack_bf16_2(u.x); f[1] = unpack_bf16_2(u.y); f[2] = unpack_bf16_2(u.z); f[3] = unpack_bf16_2(u.w);
+}
+__device__ __forceinline__ uint32_t pack_pair(f32x2 a) {
+  const float2 f = up2(a);
+  return pack_bf16(f.x, f.y);
+}
+__device__ __forceinline__ uint4 pack4x2(const f32x2* f) {
+  return make_uint4(pack_pair(f[0]), pack_pair(f[1]), pack_pair(f[2]), pack_pair(f[3]));
+}
+__device__ __forceinline__ float hsum(f32x2 a) {
+  const float2 f = up2(a);
+  return f.x + f.y;
+}
+
 constexpr int ROW_WARPS = 8;     // rows per CTA
-constexpr int ROW_CACHE = 8;     // 8 x (32 lanes x 8 elems) = 2048 columns kept in registers
 
 // ----------------------------------------------------------------------------- LayerNorm fwd
-constexpr int NF_CACHE = 4;      // forward: 4 x (32 lanes x 8 elems) = 1024 columns kept in registers
-template <bool RMS>
-__global__ void __launch_bounds__(ROW_WARPS * 32, 4)
+// Rows of up to 256 NV columns: a warp owns a row and keeps it in registers, NV 16-byte vectors per lane; wider rows (up to
+// 8192 columns) are shared by the eight warps of a CTA.  The row, gamma and beta are all requested before the first
+// addition, so a row costs one memory latency; a warp that re-reads columns beyond its registers, as it did from 1024
+// columns on, pays three.  Sums run over a lane's vectors in ascending order, then over the lanes (and warps) in a fixed tree.
+// Memory bound: 8192 x 768 6.9 -> 5.3 us (25 MB), 8192 x 2048 14.6 -> 11.6 us, 1500 x 1280 5.6 -> 3.2 us; pairs of values per
+// instruction (f32x2) are a third of the first: the kernel was at two thirds of its issue slots.
+template <int NV, int WPR, bool RMS>
+__global__ void __launch_bounds__(WPR == 1 ? 128 : 256)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
                 __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                 float eps) {
+  __shared__ float red[2][8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = WPR == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
+  const int v0 = WPR == 1 ? lane : (int)threadIdx.x;
+  constexpr int STEP = 32 * WPR;
+  if (row >= rows) return;
+  const int nvec = cols >> 3;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
+  const uint4* rr = resid ? reinterpret_cast<const uint4*>(resid + (size_t)row * cols) : nullptr;
+  const uint4* gv = reinterpret_cast<const uint4*>(gamma);
+  const uint4* bv = reinterpret_cast<const uint4*>(beta);
+  constexpr bool PRE = NV <= 6;      // more vectors than that: gamma and beta come from L1 at the end, for the registers' sake
+  uint4 xc[NV], rc[NV], gc[PRE ? NV : 1], bc[PRE ? NV : 1];
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    const int v = v0 + STEP * c;
+    xc[c] = rc[c] = make_uint4(0u, 0u, 0u, 0u);
+    if (v < nvec) {
+      xc[c] = xr[v];
+      if (rr) rc[c] = rr[v];
+    }
+  }
+  auto affine = [&](int c, uint4& g, uint4& b) {
+    const int v = v0 + STEP * c;
+    g = b = make_uint4(0u, 0u, 0u, 0u);
+    if (v < nvec) {
+      g = __ldg(gv + v);
+      if (beta) b = __ldg(bv + v);
+    }
+  };
+  if (PRE) {
+#pragma unroll
+    for (int c = 0; c < NV; ++c) affine(c, gc[PRE ? c : 0], bc[PRE ? c : 0]);
+  }
+  auto row_sum = [&](float v, int slot) -> float {
+    v = warp_sum(v);
+    if (WPR > 1) {
+      if (lane == 0) red[slot][warp] = v;
+      __syncthreads();
+      v = red[slot][0];
+#pragma unroll
+      for (int w = 1; w < WPR; ++w) v += red[slot][w];
+    }
+    return v;
+  };
+  f32x2 f[NV][4];
+  f32x2 s2 = pk2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    unpack4x2(xc[c], f[c]);
+    if (rr) {
+      f32x2 g[4];
+      unpack4x2(rc[c], g);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) f[c][i] = add2(f[c][i], g[i]);
+      const uint4 u = pack4x2(f[c]);
+      unpack4x2(u, f[c]);  // statistics are taken on the rounded sum that downstream kernels will read
+      if (sum_out && v0 + STEP * c < nvec) reinterpret_cast<uint4*>(sum_out + (size_t)row * cols)[v0 + STEP * c] = u;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s2 = RMS ? fma2(f[c][i], f[c][i], s2) : add2(s2, f[c][i]);
+  }
+  const float s = row_sum(hsum(s2), 0);
+  float mean = 0.f, rstd;
+  if (RMS) {
+    rstd = rsqrtf(s / cols + eps);
+  } else {
+    mean = s / cols;
+    const f32x2 nm = pk2(-mean, -mean);
+    f32x2 q2 = pk2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < NV; ++c)
+      if (v0 + STEP * c < nvec) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          f[c][i] = add2(f[c][i], nm);
+          q2 = fma2(f[c][i], f[c][i], q2);
+        }
+      }
+    rstd = rsqrtf(row_sum(hsum(q2), 1) / cols + eps);
+  }
+  if (v0 == 0) {
+    if (mean_out) mean_out[row] = mean;
+    rstd_out[row] = rstd;
+  }
+  const f32x2 rs = pk2(rstd, rstd);
+  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
+#pragma unroll
+  for (int c = 0; c < NV; ++c)
+    if (v0 + STEP * c < nvec) {
+      f32x2 g[4], b[4];
+      if (!PRE) affine(c, gc[0], bc[0]);
+      unpack4x2(gc[PRE ? c : 0], g);
+      unpack4x2(bc[PRE ? c : 0], b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const f32x2 h = mul2(f[c][i], rs);
+        f[c][i] = beta ? fma2(h, g[i], b[i]) : mul2(h, g[i]);
+      }
+      yr[v0 + STEP * c] = pack4x2(f[c]);
+    }
+}
+
+// Rows of more than 8192 columns: one warp walks the row three times.
+template <bool RMS>
+__global__ void __launch_bounds__(ROW_WARPS * 32)
+norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
+                     __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
+                     const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
+                     float eps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * ROW_WARPS + warp;
   if (row >= rows) return;
@@ -53,66 +184,39 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
   const uint4* rr = resid ? reinterpret_cast<const uint4*>(resid + (size_t)row * cols) : nullptr;
   uint4* so = sum_out ? reinterpret_cast<uint4*>(sum_out + (size_t)row * cols) : nullptr;
-  // The first NF_CACHE vectors of a lane (1024 columns) live in registers: every loop over
-  // them is fully unrolled so the array never spills to local memory, and all loads of the row
-  // are issued before any arithmetic (a lane that loads and reduces one vector at a time sits at
-  // memory latency).  Columns beyond the cache are re-read.  Sums run in ascending vector order
-  // in both parts, so results do not depend on the split.
-  uint4 cache[NF_CACHE];
-  uint4 rcache[NF_CACHE];
-#pragma unroll
-  for (int c = 0; c < NF_CACHE; ++c) {
-    const int v = lane + 32 * c;
-    if (v < nvec) {
-      cache[c] = xr[v];
-      if (rr) rcache[c] = rr[v];
-    }
-  }
+  const uint4* src = rr ? reinterpret_cast<const uint4*>(so) : xr;
   float s = 0.f;
-  auto first_pass = [&](uint4 u, const uint4& r, int v) -> uint4 {
+  for (int v = lane; v < nvec; v += 32) {
     float f[8];
-    unpack8(u, f);
+    unpack8(xr[v], f);
     if (rr) {
       float g[8];
-      unpack8(r, g);
+      unpack8(rr[v], g);
 #pragma unroll
       for (int i = 0; i < 8; ++i) f[i] += g[i];
-      u = pack8(f);
-      unpack8(u, f);  // statistics are taken on the rounded sum that downstream kernels will read
+      const uint4 u = pack8(f);
+      unpack8(u, f);
       if (so) so[v] = u;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += RMS ? f[i] * f[i] : f[i];
-    return u;
-  };
-#pragma unroll
-  for (int c = 0; c < NF_CACHE; ++c) {
-    const int v = lane + 32 * c;
-    if (v < nvec) cache[c] = first_pass(cache[c], rcache[c], v);
   }
-  for (int v = lane + 32 * NF_CACHE; v < nvec; v += 32)
-    first_pass(xr[v], rr ? rr[v] : make_uint4(0u, 0u, 0u, 0u), v);
   s = warp_sum(s);
   float mean = 0.f, rstd;
-  const uint4* src = rr ? reinterpret_cast<const uint4*>(so) : xr;
   if (RMS) {
     rstd = rsqrtf(s / cols + eps);
   } else {
     mean = s / cols;
     float q = 0.f;
-    auto second_pass = [&](const uint4& u) {
+    for (int v = lane; v < nvec; v += 32) {
       float f[8];
-      unpack8(u, f);
+      unpack8(src[v], f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        float d = f[i] - mean;
+        const float d = f[i] - mean;
         q += d * d;
       }
-    };
-#pragma unroll
-    for (int c = 0; c < NF_CACHE; ++c)
-      if (lane + 32 * c < nvec) second_pass(cache[c]);
-    for (int v = lane + 32 * NF_CACHE; v < nvec; v += 32) second_pass(src[v]);
+    }
     q = warp_sum(q);
     rstd = rsqrtf(q / cols + eps);
   }
@@ -123,22 +227,18 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   const uint4* gv = reinterpret_cast<const uint4*>(gamma);
   const uint4* bv = beta ? reinterpret_cast<const uint4*>(beta) : nullptr;
   uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
-  auto write_out = [&](const uint4& u, int v) {
+  for (int v = lane; v < nvec; v += 32) {
     float f[8], g[8], b[8];
-    unpack8(u, f);
+    unpack8(src[v], f);
     unpack8(__ldg(gv + v), g);
     if (bv) unpack8(__ldg(bv + v), b);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float h = (f[i] - mean) * rstd * g[i];
+      const float h = (f[i] - mean) * rstd * g[i];
       f[i] = bv ? h + b[i] : h;
     }
     yr[v] = pack8(f);
-  };
-#pragma unroll
-  for (int c = 0; c < NF_CACHE; ++c)
-    if (lane + 32 * c < nvec) write_out(cache[c], lane + 32 * c);
-  for (int v = lane + 32 * NF_CACHE; v < nvec; v += 32) write_out(src[v], v);
+  }
 }
 
 // ----------------------------------------------------------------------------- LayerNorm bwd dx
@@ -193,156 +293,232 @@ norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// ----------------------------------------------------------------------------- LayerNorm bwd, one pass
-// dx and the per-block column partials of dgamma / dbeta from a single read of dy and x.
-// A CTA of 8 warps owns LNB_ROWS consecutive rows; warp w takes rows w, w + 8, ... in ascending
-// order.  The loads of a warp's next row are issued before the arithmetic of the current one
-// (register double buffer), so a warp always has a row in flight; gamma is read from shared
-// memory.  Per-lane column accumulators of dy*xhat / dy are added over the 8 warps in warp order
-// through one shared-memory pass per quantity (layout [warp][i][vector]: conflict-free both ways)
-// and the CTA writes partial[blk][c].  NV = 16-byte vectors per lane.
-constexpr int LNB_ROWS = 32;
-template <int NV>
+// ----------------------------------------------------------------------------- norm bwd, one pass
+// dx and the per-block column partials of dgamma / dbeta from a single read of dy and x (and of the gradient that is added to
+// dx), rows of up to 8192 columns.  A CTA of 8 warps owns a contiguous range of rows and takes them in steps of G = 8 / WPR
+// rows, WPR warps per row, NV 16-byte vectors per lane.  The rows of a step are one contiguous piece of each array: bulk
+// copies bring it into a ring of shared-memory stages, so the bytes in flight per SM do not depend on registers.  Column
+// sums of dy * xhat and dy stay in registers; at the end the G groups' sums are added in group order and the CTA writes
+// partial[blk][c].  Rows go to CTAs and warps by index alone, so the result does not depend on scheduling.
+// Memory bound from some thousand rows on: with the gradient that is added, column sums finished, 8192 x 768 17.9 -> 15.9 us
+// (one row per warp prefetched in registers before), 8192 x 2048 62.9 -> 37.1 us and 1500 x 1280 15.8 -> 10.6 us (three
+// kernels before: rows wider than 768 columns spilled the column sums of one warp per row).
+constexpr int NB_MAX_BLOCKS = 296;       // two CTAs per SM
+constexpr int NB_RING_BYTES = 96 * 1024; // operand stages of one CTA
+template <int NV, int WPR, bool RMS>
 __global__ void __launch_bounds__(ROW_WARPS * 32, 2)
-ln_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                    const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                    const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dx_add,
-                    __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int cols,
-                    int nblk) {
-  constexpr int VEC = NV * 32;                      // vectors of a (padded) row
-  __shared__ float red[ROW_WARPS][8 * VEC];
-  __shared__ uint4 sgam[VEC];
+norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                      const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
+                      const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dx_add,
+                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int cols,
+                      int rows_per_blk, int stages, int* status) {
+  constexpr int G = ROW_WARPS / WPR;
+  extern __shared__ __align__(128) uint8_t nb_smem[];
+  __shared__ uint64_t full[8], empty[8];
+  __shared__ int abort_w;
+  __shared__ float red[2][ROW_WARPS][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = warp / WPR;                            // row of the step
+  const int v0 = (warp % WPR) * 32 + lane;               // first vector of this lane
+  constexpr int STEP = 32 * WPR;
   const int nvec = cols >> 3;
-  for (int v = threadIdx.x; v < VEC; v += blockDim.x)
-    sgam[v] = v < nvec ? __ldg(reinterpret_cast<const uint4*>(gamma) + v) : make_uint4(0u, 0u, 0u, 0u);
-  float dg[NV][8], db[NV][8];
+  const int n_arr = dx_add ? 3 : 2;
+  const uint32_t piece = (uint32_t)(G * cols * 2);       // bytes of one array in one stage
+  WaitCtx ctx{status, &abort_w};
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], ROW_WARPS);
+    }
+    abort_w = 0;
+    fence_mbar_init();
+  }
+  uint4 gam[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    gam[j] = v0 + STEP * j < nvec ? __ldg(reinterpret_cast<const uint4*>(gamma) + v0 + STEP * j) : make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  const int row_begin = blockIdx.x * rows_per_blk, row_end = min(rows, row_begin + rows_per_blk);
+  const int steps = row_end > row_begin ? (row_end - row_begin + G - 1) / G : 0;
+  auto load_step = [&](int st) {       // one thread
+    const int r = row_begin + st * G, n = min(G, row_end - r);
+    uint8_t* dst = nb_smem + (size_t)(st % stages) * n_arr * piece;
+    uint64_t* bar = &full[st % stages];
+    const uint32_t bytes = (uint32_t)(n * cols * 2);
+    mbar_arrive_expect_tx(bar, n_arr * bytes);
+    auto copy = [&](int a, const __nv_bfloat16* src) {
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"(smem_u32(dst + a * piece)), "l"(src + (size_t)r * cols), "r"(bytes), "r"(smem_u32(bar))
+                   : "memory");
+    };
+    copy(0, x);
+    copy(1, dy);
+    if (dx_add) copy(2, dx_add);
+  };
+  if ((int)threadIdx.x < stages && (int)threadIdx.x < steps) load_step((int)threadIdx.x);      // one thread per stage
+  f32x2 dg[NV][4], db[NV][4];
 #pragma unroll
   for (int j = 0; j < NV; ++j)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) dg[j][i] = db[j][i] = 0.f;
-  const int row0 = blockIdx.x * LNB_ROWS + warp;
-  const int row_end = min(rows, (int)(blockIdx.x + 1) * LNB_ROWS);
-  uint4 xn[NV], dn[NV];
+    for (int i = 0; i < 4; ++i) dg[j][i] = db[j][i] = pk2(0.f, 0.f);
+  bool ok = true;
   float mean_n = 0.f, rstd_n = 0.f;
-  auto fetch = [&](int row) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + (size_t)row * cols);
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int v = lane + 32 * j;
-      xn[j] = v < nvec ? __ldcs(xr + v) : make_uint4(0u, 0u, 0u, 0u);
-      dn[j] = v < nvec ? __ldcs(dr + v) : make_uint4(0u, 0u, 0u, 0u);
+  auto fetch_stats = [&](int st) {
+    const int row = row_begin + st * G + grp;
+    if (row < row_end) {
+      mean_n = RMS ? 0.f : __ldg(mean_in + row);
+      rstd_n = __ldg(rstd_in + row);
     }
-    mean_n = __ldg(mean_in + row);
-    rstd_n = __ldg(rstd_in + row);
   };
-  if (row0 < row_end) fetch(row0);
-  __syncthreads();                                  // gamma is in shared memory
-  for (int row = row0; row < row_end; row += ROW_WARPS) {
-    uint4 xp[NV], dp[NV];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      xp[j] = xn[j];
-      dp[j] = dn[j];
-    }
+  fetch_stats(0);
+  for (int st = 0; st < steps; ++st) {
+    const int row = row_begin + st * G + grp;
+    const bool live = row < row_end;
     const float mean = mean_n, rstd = rstd_n;
-    if (row + ROW_WARPS < row_end) fetch(row + ROW_WARPS);     // in flight during this row's arithmetic
-    float s1 = 0.f, s2 = 0.f;
+    fetch_stats(st + 1);
+    if (ok) ok = mbar_wait(&full[st % stages], (st / stages) & 1, ctx, FT_ERR_WAIT_FULL);
+    const uint8_t* src = nb_smem + (size_t)(st % stages) * n_arr * piece + (size_t)grp * cols * 2;
+    const uint4* xv = reinterpret_cast<const uint4*>(src);
+    const uint4* dv = reinterpret_cast<const uint4*>(src + piece);
+    const uint4* av = reinterpret_cast<const uint4*>(src + 2 * piece);
+    const f32x2 nm = pk2(-mean, -mean), rs = pk2(rstd, rstd);
+    f32x2 a1 = pk2(0.f, 0.f), a2 = a1;
+    if (live && ok) {
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      if (lane + 32 * j < nvec) {
-        float fx[8], fd[8], g[8];
-        unpack8(xp[j], fx);
-        unpack8(dp[j], fd);
-        unpack8(sgam[lane + 32 * j], g);
+      for (int j = 0; j < NV; ++j)
+        if (v0 + STEP * j < nvec) {
+          f32x2 fx[4], fd[4], g[4];
+          unpack4x2(xv[v0 + STEP * j], fx);
+          unpack4x2(dv[v0 + STEP * j], fd);
+          unpack4x2(gam[j], g);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float gd = g[i] * fd[i];
-          const float xh = (fx[i] - mean) * rstd;
-          s1 += gd;
-          s2 += gd * xh;
-          dg[j][i] += fd[i] * xh;
-          db[j][i] += fd[i];
+          for (int i = 0; i < 4; ++i) {
+            const f32x2 gd = mul2(g[i], fd[i]);
+            const f32x2 xh = mul2(RMS ? fx[i] : add2(fx[i], nm), rs);
+            if (!RMS) a1 = add2(a1, gd);
+            a2 = fma2(gd, xh, a2);
+            dg[j][i] = fma2(fd[i], xh, dg[j][i]);
+            if (!RMS) db[j][i] = add2(db[j][i], fd[i]);
+          }
         }
+    }
+    float s1 = RMS ? 0.f : hsum(a1), s2 = hsum(a2);
+    if (!RMS) s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (WPR > 1) {
+      if (lane == 0) {
+        red[st & 1][warp][0] = s1;
+        red[st & 1][warp][1] = s2;
+      }
+      __syncthreads();
+      s1 = s2 = 0.f;
+#pragma unroll
+      for (int w = 0; w < WPR; ++w) {
+        s1 += red[st & 1][grp * WPR + w][0];
+        s2 += red[st & 1][grp * WPR + w][1];
       }
     }
-    s1 = warp_sum(s1) / cols;
-    s2 = warp_sum(s2) / cols;
-    const uint4* av = dx_add ? reinterpret_cast<const uint4*>(dx_add + (size_t)row * cols) : nullptr;
-    uint4* ov = reinterpret_cast<uint4*>(dx + (size_t)row * cols);
+    const f32x2 m1 = pk2(-s1 / cols, -s1 / cols), m2 = pk2(-s2 / cols, -s2 / cols);
+    if (live && ok) {
+      uint4* ov = reinterpret_cast<uint4*>(dx + (size_t)row * cols);
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      const int v = lane + 32 * j;
-      if (v < nvec) {
-        float fx[8], fd[8], g[8], a[8];
-        unpack8(xp[j], fx);
-        unpack8(dp[j], fd);
-        unpack8(sgam[v], g);
-        if (av) unpack8(av[v], a);
+      for (int j = 0; j < NV; ++j)
+        if (v0 + STEP * j < nvec) {
+          f32x2 fx[4], fd[4], g[4], a[4];
+          unpack4x2(xv[v0 + STEP * j], fx);
+          unpack4x2(dv[v0 + STEP * j], fd);
+          unpack4x2(gam[j], g);
+          if (dx_add) unpack4x2(av[v0 + STEP * j], a);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float xh = (fx[i] - mean) * rstd;
-          const float r = rstd * (g[i] * fd[i] - s1 - xh * s2);
-          fx[i] = av ? r + a[i] : r;
+          for (int i = 0; i < 4; ++i) {
+            const f32x2 xh = mul2(RMS ? fx[i] : add2(fx[i], nm), rs);
+            f32x2 t = mul2(g[i], fd[i]);
+            if (!RMS) t = add2(t, m1);
+            t = fma2(xh, m2, t);
+            fx[i] = dx_add ? fma2(rs, t, a[i]) : mul2(rs, t);
+          }
+          ov[v0 + STEP * j] = pack4x2(fx);
         }
-        ov[v] = pack8(fx);
-      }
+    }
+    fence_proxy_async_smem();            // this warp has read its part of the stage
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[st % stages]);
+    // the stage of the step before (the other warps have left it by now) takes the next rows
+    if (threadIdx.x == 0 && ok && st > 0 && st - 1 + stages < steps) {
+      if (mbar_wait(&empty[(st - 1) % stages], ((st - 1) / stages) & 1, ctx, FT_ERR_WAIT_EMPTY)) load_step(st - 1 + stages);
     }
   }
-  // the 8 warps' column accumulators, added in warp order: dgamma first, then dbeta
-  float* pg = partial + (size_t)blockIdx.x * cols;
-  float* pb = partial + ((size_t)nblk + blockIdx.x) * cols;
+  // the groups' column sums, added in group order: dgamma first, then dbeta
+  if (!partial) return;
+  constexpr int NS = RMS ? 1 : 2;                        // dgamma, dbeta
+  float* acc = reinterpret_cast<float*>(nb_smem);        // [NS][G][cols], in the stages
+  __syncthreads();                                       // the stages have been read
 #pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass) __syncthreads();                      // the sums of pass 0 have been read
+  for (int k = 0; k < NS; ++k) {
+    float* d0 = G > 1 ? acc + (size_t)(k * G + grp) * cols : partial + ((size_t)k * gridDim.x + blockIdx.x) * cols;
 #pragma unroll
     for (int j = 0; j < NV; ++j)
+      if (v0 + STEP * j < nvec) {
+        float* d = d0 + (v0 + STEP * j) * 8;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) red[warp][i * VEC + lane + 32 * j] = pass ? db[j][i] : dg[j][i];
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < 8 * VEC; idx += blockDim.x) {
-      const int i = idx / VEC, v = idx - i * VEC;
-      if (v < nvec) {
-        float t = red[0][idx];
-#pragma unroll
-        for (int w = 1; w < ROW_WARPS; ++w) t += red[w][idx];
-        (pass ? pb : pg)[v * 8 + i] = t;
+        for (int h = 0; h < 2; ++h) {
+          const float2 lo = up2(k ? db[j][2 * h] : dg[j][2 * h]), hi = up2(k ? db[j][2 * h + 1] : dg[j][2 * h + 1]);
+          reinterpret_cast<float4*>(d)[h] = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
       }
+  }
+  if (G == 1) return;
+  __syncthreads();
+  for (int c = threadIdx.x * 4; c < cols; c += blockDim.x * 4) {
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      float4 t = *reinterpret_cast<const float4*>(acc + (size_t)k * G * cols + c);
+#pragma unroll
+      for (int g = 1; g < G; ++g) {
+        const float4 u = *reinterpret_cast<const float4*>(acc + (size_t)(k * G + g) * cols + c);
+        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+      }
+      *reinterpret_cast<float4*>(partial + ((size_t)k * gridDim.x + blockIdx.x) * cols + c) = t;
     }
   }
 }
 
-// Fixed-order sum over many block partials, parallel over 8 interleaved groups of blocks:
-// thread (g, c) adds partial[b][c] for b = g, g + 8, ... ascending, then the 8 group sums are
-// added in group order.  `two` arrays per launch (dgamma and dbeta).
-__global__ void __launch_bounds__(256)
+// Fixed-order sum over block partials: a CTA takes 32 columns, warp g adds partial[b][c] for b = g, g + 32, ... ascending
+// with up to eight loads of each array in flight, then the 32 group sums of a column are added by a fixed shuffle tree.  A
+// second array (dbeta) goes along.  All latency: with 8 groups of serial loads 256 partials x 768 took 4.9 us, now 3.1 us.
+__global__ void __launch_bounds__(1024)
 col_final_wide_kernel(const float* __restrict__ partial, float* __restrict__ out,
                       const float* __restrict__ partial2, float* __restrict__ out2, int cols, int nblk,
                       int accumulate) {
-  __shared__ float sm[2][8][32];
+  __shared__ float sm[2][32][33];
   const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cl;
   float s = 0.f, t = 0.f;
   if (c < cols) {
-#pragma unroll 4
-    for (int b = g; b < nblk; b += 8) {
-      s += partial[(size_t)b * cols + c];
-      if (partial2) t += partial2[(size_t)b * cols + c];
+    for (int b0 = g; b0 < nblk; b0 += 32 * 8) {
+      float u[8], w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int b = b0 + 32 * k;
+        u[k] = b < nblk ? partial[(size_t)b * cols + c] : 0.f;
+        w[k] = (partial2 && b < nblk) ? partial2[(size_t)b * cols + c] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        s += u[k];
+        t += w[k];
+      }
     }
   }
   sm[0][g][cl] = s;
   sm[1][g][cl] = t;
   __syncthreads();
-  if (g == 0 && c < cols) {
-    float a = 0.f, b2 = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      a += sm[0][k][cl];
-      b2 += sm[1][k][cl];
-    }
-    out[c] = accumulate ? out[c] + a : a;
-    if (partial2) out2[c] = accumulate ? out2[c] + b2 : b2;
+  // warp g now owns column g of the 32; lane = group
+  const float a = warp_sum(sm[0][cl][g]), b2 = partial2 ? warp_sum(sm[1][cl][g]) : 0.f;
+  const int cc = blockIdx.x * 32 + g;
+  if (cl == 0 && cc < cols) {
+    out[cc] = accumulate ? out[cc] + a : a;
+    if (partial2) out2[cc] = accumulate ? out2[cc] + b2 : b2;
   }
 }
 
@@ -402,25 +578,6 @@ col_partial_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     }
   }
 }
-// Serial (fixed-order) sum over block partials; `two` reduces a second array (dbeta) in the
-// same launch.
-__global__ void __launch_bounds__(128)
-col_final_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                 const float* __restrict__ partial2, float* __restrict__ out2, int cols, int nblk,
-                 int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f, t = 0.f;
-#pragma unroll 8
-  for (int b = 0; b < nblk; ++b) s += partial[(size_t)b * cols + c];
-  out[c] = accumulate ? out[c] + s : s;
-  if (partial2) {
-#pragma unroll 8
-    for (int b = 0; b < nblk; ++b) t += partial2[(size_t)b * cols + c];
-    out2[c] = accumulate ? out2[c] + t : t;
-  }
-}
-
 // ----------------------------------------------------------------------------- softmax
 template <typename T>
 __device__ __forceinline__ float ldf(const T* p);
@@ -681,68 +838,133 @@ using namespace ftk;
 #define BF(p) reinterpret_cast<const __nv_bfloat16*>(p)
 #define BFW(p) reinterpret_cast<__nv_bfloat16*>(p)
 
+template <bool RMS>
+static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, const void* gamma, const void* beta, void* y,
+                           float* mean, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
+#define FT_NORM_FWD(NV, WPR)                                                                                   \
+  norm_fwd_kernel<NV, WPR, RMS><<<WPR == 1 ? (rows + 3) / 4 : rows, WPR == 1 ? 128 : 256, 0, s>>>(             \
+      BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps)
+  const int nvec = cols / 8, per_lane = (nvec + 31) / 32;
+  // Up to 1536 columns a row is one warp's.  Wider rows take a CTA each, except where there are enough rows of up to 2048
+  // columns to fill the chip with warps (8192 x 2048: 11.6 against 16.4 us).
+  if (per_lane <= 1) FT_NORM_FWD(1, 1);
+  else if (per_lane <= 2) FT_NORM_FWD(2, 1);
+  else if (per_lane <= 3) FT_NORM_FWD(3, 1);
+  else if (per_lane <= 4) FT_NORM_FWD(4, 1);
+  else if (per_lane <= 6) FT_NORM_FWD(6, 1);
+  else if (per_lane <= 8 && rows >= 2048) FT_NORM_FWD(8, 1);
+  else if (nvec <= 256) FT_NORM_FWD(1, 8);
+  else if (nvec <= 512) FT_NORM_FWD(2, 8);
+  else if (nvec <= 1024) FT_NORM_FWD(4, 8);
+  else
+    norm_fwd_long_kernel<RMS><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
+        BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps);
+#undef FT_NORM_FWD
+  return (int)cudaGetLastError();
+}
 extern "C" int ftk_layernorm_fwd(const void* x, const void* resid_in, void* sum_out,
                                  const void* gamma, const void* beta, void* y, float* mean,
                                  float* rstd, int rows, int cols, float eps, void* stream) {
   if (cols % 8 || rows <= 0) return -2;
   if (resid_in && !sum_out) return -3;
-  norm_fwd_kernel<false><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, STREAM(stream)>>>(
-      BF(x), BF(resid_in), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps);
-  return (int)cudaGetLastError();
+  return norm_fwd_launch<false>(x, resid_in, sum_out, gamma, beta, y, mean, rstd, rows, cols, eps, STREAM(stream));
 }
 extern "C" int ftk_rmsnorm_fwd(const void* x, const void* gamma, void* y, float* rstd, int rows,
                                int cols, float eps, void* stream) {
   if (cols % 8 || rows <= 0) return -2;
-  norm_fwd_kernel<true><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, STREAM(stream)>>>(
-      BF(x), nullptr, nullptr, BF(gamma), nullptr, BFW(y), nullptr, rstd, rows, cols, eps);
-  return (int)cudaGetLastError();
+  return norm_fwd_launch<true>(x, nullptr, nullptr, gamma, nullptr, y, nullptr, rstd, rows, cols, eps, STREAM(stream));
 }
 // number of partial blocks the caller must provide room for (2 * blocks * cols floats)
-extern "C" int ftk_layernorm_bwd_blocks(int rows) { return (rows + LNB_ROWS - 1) / LNB_ROWS; }
 static int norm_col_blocks(int rows) { return (rows + COL_ROWS_PER_BLK - 1) / COL_ROWS_PER_BLK; }
+extern "C" int ftk_layernorm_bwd_blocks(int rows) {
+  const int fused = rows < NB_MAX_BLOCKS ? rows : NB_MAX_BLOCKS, wide = norm_col_blocks(rows);
+  return fused > wide ? fused : wide;
+}
 
+template <int NV, int WPR, bool RMS>
+static int norm_bwd_fused_launch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                                 const void* dx_add, void* dx, float* partial, int rows, int cols, int nblk, cudaStream_t s) {
+  constexpr int G = ROW_WARPS / WPR;
+  int* status = ftk_status_word();
+  if (!status) return -6;
+  const size_t stage = (size_t)(dx_add ? 3 : 2) * G * cols * 2;
+  int stages = (int)(NB_RING_BYTES / stage);
+  if (stages > 8) stages = 8;
+  if (stages < 2) stages = 2;
+  size_t smem = stages * stage;
+  const size_t sums = G > 1 ? (size_t)(RMS ? 1 : 2) * G * cols * 4 : 0;
+  if (smem < sums) smem = sums;
+  static bool done[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (!done[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(norm_bwd_fused_kernel<NV, WPR, RMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         112 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    done[dev] = true;
+  }
+  norm_bwd_fused_kernel<NV, WPR, RMS><<<nblk, ROW_WARPS * 32, smem, s>>>(
+      BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add), BFW(dx), partial, rows, cols, (rows + nblk - 1) / nblk, stages, status);
+  return (int)cudaGetLastError();
+}
+template <bool RMS>
+static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
+                           const void* dx_add, void* dx, float* dgamma, float* dbeta, float* partial, int rows, int cols,
+                           int accumulate, cudaStream_t s) {
+  const int nvec = cols / 8;
+  int nblk = 0, rc = 0;
+  if (dgamma && nvec <= 1024) {
+    // One pass.  WPR warps per row so that a lane holds at most three vectors (four at the widest) and its column sums stay
+    // in registers.
+    const int wpr = nvec <= 96 ? 1 : (nvec <= 192 ? 2 : (nvec <= 384 ? 4 : 8));
+    const int nv = (nvec + 32 * wpr - 1) / (32 * wpr), G = ROW_WARPS / wpr;
+    nblk = (rows + G - 1) / G;
+    if (nblk > NB_MAX_BLOCKS) nblk = NB_MAX_BLOCKS;
+    const int per = ((rows + nblk - 1) / nblk + G - 1) / G * G;     // whole steps
+    nblk = (rows + per - 1) / per;
+#define FT_NORM_BWD(NV, WPR) \
+  rc = norm_bwd_fused_launch<NV, WPR, RMS>(dy, x, gamma, mean, rstd, dx_add, dx, partial, rows, cols, nblk, s)
+    switch (wpr * 8 + nv) {
+      case 9: FT_NORM_BWD(1, 1); break;
+      case 10: FT_NORM_BWD(2, 1); break;
+      case 11: FT_NORM_BWD(3, 1); break;
+      case 18: FT_NORM_BWD(2, 2); break;
+      case 19: FT_NORM_BWD(3, 2); break;
+      case 34: FT_NORM_BWD(2, 4); break;
+      case 35: FT_NORM_BWD(3, 4); break;
+      case 66: FT_NORM_BWD(2, 8); break;
+      case 67: FT_NORM_BWD(3, 8); break;
+      case 68: FT_NORM_BWD(4, 8); break;
+      default: return -7;
+    }
+#undef FT_NORM_BWD
+    if (rc) return rc;
+  } else {
+    norm_bwd_dx_kernel<RMS><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
+        BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add), BFW(dx), rows, cols);
+    if (!dgamma) return (int)cudaGetLastError();
+    nblk = norm_col_blocks(rows);
+    dim3 g((cols / 2 + 31) / 32, nblk);
+    col_partial_kernel<RMS ? 1 : 0><<<g, 256, 0, s>>>(BF(dy), BF(x), mean, rstd, partial, rows, cols, cols, nblk);
+  }
+  col_final_wide_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, dgamma, RMS ? nullptr : partial + (size_t)nblk * cols,
+                                                          dbeta, cols, nblk, accumulate);
+  return (int)cudaGetLastError();
+}
 extern "C" int ftk_layernorm_bwd(const void* dy, const void* x, const void* gamma,
                                  const float* mean, const float* rstd, const void* dx_add, void* dx,
                                  float* dgamma, float* dbeta, float* partial, int rows, int cols,
                                  int accumulate, void* stream) {
   if (cols % 8 || rows <= 0) return -2;
-  cudaStream_t s = STREAM(stream);
-  if (dgamma && cols <= 768) {
-    // one pass: dx + column partials, then the fixed-order sum over blocks (wider rows would
-    // spill the per-lane column accumulators and take the three-kernel path below)
-    const int nblk = ftk_layernorm_bwd_blocks(rows);
-    ln_bwd_fused_kernel<3><<<nblk, ROW_WARPS * 32, 0, s>>>(BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add),
-                                                          BFW(dx), partial, rows, cols, nblk);
-    col_final_wide_kernel<<<(cols + 31) / 32, 256, 0, s>>>(partial, dgamma, partial + (size_t)nblk * cols, dbeta,
-                                                           cols, nblk, accumulate);
-    return (int)cudaGetLastError();
-  }
-  norm_bwd_dx_kernel<false><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
-      BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add), BFW(dx), rows, cols);
-  if (dgamma) {
-    const int nblk = norm_col_blocks(rows);
-    dim3 g((cols / 2 + 31) / 32, nblk);
-    col_partial_kernel<0><<<g, 256, 0, s>>>(BF(dy), BF(x), mean, rstd, partial, rows, cols, cols, nblk);
-    col_final_kernel<<<(cols + 127) / 128, 128, 0, s>>>(partial, dgamma, partial + (size_t)nblk * cols,
-                                                         dbeta, cols, nblk, accumulate);
-  }
-  return (int)cudaGetLastError();
+  return norm_bwd_launch<false>(dy, x, gamma, mean, rstd, dx_add, dx, dgamma, dbeta, partial, rows, cols, accumulate,
+                                STREAM(stream));
 }
 extern "C" int ftk_rmsnorm_bwd(const void* dy, const void* x, const void* gamma, const float* rstd,
                                void* dx, float* dgamma, float* partial, int rows, int cols,
                                int accumulate, void* stream) {
   if (cols % 8 || rows <= 0) return -2;
-  cudaStream_t s = STREAM(stream);
-  norm_bwd_dx_kernel<true><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
-      BF(dy), BF(x), BF(gamma), nullptr, rstd, nullptr, BFW(dx), rows, cols);
-  if (dgamma) {
-    const int nblk = norm_col_blocks(rows);
-    dim3 g((cols / 2 + 31) / 32, nblk);
-    col_partial_kernel<1><<<g, 256, 0, s>>>(BF(dy), BF(x), nullptr, rstd, partial, rows, cols, cols, nblk);
-    col_final_wide_kernel<<<(cols + 31) / 32, 256, 0, s>>>(partial, dgamma, nullptr, nullptr, cols, nblk,
-                                                           accumulate);
-  }
-  return (int)cudaGetLastError();
+  return norm_bwd_launch<true>(dy, x, gamma, nullptr, rstd, nullptr, dx, dgamma, nullptr, partial, rows, cols, accumulate,
+                               STREAM(stream));
 }
 // Plain column sums with 16-byte loads: a CTA covers 256 columns x CSW_ROWS rows as 8 row groups of
 // 32 lanes x 8 columns.  Each thread adds its rows (r0 + group, + 8, ...) in ascending order with four
@@ -819,7 +1041,7 @@ extern "C" int ftk_colsum_bf16(const void* x, float* out, float* partial, int ro
     dim3 g((cols / 2 + 31) / 32, nblk);
     col_partial_kernel<2><<<g, 256, 0, s>>>(BF(x), nullptr, nullptr, nullptr, partial, rows, cols, ld, nblk);
   }
-  col_final_wide_kernel<<<(cols + 31) / 32, 256, 0, s>>>(partial, out, nullptr, nullptr, cols, nblk, accumulate);
+  col_final_wide_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, out, nullptr, nullptr, cols, nblk, accumulate);
   return (int)cudaGetLastError();
 }
 
