@@ -39,6 +39,8 @@ __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   float* __restrict__ delta, int B, int H, int S, long long bs, long long ss,
                   long long hs, FastDiv by_h, FastDiv by_s) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int RPW = 32 / LPR;                       // rows per warp and step
   constexpr int U = 4;                                // steps: four rows' loads in flight per thread
   const int lane = threadIdx.x & 31;
@@ -161,6 +163,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   WaitCtx ctx{p.status, abort_f};
 
   if ((smem_u32(smem) & 1023u) != 0u) {
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -199,6 +202,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   const int n_hb = p.H * p.B;
   const int nq_all = (p.S + AT_T - 1) / AT_T;
@@ -567,6 +572,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   WaitCtx ctx{p.status, abort_f};
 
   if ((smem_u32(smem) & 1023u) != 0u) {
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -601,6 +607,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   // items are numbered with the most key blocks (the late query blocks under a causal mask) first
   const int n_hb = p.H * p.B;
@@ -820,13 +828,13 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   const long long nrows = (long long)a->B * a->S * a->H;
   if (nrows > 0x7fffffffll) return -2;
   constexpr int LPR = HD / 8, ROWS_PER_CTA = 8 * (32 / LPR) * 4;
-  attn_delta_kernel<LPR><<<(unsigned)((nrows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, s>>>(
+  launch_pdl(attn_delta_kernel<LPR>, (unsigned)((nrows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, s,
       reinterpret_cast<const __nv_bfloat16*>(a->o), reinterpret_cast<const __nv_bfloat16*>(a->d_o),
       a->delta, a->B, a->H, a->S, a->o_bs, a->o_ss, a->o_hs, FastDiv((uint32_t)a->H), FastDiv((uint32_t)a->S));
   unsigned grid = 0;
   if ((rc = set_items(p, a, AT_T, &grid))) return rc;
-  attn_bwd_dkv_kernel<HD><<<grid, BW_THREADS, DkvCfg<HD>::SMEM, s>>>(tq, tk, tv, tdo, p);
-  attn_bwd_dq_kernel<HD><<<grid, BW_THREADS, DqCfg<HD>::SMEM, s>>>(tq, tk, tv, tdo, p);
+  launch_pdl(attn_bwd_dkv_kernel<HD>, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);
+  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
 }
 

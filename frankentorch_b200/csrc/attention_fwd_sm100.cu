@@ -106,6 +106,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   WaitCtx ctx{p.status, abort_f};
 
   if ((smem_u32(smem) & 1023u) != 0u) {
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -136,6 +137,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
   TileWalk walk(p.n_tiles);
 
   if (warp >= 8) {
@@ -470,7 +473,7 @@ static int attn_fwd2_launch(const FtkAttnDesc* a, cudaStream_t s) {
   }
   unsigned grid = 0;
   if ((rc = set_items(p, a, 2 * AT_T, &grid))) return rc;
-  attn_fwd2_kernel<HD><<<grid, F2_THREADS, Fwd2Cfg<HD>::SMEM, s>>>(tq, tk, tv, p);
+  launch_pdl(attn_fwd2_kernel<HD>, grid, F2_THREADS, Fwd2Cfg<HD>::SMEM, s, tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 

@@ -8,6 +8,7 @@
 // im2col gather (fused.rs:262).  The runtime status word lives here too.
 #include <cuda_fp16.h>
 #include "ft_sm100.cuh"
+#include "launch.cuh"
 #include "ftk_api.h"
 
 namespace ftk {
@@ -62,6 +63,8 @@ template <int OP>
 __global__ void __launch_bounds__(256)
 ew_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                __nv_bfloat16* __restrict__ out, long long n, int tanh_form) {
+  pdl_wait();
+  pdl_trigger();
   const long long nvec = n >> 3;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += stride) {
@@ -90,6 +93,8 @@ ew_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restr
 
 __global__ void __launch_bounds__(256)
 cast_f32_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+  pdl_wait();
+  pdl_trigger();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
     y[i] = __float2bfloat16(x[i]);
@@ -97,6 +102,8 @@ cast_f32_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y,
 __global__ void __launch_bounds__(256)
 cast_bf16_f32_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ y, long long n,
                      int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     float v = __bfloat162float(x[i]);
@@ -127,6 +134,8 @@ __device__ __forceinline__ void philox4x32(uint64_t seed, uint64_t ctr, uint32_t
 __global__ void __launch_bounds__(256)
 dropout_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n,
                float p, unsigned long long seed, unsigned long long offset) {
+  pdl_wait();
+  pdl_trigger();
   const float inv = 1.f / (1.f - p);
   const long long nq = (n + 3) >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -149,6 +158,8 @@ __global__ void __launch_bounds__(128)
 embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ wte,
                      const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out, int S,
                      int d, long long vocab, int* status) {
+  pdl_wait();
+  pdl_trigger();
   const int r = blockIdx.x;
   long long id = ids[r];
   // a token id outside the table: reported through the status word, row 0 is read instead
@@ -175,6 +186,8 @@ __global__ void __launch_bounds__(128)
 embedding_bwd_wte_kernel(const long long* __restrict__ sorted_ids, const int* __restrict__ order,
                          int rows, const __nv_bfloat16* __restrict__ dout,
                          float* __restrict__ dwte, int d, long long vocab, int* status) {
+  pdl_wait();
+  pdl_trigger();
   const int b = blockIdx.x;
   const long long id = sorted_ids[b];
   if (b > 0 && sorted_ids[b - 1] == id) return;
@@ -202,6 +215,8 @@ embedding_bwd_wte_kernel(const long long* __restrict__ sorted_ids, const int* __
 __global__ void __launch_bounds__(128)
 embedding_bwd_wte_scan_kernel(const long long* __restrict__ ids, int rows, const __nv_bfloat16* __restrict__ dout,
                               float* __restrict__ dwte, int d, long long vocab, int* status) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int BLK = 1024;                               // positions looked at per vote: 8 loads in flight per thread
   __shared__ unsigned char match[BLK];
   __shared__ unsigned short list[BLK];
@@ -304,6 +319,8 @@ embedding_bwd_wte_scan_kernel(const long long* __restrict__ ids, int rows, const
 __global__ void __launch_bounds__(128)
 embedding_bwd_wpe_kernel(const __nv_bfloat16* __restrict__ dout, float* __restrict__ dwpe, int rows,
                          int S, int d) {
+  pdl_wait();
+  pdl_trigger();
   const int s = blockIdx.x;
   for (int c = threadIdx.x * 2; c < d; c += blockDim.x * 2) {
     float s0 = 0.f, s1 = 0.f;
@@ -323,6 +340,8 @@ adamw_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ shadow,
              const float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
              long long n, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2,
              float gscale) {
+  pdl_wait();
+  pdl_trigger();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const float g = grad[i] * gscale;
@@ -342,6 +361,8 @@ adamw_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ shadow,
 // hyper = {lr, bias_correction1, bias_correction2, grad_scale}; step is incremented here.
 __global__ void adamw_tick_kernel(long long* __restrict__ step, float* __restrict__ hyper, double b1,
                                   double b2) {
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const long long s = *step + 1;
     *step = s;
@@ -352,6 +373,8 @@ __global__ void adamw_tick_kernel(long long* __restrict__ step, float* __restric
 // hyper[3] = min(1, max_norm / (sqrt(sumsq) + 1e-6))  (clip_grad_norm_, ft-nn/src/lib.rs:740)
 __global__ void clip_scale_kernel(const float* __restrict__ sumsq, float max_norm,
                                   float* __restrict__ hyper, float* __restrict__ norm_out) {
+  pdl_wait();
+  pdl_trigger();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const float nrm = sqrtf(*sumsq);
     if (norm_out) *norm_out = nrm;
@@ -364,6 +387,8 @@ adamw_dev_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ shadow,
                  const float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
                  long long n, const float* __restrict__ hyper, float b1, float b2, float eps,
                  float wd) {
+  pdl_wait();
+  pdl_trigger();
   const float lr = hyper[0], bc1 = hyper[1], bc2 = hyper[2], gscale = hyper[3];
   const long long n4 = n >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -407,6 +432,8 @@ adamw_dev_kernel(float* __restrict__ master, __nv_bfloat16* __restrict__ shadow,
   }
 }
 __global__ void __launch_bounds__(256) fill_f32_kernel(float* __restrict__ x, long long n, float v) {
+  pdl_wait();
+  pdl_trigger();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = v;
 }
@@ -431,6 +458,8 @@ __global__ void present_rgba8_kernel(const unsigned char* __restrict__ src, void
 }
 __global__ void im2col_1d_kernel(const float* __restrict__ x, float* __restrict__ y, int t_in,
                                  int cin, int k, int stride, int pad, int t_out) {
+  pdl_wait();
+  pdl_trigger();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;  // index into cin*k
   const int t = blockIdx.y * blockDim.y + threadIdx.y;
   if (col >= cin * k || t >= t_out) return;
@@ -455,41 +484,41 @@ static inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) 
 
 extern "C" int ftk_gelu_fwd(const void* x, void* y, long long n, int tanh_form, void* stream) {
   if (n <= 0 || !al16(x) || !al16(y)) return -2;
-  ew_bf16_kernel<0><<<ew_grid(n >> 3, 256), 256, 0, STREAM(stream)>>>(BF(x), nullptr, BFW(y), n, tanh_form);
+  launch_pdl(ew_bf16_kernel<0>, ew_grid(n >> 3, 256), 256, 0, STREAM(stream), BF(x), nullptr, BFW(y), n, tanh_form);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_gelu_bwd(const void* x, const void* dy, void* dx, long long n, int tanh_form,
                             void* stream) {
   if (n <= 0 || !al16(x) || !al16(dy) || !al16(dx)) return -2;
-  ew_bf16_kernel<1><<<ew_grid(n >> 3, 256), 256, 0, STREAM(stream)>>>(BF(x), BF(dy), BFW(dx), n, tanh_form);
+  launch_pdl(ew_bf16_kernel<1>, ew_grid(n >> 3, 256), 256, 0, STREAM(stream), BF(x), BF(dy), BFW(dx), n, tanh_form);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_add_bf16(const void* a, const void* b, void* out, long long n, void* stream) {
   if (n <= 0 || !al16(a) || !al16(b) || !al16(out)) return -2;
-  ew_bf16_kernel<2><<<ew_grid(n >> 3, 256), 256, 0, STREAM(stream)>>>(BF(a), BF(b), BFW(out), n, 0);
+  launch_pdl(ew_bf16_kernel<2>, ew_grid(n >> 3, 256), 256, 0, STREAM(stream), BF(a), BF(b), BFW(out), n, 0);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_cast_f32_to_bf16(const float* x, void* y, long long n, void* stream) {
   if (n <= 0) return -2;
-  cast_f32_bf16_kernel<<<ew_grid(n, 256), 256, 0, STREAM(stream)>>>(x, BFW(y), n);
+  launch_pdl(cast_f32_bf16_kernel, ew_grid(n, 256), 256, 0, STREAM(stream), x, BFW(y), n);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_cast_bf16_to_f32(const void* x, float* y, long long n, int accumulate,
                                     void* stream) {
   if (n <= 0) return -2;
-  cast_bf16_f32_kernel<<<ew_grid(n, 256), 256, 0, STREAM(stream)>>>(BF(x), y, n, accumulate);
+  launch_pdl(cast_bf16_f32_kernel, ew_grid(n, 256), 256, 0, STREAM(stream), BF(x), y, n, accumulate);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_dropout_bf16(const void* x, void* y, long long n, float p,
                                 unsigned long long seed, unsigned long long offset, void* stream) {
   if (n <= 0 || !(p >= 0.f && p < 1.f)) return -2;
-  dropout_kernel<<<ew_grid((n + 3) >> 2, 256), 256, 0, STREAM(stream)>>>(BF(x), BFW(y), n, p, seed, offset);
+  launch_pdl(dropout_kernel, ew_grid((n + 3) >> 2, 256), 256, 0, STREAM(stream), BF(x), BFW(y), n, p, seed, offset);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_embedding_fwd(const long long* ids, const void* wte, const void* wpe, void* out,
                                  int rows, int S, int d, long long vocab, void* stream) {
   if (rows <= 0 || d % 8 || S <= 0 || vocab <= 0) return -2;
-  embedding_fwd_kernel<<<rows, 128, 0, STREAM(stream)>>>(ids, BF(wte), BF(wpe), BFW(out), S, d, vocab,
+  launch_pdl(embedding_fwd_kernel, rows, 128, 0, STREAM(stream), ids, BF(wte), BF(wpe), BFW(out), S, d, vocab,
                                                          ftk_status_word());
   return (int)cudaGetLastError();
 }
@@ -497,9 +526,9 @@ extern "C" int ftk_embedding_bwd(const long long* sorted_ids, const int* order, 
                                  float* dwte, float* dwpe, int rows, int S, int d, long long vocab, void* stream) {
   if (rows <= 0 || d % 2 || (dwte && vocab <= 0)) return -2;
   if (dwte)
-    embedding_bwd_wte_kernel<<<rows, 128, 0, STREAM(stream)>>>(sorted_ids, order, rows, BF(dout), dwte, d, vocab,
+    launch_pdl(embedding_bwd_wte_kernel, rows, 128, 0, STREAM(stream), sorted_ids, order, rows, BF(dout), dwte, d, vocab,
                                                                ftk_status_word());
-  if (dwpe) embedding_bwd_wpe_kernel<<<S, 128, 0, STREAM(stream)>>>(BF(dout), dwpe, rows, S, d);
+  if (dwpe) launch_pdl(embedding_bwd_wpe_kernel, S, 128, 0, STREAM(stream), BF(dout), dwpe, rows, S, d);
   return (int)cudaGetLastError();
 }
 // Sort-free form: `ids` in their original order (int64 [rows]); d <= 1024 (wider tables use the sorted form).
@@ -507,16 +536,16 @@ extern "C" int ftk_embedding_bwd_scan(const long long* ids, const void* dout, fl
                                       int S, int d, long long vocab, void* stream) {
   if (rows <= 0 || d % 2 || d > 1024 || (dwte && vocab <= 0)) return -2;
   if (dwte)
-    embedding_bwd_wte_scan_kernel<<<rows, 128, 0, STREAM(stream)>>>(ids, rows, BF(dout), dwte, d, vocab,
+    launch_pdl(embedding_bwd_wte_scan_kernel, rows, 128, 0, STREAM(stream), ids, rows, BF(dout), dwte, d, vocab,
                                                                     ftk_status_word());
-  if (dwpe) embedding_bwd_wpe_kernel<<<S, 128, 0, STREAM(stream)>>>(BF(dout), dwpe, rows, S, d);
+  if (dwpe) launch_pdl(embedding_bwd_wpe_kernel, S, 128, 0, STREAM(stream), BF(dout), dwpe, rows, S, d);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_adamw(float* master, void* shadow, const float* grad, float* m, float* v,
                          long long n, float lr, float b1, float b2, float eps, float wd, float bc1,
                          float bc2, float gscale, void* stream) {
   if (n <= 0) return -2;
-  adamw_kernel<<<ew_grid(n, 256), 256, 0, STREAM(stream)>>>(master, BFW(shadow), grad, m, v, n, lr,
+  launch_pdl(adamw_kernel, ew_grid(n, 256), 256, 0, STREAM(stream), master, BFW(shadow), grad, m, v, n, lr,
                                                              b1, b2, eps, wd, bc1, bc2, gscale);
   return (int)cudaGetLastError();
 }
@@ -534,17 +563,17 @@ extern "C" int ftk_im2col_1d(const float* x, float* y, int t_in, int cin, int k,
                              int pad, int t_out, void* stream) {
   if (t_in <= 0 || cin <= 0 || k <= 0 || t_out <= 0 || stride <= 0) return -2;
   dim3 b(32, 8), g((cin * k + 31) / 32, (t_out + 7) / 8);
-  im2col_1d_kernel<<<g, b, 0, STREAM(stream)>>>(x, y, t_in, cin, k, stride, pad, t_out);
+  launch_pdl(im2col_1d_kernel, g, b, 0, STREAM(stream), x, y, t_in, cin, k, stride, pad, t_out);
   return (int)cudaGetLastError();
 }
 
 extern "C" int ftk_adamw_tick(long long* step, float* hyper, double b1, double b2, void* stream) {
-  adamw_tick_kernel<<<1, 32, 0, STREAM(stream)>>>(step, hyper, b1, b2);
+  launch_pdl(adamw_tick_kernel, 1, 32, 0, STREAM(stream), step, hyper, b1, b2);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_clip_scale(const float* sumsq, float max_norm, float* hyper, float* norm_out,
                               void* stream) {
-  clip_scale_kernel<<<1, 32, 0, STREAM(stream)>>>(sumsq, max_norm, hyper, norm_out);
+  launch_pdl(clip_scale_kernel, 1, 32, 0, STREAM(stream), sumsq, max_norm, hyper, norm_out);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_adamw_dev(float* master, void* shadow, const float* grad, float* m, float* v,
@@ -553,7 +582,7 @@ extern "C" int ftk_adamw_dev(float* master, void* shadow, const float* grad, flo
   if (n <= 0) return -2;
   if (!al16(master) || !al16(grad) || !al16(m) || !al16(v) || (shadow && (reinterpret_cast<uintptr_t>(shadow) & 7)))
     return -3;
-  adamw_dev_kernel<<<ew_grid(n >> 2, 256), 256, 0, STREAM(stream)>>>(master, BFW(shadow), grad, m, v, n,
+  launch_pdl(adamw_dev_kernel, ew_grid(n >> 2, 256), 256, 0, STREAM(stream), master, BFW(shadow), grad, m, v, n,
                                                                       hyper, b1, b2, eps, wd);
   return (int)cudaGetLastError();
 }
@@ -571,7 +600,7 @@ extern "C" int ftk_timestamp(unsigned long long* out, void* stream) {
 }
 extern "C" int ftk_fill_f32(float* x, long long n, float v, void* stream) {
   if (n <= 0) return -2;
-  fill_f32_kernel<<<ew_grid(n, 256), 256, 0, STREAM(stream)>>>(x, n, v);
+  launch_pdl(fill_f32_kernel, ew_grid(n, 256), 256, 0, STREAM(stream), x, n, v);
   return (int)cudaGetLastError();
 }
 

@@ -164,6 +164,7 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
   extern __shared__ __align__(1024) uint8_t smem[];
   // (the dynamic shared-memory base has the same offset in both CTAs, so both take the same branch)
   if ((smem_u32(smem) & 1023u) != 0u) {
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -175,6 +176,8 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     tma_prefetch_desc(&tmB);
   }
   cta.setup();
+  pdl_wait();
+  if (warp != 0) pdl_trigger();      // (these warps have seen the tensor-memory allocation)
 
   const int pair = (int)blockIdx.x >> 1;
   const int n_pairs = (int)gridDim.x >> 1;

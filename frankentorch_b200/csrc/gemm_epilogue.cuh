@@ -18,6 +18,7 @@
 #pragma once
 #include "ft_sm100.cuh"
 #include "ftk_api.h"
+#include "launch.cuh"
 
 namespace ftk {
 

@@ -61,6 +61,7 @@ gemm_group_bf16_sm100_kernel(const __grid_constant__ GroupMaps maps, const Group
   using Cfg = PairCfg<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(g.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -68,6 +69,8 @@ gemm_group_bf16_sm100_kernel(const __grid_constant__ GroupMaps maps, const Group
   const int warp = cta.warp, lane = cta.lane, rank = cta.rank;
   WaitCtx ctx{g.status, cta.abort_f};
   cta.setup();
+  pdl_wait();
+  if (warp != 0) pdl_trigger();      // (these warps have seen the tensor-memory allocation)
 
   const int pair = (int)blockIdx.x >> 1;
   const int n_pairs = (int)gridDim.x >> 1;

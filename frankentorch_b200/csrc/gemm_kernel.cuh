@@ -563,6 +563,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
   const int lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
   if ((smem_u32(smem) & 1023u) != 0u) {      // swizzled tiles need 1024-byte aligned bases
+    pdl_wait();
     if (threadIdx.x == 0) atomicCAS(p.status, 0, FT_ERR_BAD_ARG);
     return;
   }
@@ -622,6 +623,10 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     setup_barrier(G_THREADS - 32);
     tc_fence_after();
     tmem_base = *tmem_slot;
+  }
+  if (!COMM) {
+    pdl_wait();
+    if (warp != 0) pdl_trigger();      // (these warps have seen the tensor-memory allocation)
   }
 
   const int tiles_m = (int)p.by_tiles_m.d;

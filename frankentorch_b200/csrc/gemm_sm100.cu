@@ -30,6 +30,8 @@ namespace ftk {
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ D, long long M, long long N,
                      long long ldd, int splits, int out_fp32, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   const long long total4 = (M * N) >> 2;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += stride) {
@@ -189,7 +191,7 @@ static int launch_gemm_kind(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm
   if (grid <= 0) return 0;
   CommArgs none;
   memset(&none, 0, sizeof(none));
-  gemm_bf16_sm100_kernel<BN, 0, KIND><<<grid, G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, tmA, a, none);
+  launch_pdl(gemm_bf16_sm100_kernel<BN, 0, KIND>, grid, G_THREADS, Cfg::SMEM, stream, tmA, tmB, tmA, a, none);
   return (int)cudaGetLastError();
 }
 
@@ -222,7 +224,7 @@ static int launch_gemm_pair_kind(const CUtensorMap& tmA, const CUtensorMap& tmB,
   long long pairs = max_ctas / 2;
   if (items < pairs) pairs = items;
   if (pairs <= 0) return 0;
-  gemm2_bf16_sm100_kernel<BN, KIND><<<(unsigned)(2 * pairs), G_THREADS, Cfg::SMEM, stream>>>(tmA, tmB, a);
+  launch_pdl(gemm2_bf16_sm100_kernel<BN, KIND>, (unsigned)(2 * pairs), G_THREADS, Cfg::SMEM, stream, tmA, tmB, a);
   return (int)cudaGetLastError();
 }
 
@@ -401,7 +403,7 @@ static int launch_group(const GroupMaps& maps, const GroupArgs& ga, int pairs, c
     if (e != cudaSuccess) return (int)e;
     *attr_set_p = true;
   }
-  gemm_group_bf16_sm100_kernel<KIND><<<2 * pairs, G_THREADS, SMEM, stream>>>(maps, ga);
+  launch_pdl(gemm_group_bf16_sm100_kernel<KIND>, 2 * pairs, G_THREADS, SMEM, stream, maps, ga);
   return (int)cudaGetLastError();
 }
 
@@ -496,7 +498,7 @@ extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
     if (e == cudaSuccess) e = cudaStreamWaitEvent(rs, ev[dev], 0);
     if (e != cudaSuccess) return (int)e;
   }
-  splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, rs>>>(a.ws, g->D, g->M, g->N, g->ldd, splits,
+  launch_pdl(splitk_reduce_kernel, (unsigned)blocks, 256, 0, rs, a.ws, g->D, g->M, g->N, g->ldd, splits,
                                                          g->out_fp32, g->accumulate);
   return (int)cudaGetLastError();
 }

@@ -9,6 +9,7 @@
 // Parameter-gradient reductions run in a fixed order (row blocks, then a serial
 // pass over the block partials), so two runs give identical bits.
 #include "ft_sm100.cuh"
+#include "launch.cuh"
 #include "ftk_api.h"
 
 namespace ftk {
@@ -66,6 +67,8 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                 float eps) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = WPR == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
@@ -177,6 +180,8 @@ norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
                      const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                      float eps) {
+  pdl_wait();
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * ROW_WARPS + warp;
   if (row >= rows) return;
@@ -248,6 +253,8 @@ norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                    const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dx_add,
                    __nv_bfloat16* __restrict__ dx, int rows, int cols) {
+  pdl_wait();
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * ROW_WARPS + warp;
   if (row >= rows) return;
@@ -333,6 +340,8 @@ norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16*
     abort_w = 0;
     fence_mbar_init();
   }
+  pdl_wait();
+  pdl_trigger();
   uint4 gam[NV];
 #pragma unroll
   for (int j = 0; j < NV; ++j)
@@ -490,6 +499,8 @@ __global__ void __launch_bounds__(1024)
 col_final_wide_kernel(const float* __restrict__ partial, float* __restrict__ out,
                       const float* __restrict__ partial2, float* __restrict__ out2, int cols, int nblk,
                       int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sm[2][32][33];
   const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cl;
@@ -534,6 +545,8 @@ __global__ void __launch_bounds__(256)
 col_partial_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                    float* __restrict__ partial, int rows, int cols, long long ld, int nblk) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sm[4][COL_GROUPS][32];
   const int cp = threadIdx.x & 31, rg = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + cp) * 2;
@@ -616,6 +629,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 softmax_rows_kernel(const T* __restrict__ x, T* __restrict__ y, int cols, int S_causal,
                     float scale) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   const int limit = S_causal > 0 ? (int)(row % S_causal) + 1 : cols;
@@ -639,6 +654,8 @@ softmax_rows_kernel(const T* __restrict__ x, T* __restrict__ y, int cols, int S_
 __global__ void __launch_bounds__(256)
 softmax_bwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ dy,
                    __nv_bfloat16* __restrict__ dx, int cols, float scale) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[33];
   const size_t row = blockIdx.x;
   const __nv_bfloat16* yr = y + row * cols;
@@ -676,6 +693,8 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
 cross_entropy_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
                      float* __restrict__ losses, __nv_bfloat16* __restrict__ dlogits, int vocab,
                      int ld, float grad_scale, int use_smem) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ uint4 ce_smem[];
   __shared__ float red[33];
   const size_t row = blockIdx.x;
@@ -806,6 +825,8 @@ template <bool SQUARE>
 __global__ void __launch_bounds__(1024)
 reduce_one_block_kernel(const float* __restrict__ x, float* __restrict__ out, long long n,
                         float scale, int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[33];
   float s = 0.f;
   for (long long i = threadIdx.x; i < n; i += 1024) {
@@ -819,6 +840,8 @@ reduce_one_block_kernel(const float* __restrict__ x, float* __restrict__ out, lo
 template <bool SQUARE>
 __global__ void __launch_bounds__(256)
 reduce_level1_kernel(const float* __restrict__ x, float* __restrict__ partial, long long n) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float red[33];
   const long long per = (n + gridDim.x - 1) / gridDim.x;
   const long long b = per * blockIdx.x, e = (b + per < n) ? b + per : n;
@@ -842,7 +865,7 @@ template <bool RMS>
 static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, const void* gamma, const void* beta, void* y,
                            float* mean, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
 #define FT_NORM_FWD(NV, WPR)                                                                                   \
-  norm_fwd_kernel<NV, WPR, RMS><<<WPR == 1 ? (rows + 3) / 4 : rows, WPR == 1 ? 128 : 256, 0, s>>>(             \
+  launch_pdl(norm_fwd_kernel<NV, WPR, RMS>, WPR == 1 ? (rows + 3) / 4 : rows, WPR == 1 ? 128 : 256, 0, s,             \
       BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps)
   const int nvec = cols / 8, per_lane = (nvec + 31) / 32;
   // Up to 1536 columns a row is one warp's.  Wider rows take a CTA each, except where there are enough rows of up to 2048
@@ -857,7 +880,7 @@ static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, cons
   else if (nvec <= 512) FT_NORM_FWD(2, 8);
   else if (nvec <= 1024) FT_NORM_FWD(4, 8);
   else
-    norm_fwd_long_kernel<RMS><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
+    launch_pdl(norm_fwd_long_kernel<RMS>, (rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s,
         BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps);
 #undef FT_NORM_FWD
   return (int)cudaGetLastError();
@@ -903,7 +926,7 @@ static int norm_bwd_fused_launch(const void* dy, const void* x, const void* gamm
     if (e != cudaSuccess) return (int)e;
     done[dev] = true;
   }
-  norm_bwd_fused_kernel<NV, WPR, RMS><<<nblk, ROW_WARPS * 32, smem, s>>>(
+  launch_pdl(norm_bwd_fused_kernel<NV, WPR, RMS>, nblk, ROW_WARPS * 32, smem, s,
       BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add), BFW(dx), partial, rows, cols, (rows + nblk - 1) / nblk, stages, status);
   return (int)cudaGetLastError();
 }
@@ -940,14 +963,14 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
 #undef FT_NORM_BWD
     if (rc) return rc;
   } else {
-    norm_bwd_dx_kernel<RMS><<<(rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s>>>(
+    launch_pdl(norm_bwd_dx_kernel<RMS>, (rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s,
         BF(dy), BF(x), BF(gamma), mean, rstd, BF(dx_add), BFW(dx), rows, cols);
     if (!dgamma) return (int)cudaGetLastError();
     nblk = norm_col_blocks(rows);
     dim3 g((cols / 2 + 31) / 32, nblk);
-    col_partial_kernel<RMS ? 1 : 0><<<g, 256, 0, s>>>(BF(dy), BF(x), mean, rstd, partial, rows, cols, cols, nblk);
+    launch_pdl(col_partial_kernel<RMS ? 1 : 0>, g, 256, 0, s, BF(dy), BF(x), mean, rstd, partial, rows, cols, cols, nblk);
   }
-  col_final_wide_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, dgamma, RMS ? nullptr : partial + (size_t)nblk * cols,
+  launch_pdl(col_final_wide_kernel, (cols + 31) / 32, 1024, 0, s, partial, dgamma, RMS ? nullptr : partial + (size_t)nblk * cols,
                                                           dbeta, cols, nblk, accumulate);
   return (int)cudaGetLastError();
 }
@@ -973,6 +996,8 @@ constexpr int CSW_ROWS = 64;
 __global__ void __launch_bounds__(256)
 colsum_wide_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ partial, int rows, int cols,
                    long long ld) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sm[COL_GROUPS][32][9];
   const int lane = threadIdx.x & 31, rg = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * 8;
@@ -1034,14 +1059,14 @@ extern "C" int ftk_colsum_bf16(const void* x, float* out, float* partial, int ro
   if (wide) {
     nblk = ftk_colsum_blocks(rows);
     dim3 g((cols / 8 + 31) / 32, nblk);
-    colsum_wide_kernel<<<g, 256, 0, s>>>(BF(x), partial, rows, cols, ld);
+    launch_pdl(colsum_wide_kernel, g, 256, 0, s, BF(x), partial, rows, cols, ld);
   } else {
     // odd extents / alignments: two columns per thread; needs fewer row blocks than were provided for
     nblk = (rows + COL_ROWS_PER_BLK - 1) / COL_ROWS_PER_BLK;
     dim3 g((cols / 2 + 31) / 32, nblk);
-    col_partial_kernel<2><<<g, 256, 0, s>>>(BF(x), nullptr, nullptr, nullptr, partial, rows, cols, ld, nblk);
+    launch_pdl(col_partial_kernel<2>, g, 256, 0, s, BF(x), nullptr, nullptr, nullptr, partial, rows, cols, ld, nblk);
   }
-  col_final_wide_kernel<<<(cols + 31) / 32, 1024, 0, s>>>(partial, out, nullptr, nullptr, cols, nblk, accumulate);
+  launch_pdl(col_final_wide_kernel, (cols + 31) / 32, 1024, 0, s, partial, out, nullptr, nullptr, cols, nblk, accumulate);
   return (int)cudaGetLastError();
 }
 
@@ -1049,23 +1074,23 @@ extern "C" int ftk_softmax_rows(const void* x, void* y, int rows, int cols, int 
                                 void* stream) {
   if (rows <= 0 || cols <= 0) return -2;
   if (is_bf16)
-    softmax_rows_kernel<__nv_bfloat16><<<rows, 256, 0, STREAM(stream)>>>(BF(x), BFW(y), cols, 0, 1.f);
+    launch_pdl(softmax_rows_kernel<__nv_bfloat16>, rows, 256, 0, STREAM(stream), BF(x), BFW(y), cols, 0, 1.f);
   else
-    softmax_rows_kernel<float><<<rows, 256, 0, STREAM(stream)>>>(
+    launch_pdl(softmax_rows_kernel<float>, rows, 256, 0, STREAM(stream),
         reinterpret_cast<const float*>(x), reinterpret_cast<float*>(y), cols, 0, 1.f);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_softmax_causal_bf16(const void* x, void* y, int L, int S, float scale,
                                        void* stream) {
   if (L <= 0 || S <= 0) return -2;
-  softmax_rows_kernel<__nv_bfloat16><<<(unsigned)((size_t)L * S), 256, 0, STREAM(stream)>>>(
+  launch_pdl(softmax_rows_kernel<__nv_bfloat16>, (unsigned)((size_t)L * S), 256, 0, STREAM(stream),
       BF(x), BFW(y), S, S, scale);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_softmax_bwd_bf16(const void* y, const void* dy, void* dx, long long rows,
                                     int cols, float scale, void* stream) {
   if (rows <= 0 || cols <= 0) return -2;
-  softmax_bwd_kernel<<<(unsigned)rows, 256, 0, STREAM(stream)>>>(BF(y), BF(dy), BFW(dx), cols, scale);
+  launch_pdl(softmax_bwd_kernel, (unsigned)rows, 256, 0, STREAM(stream), BF(y), BF(dy), BFW(dx), cols, scale);
   return (int)cudaGetLastError();
 }
 
@@ -1082,7 +1107,7 @@ extern "C" int ftk_cross_entropy_fwd_bwd(const void* logits, const long long* ta
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  cross_entropy_kernel<<<rows, CE_THREADS, use_smem ? bytes : 0, STREAM(stream)>>>(
+  launch_pdl(cross_entropy_kernel, rows, CE_THREADS, use_smem ? bytes : 0, STREAM(stream),
       BF(logits), targets, losses, BFW(dlogits), vocab, ld, grad_scale, use_smem);
   return (int)cudaGetLastError();
 }
@@ -1090,18 +1115,18 @@ extern "C" int ftk_cross_entropy_fwd_bwd(const void* logits, const long long* ta
 extern "C" int ftk_reduce_mean_f32(const float* x, float* out, long long n, float scale,
                                    void* stream) {
   if (n <= 0) return -2;
-  reduce_one_block_kernel<false><<<1, 1024, 0, STREAM(stream)>>>(x, out, n, scale, 0);
+  launch_pdl(reduce_one_block_kernel<false>, 1, 1024, 0, STREAM(stream), x, out, n, scale, 0);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_sumsq_f32(const float* x, float* out, float* partial, long long n,
                              int accumulate, void* stream) {
   if (n <= 0) return -2;
   if (n < (1 << 16) || !partial) {
-    reduce_one_block_kernel<true><<<1, 1024, 0, STREAM(stream)>>>(x, out, n, 1.f, accumulate);
+    launch_pdl(reduce_one_block_kernel<true>, 1, 1024, 0, STREAM(stream), x, out, n, 1.f, accumulate);
   } else {
     // level 1: FTK_SUMSQ_PARTIALS fixed slices; level 2: one block over the partials
-    reduce_level1_kernel<true><<<FTK_SUMSQ_PARTIALS, 256, 0, STREAM(stream)>>>(x, partial, n);
-    reduce_one_block_kernel<false><<<1, 1024, 0, STREAM(stream)>>>(partial, out, FTK_SUMSQ_PARTIALS,
+    launch_pdl(reduce_level1_kernel<true>, FTK_SUMSQ_PARTIALS, 256, 0, STREAM(stream), x, partial, n);
+    launch_pdl(reduce_one_block_kernel<false>, 1, 1024, 0, STREAM(stream), partial, out, FTK_SUMSQ_PARTIALS,
                                                                     1.f, accumulate);
   }
   return (int)cudaGetLastError();
