@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from pathlib import Path
 
 _LIB = None
@@ -51,6 +52,12 @@ class FtkAttnDesc(C.Structure):
         ("dq", C.c_void_p), ("dk", C.c_void_p), ("dv", C.c_void_p),
     ]
 
+
+# The same two layouts for struct.pack: filling a ctypes structure field by field costs more than the launch of a small
+# kernel (the fields in declaration order, zero for a null pointer).
+GEMM_DESC = struct.Struct("@7iP3qP3qP3qPP3qPf5iPqiPPi0q")
+ATTN_DESC = struct.Struct("@5if3P9qP3q3P3P")
+assert GEMM_DESC.size == C.sizeof(FtkGemmDesc) and ATTN_DESC.size == C.sizeof(FtkAttnDesc)
 
 FTK_MAX_RANKS = 8
 COMM_GATHER_A, COMM_GATHER_B, COMM_SCATTER_D = 1, 2, 3
@@ -154,6 +161,12 @@ def load(build_if_missing: bool = True):
         "ftk_im2col_1d": [vp, vp, i, i, i, i, i, i, vp],
         "ftk_wait_probe": [vp, i, ll, vp, vp],
     }
+    # descriptors packed by GEMM_DESC / ATTN_DESC (a second function object per entry: argument types are per object)
+    for name, sym in (("gemm_packed", "ftk_gemm_bf16"), ("attn_fwd_packed", "ftk_attn_fwd"),
+                      ("attn_bwd_packed", "ftk_attn_bwd")):
+        fn = lib[sym]
+        fn.argtypes, fn.restype = [C.c_char_p, C.c_void_p], C.c_int
+        setattr(lib, name, fn)
     for name, args in sigs.items():
         fn = getattr(lib, name)
         fn.argtypes = args

@@ -180,6 +180,15 @@ def _bgrad_into(targets, idx, dy2d, side: Optional["SideWork"] = None):
     return run(dy2d)
 
 
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as ``[rows, last extent]``."""
+    return t if t.dim() == 2 else t.reshape(-1, t.shape[-1])
+
+
+def _as(t: torch.Tensor, ref: torch.Tensor) -> torch.Tensor:
+    return t if t.shape == ref.shape else t.reshape(ref.shape)
+
+
 def linear(tape: TensorTape, x: int, w: int, b: Optional[int] = None, *, act: Optional[str] = None,
            resid: Optional[int] = None) -> int:
     """``y = act(x @ w^T + b) (+ resid)``; ``w`` is ``[out, in]`` (ft-nn/src/lib.rs:902).
@@ -190,20 +199,21 @@ def linear(tape: TensorTape, x: int, w: int, b: Optional[int] = None, *, act: Op
     xv, wv = tape.value(x), tape.value(w)
     bv = tape.value(b) if b is not None else None
     rv = tape.value(resid) if resid is not None else None
-    x2 = xv.reshape(-1, xv.shape[-1])
+    x2 = _rows(xv)
     epi = {None: K.EPI_NONE, "gelu_tanh": K.EPI_GELU_TANH, "gelu_erf": K.EPI_GELU_ERF, "relu": K.EPI_RELU}[act]
     depi = {None: K.EPI_NONE, "gelu_tanh": K.EPI_MUL_DGELU_TANH, "gelu_erf": K.EPI_MUL_DGELU_ERF,
             "relu": K.EPI_MUL_DRELU}[act]
     aux = torch.empty((x2.shape[0], wv.shape[0]), dtype=torch.bfloat16, device=xv.device) if act else None
-    r2 = rv.reshape(-1, rv.shape[-1]) if rv is not None else None
+    r2 = _rows(rv) if rv is not None else None
     y = K.linear_fwd(x2, wv, bv, epi=epi, resid=r2, aux=aux)
-    y = y.reshape(*xv.shape[:-1], wv.shape[0])
+    if xv.dim() != 2:
+        y = y.reshape(*xv.shape[:-1], wv.shape[0])
     inputs = [x, w] + ([b] if b is not None else []) + ([resid] if resid is not None else [])
     has_b, has_r = b is not None, resid is not None
     x_needs = tape.nodes[x].requires_grad
 
     def vjp(gy, targets):
-        g2 = gy.reshape(-1, gy.shape[-1])
+        g2 = _rows(gy)
         if act:
             # dU = dY * act'(U): elementwise on the saved pre-activation
             g2 = K.gelu_bwd(aux, g2, tanh_form=(act == "gelu_tanh")) if act != "relu" else \
@@ -212,7 +222,7 @@ def linear(tape: TensorTape, x: int, w: int, b: Optional[int] = None, *, act: Op
         with SideWork(tape, g2.device) as side:
             db = _bgrad_into(targets, 2, g2, side) if has_b else None      # column sums next to the GEMMs
             dw = _wgrad_into(targets, 1, g2, x2, side)
-            dx = K.linear_dgrad(g2, wv).reshape(xv.shape) if x_needs else None
+            dx = _as(K.linear_dgrad(g2, wv), xv) if x_needs else None
         out.append(dx)
         out.append(dw)
         if has_b:
@@ -233,16 +243,16 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
     ``dU = (dY @ w2) * act'(U)`` is one kernel (no separate elementwise pass).
     """
     xv, w1v, b1v, w2v, b2v, rv = (tape.value(i) for i in (x, w1, b1, w2, b2, resid))
-    x2 = xv.reshape(-1, xv.shape[-1])
-    r2 = rv.reshape(-1, rv.shape[-1])
+    x2 = _rows(xv)
+    r2 = _rows(rv)
     epi = {"gelu_tanh": K.EPI_GELU_TANH, "gelu_erf": K.EPI_GELU_ERF, "relu": K.EPI_RELU}[act]
     depi = {"gelu_tanh": K.EPI_MUL_DGELU_TANH, "gelu_erf": K.EPI_MUL_DGELU_ERF, "relu": K.EPI_MUL_DRELU}[act]
     u = torch.empty((x2.shape[0], w1v.shape[0]), dtype=torch.bfloat16, device=xv.device)
     h = K.linear_fwd(x2, w1v, b1v, epi=epi, aux=u)
-    y = K.linear_fwd(h, w2v, b2v, resid=r2).reshape(rv.shape)
+    y = _as(K.linear_fwd(h, w2v, b2v, resid=r2), rv)
 
     def vjp(gy, targets):
-        g2 = gy.reshape(-1, gy.shape[-1])
+        g2 = _rows(gy)
         with SideWork(tape, g2.device) as side:
             db2 = _bgrad_into(targets, 4, g2, side)
             dw2 = _wgrad_into(targets, 3, g2, h, side)
@@ -254,7 +264,7 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
                 side.side.wait_event(ev)
             db1 = _bgrad_into(targets, 2, du, side)
             dw1 = _wgrad_into(targets, 1, du, x2, side)
-            dx = K.linear_dgrad(du, w1v).reshape(xv.shape)
+            dx = _as(K.linear_dgrad(du, w1v), xv)
         return [dx, dw1, db1, dw2, db2, gy]
 
     return tape.record("mlp", [x, w1, b1, w2, b2, resid], y, vjp,
@@ -264,43 +274,43 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
 def layernorm(tape: TensorTape, x: int, gamma: int, beta: int, eps: float = 1e-5) -> int:
     """LayerNorm over the last dim (ft-nn/src/lib.rs:2042; kernel math lib.rs:5824/6052)."""
     xv, gv, bv = tape.value(x), tape.value(gamma), tape.value(beta)
-    x2 = xv.reshape(-1, xv.shape[-1])
+    x2 = _rows(xv)
     y, mean, rstd, _ = K.layernorm_fwd(x2, gv, bv, eps)
 
     def vjp(gy, targets):
-        g2 = gy.reshape(-1, gy.shape[-1])
+        g2 = _rows(gy)
         # fuse the running gradient of x (the residual branch) into the dx kernel
         cur = targets.take_current(0)
         tg, tb = targets.leaf_target(1), targets.leaf_target(2)
         if tg is not None and tb is not None and tg[1] == tb[1]:
-            dx, _, _ = K.layernorm_bwd(g2, x2, gv, mean, rstd, dx_add=None if cur is None else cur.reshape(x2.shape),
+            dx, _, _ = K.layernorm_bwd(g2, x2, gv, mean, rstd, dx_add=None if cur is None else _as(cur, x2),
                                        dgamma=tg[0], dbeta=tb[0], accumulate=tg[1])
             targets.mark_accumulated(1)
             targets.mark_accumulated(2)
-            return [dx.reshape(xv.shape), ACCUMULATED, ACCUMULATED]
-        dx, dg, db = K.layernorm_bwd(g2, x2, gv, mean, rstd, dx_add=None if cur is None else cur.reshape(x2.shape))
-        return [dx.reshape(xv.shape), dg, db]
+            return [_as(dx, xv), ACCUMULATED, ACCUMULATED]
+        dx, dg, db = K.layernorm_bwd(g2, x2, gv, mean, rstd, dx_add=None if cur is None else _as(cur, x2))
+        return [_as(dx, xv), dg, db]
 
-    return tape.record("layer_norm", [x, gamma, beta], y.reshape(xv.shape), vjp, "d(layer_norm(x))/dx,dgamma,dbeta")
+    return tape.record("layer_norm", [x, gamma, beta], _as(y, xv), vjp, "d(layer_norm(x))/dx,dgamma,dbeta")
 
 
 def rmsnorm(tape: TensorTape, x: int, gamma: int, eps: float = 1e-6) -> int:
     """RMSNorm (ft-nn/src/lib.rs:6843; kernel math ft-kernel-cpu/src/lib.rs:6418/6503)."""
     xv, gv = tape.value(x), tape.value(gamma)
-    x2 = xv.reshape(-1, xv.shape[-1])
+    x2 = _rows(xv)
     y, rstd = K.rmsnorm_fwd(x2, gv, eps)
 
     def vjp(gy, targets):
-        g2 = gy.reshape(-1, gy.shape[-1])
+        g2 = _rows(gy)
         tg = targets.leaf_target(1)
         if tg is not None:
             dx, _ = K.rmsnorm_bwd(g2, x2, gv, rstd, dgamma=tg[0], accumulate=tg[1])
             targets.mark_accumulated(1)
-            return [dx.reshape(xv.shape), ACCUMULATED]
+            return [_as(dx, xv), ACCUMULATED]
         dx, dg = K.rmsnorm_bwd(g2, x2, gv, rstd)
-        return [dx.reshape(xv.shape), dg]
+        return [_as(dx, xv), dg]
 
-    return tape.record("rms_norm", [x, gamma], y.reshape(xv.shape), vjp, "d(rms_norm(x))/dx,dgamma")
+    return tape.record("rms_norm", [x, gamma], _as(y, xv), vjp, "d(rms_norm(x))/dx,dgamma")
 
 
 def attention_packed(tape: TensorTape, qkv: int, n_heads: int, *, causal: bool = True,

@@ -13,7 +13,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import FtkAttnDesc, FtkGemmDesc
+from ._lib import FtkGemmDesc
 
 EPI_NONE, EPI_GELU_TANH, EPI_GELU_ERF, EPI_RELU = 0, 1, 2, 3
 EPI_MUL_DGELU_TANH, EPI_MUL_DGELU_ERF, EPI_MUL_DRELU = 4, 5, 6
@@ -44,8 +44,14 @@ def reset_launch_count() -> None:
     _launches = 0
 
 
+# Raw handle of the current device's current stream.  torch.cuda.current_stream() builds a Stream object and resolves the
+# device through several layers: 4 - 5 us, as much as the rest of a launch.
+_get_device = torch._C._cuda_getDevice
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_get_device())
 
 
 def _ptr(t: Optional[torch.Tensor]):
@@ -120,66 +126,72 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     _bf16(a, "a"), _bf16(b, "b")
     if a.dim() != 2 or b.dim() != 2 or a.stride(1) != 1 or b.stride(1) != 1:
         raise KernelError("gemm operands must be 2-D with unit inner stride")
-    M, K = (a.shape[1], a.shape[0]) if a_mn else (a.shape[0], a.shape[1])
-    N, Kb = (b.shape[1], b.shape[0]) if b_mn else (b.shape[0], b.shape[1])
+    M, K = a.shape
+    if a_mn:
+        M, K = K, M
+    N, Kb = b.shape
+    if b_mn:
+        N, Kb = Kb, N
     if K != Kb:
         raise KernelError(f"gemm K mismatch: {K} vs {Kb}")
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    if out.shape != (M, N) or out.stride(1) != 1:
+    ldd, out_inner = out.stride() if out.dim() == 2 else (0, 0)
+    if out.shape != (M, N) or out_inner != 1:
         raise KernelError("gemm output must be [M, N] with unit inner stride")
-    g = FtkGemmDesc()
-    g.M, g.N, g.K, g.L0, g.L1 = M, N, K, 1, 1
-    g.a_mn, g.b_mn = int(a_mn), int(b_mn)
-    g.A, g.lda = a.data_ptr(), a.stride(0)
-    g.B, g.ldb = b.data_ptr(), b.stride(0)
-    g.D, g.ldd = out.data_ptr(), out.stride(0)
-    g.bias = _ptr(bias)
+    resid_ptr = ldr = aux_ptr = 0
     if resid is not None:
         _bf16(resid, "resid")
-        g.resid, g.ldr = resid.data_ptr(), resid.stride(0)
+        resid_ptr, ldr = resid.data_ptr(), resid.stride(0)
     if aux is not None:
         _bf16(aux, "aux")
-        if aux.stride(0) != out.stride(0):
+        if aux.stride(0) != ldd:
             raise KernelError("aux must share the row stride of the output")
-        g.aux = aux.data_ptr()
-    g.alpha, g.epi = float(alpha), int(epi)
-    g.out_fp32 = 1 if out.dtype == torch.float32 else 0
+        aux_ptr = aux.data_ptr()
     if out.dtype not in (torch.float32, torch.bfloat16):
         raise KernelError("gemm output must be bf16 or fp32")
-    g.accumulate, g.force_bn, g.max_ctas = int(accumulate), int(force_bn), int(max_ctas)
-    g.split_k = int(split_k)
-    g.reduce_stream = reduce_stream
+    seg_ptr = 0
     if seg_counts is not None:
         if seg_counts.dtype != torch.int32 or not seg_counts.is_cuda or seg_rows <= 0:
             raise KernelError("seg_counts must be a CUDA int32 tensor and seg_rows positive")
         if a_mn or seg_counts.numel() < -(-M // seg_rows):
             raise KernelError("seg_counts needs one entry per segment of rows of a row-major A operand")
-        g.seg_counts, g.seg_rows = seg_counts.data_ptr(), int(seg_rows)
+        seg_ptr = seg_counts.data_ptr()
     lib = _lib.load()
-    dev_key = a.device.index if a.device.index is not None else torch.cuda.current_device()
+    ws_ptr = ws_bytes = 0
+
+    def pack() -> bytes:
+        return _lib.GEMM_DESC.pack(
+            M, N, K, 1, 1, int(a_mn), int(b_mn), a.data_ptr(), a.stride(0), 0, 0, b.data_ptr(), b.stride(0), 0, 0,
+            out.data_ptr(), ldd, 0, 0, 0 if bias is None else bias.data_ptr(), resid_ptr, ldr, 0, 0, aux_ptr, float(alpha),
+            int(epi), 1 if out.dtype == torch.float32 else 0, int(accumulate), int(force_bn), int(max_ctas), ws_ptr,
+            ws_bytes, int(split_k), reduce_stream or 0, seg_ptr, int(seg_rows) if seg_ptr else 0)
+
+    def plan():
+        bn, sp = C.c_int(0), C.c_int(1)
+        rc = lib.ftk_gemm_plan(C.byref(FtkGemmDesc.from_buffer_copy(pack())), C.byref(bn), C.byref(sp))
+        return rc, bn.value, sp.value
     if split_k != 1 and bias is None and resid is None and aux is None and epi == EPI_NONE:
+        dev_key = a.device.index if a.device.index is not None else torch.cuda.current_device()
         ws = _gemm_workspace(a.device)
-        g.workspace, g.workspace_bytes = ws.data_ptr(), ws.numel() * 4
+        ws_ptr, ws_bytes = ws.data_ptr(), ws.numel() * 4
         busy = _WS_BUSY.get(dev_key)
         if busy is not None or reduce_stream is not None:
-            bn, sp = C.c_int(0), C.c_int(1)
-            lib.ftk_gemm_plan(C.byref(g), C.byref(bn), C.byref(sp))
-            if sp.value > 1:
+            if plan()[2] > 1:
                 if busy is not None:
                     # a reduction on another stream still reads the split-K workspace this GEMM will write
                     torch.cuda.current_stream(a.device).wait_event(busy)
                     _WS_BUSY.pop(dev_key, None)
             else:
-                g.reduce_stream = reduce_stream = None
+                reduce_stream = None
     what = "ftk_gemm_bf16"
     if _TRACE is not None:          # name the tile the planner picks for this problem
-        bn, sp = C.c_int(0), C.c_int(1)
-        if lib.ftk_gemm_plan(C.byref(g), C.byref(bn), C.byref(sp)) == 0:
-            what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn.value - 256, sp.value)) if bn.value > 256 else \
-                ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn.value, sp.value))
-    _chk(lib.ftk_gemm_bf16(C.byref(g), _stream()), what)
-    if reduce_stream is not None and g.workspace:
+        rc, bn, sp = plan()
+        if rc == 0:
+            what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn - 256, sp)) if bn > 256 else \
+                ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn, sp))
+    _chk(lib.gemm_packed(pack(), _stream()), what)
+    if reduce_stream is not None and ws_ptr:
         ev = torch.cuda.Event()
         ev.record(torch.cuda.ExternalStream(reduce_stream, device=a.device))
         _WS_BUSY[dev_key] = ev
@@ -276,22 +288,21 @@ def linear_wgrad(dy, x, *, out=None, accumulate=False, reduce_stream=None):
 
 
 # --------------------------------------------------------------------------------------- attention
-def _attn_desc(q, k, v, o, lse, causal, scale):
+def _attn_desc(q, k, v, o, lse, causal, scale, d_o=0, delta=0, dq=0, dk=0, dv=0) -> bytes:
     # q/k/v/o: views of shape [B, S, H, hd] (any strides with unit inner stride)
-    B, S, H, hd = q.shape
-    d = FtkAttnDesc()
-    d.B, d.H, d.S, d.hd, d.causal = B, H, S, hd, int(causal)
-    d.scale = float(scale if scale is not None else 1.0 / math.sqrt(hd))
+    shape = q.shape
+    B, S, H, hd = shape
+    ptrs, strides = [], []
     for name, t in (("q", q), ("k", k), ("v", v), ("o", o)):
         _bf16(t, name)
-        if t.shape != q.shape or t.stride(3) != 1:
+        bs, ss, hs, inner = t.stride() if t.dim() == 4 else (0, 0, 0, 0)
+        if t.shape != shape or inner != 1:
             raise KernelError(f"attention operand {name} must be [B,S,H,hd] with unit inner stride")
-        setattr(d, name, t.data_ptr())
-        setattr(d, name + "_bs", t.stride(0))
-        setattr(d, name + "_ss", t.stride(1))
-        setattr(d, name + "_hs", t.stride(2))
-    d.lse = lse.data_ptr()
-    return d
+        ptrs.append(t.data_ptr())
+        strides += (bs, ss, hs)
+    return _lib.ATTN_DESC.pack(B, H, S, hd, int(causal), float(scale if scale is not None else 1.0 / math.sqrt(hd)),
+                               ptrs[0], ptrs[1], ptrs[2], *strides[:9], ptrs[3], *strides[9:], lse.data_ptr(), d_o, delta,
+                               dq, dk, dv)
 
 
 def attention_fwd(q, k, v, *, causal=True, scale=None, out=None):
@@ -301,7 +312,7 @@ def attention_fwd(q, k, v, *, causal=True, scale=None, out=None):
         out = torch.empty((B, S, H, hd), dtype=torch.bfloat16, device=q.device)
     lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
     d = _attn_desc(q, k, v, out, lse, causal, scale)
-    _chk(_lib.load().ftk_attn_fwd(C.byref(d), _stream()), "ftk_attn_fwd")
+    _chk(_lib.load().attn_fwd_packed(d, _stream()), "ftk_attn_fwd")
     return out, lse
 
 
@@ -315,10 +326,9 @@ def attention_bwd(q, k, v, o, lse, d_o, *, causal=True, scale=None, dq=None, dk=
         if t.stride() != ref.stride():
             raise KernelError(f"{name} must share the strides of its primal")
     delta = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-    d = _attn_desc(q, k, v, o, lse, causal, scale)
-    d.d_o, d.delta = d_o.data_ptr(), delta.data_ptr()
-    d.dq, d.dk, d.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    _chk(_lib.load().ftk_attn_bwd(C.byref(d), _stream()), "ftk_attn_bwd")
+    d = _attn_desc(q, k, v, o, lse, causal, scale, d_o.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                   dv.data_ptr())
+    _chk(_lib.load().attn_bwd_packed(d, _stream()), "ftk_attn_bwd")
     return dq, dk, dv
 
 
