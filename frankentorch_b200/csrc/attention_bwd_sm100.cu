@@ -222,14 +222,19 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // fetched into registers one iteration ahead, so their global-memory latency is spent while
       // this warp waits for the stage, not between the stage becoming free and its TMA loads.
       const long long sbase = ((long long)b * p.H + h) * p.S;
-      float nl_r[4], dl_r[4];
+      // (signs are changed where the values are stored: an operation on a value in flight would wait for it here)
+      float lse_r[4], dl_r[4];
       auto fetch_stats = [&](int it) {
         const int q0 = (qb_first + it) * AT_T;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int gq = q0 + lane + 32 * u;
-          nl_r[u] = gq < p.S ? -p.lse[sbase + gq] : -INFINITY;
-          dl_r[u] = gq < p.S ? -p.delta[sbase + gq] : 0.f;
+          lse_r[u] = INFINITY;
+          dl_r[u] = 0.f;
+          if (gq < p.S) {
+            lse_r[u] = p.lse[sbase + gq];
+            dl_r[u] = p.delta[sbase + gq];
+          }
         }
       };
       fetch_stats(0);
@@ -256,8 +261,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         float* sl = stat + st * 256;          // published by the arrive below
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          sl[lane + 32 * u] = nl_r[u];
-          sl[128 + lane + 32 * u] = dl_r[u];
+          sl[lane + 32 * u] = -lse_r[u];
+          sl[128 + lane + 32 * u] = -dl_r[u];
         }
         __syncwarp();
         if (elect_one()) {
@@ -536,11 +541,15 @@ template <int HD>
 struct DqCfg {
   static constexpr int TILE = (HD / 64) * AT_REGION;
   static constexpr int QB = (HD == 64) ? 2 : 1;          // Q / dO buffers (one per work item)
-  static constexpr int NSLOT = (HD == 64) ? 8 : 4;       // ring of single K / V tiles: a V slot is free after dP, a K slot after dQ
-  static constexpr int OFF_QDO = 0;                      // [QB] Q, dO
-  static constexpr int OFF_KV = QB * 2 * TILE;           // [NSLOT]
-  static constexpr int OFF_OUT = OFF_KV + NSLOT * TILE;  // output staging
-  static constexpr int OFF_BAR = OFF_OUT + 2 * AT_REGION;
+  // K and V have a ring each: a V tile is free after dP, a K tile only after dQ, most of two blocks later.  (In one ring of
+  // four tiles the load of every second K started when it was needed: 2000 cycles per pair of blocks.  B4 S2048 H16 causal, head
+  // size 128: 126 -> 110 us.)
+  static constexpr int KS = (HD == 64) ? 4 : 3;
+  static constexpr int VS = (HD == 64) ? 4 : 2;
+  static constexpr int OFF_QDO = 0;                      // [QB] Q, dO; the item's output leaves through them
+  static constexpr int OFF_K = QB * 2 * TILE;            // [KS]
+  static constexpr int OFF_V = OFF_K + KS * TILE;        // [VS]
+  static constexpr int OFF_BAR = OFF_V + VS * TILE;
   static constexpr int SMEM = OFF_BAR + 512;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256;
@@ -558,9 +567,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* qdo_full = bars;        // [2]
-  uint64_t* qdo_empty = bars + 2;   // [2] the item's score products are done
-  uint64_t* kv_full = bars + 4;     // [8]
-  uint64_t* kv_empty = bars + 12;   // [8]
+  uint64_t* qdo_empty = bars + 2;   // [2] the item's output has left (one arrival per warp)
+  uint64_t* k_full = bars + 4;      // [4]
+  uint64_t* k_empty = bars + 8;     // [4]
+  uint64_t* v_full = bars + 12;     // [4]
+  uint64_t* v_empty = bars + 16;    // [4]
   uint64_t* s_full = bars + 20;     // S and dP in TMEM
   uint64_t* s_free = bars + 21;     // both copied to registers (one arrival per warp)
   uint64_t* ds_ready = bars + 22;   // [2] dS handed to the tensor core (one arrival per warp)
@@ -579,14 +590,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
+      mbar_init(&qdo_empty[i], BW_MATH);
       mbar_init(&ds_ready[i], BW_MATH);
       mbar_init(&acc_done[i], 1);
     }
-    for (int i = 0; i < 8; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-    }
+    for (int i = 0; i < 16; ++i) mbar_init(&k_full[i], 1);      // the four arrays of the rings
     mbar_init(s_full, 1);
     mbar_init(s_free, BW_MATH);
     mbar_init(acc_free, BW_MATH);
@@ -619,7 +627,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == BW_WARP_TMA) {
     Ring<C::QB> rq;
-    Ring<C::NSLOT> rk;
+    Ring<C::KS> rk;
+    Ring<C::VS> rv;
     bool ok = true;
 #pragma unroll 1
     for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
@@ -635,22 +644,31 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       __syncwarp();
       rq.step();
 #pragma unroll 1
-      for (int n = 0; n < 2 * nkv; ++n) {      // K_0, V_0, K_1, V_1, ...
-        if (!mbar_wait_warp(&kv_empty[rk.s], rk.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+      for (int j = 0; j < nkv; ++j) {
+        if (!mbar_wait_warp(&k_empty[rk.s], rk.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
         if (elect_one()) {
-          mbar_arrive_expect_tx(&kv_full[rk.s], C::TILE);
-          load_tile<HD>(smem + C::OFF_KV + rk.s * C::TILE, (n & 1) ? &tmV : &tmK, &kv_full[rk.s], (n >> 1) * AT_T, h, b);
+          mbar_arrive_expect_tx(&k_full[rk.s], C::TILE);
+          load_tile<HD>(smem + C::OFF_K + rk.s * C::TILE, &tmK, &k_full[rk.s], j * AT_T, h, b);
         }
         __syncwarp();
         rk.step();
+        if (!mbar_wait_warp(&v_empty[rv.s], rv.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
+          mbar_arrive_expect_tx(&v_full[rv.s], C::TILE);
+          load_tile<HD>(smem + C::OFF_V + rv.s * C::TILE, &tmV, &v_full[rv.s], j * AT_T, h, b);
+        }
+        __syncwarp();
+        rv.step();
       }
     }
   } else if (warp == BW_WARP_MMA) {
     // ---------------------------------------------------------- issuer 1: S = Q K^T, dP = dO V^T
     const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
-    const uint32_t qdo_addr = smem_u32(smem + C::OFF_QDO), kv_addr = smem_u32(smem + C::OFF_KV);
+    const uint32_t qdo_addr = smem_u32(smem + C::OFF_QDO);
+    const uint32_t k_addr = smem_u32(smem + C::OFF_K), v_addr = smem_u32(smem + C::OFF_V);
     Ring<C::QB> rq;
-    Ring<C::NSLOT> rk;
+    Ring<C::KS> rk;
+    Ring<C::VS> rv;
     uint32_t ph = 0;
     bool ok = true, first = true;
 #pragma unroll 1
@@ -660,32 +678,31 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t q_addr = qdo_addr + rq.s * 2 * C::TILE, do_addr = q_addr + C::TILE;
 #pragma unroll 1
       for (int j = 0; j < nkv; ++j) {
-        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL) ||
+        if (!mbar_wait_warp(&k_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL) ||
             (!first && !mbar_wait_warp(s_free, ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
         if (!first) ph ^= 1u;
         first = false;
         tc_fence_after();
-        if (elect_one()) mma_kmajor<HD>(tmem_base + C::TM_S, q_addr, kv_addr + rk.s * C::TILE, idesc_s);
+        if (elect_one()) mma_kmajor<HD>(tmem_base + C::TM_S, q_addr, k_addr + rk.s * C::TILE, idesc_s);
         __syncwarp();
         rk.step();
-        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(&v_full[rv.s], rv.ph, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-          mma_kmajor<HD>(tmem_base + C::TM_DP, do_addr, kv_addr + rk.s * C::TILE, idesc_s);
+          mma_kmajor<HD>(tmem_base + C::TM_DP, do_addr, v_addr + rv.s * C::TILE, idesc_s);
           umma_commit(s_full);
-          umma_commit(&kv_empty[rk.s]);
-          if (j == nkv - 1) umma_commit(&qdo_empty[rq.s]);
+          umma_commit(&v_empty[rv.s]);
         }
         __syncwarp();
-        rk.step();
+        rv.step();
       }
       rq.step();
     }
   } else if (warp == BW_WARP_MMA2) {
     // ---------------------------------------------------------- issuer 2: dQ += dS K
     const uint32_t idesc_acc = make_idesc_bf16(128, HD, 0, 1);
-    const uint32_t kv_addr = smem_u32(smem + C::OFF_KV);
-    Ring<C::NSLOT> rk;
+    const uint32_t k_addr = smem_u32(smem + C::OFF_K);
+    Ring<C::KS> rk;
     Ring<2> rd;
     uint32_t tile_ph = 0;
     bool ok = true, first_item = true;
@@ -694,18 +711,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int nkv = key_blocks(query_block(item));
 #pragma unroll 1
       for (int j = 0; j < nkv; ++j) {
-        if (!mbar_wait_warp(&kv_full[rk.s], rk.ph, ctx, FT_ERR_WAIT_FULL) ||
-            !mbar_wait_warp(&ds_ready[rd.s], rd.ph, ctx, FT_ERR_WAIT_SOFTMAX) ||
+        // (K_j landed before the scores that dS_j was made from)
+        if (!mbar_wait_warp(&ds_ready[rd.s], rd.ph, ctx, FT_ERR_WAIT_SOFTMAX) ||
             (j == 0 && !first_item && !mbar_wait_warp(acc_free, tile_ph, ctx, FT_ERR_WAIT_TMEM_EMPTY))) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-          mma_ptmem_times_rows(tmem_base + C::TM_DQ, tmem_base + C::TM_DS + 64 * rd.s, kv_addr + rk.s * C::TILE,
+          mma_ptmem_times_rows(tmem_base + C::TM_DQ, tmem_base + C::TM_DS + 64 * rd.s, k_addr + rk.s * C::TILE,
                                idesc_acc, j > 0);
           umma_commit(&acc_done[rd.s]);
-          umma_commit(&kv_empty[rk.s]);      // S of this tile finished before the math ran
+          umma_commit(&k_empty[rk.s]);       // S of this tile finished before the math ran
         }
         __syncwarp();
-        rk.step();
         rk.step();
         rd.step();
       }
@@ -724,21 +740,26 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     int filled = 0;                        // dS buffers written so far (2 = both have had a reader)
     bool ok = true;
     // statistics of this thread's row, fetched one item ahead
-    float nl_n = 0.f, dl_n = 0.f;
+    float lse_n = 0.f, dl_n = 0.f;
     auto fetch_stats = [&](int item) {
       if (item < 0) return;
       const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb;
       const int grow = qb * AT_T + row;
       const long long s = (long long)hb * p.S + grow;      // lse and delta are [B, H, S]
-      nl_n = grow < p.S ? -p.lse[s] : -INFINITY;
-      dl_n = grow < p.S ? -p.delta[s] : 0.f;
+      lse_n = INFINITY;
+      dl_n = 0.f;
+      if (grow < p.S) {          // (used, and their signs changed, one item later)
+        lse_n = p.lse[s];
+        dl_n = p.delta[s];
+      }
     };
+    Ring<C::QB> rq;
     int item = walk.next();
     fetch_stats(item);
     while (ok && item >= 0) {
       const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
       const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
-      const f32x2 nl = pk2(nl_n, nl_n), dl = pk2(dl_n, dl_n);
+      const f32x2 nl = pk2(-lse_n, -lse_n), dl = pk2(-dl_n, -dl_n);
       item = walk.next();
       fetch_stats(item);
       const int last_col = p.causal ? min(grow, p.S - 1) : p.S - 1;                 // last valid key of this row
@@ -792,11 +813,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_free);
         const int r0 = q0 + qd * 32;
-        store_out32(smem + C::OFF_OUT, qd, c0, lane, r, p.scale,
+        store_out32(smem + C::OFF_QDO + rq.s * 2 * C::TILE, qd, c0, lane, r, p.scale,
                     p.dq + b * p.dq_bs + r0 * p.dq_ss + h * p.dq_hs + c0, p.dq_ss, p.S - r0);
+        fence_proxy_async_smem();        // the tiles go back to the loader
+        __syncwarp();
       } else if (lane == 0) {
         mbar_arrive(acc_free);
       }
+      if (lane == 0) mbar_arrive(&qdo_empty[rq.s]);
+      rq.step();
     }
   }
 
