@@ -31,49 +31,6 @@ constexpr int BW_WARP_TMA = 16;
 constexpr int BW_WARP_MMA = 17;      // issues the score products, owns TMEM
 constexpr int BW_WARP_MMA2 = 18;     // issues the accumulating products
 
-// =============================================================================== delta
-// delta[b,h,s] = sum_e dO * O.  LPR = hd / 8 lanes share one (b, s, h) row (16 bytes each), so
-// a warp covers 32 / LPR rows and every lane loads.
-template <int LPR>
-__global__ void __launch_bounds__(256)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                  float* __restrict__ delta, int B, int H, int S, long long bs, long long ss,
-                  long long hs, FastDiv by_h, FastDiv by_s) {
-  pdl_wait();
-  pdl_trigger();
-  constexpr int RPW = 32 / LPR;                       // rows per warp and step
-  constexpr int U = 4;                                // steps: four rows' loads in flight per thread
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % LPR;
-  const long long total = (long long)B * S * H;
-  const long long w0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * (RPW * U) + lane / LPR;
-  uint4 a[U], g[U];
-  long long dst[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const long long w = w0 + u * RPW;
-    dst[u] = -1;
-    a[u] = g[u] = make_uint4(0u, 0u, 0u, 0u);
-    if (w < total) {
-      const int t = by_h.div((int)w), h = (int)w - t * H, b = by_s.div(t), s = t - b * S;
-      const long long off = (long long)b * bs + (long long)s * ss + (long long)h * hs + sub * 8;
-      a[u] = *reinterpret_cast<const uint4*>(o + off);
-      g[u] = *reinterpret_cast<const uint4*>(d_o + off);
-      dst[u] = ((long long)b * H + h) * S + s;
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    float2 a0 = unpack_bf16(a[u].x), a1 = unpack_bf16(a[u].y), a2 = unpack_bf16(a[u].z), a3 = unpack_bf16(a[u].w);
-    float2 g0 = unpack_bf16(g[u].x), g1 = unpack_bf16(g[u].y), g2 = unpack_bf16(g[u].z), g3 = unpack_bf16(g[u].w);
-    float acc = a0.x * g0.x + a0.y * g0.y + a1.x * g1.x + a1.y * g1.y + a2.x * g2.x + a2.y * g2.y +
-                a3.x * g3.x + a3.y * g3.y;
-#pragma unroll
-    for (int d = LPR / 2; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-    if (dst[u] >= 0 && sub == 0) delta[dst[u]] = acc;
-  }
-}
-
 // Store 32 packed-bf16 columns (16 words) of one tile row into the swizzled K-major tile.
 __device__ __forceinline__ void store_row32_packed(uint8_t* tile, int row, int col0,
                                                    const uint32_t* w) {
@@ -550,7 +507,10 @@ struct DqCfg {
   static constexpr int OFF_K = QB * 2 * TILE;            // [KS]
   static constexpr int OFF_V = OFF_K + KS * TILE;        // [VS]
   static constexpr int OFF_BAR = OFF_V + VS * TILE;
-  static constexpr int SMEM = OFF_BAR + 512;
+  static constexpr int OFF_DELTA = OFF_BAR + 512;        // [2] rowsum(dO o O) of an item's rows
+  static constexpr int SMEM = OFF_DELTA + 2 * AT_T * 4;
+  // rowsum(dO o O): LPR lanes share a row, each of the 16 math warps takes 8 rows in U steps
+  static constexpr int LPR = HD / 8, RPS = 32 / LPR, U = 8 / RPS;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256;
   static constexpr int TM_DS = 384;                      // dS buffer i (packed bf16) at TM_DS + 64 i
@@ -558,6 +518,11 @@ struct DqCfg {
 };
 
 // Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.
+//
+// It also makes delta = rowsum(dO o O), which the dK / dV kernel behind it reads: dO is in shared memory here anyway and the
+// item's share of O is fetched one item ahead, so the sums run under the item's first score products.  (A kernel of its own
+// in front of both read dO once more and stood on the path of the whole backward: B8 S1024 H12 head size 64 causal 75.1 -> 72.5 us,
+// B4 S2048 H16 head size 128 252 -> 246 us, B4 S128 H2 11.7 -> 10.4 us.)
 template <int HD>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -577,7 +542,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* ds_ready = bars + 22;   // [2] dS handed to the tensor core (one arrival per warp)
   uint64_t* acc_done = bars + 24;   // [2] dQ product that read the buffer done
   uint64_t* acc_free = bars + 26;   // the item's dQ copied to registers (one arrival per warp)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
+  uint64_t* d_ready = bars + 27;    // the item's delta is in shared memory (one arrival per warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
   int* abort_f = reinterpret_cast<int*>(tmem_slot + 1);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
@@ -598,6 +564,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(s_full, 1);
     mbar_init(s_free, BW_MATH);
     mbar_init(acc_free, BW_MATH);
+    mbar_init(d_ready, BW_MATH);
     *abort_f = 0;
     fence_mbar_init();
   }
@@ -739,29 +706,62 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     uint32_t blk = 0;                      // parity of the block
     int filled = 0;                        // dS buffers written so far (2 = both have had a reader)
     bool ok = true;
-    // statistics of this thread's row, fetched one item ahead
-    float lse_n = 0.f, dl_n = 0.f;
-    auto fetch_stats = [&](int item) {
+    // log-sum-exp of this thread's row and this lane's segments of O, fetched one item ahead (used, and signs changed, then)
+    float lse_n = 0.f;
+    uint4 o_n[C::U];
+    const int d_row = 8 * warp + lane / C::LPR, d_seg = lane % C::LPR;      // row of step 0, 16-byte segment
+    float* s_delta = reinterpret_cast<float*>(smem + C::OFF_DELTA);
+    uint32_t it_ph = 0;                    // parity of the item: d_ready's phase and the buffer of s_delta
+    auto fetch_rows = [&](int item) {
       if (item < 0) return;
-      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb;
-      const int grow = qb * AT_T + row;
-      const long long s = (long long)hb * p.S + grow;      // lse and delta are [B, H, S]
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int q0 = qb * AT_T;
       lse_n = INFINITY;
-      dl_n = 0.f;
-      if (grow < p.S) {          // (used, and their signs changed, one item later)
-        lse_n = p.lse[s];
-        dl_n = p.delta[s];
+      if (q0 + row < p.S) lse_n = p.lse[(long long)hb * p.S + q0 + row];      // [B, H, S]
+      const __nv_bfloat16* op = p.o + b * p.o_bs + (long long)(q0 + d_row) * p.o_ss + h * p.o_hs + d_seg * 8;
+#pragma unroll
+      for (int u = 0; u < C::U; ++u) {
+        o_n[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (q0 + d_row + u * C::RPS < p.S) o_n[u] = *reinterpret_cast<const uint4*>(op + (long long)(u * C::RPS) * p.o_ss);
       }
     };
     Ring<C::QB> rq;
     int item = walk.next();
-    fetch_stats(item);
+    fetch_rows(item);
     while (ok && item >= 0) {
       const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
       const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
-      const f32x2 nl = pk2(-lse_n, -lse_n), dl = pk2(-dl_n, -dl_n);
+      const f32x2 nl = pk2(-lse_n, -lse_n);
+      if (!mbar_wait_warp(&qdo_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
+      const uint8_t* do_tile = smem + C::OFF_QDO + (rq.s * 2 + 1) * C::TILE + (d_seg >> 3) * AT_REGION;
+      float* s_dl = s_delta + it_ph * AT_T;
+#pragma unroll
+      for (int u = 0; u < C::U; ++u) {
+        const int r = d_row + u * C::RPS;
+        const uint4 g = *reinterpret_cast<const uint4*>(do_tile + r * 128 + (((d_seg & 7) ^ (r & 7)) << 4));
+        const uint32_t ow[4] = {o_n[u].x, o_n[u].y, o_n[u].z, o_n[u].w}, gw[4] = {g.x, g.y, g.z, g.w};
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = unpack_bf16(ow[i]), y = unpack_bf16(gw[i]);
+          acc = fmaf(x.x, y.x, acc);
+          acc = fmaf(x.y, y.y, acc);
+        }
+#pragma unroll
+        for (int m = C::LPR / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+        if (d_seg == 0) {
+          s_dl[r] = acc;
+          if (q0 + r < p.S) p.delta[(long long)hb * p.S + q0 + r] = acc;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(d_ready);
       item = walk.next();
-      fetch_stats(item);
+      fetch_rows(item);
+      if (!mbar_wait_warp(d_ready, it_ph, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
+      it_ph ^= 1u;
+      const float dl_row = -s_dl[row];
+      const f32x2 dl = pk2(dl_row, dl_row);
       const int last_col = p.causal ? min(grow, p.S - 1) : p.S - 1;                 // last valid key of this row
       const int warp_last = p.causal ? min(q0 + qd * 32, p.S - 1) : p.S - 1;       // of the warp's first row
 #pragma unroll 1
@@ -852,14 +852,10 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   }
   const long long nrows = (long long)a->B * a->S * a->H;
   if (nrows > 0x7fffffffll) return -2;
-  constexpr int LPR = HD / 8, ROWS_PER_CTA = 8 * (32 / LPR) * 4;
-  launch_pdl(attn_delta_kernel<LPR>, (unsigned)((nrows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, s,
-      reinterpret_cast<const __nv_bfloat16*>(a->o), reinterpret_cast<const __nv_bfloat16*>(a->d_o),
-      a->delta, a->B, a->H, a->S, a->o_bs, a->o_ss, a->o_hs, FastDiv((uint32_t)a->H), FastDiv((uint32_t)a->S));
   unsigned grid = 0;
   if ((rc = set_items(p, a, AT_T, &grid))) return rc;
+  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);      // writes delta
   launch_pdl(attn_bwd_dkv_kernel<HD>, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);
-  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
 }
 

@@ -23,7 +23,7 @@ struct AttnArgs {
   __nv_bfloat16* o;
   long long o_bs, o_ss, o_hs;
   float* lse;
-  const float* delta;
+  float* delta;             // written by the dQ kernel, read by the dK / dV kernel
   __nv_bfloat16 *dq, *dk, *dv;
   long long dq_bs, dq_ss, dq_hs, dk_bs, dk_ss, dk_hs, dv_bs, dv_ss, dv_hs;
   int* status;
