@@ -14,13 +14,13 @@
 // columns; a thread owns one tile row inside its group's columns), so one tcgen05.ld per
 // operand brings a thread's whole share into registers, the TMEM score tiles are released at
 // once and the tensor core computes the next block's scores under the exponentials of this
-// one.  With head_dim 64, P^T / dS^T (or dS) go back to the tensor core through tensor memory
-// (tcgen05.st by the row's thread, MMA with its A operand in TMEM); with head_dim 128 all 512
-// columns hold accumulators and they go through 128B-swizzled bf16 tiles in shared memory.
+// one.  P^T and dS go back to the tensor core through tensor memory (tcgen05.st by the row's thread, MMA with its A operand in
+// TMEM), dS^T too with head_dim 64; with head_dim 128 the accumulators leave no columns for dS^T, which goes through
+// 128B-swizzled bf16 tiles in shared memory.
 //
-// Determinism: dK/dV are accumulated in TMEM by the CTA that owns the key block, dQ by the
-// CTA that owns the query block (second kernel), both in ascending block order; there are
-// no atomics, so gradients are bit-identical run to run.
+// Determinism: dQ is accumulated in TMEM by the CTA that owns the query block (first kernel, which also writes
+// delta = rowsum(dO o O)), dK / dV by the CTA that owns the key block, all in ascending block order; there are no atomics, so
+// gradients are bit-identical run to run.
 #include "attn_common.cuh"
 
 namespace ftk {
