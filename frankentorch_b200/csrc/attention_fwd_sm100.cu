@@ -22,6 +22,7 @@
 // columns are taken by S and O, so P overwrites the scores it was made from and a tile's next scores follow its P V - the
 // two tiles take turns on the tensor core and on the exponentials.
 #include "attn_common.cuh"
+#include "attn_turns.h"
 
 namespace ftk {
 
@@ -99,7 +100,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* p_ready = bars + 28;       // [2][2] per half and tile: probabilities in TMEM (one arrival per warp)
   uint64_t* pv_done = bars + 32;       // [2] per tile: PV finished (P free, O tile settled)
   uint64_t* o_free = bars + 34;        // [2] per tile: the item's O copied to registers (one arrival per warp)
-  uint64_t* e_done = bars + 36;        // [2] per tile: exponentials of the block done (one arrival per warp)
+  uint64_t* e_done = bars + 36;        // [2] per tile: the group's turn is over (one arrival per warp)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 38);
   int* abort_f = reinterpret_cast<int*>(tmem_slot + 1);
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -289,14 +290,13 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const f32x2 sl2 = pk2(p.sl2, p.sl2);
     uint32_t blk = 0;                        // parity of the tile's block
     Ring<C::QS> rq;                          // the Q tile of the group's next item
-    uint32_t other = 0;                      // blocks of the other group in the items before this one
+    AttnTurns turns;
     bool ok = true;
 #pragma unroll 1
     for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
       const FwdItem it(item, p);
       const int n_my = t == 0 ? it.nb[0] : it.nb[1], n_other = t == 0 ? it.nb[1] : it.nb[0];
-      const uint32_t other0 = other;
-      other += (uint32_t)n_other;
+      turns.item(n_my, n_other);
       if (t == 1 && n_other > 0) rq.step();         // tile 0's Q comes first
       const int q_slot = rq.s;
       if (n_my > 0) rq.step();
@@ -377,13 +377,14 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
           }
         }
-        // The groups take turns: A's exponentials of block j, B's of block j, A's of block j + 1.  Side by side they halve
-        // each other's rate on the one unit that evaluates them, and both groups' other work then leaves it idle
-        // (1 x 1500 x 20 heads of 64: 26.0 us side by side, 23.5 us in turns).  With head_dim 128 the score products keep the
-        // groups apart by themselves (4 x 2048 x 16, causal: 77.5 us in turns, 75.3 us without).
-        if (C::TURNS && (t == 0 ? (j > 0 && n_other > 0) : j < n_other)) {
-          const uint32_t want = other0 + (uint32_t)(t == 0 ? j - 1 : j);      // index of the other group's block
-          if (!mbar_wait_warp(&e_done[t ^ 1], want & 1u, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
+        // The groups take turns (see AttnTurns).  Side by side they halve each other's rate on the one unit that evaluates
+        // exponentials, and both groups' other work then leaves it idle (1 x 1500 x 20 heads of 64: 26.0 us side by side,
+        // 23.5 us in turns).  With head_dim 128 the score products keep the groups apart by themselves (4 x 2048 x 16, causal:
+        // 77.5 us in turns, 75.3 us without).  Every wait is for work that precedes this block in the order (item, block,
+        // tile) in which scores, products and turns are issued, so the turns add no cycle to the other barriers.
+        uint32_t turn;
+        if (C::TURNS && turns.waits(t, j, turn)) {
+          if (!mbar_wait_warp(&e_done[t ^ 1], turn, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
         }
         // probabilities go to tensor memory, each half as soon as it is computed
         exp_half(0);
@@ -393,7 +394,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_ready[t]);
         exp_half(64);
-        if (C::TURNS && lane == 0) mbar_arrive(&e_done[t]);
+        if (C::TURNS && turns.takes(j) && lane == 0) mbar_arrive(&e_done[t]);
         tmem_st32(p_tmem + 32, r + 32);
         const float2 s0 = up2(add2(rs0, rs1));
         l = l * alpha + (s0.x + s0.y);
