@@ -486,8 +486,9 @@ extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
   if (blocks > 148 * 8) blocks = 148 * 8;
   cudaStream_t rs = g->reduce_stream ? reinterpret_cast<cudaStream_t>(g->reduce_stream) : stream;
   if (rs != stream) {
-    // reduction on its own stream, ordered behind the GEMM (one event per device, re-recorded per call)
-    static cudaEvent_t ev[64] = {nullptr};
+    // reduction on its own stream, ordered behind the GEMM (one event per device and thread, re-recorded per call: another
+    // thread's record between this one's record and wait would order the reduction behind the wrong GEMM)
+    static thread_local cudaEvent_t ev[64] = {nullptr};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!ev[dev]) {

@@ -41,6 +41,7 @@ class SideWork:
         self.tape, self.device = tape, device
         self.on = SideWork.enabled and device.type == "cuda"
         self._marks = []
+        self._held = []            # partial tiles of split products, read on the side stream until the join
         self._saved_fn = None
 
     @classmethod
@@ -67,7 +68,7 @@ class SideWork:
             ev = torch.cuda.Event()
             ev.record(self.side)
             self.main.wait_event(ev)
-            K.workspace_idle(self.device)
+            self._held.clear()
             self.tape.leaf_grad_written_fn = self._saved_fn
             if self._saved_fn is not None and exc[0] is None:
                 for nid in self._marks:
@@ -78,7 +79,8 @@ class SideWork:
         """Weight gradient GEMM on the main stream; its split-K reduction (if any) on the side stream."""
         if not self.on:
             return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate)
-        return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate, reduce_stream=self.side.cuda_stream)
+        return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate, reduce_stream=self.side.cuda_stream,
+                              keep=self._held)
 
     def colsum(self, dy2d, out=None, accumulate=False):
         if not self.on:

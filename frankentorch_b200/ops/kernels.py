@@ -112,13 +112,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
          accumulate: bool = False, force_bn: int = 0, max_ctas: int = 0, split_k: int = 0,
          reduce_stream: Optional[int] = None, seg_counts: Optional[torch.Tensor] = None,
-         seg_rows: int = 0) -> torch.Tensor:
+         seg_rows: int = 0, keep: Optional[list] = None) -> torch.Tensor:
     """``D = epi(alpha * A @ B^T + bias) (+ resid) (+ D)`` on the tcgen05 GEMM.
 
     ``a`` is ``[M, K]`` (``a_mn=False``) or ``[K, M]`` (``a_mn=True``); ``b`` is
     ``[N, K]`` or ``[K, N]`` likewise.  Both must be bf16 with unit inner stride.
-    ``reduce_stream`` (a raw stream handle) moves a split-K reduction off the launching stream;
-    the caller joins that stream before reading the output or launching the next split-K GEMM.
+    ``reduce_stream`` (a raw stream handle) moves a split-K reduction off the launching stream; the caller joins
+    that stream before reading the output.  The partial tiles then live until the reduction is done, or, where
+    ``keep`` is given, in that list until the caller drops it behind the join.
     ``seg_counts`` (int32, device) with ``seg_rows``: the rows are segments of ``seg_rows`` rows of which
     only the first ``seg_counts[s]`` are in use; 128-row tiles without a used row are skipped and
     their output rows are left as they were (expert batches with capacity padding).
@@ -158,7 +159,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise KernelError("seg_counts needs one entry per segment of rows of a row-major A operand")
         seg_ptr = seg_counts.data_ptr()
     lib = _lib.load()
-    ws_ptr = ws_bytes = 0
+    ws, ws_ptr, ws_bytes = None, 0, 0
 
     def pack() -> bytes:
         return _lib.GEMM_DESC.pack(
@@ -171,19 +172,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         bn, sp = C.c_int(0), C.c_int(1)
         rc = lib.ftk_gemm_plan(C.byref(FtkGemmDesc.from_buffer_copy(pack())), C.byref(bn), C.byref(sp))
         return rc, bn.value, sp.value
-    if split_k != 1 and bias is None and resid is None and aux is None and epi == EPI_NONE:
-        dev_key = a.device.index if a.device.index is not None else torch.cuda.current_device()
-        ws = _gemm_workspace(a.device)
-        ws_ptr, ws_bytes = ws.data_ptr(), ws.numel() * 4
-        busy = _WS_BUSY.get(dev_key)
-        if busy is not None or reduce_stream is not None:
-            if plan()[2] > 1:
-                if busy is not None:
-                    # a reduction on another stream still reads the split-K workspace this GEMM will write
-                    torch.cuda.current_stream(a.device).wait_event(busy)
-                    _WS_BUSY.pop(dev_key, None)
-            else:
-                reduce_stream = None
+    if split_k != 1 and K > SPLIT_ABOVE_K and bias is None and resid is None and aux is None and epi == EPI_NONE and \
+            seg_counts is None:
+        # Partial tiles go to scratch of this call alone, in the order of the launching stream: products of other
+        # streams, threads and captured graphs are never written over.
+        ws_ptr, ws_bytes = 256, GEMM_WORKSPACE_BYTES      # a stand-in: the plan looks at the size
+        rc, _, sp = plan()
+        ws_ptr = ws_bytes = 0
+        if rc == 0 and sp > 1:
+            ws = torch.empty(sp * M * N, dtype=torch.float32, device=a.device)
+            ws_ptr, ws_bytes = ws.data_ptr(), sp * M * N * 4
     what = "ftk_gemm_bf16"
     if _TRACE is not None:          # name the tile the planner picks for this problem
         rc, bn, sp = plan()
@@ -191,10 +189,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn - 256, sp)) if bn > 256 else \
                 ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn, sp))
     _chk(lib.gemm_packed(pack(), _stream()), what)
-    if reduce_stream is not None and ws_ptr:
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.ExternalStream(reduce_stream, device=a.device))
-        _WS_BUSY[dev_key] = ev
+    if reduce_stream is not None and ws is not None:
+        if keep is not None:
+            keep.append(ws)
+        else:
+            ws.record_stream(torch.cuda.ExternalStream(reduce_stream, device=a.device))
     return out
 
 
@@ -229,27 +228,10 @@ def gemm_grouped(problems, *, a_mn: bool = True, b_mn: bool = True, max_ctas: in
          "ftk::gemm_group_bf16_sm100<128x192,problems=%d>" % n)
 
 
-_WORKSPACES = {}
+# Most bytes of partial tiles that the tile planner may spend on one product, and the reduction length up to which it never
+# splits (a split keeps at least eight k-blocks of 64), so that short products do not ask it.
 GEMM_WORKSPACE_BYTES = 64 << 20
-# per device: event recorded behind a split-K reduction that runs on a stream other than its GEMM's;
-# the next split-K GEMM waits for it, and whoever joins that stream calls workspace_idle()
-_WS_BUSY = {}
-
-
-def workspace_idle(device) -> None:
-    """The caller has joined the stream that ran split-K reductions: the workspace is free again."""
-    key = device.index if getattr(device, "index", None) is not None else torch.cuda.current_device()
-    _WS_BUSY.pop(key, None)
-
-
-def _gemm_workspace(device) -> torch.Tensor:
-    """Per-device fp32 scratch for split-K partial tiles (allocated once, outside any capture)."""
-    key = (device.type, device.index if device.index is not None else torch.cuda.current_device())
-    ws = _WORKSPACES.get(key)
-    if ws is None:
-        ws = torch.empty(GEMM_WORKSPACE_BYTES // 4, dtype=torch.float32, device=device)
-        _WORKSPACES[key] = ws
-    return ws
+SPLIT_ABOVE_K = 15 * 64
 
 
 def gemm_batched(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, M: int, N: int, K: int,
@@ -281,10 +263,10 @@ def linear_dgrad(dy, w, *, epi=EPI_NONE, resid=None, out=None, seg_counts=None, 
     return gemm(dy, w, b_mn=True, epi=epi, resid=resid, out=out, seg_counts=seg_counts, seg_rows=seg_rows)
 
 
-def linear_wgrad(dy, x, *, out=None, accumulate=False, reduce_stream=None):
+def linear_wgrad(dy, x, *, out=None, accumulate=False, reduce_stream=None, keep=None):
     """``dw[out, in] (+)= dy^T @ x`` in fp32; both operands are consumed MN-major."""
     return gemm(dy, x, a_mn=True, b_mn=True, out=out, out_dtype=torch.float32, accumulate=accumulate,
-                reduce_stream=reduce_stream)
+                reduce_stream=reduce_stream, keep=keep)
 
 
 # --------------------------------------------------------------------------------------- attention
