@@ -13,8 +13,8 @@
 // 32 x 2048 x 512 with bias 11.3 -> 5.1 us, 8192 x 3072 x 768 with bias, GELU and pre-activation 75.3 -> 39.7 us, with GELU'
 // of a residual operand 66.3 -> 42.0 us (both together with the issue loops of the kernels, see mbar_wait_warp).
 //
-// Outputs whose extents or alignment do not allow 16-byte segments (and bf16 accumulation) take the general path: the
-// chunk goes to the tile in fp32 and is written row by row, lane = column, in a rolled loop.
+// Outputs and operands whose extents or alignment do not allow 16-byte segments take the general path: the chunk goes to
+// the tile in fp32 and is written row by row, lane = column, eight rows at a time.
 #pragma once
 #include "ft_sm100.cuh"
 #include "ftk_api.h"
@@ -150,7 +150,9 @@ struct TileEpilogue {
   long long ldd_;
   const __nv_bfloat16* resid;    // row `row0`, column 0
   __nv_bfloat16* aux;
-  uint4 rq[4];                   // residual chunk in flight: rows 8 i + lane / 4, segment lane % 4
+  bool r_vec_;                   // the residual's rows are whole 16-byte segments
+  uint32_t rw[16];               // residual chunk in flight: words 4 i .. of row 8 i + lane / 4, segment lane % 4, or
+                                 // (rows that are not whole segments) column `lane` of rows 2 i and 2 i + 1
 
   __device__ __forceinline__ TileEpilogue(const GemmArgs& args, uint8_t* st, __nv_bfloat16* sb, int ln)
       : p(args), stage(st), sbias(sb), lane(ln) {}
@@ -187,7 +189,7 @@ struct TileEpilogue {
     if (CAN_R) resid = p.resid + l0 * p.r_s0 + l1 * p.r_s1 + (long long)row * p.ldr;
     if (ANY) {
       bool ok = ((reinterpret_cast<uintptr_t>(d) & 15) == 0) && p.ldd % (16 / es) == 0 && p.N % (16 / es) == 0;
-      if (has_r()) ok = ok && ((reinterpret_cast<uintptr_t>(resid) & 15) == 0) && p.ldr % 8 == 0 && p.N % 8 == 0;
+      r_vec_ = ((reinterpret_cast<uintptr_t>(resid) & 15) == 0) && p.ldr % 8 == 0 && p.N % 8 == 0;
       if (has_aux()) ok = ok && !p.out_fp32 && ((reinterpret_cast<uintptr_t>(aux) & 15) == 0);
       if (p.accumulate && !p.out_fp32) ok = false;
       mode_ = !ok ? SLOW : (p.out_fp32 ? F32 : BF16);
@@ -203,14 +205,40 @@ struct TileEpilogue {
     }
     if (has_r() && mode() != SLOW) fetch_resid(col);
   }
+  __device__ __forceinline__ bool r_vec() const { return !ANY || r_vec_; }
+  // Rows that are not whole 16-byte segments come in 2 bytes per lane, 64 contiguous bytes of a row per warp, and leave the
+  // output on the staged path (8192 x 768 x 3072 with residual rows of 8 bytes 114 us on the general path, 39 so).
+  // (plain loads: the residual may be the output itself)
   __device__ __forceinline__ void fetch_resid(int n0) {
-    const int c = n0 + (lane & 3) * 8;
+    if (r_vec()) {
+      const int c = n0 + (lane & 3) * 8;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 8 * i + (lane >> 2);
-      rq[i] = (row0 + r < p.M && c < p.N)
-                  ? __ldg(reinterpret_cast<const uint4*>(resid + (long long)r * p.ldr + c))
-                  : make_uint4(0u, 0u, 0u, 0u);
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2);
+        const uint4 u = (row0 + r < p.M && c < p.N) ? *reinterpret_cast<const uint4*>(resid + (long long)r * p.ldr + c)
+                                                    : make_uint4(0u, 0u, 0u, 0u);
+        rw[4 * i] = u.x; rw[4 * i + 1] = u.y; rw[4 * i + 2] = u.z; rw[4 * i + 3] = u.w;
+      }
+    } else {
+      const unsigned short* rp = reinterpret_cast<const unsigned short*>(resid) + n0 + lane;
+      const int rows = n0 + lane < p.N ? p.M - row0 : 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t lo = 2 * i < rows ? rp[(2 * i) * p.ldr] : 0, hi = 2 * i + 1 < rows ? rp[(2 * i + 1) * p.ldr] : 0;
+        rw[i] = lo | (hi << 16);
+      }
+    }
+  }
+  // the fetched chunk into the tile
+  __device__ __forceinline__ void put_resid() const {
+    if (r_vec()) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *seg64(0, 8 * i + (lane >> 2), lane & 3) = make_uint4(rw[4 * i], rw[4 * i + 1], rw[4 * i + 2], rw[4 * i + 3]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 32; ++r)
+        reinterpret_cast<unsigned short*>(seg64(0, r, lane >> 3))[lane & 7] = (unsigned short)(rw[r >> 1] >> (16 * (r & 1)));
     }
   }
   // 64-byte rows: segment s (16 bytes) of row r
@@ -275,24 +303,40 @@ struct TileEpilogue {
     const bool live = c < p.N;
     const float b = has_bias() ? __bfloat162float(sbias[32 * j + lane]) : 0.f;
     const int rows = min(32, p.M - row0);
+    if (!live) return;
+    // Eight rows at a time, all that is read of them requested before the first is written: row by row, each waits for its
+    // own load (8192 x 769 x 3072 with bias and residual 146 -> 87 us, with fp32 accumulation 170 -> 87).
+    const bool add = p.accumulate && !split();
 #pragma unroll 1
-    for (int r = 0; r < rows; ++r) {
-      float v = reinterpret_cast<const float*>(seg128(r, lane >> 2))[lane & 3] + b;
-      if (!live) continue;
-      if (split()) {
-        reinterpret_cast<float*>(d)[(long long)r * ldd() + c] = v;
-        continue;
+    for (int r0 = 0; r0 < rows; r0 += 8) {
+      float rr[8], old[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = r0 + k;
+        rr[k] = old[k] = 0.f;
+        if (has_r() && r < rows) rr[k] = __bfloat162float(resid[(long long)r * p.ldr + c]);
+        if (add && r < rows)
+          old[k] = p.out_fp32 ? reinterpret_cast<const float*>(d)[(long long)r * ldd() + c]
+                              : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(d)[(long long)r * ldd() + c]);
       }
-      if (has_aux()) aux[(long long)r * ldd() + c] = __float2bfloat16(v);
-      const float rr = has_r() ? __bfloat162float(resid[(long long)r * p.ldr + c]) : 0.f;
-      v = apply_epi(v, rr, p.epi);
-      if (p.epi < FTK_EPI_MUL_DGELU_TANH) v += rr;
-      if (p.out_fp32) {
-        float* dp = reinterpret_cast<float*>(d) + (long long)r * ldd() + c;
-        *dp = p.accumulate ? *dp + v : v;
-      } else {
-        __nv_bfloat16* dp = reinterpret_cast<__nv_bfloat16*>(d) + (long long)r * ldd() + c;
-        *dp = __float2bfloat16(p.accumulate ? __bfloat162float(*dp) + v : v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = r0 + k;
+        if (r >= rows) break;
+        float v = reinterpret_cast<const float*>(seg128(r, lane >> 2))[lane & 3] + b;
+        const long long at = (long long)r * ldd() + c;
+        if (split()) {
+          reinterpret_cast<float*>(d)[at] = v;
+          continue;
+        }
+        if (has_aux()) aux[at] = __float2bfloat16(v);
+        v = apply_epi(v, rr[k], p.epi);
+        if (has_r() && p.epi < FTK_EPI_MUL_DGELU_TANH) v += rr[k];
+        if (add) v += old[k];
+        if (p.out_fp32)
+          reinterpret_cast<float*>(d)[at] = v;
+        else
+          reinterpret_cast<__nv_bfloat16*>(d)[at] = __float2bfloat16(v);
       }
     }
   }
@@ -308,8 +352,7 @@ struct TileEpilogue {
       uint32_t rp[16];
       if (has_r() && mode() != SLOW) {
         // residual: registers -> tile -> the row's own thread
-#pragma unroll
-        for (int i = 0; i < 4; ++i) *seg64(0, 8 * i + (lane >> 2), lane & 3) = rq[i];
+        put_resid();
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -98,6 +98,30 @@ def test_rows_without_aligned_segments(cuda_device, bn, N, ldd, off):
     assert bool((store[mask] == 7.0).all())
 
 
+@pytest.mark.parametrize("bn", WIDTHS)
+@pytest.mark.parametrize("kind", ["plain", "bias_gelu", "relu_resid", "dgelu"])
+@pytest.mark.parametrize("ldr", [72, 73, 76])
+def test_bf16_accumulation_and_residual_rows(cuda_device, bn, kind, ldr):
+    """A bf16 output that is added to, with an operand whose rows are whole 16-byte segments (72), 2 or 8 bytes off them."""
+    from frankentorch_b200.ops import kernels as k
+    M, N, K = 333, 72, 136
+    a, w, bias = _rand((M, K), 31, cuda_device), _rand((N, K), 32, cuda_device, K ** -0.5), _rand((N,), 33, cuda_device)
+    out, r = _rand((M, N), 34, cuda_device), _rand((M, ldr), 35, cuda_device)[:, :N]
+    ref, kw = a.double() @ w.double().t(), {}
+    if kind == "bias_gelu":
+        ref, kw = _gelu(ref + bias.double()), {"bias": bias, "epi": k.EPI_GELU_TANH}
+    elif kind == "relu_resid":
+        ref, kw = torch.relu(ref) + r.double(), {"epi": k.EPI_RELU, "resid": r}
+    elif kind == "dgelu":
+        ref, kw = ref * _dgelu(r.double()), {"epi": k.EPI_MUL_DGELU_TANH, "resid": r}
+    fresh = k.gemm(a, w, force_bn=bn, split_k=1, **kw)
+    ref_acc = ref + out.double()
+    k.gemm(a, w, out=out, accumulate=True, force_bn=bn, split_k=1, **kw)
+    k.check_status()
+    _close(fresh, ref, act="gelu" in kind)
+    _close(out, ref_acc, act="gelu" in kind)
+
+
 def test_grouped_products_with_unaligned_outputs(cuda_device):
     from frankentorch_b200.ops import kernels as k
     K, shapes = 264, [(264, 200), (16, 8), (520, 40)]
