@@ -6,8 +6,8 @@
 // variance (ft-kernel-cpu/src/lib.rs:5824), RMSNorm (:6418, backward :6503),
 // cross-entropy = lse - logit[target] with gradient softmax - onehot (:6649,:6679),
 // guarded row softmax of the Metal shader (ft-kernel-metal/src/fused.rs:321).
-// Parameter-gradient reductions run in a fixed order (row blocks, then a serial
-// pass over the block partials), so two runs give identical bits.
+// Parameter-gradient reductions run in a fixed order (row blocks, then a fixed tree over
+// the block partials), so two runs give identical bits.
 #include "ft_sm100.cuh"
 #include "launch.cuh"
 #include "ftk_api.h"
@@ -492,25 +492,28 @@ norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16*
   }
 }
 
-// Fixed-order sum over block partials: a CTA takes 32 columns, warp g adds partial[b][c] for b = g, g + 32, ... ascending
-// with up to eight loads of each array in flight, then the 32 group sums of a column are added by a fixed shuffle tree.  A
-// second array (dbeta) goes along.  All latency: with 8 groups of serial loads 256 partials x 768 took 4.9 us, now 3.1 us.
-__global__ void __launch_bounds__(1024)
-col_final_wide_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                      const float* __restrict__ partial2, float* __restrict__ out2, int cols, int nblk,
-                      int accumulate) {
+// Fixed-order sum over block partials.  G groups share a column: group g adds partial[b][c] for b = g, g + G, ... ascending with
+// up to eight loads of each array in flight, then the group sums are added, in group order (G = 8) or by a fixed shuffle tree
+// (G = 32).  A second array (dbeta) goes along.  All latency, so the number of groups follows the number of partials, see
+// col_final().
+template <int G>
+__global__ void __launch_bounds__(G == 1 ? 128 : 32 * G)
+col_final_kernel(const float* __restrict__ partial, float* __restrict__ out,
+                 const float* __restrict__ partial2, float* __restrict__ out2, int cols, int nblk,
+                 int accumulate) {
   pdl_wait();
   pdl_trigger();
-  __shared__ float sm[2][32][33];
-  const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + cl;
+  constexpr int CW = G == 1 ? 128 : 32;                  // columns of a CTA
+  __shared__ float sm[2][G][CW + 1];
+  const int cl = threadIdx.x % CW, g = threadIdx.x / CW;
+  const int c = blockIdx.x * CW + cl;
   float s = 0.f, t = 0.f;
   if (c < cols) {
-    for (int b0 = g; b0 < nblk; b0 += 32 * 8) {
+    for (int b0 = g; b0 < nblk; b0 += G * 8) {
       float u[8], w[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int b = b0 + 32 * k;
+        const int b = b0 + G * k;
         u[k] = b < nblk ? partial[(size_t)b * cols + c] : 0.f;
         w[k] = (partial2 && b < nblk) ? partial2[(size_t)b * cols + c] : 0.f;
       }
@@ -521,15 +524,27 @@ col_final_wide_kernel(const float* __restrict__ partial, float* __restrict__ out
       }
     }
   }
-  sm[0][g][cl] = s;
-  sm[1][g][cl] = t;
-  __syncthreads();
-  // warp g now owns column g of the 32; lane = group
-  const float a = warp_sum(sm[0][cl][g]), b2 = partial2 ? warp_sum(sm[1][cl][g]) : 0.f;
-  const int cc = blockIdx.x * 32 + g;
-  if (cl == 0 && cc < cols) {
-    out[cc] = accumulate ? out[cc] + a : a;
-    if (partial2) out2[cc] = accumulate ? out2[cc] + b2 : b2;
+  if constexpr (G > 1) {
+    sm[0][g][cl] = s;
+    sm[1][g][cl] = t;
+    __syncthreads();
+    if constexpr (G == 32) {
+      // warp g now owns column g of the 32; lane = group
+      s = warp_sum(sm[0][cl][g]);
+      t = partial2 ? warp_sum(sm[1][cl][g]) : 0.f;
+    } else if (g == 0) {
+      s = t = 0.f;
+#pragma unroll
+      for (int k = 0; k < G; ++k) {
+        s += sm[0][k][cl];
+        t += sm[1][k][cl];
+      }
+    }
+  }
+  const int cc = G == 32 ? blockIdx.x * 32 + g : c;
+  if ((G == 32 ? cl : g) == 0 && cc < cols) {
+    out[cc] = accumulate ? out[cc] + s : s;
+    if (partial2) out2[cc] = accumulate ? out2[cc] + t : t;
   }
 }
 
@@ -904,6 +919,19 @@ extern "C" int ftk_layernorm_bwd_blocks(int rows) {
   return fused > wide ? fused : wide;
 }
 
+// One group where a single round of loads covers the partials, 8 groups up to two rounds, and for outputs that are wide enough
+// to fill the chip with them; 32 groups for many partials of a narrow output.  Column sums in us, 32 / 8 / 1 groups:
+// 500 x 8192 (8 partials) 6.5 / 5.0 / 4.0; 1500 x 3072 (24) 5.8 / 4.1 / 4.9; 8192 x 768 (128) 5.3 / 4.7 / 10.6; 8192 x 16384 56 / 51 / 60;
+// 20000 x 768 (313) 7.8 / 8.2 / 23; LayerNorm backward 1500 x 3072 (296) 13.2 / 14.5 / 26, 1500 x 8192 30.9 / 29.2 / 45.
+static int col_final(const float* partial, float* out, const float* partial2, float* out2, int cols, int nblk,
+                     int accumulate, cudaStream_t s) {
+  if (nblk <= 8)
+    return launch_pdl(col_final_kernel<1>, (cols + 127) / 128, 128, 0, s, partial, out, partial2, out2, cols, nblk, accumulate);
+  if (nblk <= 128 || cols >= 8192)
+    return launch_pdl(col_final_kernel<8>, (cols + 31) / 32, 256, 0, s, partial, out, partial2, out2, cols, nblk, accumulate);
+  return launch_pdl(col_final_kernel<32>, (cols + 31) / 32, 1024, 0, s, partial, out, partial2, out2, cols, nblk, accumulate);
+}
+
 template <int NV, int WPR, bool RMS>
 static int norm_bwd_fused_launch(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd,
                                  const void* dx_add, void* dx, float* partial, int rows, int cols, int nblk, cudaStream_t s) {
@@ -970,8 +998,7 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
     dim3 g((cols / 2 + 31) / 32, nblk);
     launch_pdl(col_partial_kernel<RMS ? 1 : 0>, g, 256, 0, s, BF(dy), BF(x), mean, rstd, partial, rows, cols, cols, nblk);
   }
-  launch_pdl(col_final_wide_kernel, (cols + 31) / 32, 1024, 0, s, partial, dgamma, RMS ? nullptr : partial + (size_t)nblk * cols,
-                                                          dbeta, cols, nblk, accumulate);
+  col_final(partial, dgamma, RMS ? nullptr : partial + (size_t)nblk * cols, dbeta, cols, nblk, accumulate, s);
   return (int)cudaGetLastError();
 }
 extern "C" int ftk_layernorm_bwd(const void* dy, const void* x, const void* gamma,
@@ -1066,7 +1093,7 @@ extern "C" int ftk_colsum_bf16(const void* x, float* out, float* partial, int ro
     dim3 g((cols / 2 + 31) / 32, nblk);
     launch_pdl(col_partial_kernel<2>, g, 256, 0, s, BF(x), nullptr, nullptr, nullptr, partial, rows, cols, ld, nblk);
   }
-  launch_pdl(col_final_wide_kernel, (cols + 31) / 32, 1024, 0, s, partial, out, nullptr, nullptr, cols, nblk, accumulate);
+  col_final(partial, out, nullptr, nullptr, cols, nblk, accumulate, s);
   return (int)cudaGetLastError();
 }
 

@@ -57,3 +57,22 @@ def test_norm(cuda_device, rows, cols, rms):
     close(got, y.detach(), bf16)
     close(dx, refs[0], bf16)
     close(dg, refs[1], f32)
+
+
+@pytest.mark.parametrize("rows,cols", [
+    (1, 2), (64, 130), (512, 96), (513, 96),       # up to and beyond eight row blocks of 64: another number of groups
+    (1537, 4104), (8192, 40), (8193, 40),          # two rounds of loads, 128 and 129 blocks
+    (8200, 8184), (8200, 8192),                    # the width from which the wide form stays
+    (300, 34), (3000, 1026),                       # rows that are not whole 16-byte segments: blocks of 256 rows
+])
+def test_column_sums(cuda_device, rows, cols):
+    from frankentorch_b200.ops import kernels as K
+    x = torch.randn(rows, cols, generator=torch.Generator(device=cuda_device).manual_seed(rows), device=cuda_device).to(torch.bfloat16)
+    ref = x.double().sum(0)
+    bound = 2.0 ** -24 * (8 + rows ** 0.5) * x.double().abs().sum(0) + 1e-6     # rounding errors of random sign, fp32 sums
+    out = K.colsum(x)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    pre = torch.full((cols,), 2.0, device=cuda_device)
+    K.colsum(x, out=pre, accumulate=True)
+    assert torch.equal(pre, out + 2.0)
+    assert torch.equal(K.colsum(x), out)
