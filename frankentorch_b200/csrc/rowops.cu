@@ -55,13 +55,13 @@ constexpr int ROW_WARPS = 8;     // rows per CTA
 
 // ----------------------------------------------------------------------------- LayerNorm fwd
 // Rows of up to 256 NV columns: a warp owns a row and keeps it in registers, NV 16-byte vectors per lane; wider rows (up to
-// 8192 columns) are shared by the eight warps of a CTA.  The row, gamma and beta are all requested before the first
+// 16384 columns) are shared by the four or eight warps of a CTA.  The row, gamma and beta are all requested before the first
 // addition, so a row costs one memory latency; a warp that re-reads columns beyond its registers, as it did from 1024
 // columns on, pays three.  Sums run over a lane's vectors in ascending order, then over the lanes (and warps) in a fixed tree.
 // Memory bound: 8192 x 768 6.9 -> 5.3 us (25 MB), 8192 x 2048 14.6 -> 11.6 us, 1500 x 1280 5.6 -> 3.2 us; pairs of values per
 // instruction (f32x2) are a third of the first: the kernel was at two thirds of its issue slots.
 template <int NV, int WPR, bool RMS>
-__global__ void __launch_bounds__(WPR == 1 ? 128 : 256)
+__global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
                 __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
@@ -172,7 +172,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     }
 }
 
-// Rows of more than 8192 columns: one warp walks the row three times.
+// Rows of more than 16384 columns: the eight warps of a CTA walk the row three times.
 template <bool RMS>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
@@ -182,16 +182,25 @@ norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
                      float eps) {
   pdl_wait();
   pdl_trigger();
+  __shared__ float red[2][ROW_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * ROW_WARPS + warp;
-  if (row >= rows) return;
+  const int row = blockIdx.x;
+  auto row_sum = [&](float v, int slot) -> float {
+    v = warp_sum(v);
+    if (lane == 0) red[slot][warp] = v;
+    __syncthreads();
+    v = red[slot][0];
+#pragma unroll
+    for (int w = 1; w < ROW_WARPS; ++w) v += red[slot][w];
+    return v;
+  };
   const int nvec = cols >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * cols);
   const uint4* rr = resid ? reinterpret_cast<const uint4*>(resid + (size_t)row * cols) : nullptr;
   uint4* so = sum_out ? reinterpret_cast<uint4*>(sum_out + (size_t)row * cols) : nullptr;
   const uint4* src = rr ? reinterpret_cast<const uint4*>(so) : xr;
   float s = 0.f;
-  for (int v = lane; v < nvec; v += 32) {
+  for (int v = threadIdx.x; v < nvec; v += ROW_WARPS * 32) {
     float f[8];
     unpack8(xr[v], f);
     if (rr) {
@@ -206,14 +215,14 @@ norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += RMS ? f[i] * f[i] : f[i];
   }
-  s = warp_sum(s);
+  s = row_sum(s, 0);
   float mean = 0.f, rstd;
   if (RMS) {
     rstd = rsqrtf(s / cols + eps);
   } else {
     mean = s / cols;
     float q = 0.f;
-    for (int v = lane; v < nvec; v += 32) {
+    for (int v = threadIdx.x; v < nvec; v += ROW_WARPS * 32) {
       float f[8];
       unpack8(src[v], f);
 #pragma unroll
@@ -222,17 +231,17 @@ norm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
         q += d * d;
       }
     }
-    q = warp_sum(q);
+    q = row_sum(q, 1);
     rstd = rsqrtf(q / cols + eps);
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     if (mean_out) mean_out[row] = mean;
     rstd_out[row] = rstd;
   }
   const uint4* gv = reinterpret_cast<const uint4*>(gamma);
   const uint4* bv = beta ? reinterpret_cast<const uint4*>(beta) : nullptr;
   uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * cols);
-  for (int v = lane; v < nvec; v += 32) {
+  for (int v = threadIdx.x; v < nvec; v += ROW_WARPS * 32) {
     float f[8], g[8], b[8];
     unpack8(src[v], f);
     unpack8(__ldg(gv + v), g);
@@ -880,11 +889,14 @@ template <bool RMS>
 static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, const void* gamma, const void* beta, void* y,
                            float* mean, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
 #define FT_NORM_FWD(NV, WPR)                                                                                   \
-  launch_pdl(norm_fwd_kernel<NV, WPR, RMS>, WPR == 1 ? (rows + 3) / 4 : rows, WPR == 1 ? 128 : 256, 0, s,             \
+  launch_pdl(norm_fwd_kernel<NV, WPR, RMS>, WPR == 1 ? (rows + 3) / 4 : rows, WPR == 8 ? 256 : 128, 0, s,             \
       BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps)
   const int nvec = cols / 8, per_lane = (nvec + 31) / 32;
   // Up to 1536 columns a row is one warp's.  Wider rows take a CTA each, except where there are enough rows of up to 2048
-  // columns to fill the chip with warps (8192 x 2048: 11.6 against 16.4 us).
+  // columns to fill the chip with warps (8192 x 2048: 11.6 against 16.4 us).  2056 to 3072 columns are three vectors a lane of
+  // four warps, where eight warps leave a quarter of the lanes idle (8192 x 3072: 19.5 against 27.4 us, RMS 17.0 against 20.5;
+  // 500 x 3072 level, below that the wider CTA is quicker).  A row stays in registers up to 16384 columns: 8192 x 16384 107 us
+  // against 226 walked three times by a warp, 1 x 16384 4.4 against 30.
   if (per_lane <= 1) FT_NORM_FWD(1, 1);
   else if (per_lane <= 2) FT_NORM_FWD(2, 1);
   else if (per_lane <= 3) FT_NORM_FWD(3, 1);
@@ -892,10 +904,12 @@ static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, cons
   else if (per_lane <= 6) FT_NORM_FWD(6, 1);
   else if (per_lane <= 8 && rows >= 2048) FT_NORM_FWD(8, 1);
   else if (nvec <= 256) FT_NORM_FWD(1, 8);
+  else if (nvec <= 384 && rows >= 500) FT_NORM_FWD(3, 4);
   else if (nvec <= 512) FT_NORM_FWD(2, 8);
   else if (nvec <= 1024) FT_NORM_FWD(4, 8);
+  else if (nvec <= 2048) FT_NORM_FWD(8, 8);
   else
-    launch_pdl(norm_fwd_long_kernel<RMS>, (rows + ROW_WARPS - 1) / ROW_WARPS, ROW_WARPS * 32, 0, s,
+    launch_pdl(norm_fwd_long_kernel<RMS>, rows, ROW_WARPS * 32, 0, s,
         BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps);
 #undef FT_NORM_FWD
   return (int)cudaGetLastError();

@@ -5,7 +5,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-COLS = [8, 256, 264, 512, 768, 776, 1024, 1536, 1544, 2048, 3072, 3080, 4096, 4104, 6144, 6152, 8192, 8200]
+COLS = [8, 256, 264, 512, 768, 776, 1024, 1536, 1544, 2048, 3072, 3080, 4096, 4104, 6144, 6152, 8192, 8200,
+        16384, 16392, 20008]
 
 
 def _norm(x, g, b, rms, eps):
