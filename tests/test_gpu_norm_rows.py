@@ -18,10 +18,10 @@ def _norm(x, g, b, rms, eps):
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("rows", [1, 7, 700, 5003])
 @pytest.mark.parametrize("cols", COLS)
-def test_norm(cuda_device, rows, cols, rms):
+def test_norm(cuda_device, rows, cols, rms, most=12_000_000):
     from frankentorch_b200.ops import kernels as K
-    if rows * cols > 12_000_000:
-        rows = 12_000_000 // cols
+    if rows * cols > most:
+        rows = most // cols
     gen = torch.Generator(device=cuda_device).manual_seed(cols + rows)
     rnd = lambda *s, sc=1.0, m=0.0: (torch.randn(*s, generator=gen, device=cuda_device) * sc + m).to(torch.bfloat16)   # noqa: E731
     x, dy, add = rnd(rows, cols, sc=2.0, m=0.3), rnd(rows, cols), rnd(rows, cols)
@@ -58,6 +58,13 @@ def test_norm(cuda_device, rows, cols, rms):
     close(got, y.detach(), bf16)
     close(dx, refs[0], bf16)
     close(dg, refs[1], f32)
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,cols", [(23999, 64), (24000, 64), (24000, 128), (24000, 136), (24000, 256), (24000, 264), (131073, 256)])
+def test_norm_of_many_narrow_rows(cuda_device, rows, cols, rms):
+    """Both sides of the rule that takes many narrow rows through separate passes."""
+    test_norm(cuda_device, rows, cols, rms, most=1 << 26)
 
 
 @pytest.mark.parametrize("rows,cols", [
