@@ -345,6 +345,10 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     const double bytes = mn * 4.0 * s + mn * (g->out_fp32 ? 4.0 : 2.0) * (g->accumulate ? 2.0 : 1.0);
     return bytes / 4.0e6 + 3.0;
   };
+  // Operands given [K, rows] whose rows are not whole 128-byte lines: every 128-byte row of a box straddles two lines, and a
+  // k-block takes ~1.35 times as long per such operand, however few SMs are busy (both operands, us per k-block: 2136 x 632
+  // 0.36 on 256 x 128 pairs against 0.20 for 2048 x 640; 200 x 200 on two tiles 0.34).
+  const double lines = (g->a_mn && g->lda % 64 ? 1.35 : 1.0) * (g->b_mn && g->ldb % 64 ? 1.35 : 1.0);
   auto cost = [&](int bn, int s) {
     const bool pair = bn > 256;
     const int w = pair ? bn - 256 : bn;
@@ -358,7 +362,7 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     // the last tile's epilogue and a pair's hand-shakes are not hidden: 128 x 192 x 64 takes 4.1 / 4.7 / 4.8 us on one
     // SM and 4.6 / 5.1 / 5.3 us on a pair
     const double exposed = (w == 256 ? 0.75 : (w == 192 ? 0.55 : 0.0)) + (pair ? 0.5 : 0.0);
-    return ((double)waves * (tile + (double)kblocks / s * (mma + (full - mma) * busy)) + exposed) *
+    return ((double)waves * (tile + (double)kblocks / s * (mma + (full - mma) * busy) * lines) + exposed) *
                (pair ? pair_cost_scale() : 1.0) + split_penalty(s);
   };
   auto split_ok = [&](int s) {
