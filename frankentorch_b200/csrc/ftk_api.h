@@ -73,6 +73,7 @@ int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits);
 // epilogue, as one persistent launch of 128 x 192 tiles: the weight gradients of a transformer block fill the
 // GPU together where each alone would need split-K and a reduction kernel.
 int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream);
+int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n);      // the CTAs it takes (<= max_ctas).  No launch.
 
 // ---- GEMM fused with a collective over NVLink peer memory --------------------------------
 // One kernel: `comm_ctas` CTAs move shards / reduce partials while the rest run the GEMM.

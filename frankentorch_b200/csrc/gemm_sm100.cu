@@ -411,6 +411,13 @@ static int launch_group(const GroupMaps& maps, const GroupArgs& ga, int pairs, c
   return (int)cudaGetLastError();
 }
 
+// CTAs for `total` pair tiles of a group: whole pairs, or one CTA where no pair is allowed.
+static int group_ctas(const FtkGemmDesc& g0, int total) {
+  const int sms = g0.max_ctas > 0 ? g0.max_ctas : num_sms();
+  const int pairs = total < sms / 2 ? total : sms / 2;
+  return pairs > 0 ? 2 * pairs : 1;
+}
+
 // Grouped launch: `n` (1..8) independent products with the same K and operand layouts, fp32 outputs with a plain
 // store or accumulate epilogue, in one persistent kernel of 256 x 192 pair tiles (see gemm_group_kernel.cuh).
 extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream_v) {
@@ -445,13 +452,31 @@ extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream
     ga.tile_end[p] = total;
   }
   for (int p = n; p < GG_MAX; ++p) ga.tile_end[p] = total;
+  const int ctas = group_ctas(g0, total);
+  if (ctas < 2) {
+    // one CTA is all the caller allows: the products in turn, same k order, so the same bits
+    for (int p = 0; p < n; ++p) {
+      FtkGemmDesc one = descs[p];
+      one.force_bn = GG_BN;
+      one.split_k = 1;
+      one.max_ctas = 1;
+      const int rc = ftk_gemm_bf16(&one, stream_v);
+      if (rc) return rc;
+    }
+    return 0;
+  }
   bool aligned = true;
   for (int p = 0; p < n; ++p)
     aligned = aligned && ga.N[p] % 4 == 0 && ga.ldd[p] % 4 == 0 && (reinterpret_cast<uintptr_t>(ga.D[p]) & 15) == 0;
-  const int sms = g0.max_ctas > 0 ? g0.max_ctas : num_sms();
-  int pairs = sms / 2 > 0 ? sms / 2 : 1;
-  if (total < pairs) pairs = total;
-  return aligned ? launch_group<EPI_KIND_F32>(maps, ga, pairs, stream) : launch_group<EPI_KIND_ANY>(maps, ga, pairs, stream);
+  return aligned ? launch_group<EPI_KIND_F32>(maps, ga, ctas / 2, stream) : launch_group<EPI_KIND_ANY>(maps, ga, ctas / 2, stream);
+}
+
+// CTAs that the grouped launch takes: never more than max_ctas.  Launches nothing.
+extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
+  if (!descs || n < 1 || n > GG_MAX) return -2;
+  int total = 0;
+  for (int p = 0; p < n; ++p) total += ((descs[p].M + 2 * G_BM - 1) / (2 * G_BM)) * ((descs[p].N + GG_BN - 1) / GG_BN);
+  return group_ctas(descs[0], total);
 }
 
 // Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile

@@ -29,3 +29,29 @@ def test_rows_off_the_lines_are_charged():
     assert _plan(2176, 640, 8192, a_mn=1, b_mn=1, f32=1)[2] == 1
     # the charge is for operands given [K, rows] alone
     assert _plan(2136, 632, 2000)[1:] == _plan(2136, 632, 2048)[1:]
+
+
+@pytest.mark.parametrize("max_ctas", [1, 2, 3, 36, 37, 148])
+@pytest.mark.parametrize("shapes", [[(64, 64)], [(2304, 768), (768, 768), (3072, 768), (768, 3072)]])
+def test_a_group_keeps_to_its_ctas(shapes, max_ctas):
+    fn = _lib.load().ftk_gemm_group_ctas
+    fn.argtypes, fn.restype = [C.POINTER(_lib.FtkGemmDesc), C.c_int], C.c_int
+    arr = (_lib.FtkGemmDesc * len(shapes))(*[_desc(m, n, 512, a_mn=1, b_mn=1, f32=1, max_ctas=max_ctas) for m, n in shapes])
+    ctas = fn(arr, len(shapes))
+    assert 1 <= ctas <= max_ctas and (ctas == 1) == (max_ctas == 1)
+
+
+@pytest.mark.gpu
+def test_a_group_on_one_cta(cuda_device):
+    import torch
+    from frankentorch_b200.ops import kernels as K
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda_device).to(torch.bfloat16)      # noqa: E731
+    probs = [(rnd(264, m), rnd(264, n)) for m, n in ((264, 200), (16, 8), (520, 40))]
+    outs = []
+    for max_ctas in (0, 1):
+        o = [torch.full((a.shape[1], b.shape[1]), 0.25, device=cuda_device) for a, b in probs]
+        K.gemm_grouped([(a, b, t, True) for (a, b), t in zip(probs, o)], max_ctas=max_ctas)
+        outs.append(o)
+    K.check_status()
+    assert all(torch.equal(x, y) for x, y in zip(*outs))
