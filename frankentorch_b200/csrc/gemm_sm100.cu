@@ -391,6 +391,8 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   }
   if (g->split_k > 1 && split_ok(g->split_k)) splits = g->split_k;
   if (bn != 128 && bn != 192 && bn != 256 && bn != 384 && bn != 448 && bn != 512) return -5;
+  // a forced pair tile needs two CTAs (without them nothing would run), and pair tiles know no rows that are not in use
+  if (bn > 256 && (sms < 2 || g->seg_counts)) return -5;
   *bn_out = bn;
   *splits_out = splits;
   return 0;

@@ -31,6 +31,17 @@ def test_rows_off_the_lines_are_charged():
     assert _plan(2136, 632, 2000)[1:] == _plan(2136, 632, 2048)[1:]
 
 
+@pytest.mark.parametrize("bn", [384, 448, 512])
+def test_a_pair_tile_that_cannot_run_is_refused(bn):
+    assert _plan(256, 256, 64, force_bn=bn)[:2] == (0, bn)
+    assert _plan(256, 256, 64, force_bn=bn, max_ctas=2)[:2] == (0, bn)
+    assert _plan(256, 256, 64, force_bn=bn, max_ctas=1)[0] == -5
+    g = _desc(256, 256, 64, force_bn=bn)
+    g.seg_counts, g.seg_rows = 256, 128
+    out = C.c_int(0), C.c_int(1)
+    assert _lib.load().ftk_gemm_plan(C.byref(g), C.byref(out[0]), C.byref(out[1])) == -5
+
+
 @pytest.mark.parametrize("max_ctas", [1, 2, 3, 36, 37, 148])
 @pytest.mark.parametrize("shapes", [[(64, 64)], [(2304, 768), (768, 768), (3072, 768), (768, 3072)]])
 def test_a_group_keeps_to_its_ctas(shapes, max_ctas):
