@@ -159,7 +159,7 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __r
                      const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out, int S,
                      int d, long long vocab, int* status) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work(d * (wpe ? 6 : 4));
   const int r = blockIdx.x;
   long long id = ids[r];
   // a token id outside the table: reported through the status word, row 0 is read instead

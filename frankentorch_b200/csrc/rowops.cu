@@ -68,7 +68,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                 float eps) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work((WPR == 1 ? 4 : 1) * cols * 4);
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = WPR == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
@@ -263,7 +263,7 @@ norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dx_add,
                    __nv_bfloat16* __restrict__ dx, int rows, int cols) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work(ROW_WARPS * cols * 6);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * ROW_WARPS + warp;
   if (row >= rows) return;
