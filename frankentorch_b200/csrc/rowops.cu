@@ -981,10 +981,11 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
   // Tens of thousands of rows of a vector per lane or less: a warp per row in lock step with its CTA spends 1.4 us on a step of
   // eight, most of it latency, where the separate passes have all their warps in flight and find the rows in L2 again.  In us,
   // one pass / three kernels: RMS 8192 x 64 7.3 / 9.7, 30000 x 64 17.1 / 15.9, 65536 x 64 39.5 / 25.6, 65536 x 256 41.5 / 38.9,
-  // 65536 x 384 48 / 79, 200000 x 128 115 / 101, 200000 x 256 116 / 129; LayerNorm 30000 x 64 19.4 / 19.8, 65536 x 64 45 / 32.
+  // 65536 x 384 48 / 79, 200000 x 128 115 / 101, 200000 x 256 116 / 129; LayerNorm 30000 x 64 19.4 / 19.8, 65536 x 64 45 / 32,
+  // 65536 x 256 48 / 51 and with an added gradient 45 / 57, so 256 columns are for RMSNorm only.
   // (Row blocks ride on grid.y there.)
   const bool narrow = rows >= 24000 && norm_col_blocks(rows) <= 65535 &&
-                      (nvec <= 16 || (nvec <= 32 && (long long)rows * cols <= 32ll << 20));
+                      (nvec <= 16 || (RMS && nvec <= 32 && (long long)rows * cols <= 32ll << 20));
   if (dgamma && nvec <= 1024 && !narrow) {
     // One pass.  WPR warps per row so that a lane holds at most three vectors (four at the widest) and its column sums stay
     // in registers.
