@@ -60,8 +60,10 @@ constexpr int ROW_WARPS = 8;     // rows per CTA
 // columns on, pays three.  Sums run over a lane's vectors in ascending order, then over the lanes (and warps) in a fixed tree.
 // Memory bound: 8192 x 768 6.9 -> 5.3 us (25 MB), 8192 x 2048 14.6 -> 11.6 us, 1500 x 1280 5.6 -> 3.2 us; pairs of values per
 // instruction (f32x2) are a third of the first: the kernel was at two thirds of its issue slots.
-template <int NV, int WPR, bool RMS>
-__global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
+// LEAN: gamma and beta are read at the end, which leaves registers for 32 warps per SM instead of 20.  Only four vectors per
+// lane and many rows gain: 65536 x 1024 51.4 -> 43.4 us (RMS 46.7 -> 40.7), 4096 x 1024 4.6 -> 3.9, but 500 x 1024 2.2 -> 2.8.
+template <int NV, int WPR, bool RMS, bool LEAN = false>
+__global__ void __launch_bounds__(WPR == 8 ? 256 : 128, LEAN ? 8 : 1)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
                 __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
@@ -80,7 +82,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   const uint4* rr = resid ? reinterpret_cast<const uint4*>(resid + (size_t)row * cols) : nullptr;
   const uint4* gv = reinterpret_cast<const uint4*>(gamma);
   const uint4* bv = reinterpret_cast<const uint4*>(beta);
-  constexpr bool PRE = NV <= 6;      // more vectors than that: gamma and beta come from L1 at the end, for the registers' sake
+  constexpr bool PRE = NV <= 6 && !LEAN;      // more vectors than that: gamma and beta come from L1 at the end, for the registers' sake
   uint4 xc[NV], rc[NV], gc[PRE ? NV : 1], bc[PRE ? NV : 1];
 #pragma unroll
   for (int c = 0; c < NV; ++c) {
@@ -888,21 +890,24 @@ using namespace ftk;
 template <bool RMS>
 static int norm_fwd_launch(const void* x, const void* resid, void* sum_out, const void* gamma, const void* beta, void* y,
                            float* mean, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
-#define FT_NORM_FWD(NV, WPR)                                                                                   \
-  launch_pdl(norm_fwd_kernel<NV, WPR, RMS>, WPR == 1 ? (rows + 3) / 4 : rows, WPR == 8 ? 256 : 128, 0, s,             \
+#define FT_NORM_FWD(NV, WPR, ...)                                                                              \
+  launch_pdl(norm_fwd_kernel<NV, WPR, RMS, ##__VA_ARGS__>, WPR == 1 ? (rows + 3) / 4 : rows, WPR == 8 ? 256 : 128, 0, s,             \
       BF(x), BF(resid), BFW(sum_out), BF(gamma), BF(beta), BFW(y), mean, rstd, rows, cols, eps)
   const int nvec = cols / 8, per_lane = (nvec + 31) / 32;
   // Up to 1536 columns a row is one warp's.  Wider rows take a CTA each, except where there are enough rows of up to 2048
-  // columns to fill the chip with warps (8192 x 2048: 11.6 against 16.4 us).  2056 to 3072 columns are three vectors a lane of
+  // columns to fill the chip with warps (one / four / eight warps per row, RMS: 30000 x 2048 38.5 / 42.5 / - us, 8192 x 2048 9.9 / 10.1 /
+  // -, 4096 x 2048 7.3 / 5.8 / -, 1500 x 2048 - / 3.3 / 3.6, 64 x 2048 - / 1.7 / 1.8).  2056 to 3072 columns are three vectors a lane of
   // four warps, where eight warps leave a quarter of the lanes idle (8192 x 3072: 19.5 against 27.4 us, RMS 17.0 against 20.5;
   // 500 x 3072 level, below that the wider CTA is quicker).  A row stays in registers up to 16384 columns: 8192 x 16384 107 us
   // against 226 walked three times by a warp, 1 x 16384 4.4 against 30.
   if (per_lane <= 1) FT_NORM_FWD(1, 1);
   else if (per_lane <= 2) FT_NORM_FWD(2, 1);
   else if (per_lane <= 3) FT_NORM_FWD(3, 1);
+  else if (per_lane <= 4 && rows >= 4096) FT_NORM_FWD(4, 1, true);
   else if (per_lane <= 4) FT_NORM_FWD(4, 1);
   else if (per_lane <= 6) FT_NORM_FWD(6, 1);
-  else if (per_lane <= 8 && rows >= 2048) FT_NORM_FWD(8, 1);
+  else if (per_lane <= 8 && rows >= 8192) FT_NORM_FWD(8, 1);
+  else if (per_lane <= 8 && rows >= 500) FT_NORM_FWD(2, 4);
   else if (nvec <= 256) FT_NORM_FWD(1, 8);
   else if (nvec <= 384 && rows >= 500) FT_NORM_FWD(3, 4);
   else if (nvec <= 512) FT_NORM_FWD(2, 8);

@@ -61,9 +61,12 @@ def test_norm(cuda_device, rows, cols, rms, most=12_000_000):
 
 
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("rows,cols", [(23999, 64), (24000, 64), (24000, 128), (24000, 136), (24000, 256), (24000, 264), (131073, 256)])
-def test_norm_of_many_narrow_rows(cuda_device, rows, cols, rms):
-    """Both sides of the rule that takes many narrow rows through separate passes."""
+@pytest.mark.parametrize("rows,cols", [
+    (23999, 64), (24000, 64), (24000, 128), (24000, 136), (24000, 256), (24000, 264), (131073, 256),     # separate backward passes
+    (4095, 1024), (4096, 1024), (499, 1544), (500, 1544), (8191, 2048), (8192, 2048),                   # warps per row, forward
+])
+def test_norm_where_the_number_of_rows_decides(cuda_device, rows, cols, rms):
+    """Both sides of the rules that look at the number of rows."""
     test_norm(cuda_device, rows, cols, rms, most=1 << 26)
 
 
