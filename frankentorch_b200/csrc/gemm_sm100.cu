@@ -345,10 +345,11 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     const double bytes = mn * 4.0 * s + mn * (g->out_fp32 ? 4.0 : 2.0) * (g->accumulate ? 2.0 : 1.0);
     return bytes / 4.0e6 + 3.0;
   };
-  // Operands given [K, rows] whose rows are not whole 128-byte lines: every 128-byte row of a box straddles two lines, and a
-  // k-block takes ~1.35 times as long per such operand, however few SMs are busy (both operands, us per k-block: 2136 x 632
-  // 0.36 on 256 x 128 pairs against 0.20 for 2048 x 640; 200 x 200 on two tiles 0.34).
-  const double lines = (g->a_mn && g->lda % 64 ? 1.35 : 1.0) * (g->b_mn && g->ldb % 64 ? 1.35 : 1.0);
+  // An operand whose rows are not whole 128-byte lines: every 128-byte row of a box straddles two lines, which the wide pair
+  // tiles, with the fewest rows per MMA, feel least.  us per k-block with no, one and both operands off: 1500 x 1000 x 5000, B
+  // [K, N], on 256 x 128 pairs 0.22 / 0.28 / 0.38; 8192 x 768 x 3000 on 256 x 256 pairs 0.33 and 0.43 with both, on 128 x 192
+  // 0.31 and 0.58; weight gradients of 2048 x 640 and 2136 x 632 on 256 x 128 pairs 0.20 and 0.36.
+  const int off_lines = (g->lda % 64 != 0 ? 1 : 0) + (g->ldb % 64 != 0 ? 1 : 0);
   auto cost = [&](int bn, int s) {
     const bool pair = bn > 256;
     const int w = pair ? bn - 256 : bn;
@@ -361,6 +362,7 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     const double busy = items < units ? (double)items / (double)units : 1.0;
     // the last tile's epilogue and a pair's hand-shakes are not hidden: 128 x 192 x 64 takes 4.1 / 4.7 / 4.8 us on one
     // SM and 4.6 / 5.1 / 5.3 us on a pair
+    const double off = bn > 256 ? (w == 256 ? 1.2 : 1.3) : 1.35, lines = off_lines == 0 ? 1.0 : (off_lines == 1 ? off : off * off);
     const double exposed = (w == 256 ? 0.75 : (w == 192 ? 0.55 : 0.0)) + (pair ? 0.5 : 0.0);
     return ((double)waves * (tile + (double)kblocks / s * (mma + (full - mma) * busy) * lines) + exposed) *
                (pair ? pair_cost_scale() : 1.0) + split_penalty(s);
