@@ -62,8 +62,10 @@ constexpr int ROW_WARPS = 8;     // rows per CTA
 // instruction (f32x2) are a third of the first: the kernel was at two thirds of its issue slots.
 // LEAN: gamma and beta are read at the end, which leaves registers for 32 warps per SM instead of 20.  Only four vectors per
 // lane and many rows gain: 65536 x 1024 51.4 -> 43.4 us (RMS 46.7 -> 40.7), 4096 x 1024 4.6 -> 3.9, but 500 x 1024 2.2 -> 2.8.
+// (No bound, 0, for the others: a bound of one block lets the compiler take 130 registers for six vectors, and 8192 x 1536
+// goes from 9.5 to 10.5 us.)
 template <int NV, int WPR, bool RMS, bool LEAN = false>
-__global__ void __launch_bounds__(WPR == 8 ? 256 : 128, LEAN ? 8 : 1)
+__global__ void __launch_bounds__(WPR == 8 ? 256 : 128, LEAN ? 8 : 0)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ resid,
                 __nv_bfloat16* __restrict__ sum_out, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
