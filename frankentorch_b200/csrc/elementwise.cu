@@ -187,7 +187,7 @@ embedding_bwd_wte_kernel(const long long* __restrict__ sorted_ids, const int* __
                          int rows, const __nv_bfloat16* __restrict__ dout,
                          float* __restrict__ dwte, int d, long long vocab, int* status) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work(0);      // most CTAs leave at once: their token occurred before
   const int b = blockIdx.x;
   const long long id = sorted_ids[b];
   if (b > 0 && sorted_ids[b - 1] == id) return;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128)
 embedding_bwd_wte_scan_kernel(const long long* __restrict__ ids, int rows, const __nv_bfloat16* __restrict__ dout,
                               float* __restrict__ dwte, int d, long long vocab, int* status) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work(0);      // most CTAs leave at once: their token occurred before
   constexpr int BLK = 1024;                               // positions looked at per vote: 8 loads in flight per thread
   __shared__ unsigned char match[BLK];
   __shared__ unsigned short list[BLK];
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(128)
 embedding_bwd_wpe_kernel(const __nv_bfloat16* __restrict__ dout, float* __restrict__ dwpe, int rows,
                          int S, int d) {
   pdl_wait();
-  pdl_trigger();
+  pdl_trigger_work(d * (2 * (rows / S) + 8));
   const int s = blockIdx.x;
   for (int c = threadIdx.x * 2; c < d; c += blockDim.x * 2) {
     float s0 = 0.f, s1 = 0.f;
