@@ -72,7 +72,10 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols,
                 float eps) {
   pdl_wait();
-  pdl_trigger_work((WPR == 1 ? 4 : 1) * cols * 4);
+  if constexpr (WPR == 1)
+    pdl_trigger_work(4 * cols * 4);
+  else
+    pdl_trigger();       // 6 KB and more (and RMSNorm of two vectors a lane keeps its 48 registers)
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = WPR == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
