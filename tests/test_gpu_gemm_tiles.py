@@ -1,5 +1,6 @@
 """Every tile width of the GEMM (single CTA 128 / 192 / 256, CTA pair 256 x 128 / 192 / 256) with every epilogue
-instantiation, at the edges of its tiles, and the row-by-row path of outputs without aligned 16-byte segments."""
+instantiation at the edges of its tiles, with both operands given [K, rows], with split reductions (also such that leave the
+last split empty), and the general path of outputs without aligned 16-byte segments."""
 import pytest
 import torch
 
@@ -44,8 +45,6 @@ def _close(out, ref, act=False):
 def test_tiles_and_epilogues(cuda_device, bn, M, N, K, kind):
     from frankentorch_b200.ops import kernels as k
     b_mn = kind in ("dgelu", "plain")            # the layouts that training uses: dgrad reads the weight as [K, N]
-    if b_mn and N % 8:
-        pytest.skip("an MN-major operand has rows of whole 16-byte segments")
     a, w = _rand((M, K), 1, cuda_device), _rand((K, N) if b_mn else (N, K), 2, cuda_device, K ** -0.5)
     bias, r = _rand((N,), 3, cuda_device), _rand((M, N), 4, cuda_device)
     ref = a.double() @ (w.double() if b_mn else w.double().t())
@@ -75,6 +74,50 @@ def test_tiles_and_epilogues(cuda_device, bn, M, N, K, kind):
     _close(out, ref, act="gelu" in kind)
     if aux is not None:
         _close(aux, pre)
+
+
+@pytest.mark.parametrize("bn", WIDTHS)
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (264, 200, 136), (384, 584, 1096), (520, 264, 72)])
+def test_weight_gradient_form(cuda_device, bn, M, N, K, accumulate):
+    """Both operands [K, rows], fp32 output: what a weight gradient runs."""
+    from frankentorch_b200.ops import kernels as k
+    a, b = _rand((K, M), 11, cuda_device), _rand((K, N), 12, cuda_device, K ** -0.5)
+    ref = a.double().t() @ b.double()
+    out = torch.full((M, N), 0.5 if accumulate else float("nan"), device=cuda_device)
+    k.gemm(a, b, a_mn=True, b_mn=True, out=out, accumulate=accumulate, force_bn=bn, split_k=1)
+    k.check_status()
+    _close(out, ref + 0.5 if accumulate else ref)
+
+
+@pytest.mark.parametrize("bn", WIDTHS)
+@pytest.mark.parametrize("form", ["nt", "tn", "bf16_acc"])
+@pytest.mark.parametrize("splits,K", [
+    (2, 1024),            # the shortest that may be split: eight k-blocks each
+    (3, 1600),            # 25 k-blocks: 9, 9 and 7
+    (12, 6200),           # 97 k-blocks, nine each: the twelfth split has none
+])
+def test_split_reductions(cuda_device, bn, form, splits, K):
+    from frankentorch_b200.ops import kernels as k
+    M, N = 264, 200
+    mn = form == "tn"
+    a, b = _rand((K, M) if mn else (M, K), 13, cuda_device), _rand((K, N) if mn else (N, K), 14, cuda_device, K ** -0.5)
+    ref = a.double().t() @ b.double() if mn else a.double() @ b.double().t()
+    out = torch.full((M, N), 0.25, dtype=torch.bfloat16 if form == "bf16_acc" else torch.float32, device=cuda_device)
+    kw = dict(a_mn=mn, b_mn=mn, force_bn=bn, split_k=splits)
+    k.trace_begin()
+    k.gemm(a, b, out=out, accumulate=form != "nt", **kw)
+    name, = k.trace_end()
+    assert name.endswith("splitK=%d>" % splits)
+    k.check_status()
+    if form != "nt":
+        ref = ref + 0.25
+    # as _close, with fp32 sums of K products (6200 * 2^-24 at most) and the bf16 output's rounding
+    bound = (2.0 ** -8 if out.dtype == torch.bfloat16 else 2.0 ** -20) * ref.abs() + 4e-4
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    again = torch.full_like(out, 0.25)
+    k.gemm(a, b, out=again, accumulate=form != "nt", **kw)
+    assert torch.equal(again, out)
 
 
 @pytest.mark.parametrize("bn", WIDTHS)
