@@ -10,7 +10,8 @@
 //
 // Two kernels, each 19 warps: warps 0-15 do the elementwise math, warp 16 is the TMA
 // producer, warp 17 issues the score products (and owns TMEM), warp 18 the accumulating
-// products.  The 16 math warps split every 128 x 128 score tile by columns (four groups of 32
+// products - but for dK / dV with head_dim 128, where the four products of a block follow one another and warp 17 issues
+// them all.  The 16 math warps split every 128 x 128 score tile by columns (four groups of 32
 // columns; a thread owns one tile row inside its group's columns), so one tcgen05.ld per
 // operand brings a thread's whole share into registers, the TMEM score tiles are released at
 // once and the tensor core computes the next block's scores under the exponentials of this
@@ -29,7 +30,7 @@ constexpr int BW_THREADS = 608;
 constexpr int BW_MATH = 16;         // one arrival per math warp on the math barriers
 constexpr int BW_WARP_TMA = 16;
 constexpr int BW_WARP_MMA = 17;      // issues the score products, owns TMEM
-constexpr int BW_WARP_MMA2 = 18;     // issues the accumulating products
+constexpr int BW_WARP_MMA2 = 18;     // issues the accumulating products (idle in dK / dV with head_dim 128)
 
 // Store 32 packed-bf16 columns (16 words) of one tile row into the swizzled K-major tile.
 __device__ __forceinline__ void store_row32_packed(uint8_t* tile, int row, int col0,

@@ -196,8 +196,8 @@ static int launch_gemm_kind(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm
 }
 
 // CTA-pair kernel: grid = 2 CTAs per cluster, at most sms / 2 clusters.
-// Weight of the pair tiles in the tile-choice model, 0.92 = as measured; the environment variable FT_GEMM_PAIR_COST
-// overrides it (a large value disables the pair kernel).
+// Weight of the pair tiles in the tile-choice model: 1, the model's times are measured ones.  The environment variable
+// FT_GEMM_PAIR_COST changes it to its value / 0.92 (0.92 is neutral; a large value rules the pair kernel out).
 static double pair_cost_scale() {
   static double c = -1.0;
   if (c < 0.0) {
@@ -313,7 +313,7 @@ extern "C" int ftk_tick_i32(int* word, void* stream_v) {
 }
 
 // Argument checks and tile choice shared by the launcher and the plan query.  Returns 0 and
-// (bn, splits), or a negative argument error.  bn == 512 stands for the CTA-pair kernel.
+// (bn, splits), or a negative argument error.  bn > 256 stands for the CTA-pair kernel with 256 x (bn - 256) tiles.
 static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   if (!g || g->M <= 0 || g->N <= 0 || g->K <= 0) return -2;
   const int L0 = g->L0 > 0 ? g->L0 : 1, L1 = g->L1 > 0 ? g->L1 : 1;
@@ -483,8 +483,8 @@ extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
   return group_ctas(descs[0], total);
 }
 
-// Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile
-// 128 x bn) or 512 (CTA-pair kernel, 256 x 256 tiles); *splits = split-K factor.  Launches nothing.
+// Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile 128 x bn) or
+// 384 / 448 / 512 (CTA-pair kernel, tiles of 256 x 128 / 192 / 256); *splits = split-K factor.  Launches nothing.
 extern "C" int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits) {
   if (!bn || !splits) return -2;
   return plan_gemm(g, bn, splits);

@@ -58,7 +58,7 @@ constexpr int ROW_WARPS = 8;     // rows per CTA
 // 16384 columns) are shared by the four or eight warps of a CTA.  The row, gamma and beta are all requested before the first
 // addition, so a row costs one memory latency; a warp that re-reads columns beyond its registers, as it did from 1024
 // columns on, pays three.  Sums run over a lane's vectors in ascending order, then over the lanes (and warps) in a fixed tree.
-// Memory bound: 8192 x 768 6.9 -> 5.3 us (25 MB), 8192 x 2048 14.6 -> 11.6 us, 1500 x 1280 5.6 -> 3.2 us; pairs of values per
+// Memory bound (captured loop, L2 warm): 8192 x 768 6.9 -> 5.3 us (25 MB), 8192 x 2048 14.6 -> 11.6, 1500 x 1280 5.6 -> 3.3; pairs of values per
 // instruction (f32x2) are a third of the first: the kernel was at two thirds of its issue slots.
 // LEAN: gamma and beta are read at the end, which leaves registers for 32 warps per SM instead of 20.  Only four vectors per
 // lane and many rows gain: 65536 x 1024 51.4 -> 43.4 us (RMS 46.7 -> 40.7), 4096 x 1024 4.6 -> 3.9, but 500 x 1024 2.2 -> 2.8.

@@ -93,8 +93,8 @@ class WgradQueue:
     """Weight gradients of consecutive backward rules, collected and launched together.
 
     A weight gradient ``dW = dy^T x`` of a transformer block has 24 - 96 output tiles: alone it needs split-K
-    and a reduction kernel to occupy 148 SMs.  The four of a block together are two full waves of 128 x 192
-    tiles (``K.gemm_grouped``), each output element reduced over the tokens by one CTA in order.  A rule hands
+    and a reduction kernel to occupy 148 SMs.  The four of a block together are two full waves of 256 x 192 tiles
+    on 74 CTA pairs (``K.gemm_grouped``), each output element reduced over the tokens by one pair in order.  A rule hands
     its weight gradient to the queue instead of launching it; the queue launches when it holds enough tiles
     (or eight problems) and when the backward pass ends (``TensorTape.backward`` calls :meth:`flush`).  The
     operands stay referenced until then; nothing in a backward pass writes them in place.  The observer of
@@ -103,7 +103,8 @@ class WgradQueue:
     ``FT_WGRAD_GROUP=0`` turns the queue off."""
 
     enabled = os.environ.get("FT_WGRAD_GROUP", "1") != "0"
-    FLUSH_TILES = 266          # ~0.9 x two waves of 148
+    # counted in halves of a pair tile, 128 x 192: ~0.9 x two waves of 148
+    FLUSH_TILES = 266
     MAX_TILES_PER_PROBLEM = 200
 
     def __init__(self, tape: TensorTape):

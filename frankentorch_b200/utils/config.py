@@ -36,7 +36,7 @@ ENV_FLAGS: Dict[str, EnvFlag] = {f.name: f for f in (
     EnvFlag("FT_NO_AUTOBUILD", False, _bool,
             "do not compile the kernel library on first use; raise if it is missing"),
     EnvFlag("FT_GEMM_PAIR_COST", 0.92, float,
-            "relative cost of a 256x256 CTA-pair GEMM tile against two 128x256 tiles in the tile model"),
+            "weight of the CTA-pair GEMM tiles (256 x 128 / 192 / 256) in the tile model; 0.92 = as measured"),
     EnvFlag("FT_NVTX", False, _bool, "emit an NVTX range per tape node and per engine phase"),
     EnvFlag("FT_DP_IMPL", "fused", str, "data-parallel gradient path: fused (peer memory) or nccl"),
     EnvFlag("FT_COMM_CTAS", 20, int, "copy CTAs of the gather-fused GEMMs"),
