@@ -156,6 +156,14 @@ struct PairCta {
   }
 };
 
+// Tile t of a product: groups of by_gm.d m tiles, within a group m fastest, then n (the host's set_pair_groups has the reason).
+__device__ __forceinline__ void pair_tile(const GemmArgs& p, int t, int tiles_m2, int& m_t, int& n_t) {
+  const int g = p.by_group.div(t), r = t - g * (int)p.by_group.d, m0 = g * (int)p.by_gm.d;
+  const bool full = m0 + (int)p.by_gm.d <= tiles_m2;
+  n_t = full ? p.by_gm.div(r) : p.by_gm_last.div(r);
+  m_t = m0 + r - n_t * (int)(full ? p.by_gm.d : p.by_gm_last.d);
+}
+
 template <int BN, int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
 gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -194,8 +202,9 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     for (int item = pair; ok && item < total; item += n_pairs) {
       const int sl = p.by_tiles_mn.div(item), t = item - sl * tiles_mn;      // (split, batch), tile
       const int sp = p.by_batches.div(sl), l = sl - sp * nbatch;
-      const int n_t = p.by_tiles_m.div(t);
-      const int a_row = (2 * (t - n_t * tiles_m2) + rank) * G_BM;
+      int m_t, n_t;
+      pair_tile(p, t, tiles_m2, m_t, n_t);
+      const int a_row = (2 * m_t + rank) * G_BM;
       const int b_row = n_t * BN + rank * Cfg::HALF;
       const int l1 = p.by_l0.div(l), l0 = l - l1 * p.L0;
       const int kb0 = sp * kb_per_split;
@@ -243,8 +252,9 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     for (int item = pair; item < total; item += n_pairs) {
       const int sl = p.by_tiles_mn.div(item), t = item - sl * tiles_mn;
       const int sp = p.by_batches.div(sl), l = sl - sp * nbatch;
-      const int n_t = p.by_tiles_m.div(t);
-      epi.begin(sp, l, (2 * (t - n_t * tiles_m2) + rank) * G_BM + q * 32, n_t * BN + c_begin * 32, Cfg::C_HALF,
+      int m_t, n_t;
+      pair_tile(p, t, tiles_m2, m_t, n_t);
+      epi.begin(sp, l, (2 * m_t + rank) * G_BM + q * 32, n_t * BN + c_begin * 32, Cfg::C_HALF,
                 sp * kb_per_split >= kblocks_all);
       if (!mbar_wait(&cta.tfull[acc], (acc_ph >> acc) & 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();

@@ -46,8 +46,9 @@ struct GemmArgs {
   // skipped by every role (no loads, no MMAs, no stores).  NULL = all rows in use.
   const int* seg_counts;
   int seg_rows;
-  // work item = ((split * batches + batch) * n tiles + n tile) * m tiles + m tile
-  FastDiv by_tiles_m, by_tiles_mn, by_batches, by_l0;
+  // work item = ((split * batches + batch) * n tiles + n tile) * m tiles + m tile; pair tiles take the m tiles in groups of
+  // by_gm.d (the last group by_gm_last.d) that walk all n tiles
+  FastDiv by_tiles_m, by_tiles_mn, by_batches, by_l0, by_group, by_gm, by_gm_last;
 };
 
 __device__ __forceinline__ float tanh_fast(float x) {

@@ -152,6 +152,25 @@ static void set_divisors(GemmArgs& a, int bm, int bn) {
   a.by_l0 = FastDiv((uint32_t)a.L0);
 }
 
+// m tiles per group of the pair kernel's walk.  With m fastest over all of them, the 74 tiles in flight hold up to 74 different
+// row blocks of A against one or two column blocks of B, and an A that is larger than what L2 keeps is read again for every
+// few columns: from memory, which costs time and, where the power limit sets the clock, the clock of the tensor pipe.  In
+// groups, the tiles in flight are a patch of the output and A is read once (B again for each group, but from L2 if it fits).
+// us in a loop at the power limit, m fastest / groups of 4 / of 8: 8192 x 2048 x 8192 240 / 218 / 216, 16384 x 2048 x 4096
+// 274 / 201 / 200, 16384 x 8192 x 4096 1040 / 839 / 819, 50304 x 768 x 8192 (weight gradient of a GPT-2 head) 620 / 499 / 519,
+// 50304 x 1024 x 4096 445 / 291 / 334.  An A of up to half of L2 stays there as it is and B streams past it once: 4096 x 4096 x
+// 4096 108 / 113 / 111, and 8192 x 50304 x 768, whose B is the larger operand, 535 / 585 / 549.
+static void set_pair_groups(GemmArgs& a) {
+  const uint32_t tm = a.by_tiles_m.d, tn = a.by_tiles_mn.d / tm;
+  uint32_t gm = tm;
+  if (2ll * a.M * a.K > (64ll << 20)) gm = tn < 16 ? 4 : 8;
+  if (gm > tm) gm = tm;
+  const uint32_t last = tm % gm ? tm % gm : gm;
+  a.by_group = FastDiv(gm * tn);
+  a.by_gm = FastDiv(gm);
+  a.by_gm_last = FastDiv(last);
+}
+
 // The epilogue instantiation of a problem: a special kind where its parts are exactly those of the kind and every row is
 // made of 16-byte segments, else the general one.
 static int epilogue_kind(const GemmArgs& a) {
@@ -219,6 +238,7 @@ static int launch_gemm_pair_kind(const CUtensorMap& tmA, const CUtensorMap& tmB,
     *attr_set_p = true;
   }
   set_divisors(a, 2 * G_BM, BN);
+  set_pair_groups(a);
   const long long items = (long long)((a.M + 255) / 256) * ((a.N + BN - 1) / BN) * a.L0 * a.L1 * a.splits;
   if (items > 0x7fffffffll) return -2;
   long long pairs = max_ctas / 2;

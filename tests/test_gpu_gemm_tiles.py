@@ -178,3 +178,23 @@ def test_grouped_products_with_unaligned_outputs(cuda_device):
     k.check_status()
     for (_, _, out, _), ref in zip(probs, refs):
         _close(out, ref)
+
+
+@pytest.mark.parametrize("bn", [256 + 128, 256 + 192, 256 + 256])
+@pytest.mark.parametrize("M,N,K", [
+    (4 * 256 + 8, 264, 32768),        # five row blocks of a large A in groups of four: a last group of one
+    (7 * 256, 8 * 256 + 136, 24576),  # more column blocks, a last group of three
+    (10 * 256 + 136, 17 * 256, 13312),  # groups of eight where the column blocks are many
+])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_row_block_groups(cuda_device, bn, M, N, K, splits):
+    """An A beyond half of L2 is walked in groups of row blocks: every tile once, also with a last group that is not whole."""
+    from frankentorch_b200.ops import kernels as k
+    assert 2 * M * K > 64 << 20
+    a, w = _rand((M, K), 21, cuda_device), _rand((N, K), 22, cuda_device, K ** -0.5)
+    ref = a.double() @ w.double().t()
+    out = torch.full((M, N), float("nan"), device=cuda_device)
+    k.gemm(a, w, out=out, force_bn=bn, split_k=splits)
+    k.check_status()
+    # fp32 sums of K products whose squares add up to about one: at most K * 2^-24 of them, 2e-3
+    assert float((out.double() - ref).abs().max()) <= K * 2.0 ** -24
