@@ -29,7 +29,8 @@ struct PairCfg {
   static constexpr int MN_CHUNKS = (HALF + 63) / 64;   // 64-column boxes of an MN-major B half (BN = 192 loads 32 spare columns)
   static constexpr int A_BYTES = G_BM * G_BK * 2;  // per CTA and stage
   static constexpr int B_BYTES = MN_CHUNKS * 64 * G_BK * 2;
-  static constexpr int STAGES = BN == 128 ? 8 : 6;
+  static constexpr int STAGES = BN == 384 ? 4 : (BN == 128 ? 8 : 6);
+  static constexpr int ACCS = BN > 256 ? 1 : 2;    // accumulators
   static constexpr int ACC_STRIDE = BN == 128 ? 128 : 256;
   static constexpr int TMEM_COLS = BN == 128 ? 256 : 512;
   static constexpr int OFF_BARS = STAGES * (A_BYTES + B_BYTES);
@@ -118,7 +119,9 @@ struct PairCta {
   // The MMA loop of one tile over k-blocks [kb0, kb1): leader CTA, whole warp.  Returns false on an abort.
   __device__ __forceinline__ bool mma_tile(uint32_t d_tmem, int kb0, int kb1, int a_mn, int b_mn, uint64_t* done, int& s,
                                            uint32_t& ph, const WaitCtx& ctx) {
-    const uint32_t idesc = make_idesc_bf16(2 * G_BM, BN, a_mn, b_mn);
+    // (an instruction has 256 columns at most: a wider tile takes the first 128 columns of both halves, then the rest)
+    const uint32_t idesc = make_idesc_bf16(2 * G_BM, BN > 256 ? 256 : BN, a_mn, b_mn);
+    const uint32_t idesc2 = make_idesc_bf16(2 * G_BM, BN > 256 ? BN - 256 : 64, a_mn, b_mn);
     const uint32_t a_lbo = a_mn ? G_BK * 128 : 16, a_adv16 = (a_mn ? G_UMMA_K * 128 : G_UMMA_K * 2) >> 4;
     const uint32_t b_lbo = b_mn ? G_BK * 128 : 16, b_adv16 = (b_mn ? G_UMMA_K * 128 : G_UMMA_K * 2) >> 4;
     const uint32_t a_lo0 = desc_lo(smem_u32(sA), a_lbo), b_lo0 = desc_lo(smem_u32(sB), b_lbo);
@@ -132,6 +135,13 @@ struct PairCta {
 #pragma unroll
         for (int k = 1; k < G_BK / G_UMMA_K; ++k)
           umma_bf16_pair_lo(d_tmem, a_lo + k * a_adv16, b_lo + k * b_adv16, idesc, 1u);
+        if constexpr (BN > 256) {
+          const uint32_t b2_lo = b_lo + (128 * G_BK * 2 >> 4);      // K-major: row 128; MN-major: the third 64-column box
+          umma_bf16_pair_lo(d_tmem + 256, a_lo, b2_lo, idesc2, kb > kb0 ? 1u : 0u);
+#pragma unroll
+          for (int k = 1; k < G_BK / G_UMMA_K; ++k)
+            umma_bf16_pair_lo(d_tmem + 256, a_lo + k * a_adv16, b2_lo + k * b_adv16, idesc2, 1u);
+        }
         umma_commit_pair(&empty[s], 3);                       // the stage is free in both CTAs
         if (kb == kb1 - 1) umma_commit_pair(done, 3);         // both epilogues may drain
       }

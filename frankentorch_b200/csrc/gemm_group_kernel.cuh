@@ -4,8 +4,8 @@
 //
 // Purpose: the four weight gradients of a transformer block (dW = dY^T X with K = tokens) have 12 - 48
 // output tiles each, far fewer than the 74 CTA pairs, so on their own they need split-K plus a reduction kernel.
-// Together they are 144 tiles of 256 x 192: two full waves with no split at all - every output element is
-// reduced over K by one CTA pair in k-block order, which is also the simplest deterministic order there is.
+// Together they are 72 tiles of 256 x 384 or 144 of 256 x 192: one or two full waves with no split at all - every output element
+// is reduced over K by one CTA pair in k-block order, which is also the simplest deterministic order there is.
 //
 // The kernel is the CTA-pair tcgen05 GEMM of gemm2_kernel.cuh with a table of problems in the place of one: a work
 // item is (problem, n tile, m tile), items are dealt round robin to the pairs, and each problem brings its own pair of
@@ -18,14 +18,14 @@
 namespace ftk {
 
 constexpr int GG_MAX = 8;   // problems per launch
-constexpr int GG_BN = 192;
+constexpr int GG_BN = 192, GG_BN_WIDE = 384;
 
 struct GroupArgs {
   int n;                       // number of problems
   int K;
   int a_mn, b_mn;
   int M[GG_MAX], N[GG_MAX];
-  int tile_end[GG_MAX];        // running total of 256 x GG_BN tiles up to and including problem p
+  int tile_end[GG_MAX];        // running total of tiles up to and including problem p
   float* D[GG_MAX];
   long long ldd[GG_MAX];
   int accumulate[GG_MAX];
@@ -53,11 +53,11 @@ __device__ __forceinline__ GroupTile group_decode(int item, const GroupArgs& g) 
   return t;
 }
 
-// KIND: EPI_KIND_F32, or EPI_KIND_ANY when an output's rows are not made of aligned 16-byte segments
-template <int KIND>
+// KIND: EPI_KIND_F32, or EPI_KIND_ANY when an output's rows are not made of aligned 16-byte segments.
+// BN = 192: two accumulators, the epilogue of a tile under the main loop of the next.  BN = 384: one accumulator.
+template <int BN, int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G_THREADS, 1)
 gemm_group_bf16_sm100_kernel(const __grid_constant__ GroupMaps maps, const GroupArgs g) {
-  constexpr int BN = GG_BN;
   using Cfg = PairCfg<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0u) {
@@ -117,14 +117,14 @@ gemm_group_bf16_sm100_kernel(const __grid_constant__ GroupMaps maps, const Group
         if (!cta.mma_tile(cta.tmem_base + acc * Cfg::ACC_STRIDE, 0, kblocks, g.a_mn, g.b_mn, &cta.tfull[acc], s, ph, ctx))
           break;
         acc_ph ^= (1u << acc);
-        acc ^= 1;
+        if (Cfg::ACCS > 1) acc ^= 1;
       }
     }
   } else {
     // ------------------------------------------------------------ epilogue (8 warps, both CTAs): fp32 store / accumulate
     const int ew = warp - 2;
     const int q = warp & 3;
-    const int c_begin = (ew >> 2) * Cfg::C_HALF;
+    const int half = ew >> 2;             // column half of the tile
     GemmArgs p;
     p.L0 = p.L1 = p.splits = p.out_fp32 = 1;
     p.d_s0 = p.d_s1 = p.ldr = p.r_s0 = p.r_s1 = 0;
@@ -144,16 +144,27 @@ gemm_group_bf16_sm100_kernel(const __grid_constant__ GroupMaps maps, const Group
       p.D = g.D[t.p];
       p.ldd = g.ldd[t.p];
       p.accumulate = g.accumulate[t.p];
-      epi.begin(0, 0, (2 * t.m_t + rank) * G_BM + q * 32, t.n_t * BN + c_begin * 32, Cfg::C_HALF, false);
+      const int row = (2 * t.m_t + rank) * G_BM + q * 32, col = t.n_t * BN + half * (BN / 2);
+      constexpr int FIRST = BN > 256 ? 4 : Cfg::C_HALF;      // chunks of this warp beside one another in tensor memory
+      epi.begin(0, 0, row, col, FIRST, false);
       if (!mbar_wait(&cta.tfull[acc], (acc_ph >> acc) & 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
-      epi.run(cta.tmem_base + acc * Cfg::ACC_STRIDE + c_begin * 32 + ((uint32_t)(q * 32) << 16), Cfg::C_HALF, [&] {
+      auto release = [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_leader(&cta.tempty[acc]);
-      });
+      };
+      const uint32_t lanes = cta.tmem_base + ((uint32_t)(q * 32) << 16);
+      if constexpr (BN > 256) {
+        // the tile's halves are [0, 128) and [256, 320) of the accumulator, [128, 256) and [320, 384)
+        epi.run(lanes + half * 128, FIRST, [] {});
+        epi.begin(0, 0, row, col + 128, Cfg::C_HALF - FIRST, false);
+        epi.run(lanes + 256 + half * ((BN - 256) / 2), Cfg::C_HALF - FIRST, release);
+      } else {
+        epi.run(lanes + acc * Cfg::ACC_STRIDE + half * (BN / 2), FIRST, release);
+      }
       acc_ph ^= (1u << acc);
-      acc ^= 1;
+      if (Cfg::ACCS > 1) acc ^= 1;
     }
   }
   cta.teardown();

@@ -420,30 +420,56 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   return 0;
 }
 
-template <int KIND>
+template <int BN, int KIND>
 static int launch_group(const GroupMaps& maps, const GroupArgs& ga, int pairs, cudaStream_t stream) {
-  constexpr int SMEM = PairCfg<GG_BN>::SMEM;
+  constexpr int SMEM = PairCfg<BN>::SMEM;
   static PerDeviceOnce once;
   bool* attr_set_p = once.slot();
   if (!*attr_set_p) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_group_bf16_sm100_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_group_bf16_sm100_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SMEM);
     if (e != cudaSuccess) return (int)e;
     *attr_set_p = true;
   }
-  launch_pdl(gemm_group_bf16_sm100_kernel<KIND>, 2 * pairs, G_THREADS, SMEM, stream, maps, ga);
+  launch_pdl(gemm_group_bf16_sm100_kernel<BN, KIND>, 2 * pairs, G_THREADS, SMEM, stream, maps, ga);
   return (int)cudaGetLastError();
 }
 
-// CTAs for `total` pair tiles of a group: whole pairs, or one CTA where no pair is allowed.
-static int group_ctas(const FtkGemmDesc& g0, int total) {
-  const int sms = g0.max_ctas > 0 ? g0.max_ctas : num_sms();
-  const int pairs = total < sms / 2 ? total : sms / 2;
-  return pairs > 0 ? 2 * pairs : 1;
+// Tile width of a grouped launch, its tiles and its CTAs: whole pairs, or one CTA where no pair is allowed.
+struct GroupPlan {
+  int bn, total, ctas;
+};
+// The wide tile loads 40 KB per CTA for the work that two 256 x 192 tiles load 64 KB for (an MN-major half of 96 columns comes in
+// two boxes of 64), but has one accumulator, so its epilogue is not hidden.  Modelled time: waves x (fixed + k-blocks), in us:
+// 1.2 + 0.34 per k-block of 64 and 4.5 + 0.62.  Measured, 192 / 384 columns, back to back without and with the power limit: the
+// four weight gradients of a block of 768 over 8192 rows 88.8 / 82.1 and 111.1 / 97.5, over 2048 rows 28.7 / 28.8, over 512 rows
+// 13.4 / 14.3; of a block of 1024 over 8192 rows 168.9 / 158.6 and 203.5 / 186.7, of 512 over 4096 rows (70 and 44 tiles, one wave
+// both) 25.8 / 41.2; an MLP of 2048 over 8192 rows 449 / 409 and 578 / 491; a block of 1280 over 4096 rows (6 and 4 waves)
+// 134 / 155.
+static GroupPlan plan_group(const FtkGemmDesc* descs, int n) {
+  const int sms = descs[0].max_ctas > 0 ? descs[0].max_ctas : num_sms();
+  const double kblocks = (double)((descs[0].K + G_BK - 1) / G_BK);
+  GroupPlan best = {GG_BN, 0, 1};
+  double best_us = 1e30;
+  for (int bn : {GG_BN, GG_BN_WIDE}) {
+    long long total = 0;
+    for (int p = 0; p < n; ++p)
+      total += (long long)((descs[p].M + 2 * G_BM - 1) / (2 * G_BM)) * ((descs[p].N + bn - 1) / bn);
+    const long long units = sms > 1 ? sms / 2 : 1, waves = (total + units - 1) / units;
+    const double us = waves * (bn == GG_BN ? 1.2 + 0.34 * kblocks : 4.5 + 0.62 * kblocks);
+    if (us < best_us) {
+      best_us = us;
+      best.bn = bn;
+      best.total = (int)total;
+    }
+  }
+  const int pairs = best.total < sms / 2 ? best.total : sms / 2;
+  best.ctas = pairs > 0 ? 2 * pairs : 1;
+  return best;
 }
 
 // Grouped launch: `n` (1..8) independent products with the same K and operand layouts, fp32 outputs with a plain
-// store or accumulate epilogue, in one persistent kernel of 256 x 192 pair tiles (see gemm_group_kernel.cuh).
+// store or accumulate epilogue, in one persistent kernel of pair tiles (see gemm_group_kernel.cuh).
 extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   if (!descs || n < 1 || n > GG_MAX) return -2;
@@ -454,6 +480,10 @@ extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream
   ga.n = n; ga.K = g0.K; ga.a_mn = g0.a_mn ? 1 : 0; ga.b_mn = g0.b_mn ? 1 : 0; ga.alpha = g0.alpha;
   ga.status = ftk_status_word();
   if (!ga.status) return -6;
+  for (int p = 0; p < n; ++p)
+    if (descs[p].M <= 0 || descs[p].N <= 0) return -2;
+  const GroupPlan plan = plan_group(descs, n);
+  const int bn = plan.bn;
   int total = 0;
   for (int p = 0; p < n; ++p) {
     const FtkGemmDesc* g = &descs[p];
@@ -465,19 +495,18 @@ extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream
       return -7;
     if ((reinterpret_cast<uintptr_t>(g->A) & 15) || (reinterpret_cast<uintptr_t>(g->B) & 15)) return -3;
     if ((g->lda % 8) || (g->ldb % 8)) return -4;
-    int rc = make_operand_maps(g, 1, 1, PairCfg<GG_BN>::HALF, &maps.a[p], &maps.b[p]);
+    int rc = make_operand_maps(g, 1, 1, bn / 2, &maps.a[p], &maps.b[p]);
     if (rc) return rc;
     ga.M[p] = g->M; ga.N[p] = g->N;
     ga.D[p] = reinterpret_cast<float*>(g->D);
     ga.ldd[p] = g->ldd;
     ga.accumulate[p] = g->accumulate ? 1 : 0;
     ga.by_tiles_m[p] = FastDiv((uint32_t)((g->M + 2 * G_BM - 1) / (2 * G_BM)));
-    total += ((g->M + 2 * G_BM - 1) / (2 * G_BM)) * ((g->N + GG_BN - 1) / GG_BN);
+    total += ((g->M + 2 * G_BM - 1) / (2 * G_BM)) * ((g->N + bn - 1) / bn);
     ga.tile_end[p] = total;
   }
   for (int p = n; p < GG_MAX; ++p) ga.tile_end[p] = total;
-  const int ctas = group_ctas(g0, total);
-  if (ctas < 2) {
+  if (plan.ctas < 2) {
     // one CTA is all the caller allows: the products in turn, same k order, so the same bits
     for (int p = 0; p < n; ++p) {
       FtkGemmDesc one = descs[p];
@@ -492,15 +521,18 @@ extern "C" int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream
   bool aligned = true;
   for (int p = 0; p < n; ++p)
     aligned = aligned && ga.N[p] % 4 == 0 && ga.ldd[p] % 4 == 0 && (reinterpret_cast<uintptr_t>(ga.D[p]) & 15) == 0;
-  return aligned ? launch_group<EPI_KIND_F32>(maps, ga, ctas / 2, stream) : launch_group<EPI_KIND_ANY>(maps, ga, ctas / 2, stream);
+  const int pairs = plan.ctas / 2;
+  if (bn == GG_BN_WIDE)
+    return aligned ? launch_group<GG_BN_WIDE, EPI_KIND_F32>(maps, ga, pairs, stream)
+                   : launch_group<GG_BN_WIDE, EPI_KIND_ANY>(maps, ga, pairs, stream);
+  return aligned ? launch_group<GG_BN, EPI_KIND_F32>(maps, ga, pairs, stream)
+                 : launch_group<GG_BN, EPI_KIND_ANY>(maps, ga, pairs, stream);
 }
 
 // CTAs that the grouped launch takes: never more than max_ctas.  Launches nothing.
 extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
   if (!descs || n < 1 || n > GG_MAX) return -2;
-  int total = 0;
-  for (int p = 0; p < n; ++p) total += ((descs[p].M + 2 * G_BM - 1) / (2 * G_BM)) * ((descs[p].N + GG_BN - 1) / GG_BN);
-  return group_ctas(descs[0], total);
+  return plan_group(descs, n).ctas;
 }
 
 // Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile 128 x bn) or

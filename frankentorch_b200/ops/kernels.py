@@ -225,7 +225,7 @@ def gemm_grouped(problems, *, a_mn: bool = True, b_mn: bool = True, max_ctas: in
         g.D, g.ldd = out.data_ptr(), out.stride(0)
         g.alpha, g.out_fp32, g.accumulate, g.max_ctas = 1.0, 1, int(bool(accumulate)), int(max_ctas)
     _chk(_lib.load().ftk_gemm_group_bf16(arr, n, _stream()),
-         "ftk::gemm_group_bf16_sm100<256x192,cta_group2,problems=%d>" % n)
+         "ftk::gemm_group_bf16_sm100<cta_group2,problems=%d>" % n)
 
 
 # Most bytes of partial tiles that the tile planner may spend on one product, and the reduction length up to which it never

@@ -52,6 +52,17 @@ def test_a_group_keeps_to_its_ctas(shapes, max_ctas):
     assert 1 <= ctas <= max_ctas and (ctas == 1) == (max_ctas == 1)
 
 
+def test_wide_tiles_of_a_group():
+    """256 x 384 tiles where they fill the pairs and the reduction is long: the weight gradients of a block of 768 are 72 of them
+    (144 CTAs) over 8192 rows, and 144 narrow ones on all CTAs over 512."""
+    fn = _lib.load().ftk_gemm_group_ctas
+    fn.argtypes, fn.restype = [C.POINTER(_lib.FtkGemmDesc), C.c_int], C.c_int
+    for rows, ctas in ((8192, 144), (512, 148)):
+        shapes = [(2304, 768), (768, 768), (3072, 768), (768, 3072)]
+        arr = (_lib.FtkGemmDesc * 4)(*[_desc(m, n, rows, a_mn=1, b_mn=1, f32=1) for m, n in shapes])
+        assert fn(arr, 4) == ctas
+
+
 @pytest.mark.gpu
 def test_a_group_on_one_cta(cuda_device):
     import torch

@@ -198,3 +198,28 @@ def test_row_block_groups(cuda_device, bn, M, N, K, splits):
     k.check_status()
     # fp32 sums of K products whose squares add up to about one: at most K * 2^-24 of them, 2e-3
     assert float((out.double() - ref).abs().max()) <= K * 2.0 ** -24
+
+
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("mn", [True, False])
+def test_wide_grouped_tiles(cuda_device, pad, accumulate, mn):
+    """Groups with long reductions on few CTAs take 256 x 384 tiles: several per pair, ragged rows, columns and k-blocks."""
+    from frankentorch_b200.ops import kernels as k
+    K, shapes = 4104, [(264, 384), (520, 760), (256, 392)]
+    probs, refs = [], []
+    for i, (M, N) in enumerate(shapes):
+        a, b = _rand((K, M), 30 + i, cuda_device), _rand((K, N), 40 + i, cuda_device, K ** -0.5)
+        if not mn:
+            a, b = a.t().contiguous(), b.t().contiguous()
+        out = torch.full((M, N + pad), 0.25 if accumulate else float("nan"), device=cuda_device)[:, :N]
+        probs.append((a, b, out, accumulate))
+        refs.append((a.double().t() @ b.double() if mn else a.double() @ b.double().t()) + (0.25 if accumulate else 0.0))
+    for ctas in (4, 0):
+        for _, _, out, _ in probs:
+            out.fill_(0.25)
+        k.gemm_grouped(probs, a_mn=mn, b_mn=mn, max_ctas=ctas)
+        k.check_status()
+        for (_, _, out, _), ref in zip(probs, refs):
+            # fp32 sums of K products whose squares add up to about one
+            assert float((out.double() - ref).abs().max()) <= K * 2.0 ** -24 + 2.0 ** -20 * float(ref.abs().max())
