@@ -43,7 +43,7 @@ typedef struct FtkGemmDesc {
   int epi;
   int out_fp32;
   int accumulate;        // D += result
-  int force_bn;          // 0 = heuristic, 128 / 192 / 256 = single-CTA tile, 256 + 128 / 192 / 256 = CTA-pair tile
+  int force_bn;          // 0 = heuristic, 128 / 192 / 256 = single-CTA tile, 256 + 128 to 256 in steps of 32 = CTA-pair tile
   int max_ctas;          // 0 = all SMs
   // Deterministic split-K (plain fp32/bf16 store epilogues only): partial tiles go to
   // `workspace` (fp32, split_count*M*N*4 bytes needed) and are summed in ascending split order.
@@ -66,7 +66,7 @@ typedef struct FtkGemmDesc {
 int* ftk_status_word(void);               // device pointer (allocated on first use, per device)
 int ftk_read_status(int reset);           // synchronises the device; returns the status word
 int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream);
-// Which kernel ftk_gemm_bf16 would launch: *bn = 128 / 192 / 256 (one CTA per 128 x bn tile) or 384 / 448 / 512
+// Which kernel ftk_gemm_bf16 would launch: *bn = 128 / 192 / 256 (one CTA per 128 x bn tile) or 384 to 512
 // (CTA-pair kernel, tiles of 256 x (bn - 256), cta_group::2); *splits = split-K factor.  No launch.
 int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits);
 // `n` (1..8) products with one K and one pair of operand layouts, fp32 outputs (store or accumulate), no other

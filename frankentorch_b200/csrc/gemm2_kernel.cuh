@@ -1,4 +1,4 @@
-// bf16 GEMM on CTA pairs (tcgen05 cta_group::2): one 256 x BN output tile per 2-CTA cluster, BN = 256, 192 or 128.
+// bf16 GEMM on CTA pairs (tcgen05 cta_group::2): one 256 x BN output tile per 2-CTA cluster, BN = 128 to 256 in steps of 32.
 //
 // Each CTA of the pair loads its own 128 rows of A and its own BN / 2 columns of B per k-block
 // (32 KB per stage at BN = 256 instead of the 48 KB a lone 128 x 256 tile needs), which cuts the L2 -> SM
@@ -26,7 +26,7 @@ template <int BN_>
 struct PairCfg {
   static constexpr int BN = BN_;                   // tile columns (BN / 2 staged per CTA)
   static constexpr int HALF = BN / 2;
-  static constexpr int MN_CHUNKS = (HALF + 63) / 64;   // 64-column boxes of an MN-major B half (BN = 192 loads 32 spare columns)
+  static constexpr int MN_CHUNKS = (HALF + 63) / 64;   // 64-column boxes of an MN-major B half (a half of 80, 96 or 112 loads 128 columns)
   static constexpr int A_BYTES = G_BM * G_BK * 2;  // per CTA and stage
   static constexpr int B_BYTES = MN_CHUNKS * 64 * G_BK * 2;
   static constexpr int STAGES = BN == 384 ? 4 : (BN == 128 ? 8 : 6);
@@ -38,7 +38,7 @@ struct PairCfg {
   static constexpr int OFF_BIAS = OFF_STAGE + G_EPI_WARPS * EPI_STAGE_BYTES;
   static constexpr int SMEM = OFF_BIAS + G_EPI_WARPS * EPI_BIAS_BYTES;
   static constexpr int CHUNKS = BN / 32;
-  static constexpr int C_HALF = CHUNKS / 2;
+  static constexpr int C_HALF = (CHUNKS + 1) / 2;    // chunks of the first four epilogue warps, the others take the rest
   static_assert((2 * STAGES + 4) * 8 + 8 <= 256, "barrier space");
   static_assert(SMEM <= 232448, "shared memory");
 };
@@ -254,7 +254,7 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
     // ------------------------------------------------------------ epilogue (8 warps, both CTAs)
     const int ew = warp - 2;
     const int q = warp & 3;
-    const int c_begin = (ew >> 2) * Cfg::C_HALF;
+    const int c_begin = (ew >> 2) * Cfg::C_HALF, chunks = (ew >> 2) ? Cfg::CHUNKS - Cfg::C_HALF : Cfg::C_HALF;
     TileEpilogue<KIND> epi(p, smem + Cfg::OFF_STAGE + ew * EPI_STAGE_BYTES,
                      reinterpret_cast<__nv_bfloat16*>(smem + Cfg::OFF_BIAS + ew * EPI_BIAS_BYTES), lane);
     int acc = 0;
@@ -264,11 +264,11 @@ gemm2_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmA,
       const int sp = p.by_batches.div(sl), l = sl - sp * nbatch;
       int m_t, n_t;
       pair_tile(p, t, tiles_m2, m_t, n_t);
-      epi.begin(sp, l, (2 * m_t + rank) * G_BM + q * 32, n_t * BN + c_begin * 32, Cfg::C_HALF,
+      epi.begin(sp, l, (2 * m_t + rank) * G_BM + q * 32, n_t * BN + c_begin * 32, chunks,
                 sp * kb_per_split >= kblocks_all);
       if (!mbar_wait(&cta.tfull[acc], (acc_ph >> acc) & 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
-      epi.run(cta.tmem_base + acc * Cfg::ACC_STRIDE + c_begin * 32 + ((uint32_t)(q * 32) << 16), Cfg::C_HALF, [&] {
+      epi.run(cta.tmem_base + acc * Cfg::ACC_STRIDE + c_begin * 32 + ((uint32_t)(q * 32) << 16), chunks, [&] {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_leader(&cta.tempty[acc]);   // the MMA warp lives in the leader CTA

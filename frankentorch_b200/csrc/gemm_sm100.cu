@@ -24,6 +24,8 @@
 #include "gemm2_kernel.cuh"
 #include "gemm_group_kernel.cuh"
 
+#include <type_traits>
+
 namespace ftk {
 
 // D (+)= sum over splits (ascending) of ws[split]; 4 outputs per thread.
@@ -251,10 +253,14 @@ static int launch_gemm_pair_kind(const CUtensorMap& tmA, const CUtensorMap& tmB,
 template <int BN, bool PAIR>
 static int launch_gemm(int kind, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, int max_ctas,
                        cudaStream_t stream) {
-#define FT_LAUNCH_KIND(K)                                                                  \
-  case K:                                                                                  \
-    return PAIR ? launch_gemm_pair_kind<BN, K>(tmA, tmB, a, max_ctas, stream)              \
-                : launch_gemm_kind<BN, K>(tmA, tmB, a, max_ctas, stream);
+  auto launch = [&](auto k) {
+    if constexpr (PAIR)
+      return launch_gemm_pair_kind<BN, decltype(k)::value>(tmA, tmB, a, max_ctas, stream);
+    else
+      return launch_gemm_kind<BN, decltype(k)::value>(tmA, tmB, a, max_ctas, stream);
+  };
+#define FT_LAUNCH_KIND(K) \
+  case K: return launch(std::integral_constant<int, K>());
   switch (kind) {
     FT_LAUNCH_KIND(EPI_KIND_PLAIN)
     FT_LAUNCH_KIND(EPI_KIND_RESID)
@@ -262,9 +268,7 @@ static int launch_gemm(int kind, const CUtensorMap& tmA, const CUtensorMap& tmB,
     FT_LAUNCH_KIND(EPI_KIND_GELU_AUX)
     FT_LAUNCH_KIND(EPI_KIND_DGELU)
     FT_LAUNCH_KIND(EPI_KIND_F32)
-    default:
-      return PAIR ? launch_gemm_pair_kind<BN, EPI_KIND_ANY>(tmA, tmB, a, max_ctas, stream)
-                  : launch_gemm_kind<BN, EPI_KIND_ANY>(tmA, tmB, a, max_ctas, stream);
+    default: return launch(std::integral_constant<int, EPI_KIND_ANY>());
   }
 #undef FT_LAUNCH_KIND
 }
@@ -349,7 +353,8 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   // measured amounts below, in proportion to the SMs in use.  Measured against the model (us, 256 x 256 / 256 x 192 /
   // 256 x 128 pairs, then 128 x 256 / 192 / 128; all L2-resident): 8192 x 768 x 3072 36.7 / 31.3 / 34.5, 40.6 / 37.6 / 38.9;
   // 1500 x 1280 x 5120 29.6 / 23.7 / 19.3, 29.2 / 23.4 / 21.6; 1500 x 3840 x 1280 17.8 / 14.7 / 16.0, 18.6 / 15.5 / 17.9;
-  // 8192 x 2304 x 768 21.9 / 23.0 / 25.0, 24.4 / 26.6 / 27.7.
+  // 8192 x 2304 x 768 21.9 / 23.0 / 25.0, 24.4 / 26.6 / 27.7.  224 and 160 columns (pairs only): 8192 x 2304 x 768 23.3 / 23.8,
+  // 1500 x 1280 x 5120 26.7 / 21.7 beside 29.8 / 25.4 / 20.1, 512 x 8192 x 8192 46.9 / 63.4 beside 50.1 / 67.0 / 55.6.
   // Split-K (weight-gradient shapes: few output tiles, long reduction) is considered when the
   // epilogue is a plain store and the caller supplied a workspace.
   const int kblocks = (g->K + G_BK - 1) / G_BK;
@@ -373,9 +378,12 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   auto cost = [&](int bn, int s) {
     const bool pair = bn > 256;
     const int w = pair ? bn - 256 : bn;
-    const double tile = w == 256 ? 0.4 : (w == 192 ? 0.1 : 0.3);
-    const double mma = w == 256 ? 0.278 : (w == 192 ? 0.21 : 0.143);
-    const double full = pair ? (w == 256 ? 0.375 : (w == 192 ? 0.32 : 0.235)) : (w == 256 ? 0.42 : (w == 192 ? 0.385 : 0.27));
+    // 256, 224, 192, 160, 128 columns
+    const int wi = (256 - w) / 32;
+    static const double tile_us[5] = {0.4, 0.3, 0.1, 0.2, 0.3}, mma_us[5] = {0.278, 0.244, 0.21, 0.176, 0.143};
+    static const double pair_us[5] = {0.375, 0.35, 0.32, 0.30, 0.235}, one_us[5] = {0.42, 0.0, 0.385, 0.0, 0.27};
+    static const double exposed_us[5] = {0.75, 0.7, 0.55, 0.3, 0.0};
+    const double tile = tile_us[wi], mma = mma_us[wi], full = pair ? pair_us[wi] : one_us[wi];
     const long long items = ((g->M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * (long long)((g->N + w - 1) / w) * L0 * L1 * s;
     const long long units = pair ? sms / 2 : sms;
     const long long waves = (items + units - 1) / units;
@@ -383,7 +391,7 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     // the last tile's epilogue and a pair's hand-shakes are not hidden: 128 x 192 x 64 takes 4.1 / 4.7 / 4.8 us on one
     // SM and 4.6 / 5.1 / 5.3 us on a pair
     const double off = bn > 256 ? (w == 256 ? 1.2 : 1.3) : 1.35, lines = off_lines == 0 ? 1.0 : (off_lines == 1 ? off : off * off);
-    const double exposed = (w == 256 ? 0.75 : (w == 192 ? 0.55 : 0.0)) + (pair ? 0.5 : 0.0);
+    const double exposed = exposed_us[wi] + (pair ? 0.5 : 0.0);
     return ((double)waves * (tile + (double)kblocks / s * (mma + (full - mma) * busy) * lines) + exposed) *
                (pair ? pair_cost_scale() : 1.0) + split_penalty(s);
   };
@@ -392,13 +400,17 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     if (!splittable || g->split_k == 1 || kblocks / s < 8) return false;
     return (long long)s * g->M * g->N * 4 <= g->workspace_bytes;
   };
-  static const int bn_opts[6] = {512, 448, 384, 256, 192, 128};
+  static const int bn_opts[8] = {512, 480, 448, 416, 384, 256, 192, 128};
   static const int s_opts[8] = {1, 2, 3, 4, 6, 8, 12, 16};
   int bn = g->force_bn, splits = 1;
   double best = 1e30;
-  for (int bi = 0; bi < 6; ++bi) {
+  for (int bi = 0; bi < 8; ++bi) {
     if (bn_opts[bi] > 256 && (sms < 2 || g->M < 256 || g->seg_counts)) continue;
     if (g->force_bn && bn_opts[bi] != g->force_bn) continue;
+    // 160 and 224 columns fill the last wave of forward products (1500 x 3840 x 1280 in 144 tiles of 160 14.0 us, 120 of 192
+    // 15.0; 1500 x 5120 x 1280 in 138 of 224 17.3, 120 of 256 19.0).  A half of 80 or 112 columns of a B given [K, N] loads 128
+    // all the same, and nothing is gained (17.2 and 17.5, 21.7 and 20.5).
+    if ((bn_opts[bi] == 416 || bn_opts[bi] == 480) && g->b_mn && !g->force_bn) continue;
     for (int si = 0; si < 8; ++si) {
       const int s = s_opts[si];
       if (g->split_k > 1 && s != g->split_k && s != 1) continue;
@@ -412,7 +424,7 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
     }
   }
   if (g->split_k > 1 && split_ok(g->split_k)) splits = g->split_k;
-  if (bn != 128 && bn != 192 && bn != 256 && bn != 384 && bn != 448 && bn != 512) return -5;
+  if (bn != 128 && bn != 192 && bn != 256 && bn != 384 && bn != 416 && bn != 448 && bn != 480 && bn != 512) return -5;
   // a forced pair tile needs two CTAs (without them nothing would run), and pair tiles know no rows that are not in use
   if (bn > 256 && (sms < 2 || g->seg_counts)) return -5;
   *bn_out = bn;
@@ -536,7 +548,7 @@ extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
 }
 
 // Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile 128 x bn) or
-// 384 / 448 / 512 (CTA-pair kernel, tiles of 256 x 128 / 192 / 256); *splits = split-K factor.  Launches nothing.
+// 384 to 512 in steps of 32 (CTA-pair kernel, tiles of 256 x (bn - 256)); *splits = split-K factor.  Launches nothing.
 extern "C" int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits) {
   if (!bn || !splits) return -2;
   return plan_gemm(g, bn, splits);
@@ -569,7 +581,9 @@ extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
   }
   const int kind = epilogue_kind(a);
   rc = bn == 512   ? launch_gemm<256, true>(kind, tmA, tmB, a, sms, stream)
+       : bn == 480 ? launch_gemm<224, true>(kind, tmA, tmB, a, sms, stream)
        : bn == 448 ? launch_gemm<192, true>(kind, tmA, tmB, a, sms, stream)
+       : bn == 416 ? launch_gemm<160, true>(kind, tmA, tmB, a, sms, stream)
        : bn == 384 ? launch_gemm<128, true>(kind, tmA, tmB, a, sms, stream)
        : bn == 256 ? launch_gemm<256, false>(kind, tmA, tmB, a, sms, stream)
        : bn == 192 ? launch_gemm<192, false>(kind, tmA, tmB, a, sms, stream)

@@ -52,6 +52,14 @@ def test_a_group_keeps_to_its_ctas(shapes, max_ctas):
     assert 1 <= ctas <= max_ctas and (ctas == 1) == (max_ctas == 1)
 
 
+def test_widths_that_fill_the_last_wave():
+    """1500 x 5120 x 1280 is 138 tiles of 256 x 224 on 74 pairs, 1500 x 3840 x 1280 144 of 256 x 160; a B given [K, N] loads whole
+    64-column boxes, so these widths are left out there."""
+    assert _plan(1500, 5120, 1280)[:2] == (0, 480) and _plan(1500, 3840, 1280)[:2] == (0, 416)
+    assert _plan(1500, 5120, 1280, b_mn=1)[1] not in (416, 480) and _plan(1500, 3840, 1280, b_mn=1)[1] not in (416, 480)
+    assert _plan(8192, 2304, 768)[:2] == (0, 512) and _plan(8192, 3072, 768)[:2] == (0, 448)
+
+
 def test_wide_tiles_of_a_group():
     """256 x 384 tiles where they fill the pairs and the reduction is long: the weight gradients of a block of 768 are 72 of them
     (144 CTAs) over 8192 rows, and 144 narrow ones on all CTAs over 512."""

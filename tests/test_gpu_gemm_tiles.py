@@ -223,3 +223,21 @@ def test_wide_grouped_tiles(cuda_device, pad, accumulate, mn):
         for (_, _, out, _), ref in zip(probs, refs):
             # fp32 sums of K products whose squares add up to about one
             assert float((out.double() - ref).abs().max()) <= K * 2.0 ** -24 + 2.0 ** -20 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("bn", [256 + 160, 256 + 224])
+@pytest.mark.parametrize("M,N,K", [(256, 64, 64), (257, 200, 136), (384, 584, 1096), (512, 160, 72), (300, 232, 64)])
+@pytest.mark.parametrize("kind", ["plain", "bias_resid", "gelu_aux", "dgelu", "relu_resid", "f32_acc"])
+def test_widths_of_an_odd_number_of_chunks(cuda_device, bn, M, N, K, kind):
+    """Pair tiles of 160 and 224 columns: the two warps of a lane quarter drain unequal shares."""
+    test_tiles_and_epilogues(cuda_device, bn=bn, M=M, N=N, K=K, kind=kind)
+
+
+@pytest.mark.parametrize("bn", [256 + 160, 256 + 224])
+def test_widths_of_an_odd_number_of_chunks_other_forms(cuda_device, bn):
+    for M, N, K in ((264, 200, 136), (384, 584, 1096)):
+        test_weight_gradient_form(cuda_device, bn=bn, accumulate=True, M=M, N=N, K=K)
+    test_split_reductions(cuda_device, bn=bn, form="tn", splits=3, K=1600)
+    test_rows_without_aligned_segments(cuda_device, bn=bn, N=37, ldd=37, off=0)
+    test_bf16_accumulation_and_residual_rows(cuda_device, bn=bn, kind="bias_gelu", ldr=73)
+    test_row_block_groups(cuda_device, bn=bn, M=7 * 256, N=8 * 256 + 136, K=24576, splits=1)
