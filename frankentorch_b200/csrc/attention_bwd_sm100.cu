@@ -42,27 +42,28 @@ __device__ __forceinline__ void store_row32_packed(uint8_t* tile, int row, int c
     *reinterpret_cast<uint4*>(base + (((j0 + t) ^ (row & 7)) << 4)) =
         make_uint4(w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]);
 }
-// One warp's 32 rows x 32 columns of an output: scaled fp32 accumulator rows (a thread owns one) through the warp's part of
-// a swizzled [128 x 128] bf16 tile in shared memory, so that four lanes write 64 contiguous bytes of a row.  Stored straight
-// from its thread, a row 12 KB from the next costs 32 line accesses per instruction: ~9000 cycles per item of 128 x 2 x 128.
-__device__ __forceinline__ void store_out32(uint8_t* tile, int qd, int c0, int lane, const uint32_t* r, float scale,
-                                            __nv_bfloat16* row0, long long ss, int rows) {
-  uint32_t w[16];
+// One warp's 32 rows x 32 columns of an output: scaled fp32 accumulator rows (a thread owns one) as bf16 into the 2 KB `box`,
+// laid out as the TMA's 64-byte swizzle has it, and from there to (col, row0) by the TMA unit, which cuts off the rows past the end.
+// The box is free again behind bulk_wait_read_all() of lane 0.  (Four lanes writing 64 bytes of a row took 16 warps ~2000
+// cycles; straight from its thread, a row 12 KB from the next costs 32 line accesses per instruction.)
+__device__ __forceinline__ void store_out32(uint8_t* box, int lane, const uint32_t* r, float scale, const CUtensorMap* tm, int col,
+                                            int row0, int h, int b, int S) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-    w[i] = pack_bf16(__uint_as_float(r[2 * i]) * scale, __uint_as_float(r[2 * i + 1]) * scale);
-  store_row32_packed(tile, qd * 32 + lane, c0, w);
-  __syncwarp();
-  const uint8_t* base = tile + (c0 >> 6) * AT_REGION;
-  const int seg = ((c0 & 63) >> 3) + (lane & 3);
+  for (int t = 0; t < 4; ++t) {
+    uint32_t w[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = 8 * i + (lane >> 2), row = qd * 32 + rr;
-    const uint4 u = *reinterpret_cast<const uint4*>(base + row * 128 + ((seg ^ (row & 7)) << 4));
-    if (rr < rows) *reinterpret_cast<uint4*>(row0 + (long long)rr * ss + (lane & 3) * 8) = u;
+    for (int i = 0; i < 4; ++i)
+      w[i] = pack_bf16(__uint_as_float(r[8 * t + 2 * i]) * scale, __uint_as_float(r[8 * t + 2 * i + 1]) * scale);
+    *reinterpret_cast<uint4*>(box + lane * 64 + ((t ^ ((lane >> 1) & 3)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
+  fence_proxy_async_smem();
   __syncwarp();
+  if (lane == 0 && row0 < S) tma_store_4d(tm, box, col, row0, h, b);
 }
+constexpr int BW_BOX = 2048;
+struct DkvMaps {
+  CUtensorMap m[2];      // dV, dK
+};
 
 // =============================================================================== backward: dK, dV
 template <int HD>
@@ -98,7 +99,7 @@ template <int HD>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                    const AttnArgs p) {
+                    const __grid_constant__ DkvMaps out, const AttnArgs p) {
   using C = DkvCfg<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -376,6 +377,36 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     Ring<C::STAGES> rq;
     uint32_t blk = 0;                      // parity of the block
     bool ok = true, first = true;
+    uint8_t* box = smem + C::OFF_DST + warp * BW_BOX;
+    // dV and dK of a finished item: 2 HD / 32 column chunks (dV first) spread over the four groups
+    auto drain = [&](int kb, int b, int h) {
+      constexpr int NCH = 2 * HD / 32 / 4;
+      tc_fence_after();
+      uint32_t r[NCH][32];
+#pragma unroll
+      for (int u = 0; u < NCH; ++u) tmem_ld32(tmem_base + C::TM_DV + (g + 4 * u) * 32 + lane_sel, r[u]);
+      tmem_ld_wait();
+      tc_fence_before();
+      if (C::TS && lane == 0) bulk_wait_read_all();      // the box of the item before
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
+#pragma unroll
+      for (int u = 0; u < NCH; ++u) {
+        const int ch = g + 4 * u;
+        const bool is_dk = ch >= HD / 32;
+        if (u > 0) {
+          if (lane == 0) bulk_wait_read_all();
+          __syncwarp();
+        }
+        store_out32(box, lane, r[u], is_dk ? p.scale : 1.f, &out.m[is_dk ? 1 : 0], (is_dk ? ch - HD / 32 : ch) * 32,
+                    kb * AT_T + qd * 32, h, b, p.S);
+      }
+    };
+    // head_dim 64: an item's output leaves behind the first block of the next item, so the exponentials wait neither for its last
+    // products nor for the drain (between two items' blocks went ~3300 cycles, 800 of them for the products and 2100 for the
+    // output, where a block takes 1830: B8 S1024 H12 causal, five items a CTA, 45.7 -> 39.7 us).  head_dim 128: it is staged in
+    // the dS^T tile and leaves at once (B4 S2048 H16 149 -> 142 us by the TMA stores alone).
+    int late_kb = -1, late_b = 0, late_h = 0;
 #pragma unroll 1
     for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
       const int kb = p.by_hb.div(item), hb = item - kb * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
@@ -394,6 +425,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tmem_ld32(tmem_base + C::TM_DPT + c0 + lane_sel, rd);
         tmem_ld_wait();
         tc_fence_before();
+        // (head_dim 128: behind st_free every warp's output has left the dS^T tile)
+        if (!C::TS && it == 0 && lane == 0) bulk_wait_read_all();
         __syncwarp();
         if (lane == 0) mbar_arrive(st_free);      // one arrival per warp
         const float4* sl4 = reinterpret_cast<const float4*>(stat + st * 256 + c0);
@@ -428,6 +461,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(pt_ready);      // one arrival per warp
+          if (late_kb >= 0) {                        // (acc_done of its last block was waited for above)
+            drain(late_kb, late_b, late_h);
+            late_kb = -1;
+          }
         } else {
           f32x2 e[16];
 #pragma unroll
@@ -462,28 +499,18 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         rq.step();
         blk ^= 1u;
       }
-      if (!ok || !mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-      // 2 HD / 32 column chunks (dV first, then dK) spread over the four groups
-      constexpr int NCH = 2 * HD / 32 / 4;
-      uint32_t r[NCH][32];
-#pragma unroll
-      for (int u = 0; u < NCH; ++u) tmem_ld32(tmem_base + C::TM_DV + (g + 4 * u) * 32 + lane_sel, r[u]);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_free);
-#pragma unroll
-      for (int u = 0; u < NCH; ++u) {
-        const int ch = g + 4 * u;
-        const bool is_dk = ch >= HD / 32;
-        const int c = (is_dk ? ch - HD / 32 : ch) * 32;
-        const long long bs = is_dk ? p.dk_bs : p.dv_bs, ss = is_dk ? p.dk_ss : p.dv_ss, hs = is_dk ? p.dk_hs : p.dv_hs;
-        const int r0 = k0 + qd * 32;
-        store_out32(smem + C::OFF_DST, qd, c0, lane, r[u], is_dk ? p.scale : 1.f,
-                    (is_dk ? p.dk : p.dv) + b * bs + r0 * ss + h * hs + c, ss, p.S - r0);
+      if (!ok) break;
+      if (C::TS) {
+        late_kb = kb;
+        late_b = b;
+        late_h = h;
+        continue;
       }
+      if (!mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      drain(kb, b, h);
     }
+    if (ok && late_kb >= 0 && mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) drain(late_kb, late_b, late_h);
+    if (lane == 0) bulk_wait_read_all();
   }
 
   if (*abort_f) {
@@ -504,8 +531,8 @@ struct DqCfg {
   // size 128: 126 -> 110 us.)
   static constexpr int KS = (HD == 64) ? 4 : 3;
   static constexpr int VS = (HD == 64) ? 4 : 2;
-  static constexpr int OFF_QDO = 0;                      // [QB] Q, dO; the item's output leaves through them
-  static constexpr int OFF_K = QB * 2 * TILE;            // [KS]
+  static constexpr int OFF_QDO = 0;                      // [QB] Q, dO
+  static constexpr int OFF_K = QB * 2 * TILE;            // [KS]; an item's output leaves through its last one
   static constexpr int OFF_V = OFF_K + KS * TILE;        // [VS]
   static constexpr int OFF_BAR = OFF_V + VS * TILE;
   static constexpr int OFF_DELTA = OFF_BAR + 512;        // [2] rowsum(dO o O) of an item's rows
@@ -518,7 +545,11 @@ struct DqCfg {
   static_assert(SMEM <= 232448, "shared memory");
 };
 
-// Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.
+// Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.  Between two items: the Q and
+// dO tiles go back to the loader with the last score products, delta of the next item is made under the last dQ product, and
+// the output leaves through the K tile of the last block, which the loader gets back when it has left.  (Staged in the Q tile, with
+// one such buffer for head_dim 128, an item waited ~2500 cycles for its tiles and made delta behind them: B4 S2048 H16 causal
+// 111 -> 101 us, B8 S1024 H12 head size 64 43.2 -> 40.6 us.)
 //
 // It also makes delta = rowsum(dO o O), which the dK / dV kernel behind it reads: dO is in shared memory here anyway and the
 // item's share of O is fetched one item ahead, so the sums run under the item's first score products.  (A kernel of its own
@@ -528,12 +559,12 @@ template <int HD>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                   const AttnArgs p) {
+                   const __grid_constant__ CUtensorMap tmDQ, const AttnArgs p) {
   using C = DqCfg<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
   uint64_t* qdo_full = bars;        // [2]
-  uint64_t* qdo_empty = bars + 2;   // [2] the item's output has left (one arrival per warp)
+  uint64_t* qdo_empty = bars + 2;   // [2] the item's score products are done, its delta is made (one arrival per warp)
   uint64_t* k_full = bars + 4;      // [4]
   uint64_t* k_empty = bars + 8;     // [4]
   uint64_t* v_full = bars + 12;     // [4]
@@ -544,7 +575,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* acc_done = bars + 24;   // [2] dQ product that read the buffer done
   uint64_t* acc_free = bars + 26;   // the item's dQ copied to registers (one arrival per warp)
   uint64_t* d_ready = bars + 27;    // the item's delta is in shared memory (one arrival per warp)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
+  uint64_t* out_done = bars + 28;   // [4] the output that went through the K tile has left it (one arrival per warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 32);
   int* abort_f = reinterpret_cast<int*>(tmem_slot + 1);
   const int warp = warp_index(), lane = threadIdx.x & 31;
   WaitCtx ctx{p.status, abort_f};
@@ -555,9 +587,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     return;
   }
   if (threadIdx.x == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(&out_done[i], BW_MATH);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], BW_MATH);
+      mbar_init(&qdo_empty[i], BW_MATH + 1);
       mbar_init(&ds_ready[i], BW_MATH);
       mbar_init(&acc_done[i], 1);
     }
@@ -598,6 +631,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     Ring<C::KS> rk;
     Ring<C::VS> rv;
     bool ok = true;
+    uint32_t staged = 0, staged_ph = 0;      // K tiles that an output goes through, parities of out_done
 #pragma unroll 1
     for (int item = walk.next(); ok && item >= 0; item = walk.next()) {
       const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
@@ -614,6 +648,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll 1
       for (int j = 0; j < nkv; ++j) {
         if (!mbar_wait_warp(&k_empty[rk.s], rk.ph ^ 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+        if ((staged >> rk.s) & 1u) {
+          if (!mbar_wait_warp(&out_done[rk.s], (staged_ph >> rk.s) & 1u, ctx, FT_ERR_WAIT_EMPTY)) { ok = false; break; }
+          staged &= ~(1u << rk.s);
+          staged_ph ^= 1u << rk.s;
+        }
+        if (j == nkv - 1) staged |= 1u << rk.s;
         if (elect_one()) {
           mbar_arrive_expect_tx(&k_full[rk.s], C::TILE);
           load_tile<HD>(smem + C::OFF_K + rk.s * C::TILE, &tmK, &k_full[rk.s], j * AT_T, h, b);
@@ -660,6 +700,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           mma_kmajor<HD>(tmem_base + C::TM_DP, do_addr, v_addr + rv.s * C::TILE, idesc_s);
           umma_commit(s_full);
           umma_commit(&v_empty[rv.s]);
+          if (j == nkv - 1) umma_commit(&qdo_empty[rq.s]);
         }
         __syncwarp();
         rv.step();
@@ -727,15 +768,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     };
     Ring<C::QB> rq;
-    int item = walk.next();
-    fetch_rows(item);
-    while (ok && item >= 0) {
-      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
-      const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
-      const f32x2 nl = pk2(-lse_n, -lse_n);
-      if (!mbar_wait_warp(&qdo_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL)) { ok = false; break; }
+    Ring<C::KS> rk;
+    // delta of an item, from its dO tile and the rows that were fetched
+    auto make_delta = [&](int item, uint32_t buf) -> bool {
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, q0 = qb * AT_T;
+      if (!mbar_wait_warp(&qdo_full[rq.s], rq.ph, ctx, FT_ERR_WAIT_FULL)) return false;
       const uint8_t* do_tile = smem + C::OFF_QDO + (rq.s * 2 + 1) * C::TILE + (d_seg >> 3) * AT_REGION;
-      float* s_dl = s_delta + it_ph * AT_T;
+      float* s_dl = s_delta + buf * AT_T;
 #pragma unroll
       for (int u = 0; u < C::U; ++u) {
         const int r = d_row + u * C::RPS;
@@ -755,13 +794,35 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (q0 + r < p.S) p.delta[(long long)hb * p.S + q0 + r] = acc;
         }
       }
+      fence_proxy_async_smem();      // the dO tile goes back to the loader
       __syncwarp();
-      if (lane == 0) mbar_arrive(d_ready);
+      if (lane == 0) {
+        mbar_arrive(d_ready);
+        mbar_arrive(&qdo_empty[rq.s]);
+      }
+      rq.step();
+      return true;
+    };
+    int item = walk.next();
+    fetch_rows(item);
+    ok = item >= 0 && make_delta(item, 0);
+    int staged = -1;                       // K tile that this warp's last output has not yet left
+    auto output_left = [&] {
+      if (staged >= 0 && lane == 0) {
+        bulk_wait_read_all();
+        mbar_arrive(&out_done[staged]);
+      }
+      staged = -1;
+    };
+    while (ok && item >= 0) {
+      const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
+      const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
+      const f32x2 nl = pk2(-lse_n, -lse_n);
       item = walk.next();
       fetch_rows(item);
       if (!mbar_wait_warp(d_ready, it_ph, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
+      const float dl_row = -s_delta[it_ph * AT_T + row];
       it_ph ^= 1u;
-      const float dl_row = -s_dl[row];
       const f32x2 dl = pk2(dl_row, dl_row);
       const int last_col = p.causal ? min(grow, p.S - 1) : p.S - 1;                 // last valid key of this row
       const int warp_last = p.causal ? min(q0 + qd * 32, p.S - 1) : p.S - 1;       // of the warp's first row
@@ -799,7 +860,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (lane == 0) mbar_arrive(&ds_ready[rd.s]);      // one arrival per warp
         rd.step();
         blk ^= 1u;
+        if (j == 0) output_left();
+        if (j + 1 < nkv) rk.step();
       }
+      // under the last product: delta of the next item (whose tiles were loaded under the last block)
+      if (ok && item >= 0) ok = make_delta(item, it_ph);
       // the buffer of the last block is the one before rd
       if (!ok || !mbar_wait_warp(&acc_done[rd.s ^ 1], rd.s == 0 ? rd.ph ^ 1u : rd.ph, ctx, FT_ERR_WAIT_TMEM_FULL)) {
         ok = false;
@@ -813,17 +878,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_free);
-        const int r0 = q0 + qd * 32;
-        store_out32(smem + C::OFF_QDO + rq.s * 2 * C::TILE, qd, c0, lane, r, p.scale,
-                    p.dq + b * p.dq_bs + r0 * p.dq_ss + h * p.dq_hs + c0, p.dq_ss, p.S - r0);
-        fence_proxy_async_smem();        // the tiles go back to the loader
-        __syncwarp();
+        store_out32(smem + C::OFF_K + rk.s * C::TILE + warp * BW_BOX, lane, r, p.scale, &tmDQ, c0, q0 + qd * 32, h, b, p.S);
       } else if (lane == 0) {
         mbar_arrive(acc_free);
       }
-      if (lane == 0) mbar_arrive(&qdo_empty[rq.s]);
-      rq.step();
+      staged = rk.s;
+      rk.step();
     }
+    output_left();
   }
 
   if (*abort_f) {
@@ -836,12 +898,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
 template <int HD>
 static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tdq;
+  DkvMaps out;
   int rc;
   if ((rc = make_map(&tq, a->q, a, a->q_bs, a->q_ss, a->q_hs))) return rc;
   if ((rc = make_map(&tk, a->k, a, a->k_bs, a->k_ss, a->k_hs))) return rc;
   if ((rc = make_map(&tv, a->v, a, a->v_bs, a->v_ss, a->v_hs))) return rc;
   if ((rc = make_map(&tdo, a->d_o, a, a->o_bs, a->o_ss, a->o_hs))) return rc;
+  if ((rc = make_map(&tdq, a->dq, a, a->q_bs, a->q_ss, a->q_hs, true))) return rc;
+  if ((rc = make_map(&out.m[1], a->dk, a, a->k_bs, a->k_ss, a->k_hs, true))) return rc;
+  if ((rc = make_map(&out.m[0], a->dv, a, a->v_bs, a->v_ss, a->v_hs, true))) return rc;
   AttnArgs p;
   fill_args(p, a);
   if (!p.status) return -6;
@@ -855,8 +921,8 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   if (nrows > 0x7fffffffll) return -2;
   unsigned grid = 0;
   if ((rc = set_items(p, a, AT_T, &grid))) return rc;
-  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);      // writes delta
-  launch_pdl(attn_bwd_dkv_kernel<HD>, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, p);
+  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, tdq, p);      // writes delta
+  launch_pdl(attn_bwd_dkv_kernel<HD>, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, out, p);
   return (int)cudaGetLastError();
 }
 
