@@ -85,7 +85,7 @@ struct FwdItem {
 template <int HD>
 __global__ void __launch_bounds__(F2_THREADS, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                 const __grid_constant__ CUtensorMap tmV, const AttnArgs p) {
+                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const AttnArgs p) {
   using C = Fwd2Cfg<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);
@@ -414,10 +414,11 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&o_free[t]);
-      // The output leaves through the warp's 32 rows of the Q tile, which the scores no longer need: eight lanes write 128
-      // contiguous bytes of a row.
+      // The output leaves through the warp's 32 rows of the Q tile, which the scores no longer need, by the TMA unit, which cuts
+      // off the rows past the end.  (Read back and stored 128 bytes of a row by eight lanes: B8 S1024 H12 head size 64 causal 27.6 us,
+      // 26.6 so; 1 x 1500 x 20 21.8 and 21.6; head size 128 unchanged.  Leaving it behind the next item's first block, as the
+      // backward kernels do, cost the block loop registers: 30.3 -> 32.1 us.)
       const int r0 = it.q0 + t * AT_T + qd * 32;
-      __nv_bfloat16* op = p.o + it.b * p.o_bs + r0 * p.o_ss + it.h * p.o_hs;
       uint8_t* stage = smem + C::OFF_Q + q_slot * C::TILE + qd * 32 * 128;
 #pragma unroll
       for (int c = 0; c < HD; c += 64) {
@@ -431,19 +432,16 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           *reinterpret_cast<uint4*>(stage + (c / 64) * AT_REGION + lane * 128 + (((i >> 3) ^ (lane & 7)) << 4)) = u;
         }
       }
+      fence_proxy_async_smem();
       __syncwarp();
+      if (lane == 0) {
+        if (r0 < p.S) {
 #pragma unroll
-      for (int c = 0; c < HD; c += 64) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int rr = 4 * i + (lane >> 3), seg = lane & 7;
-          const uint4 u = *reinterpret_cast<const uint4*>(stage + (c / 64) * AT_REGION + rr * 128 + ((seg ^ (rr & 7)) << 4));
-          if (r0 + rr < p.S) *reinterpret_cast<uint4*>(op + rr * p.o_ss + c + seg * 8) = u;
+          for (int c = 0; c < HD; c += 64) tma_store_4d(&tmO, stage + (c / 64) * AT_REGION, c, r0, it.h, it.b);
+          bulk_wait_read_all();
         }
+        mbar_arrive(&q_empty[q_slot]);       // the tile goes back to the loader
       }
-      fence_proxy_async_smem();        // the tile goes back to the loader
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&q_empty[q_slot]);
       if (p.lse && grow < p.S)
         p.lse[((long long)it.b * p.H + it.h) * p.S + grow] = (l > 0.f) ? m2 + log2f(l) : -INFINITY;
     }
@@ -459,11 +457,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 template <int HD>
 static int attn_fwd2_launch(const FtkAttnDesc* a, cudaStream_t s) {
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   int rc;
   if ((rc = make_map(&tq, a->q, a, a->q_bs, a->q_ss, a->q_hs))) return rc;
   if ((rc = make_map(&tk, a->k, a, a->k_bs, a->k_ss, a->k_hs))) return rc;
   if ((rc = make_map(&tv, a->v, a, a->v_bs, a->v_ss, a->v_hs))) return rc;
+  if ((rc = make_map(&to, a->o, a, a->o_bs, a->o_ss, a->o_hs, 64, 32))) return rc;
   AttnArgs p;
   fill_args(p, a);
   if (!p.status) return -6;
@@ -474,7 +473,7 @@ static int attn_fwd2_launch(const FtkAttnDesc* a, cudaStream_t s) {
   }
   unsigned grid = 0;
   if ((rc = set_items(p, a, 2 * AT_T, &grid))) return rc;
-  launch_pdl(attn_fwd2_kernel<HD>, grid, F2_THREADS, Fwd2Cfg<HD>::SMEM, s, tq, tk, tv, p);
+  launch_pdl(attn_fwd2_kernel<HD>, grid, F2_THREADS, Fwd2Cfg<HD>::SMEM, s, tq, tk, tv, to, p);
   return (int)cudaGetLastError();
 }
 

@@ -122,9 +122,9 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, u
 
 
 // ------------------------------------------------------------------------------- host helpers
-// `out`: boxes of 32 columns x 32 rows that a warp stores, else the tiles that are loaded.
+// Boxes of `cols` x `rows`: the tiles that are loaded, or what a warp stores (32 columns: 64-byte swizzle).
 static inline int make_map(CUtensorMap* m, const void* base, const FtkAttnDesc* a, long long bs,
-                    long long ss, long long hs, bool out = false) {
+                    long long ss, long long hs, unsigned cols = 64, unsigned rows = AT_T) {
   // dims {hd, S, H, B}; strides in elements
   typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                          const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -143,10 +143,10 @@ static inline int make_map(CUtensorMap* m, const void* base, const FtkAttnDesc* 
   cuuint64_t dims[4] = {(cuuint64_t)a->hd, (cuuint64_t)a->S, (cuuint64_t)a->H, (cuuint64_t)a->B};
   cuuint64_t strides[3] = {(cuuint64_t)ss * 2, (cuuint64_t)(a->H > 1 ? hs : a->hd) * 2,
                            (cuuint64_t)(a->B > 1 ? bs : (long long)a->S * ss) * 2};
-  cuuint32_t box[4] = {out ? 32u : 64u, out ? 32u : (cuuint32_t)AT_T, 1, 1};
+  cuuint32_t box[4] = {cols, rows, 1, 1};
   cuuint32_t es[4] = {1, 1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides,
-                   box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, out ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                   box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
 }
