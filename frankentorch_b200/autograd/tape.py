@@ -15,6 +15,7 @@ golden ft_autograd__tests__tensor_scheduler_telemetry_golden.snap.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass, field, replace
 from typing import Any, Callable, Dict, List, Optional, Sequence, Tuple
 
@@ -329,6 +330,15 @@ class TensorHookHandle:
     hook_id: int
 
 
+_DEFAULT_OPTIONS = BackwardOptions()
+
+
+@functools.lru_cache(maxsize=256)
+def _i64_array(n: int):
+    """The ctypes array type (making one costs more than an instance)."""
+    return C.c_int64 * n
+
+
 class TensorTape:
     """Append-only tape of tensor operations with a deterministic backward pass."""
 
@@ -374,7 +384,7 @@ class TensorTape:
         return len(self.nodes)
 
     def _append(self, op, inputs, value, requires_grad, is_leaf, vjp, rule) -> int:
-        arr = (C.c_int64 * max(1, len(inputs)))(*inputs)
+        arr = _i64_array(max(1, len(inputs)))(*inputs)
         nid = self._lib.ftc_tape_add_node(self._h, arr, len(inputs), int(requires_grad), int(is_leaf))
         if nid < 0:
             raise UnknownTensorNode(f"invalid input ids {inputs}")
@@ -685,9 +695,7 @@ class TensorTape:
     # ------------------------------------------------------------------ backward
     def schedule(self, root: int, check_consumed: bool = True):
         n = len(self.nodes)
-        order = (C.c_int64 * max(1, n))()
-        deps = (C.c_int64 * max(1, n))()
-        stats = (C.c_int64 * 3)()
+        order, deps, stats = _i64_array(max(1, n))(), _i64_array(max(1, n))(), _i64_array(3)()
         cnt = self._lib.ftc_tape_schedule(self._h, root, int(check_consumed), order, deps, stats)
         if cnt == -1:
             raise UnknownTensorNode(f"node {root}")
@@ -706,7 +714,7 @@ class TensorTape:
 
     def backward(self, root: int, options: Optional[BackwardOptions] = None,
                  seed: Optional[torch.Tensor] = None) -> TensorBackwardReport:
-        opts = options or BackwardOptions()
+        opts = options or _DEFAULT_OPTIONS
         guard = fallback = False
         if opts.current_reentrant_depth > opts.max_reentrant_depth:
             if opts.policy == ReentrantPolicy.StrictFail:

@@ -554,6 +554,21 @@ extern "C" int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits) {
   return plan_gemm(g, bn, splits);
 }
 
+// (one event per device and thread, re-recorded per call: another thread's record between this one's record and wait would
+// order the second stream behind the wrong work)
+extern "C" int ftk_stream_order(void* first, void* then) {
+  static thread_local cudaEvent_t ev[64] = {nullptr};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+  if (!ev[dev]) {
+    cudaError_t e = cudaEventCreateWithFlags(&ev[dev], cudaEventDisableTiming);
+    if (e != cudaSuccess) return (int)e;
+  }
+  cudaError_t e = cudaEventRecord(ev[dev], reinterpret_cast<cudaStream_t>(first));
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(then), ev[dev], 0);
+  return (int)e;
+}
+
 extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   int bn = 0, splits = 1;
@@ -594,18 +609,8 @@ extern "C" int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream_v) {
   if (blocks > 148 * 8) blocks = 148 * 8;
   cudaStream_t rs = g->reduce_stream ? reinterpret_cast<cudaStream_t>(g->reduce_stream) : stream;
   if (rs != stream) {
-    // reduction on its own stream, ordered behind the GEMM (one event per device and thread, re-recorded per call: another
-    // thread's record between this one's record and wait would order the reduction behind the wrong GEMM)
-    static thread_local cudaEvent_t ev[64] = {nullptr};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    if (!ev[dev]) {
-      cudaError_t e = cudaEventCreateWithFlags(&ev[dev], cudaEventDisableTiming);
-      if (e != cudaSuccess) return (int)e;
-    }
-    cudaError_t e = cudaEventRecord(ev[dev], stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(rs, ev[dev], 0);
-    if (e != cudaSuccess) return (int)e;
+    const int erc = ftk_stream_order(stream, rs);      // reduction on its own stream, ordered behind the GEMM
+    if (erc) return erc;
   }
   launch_pdl(splitk_reduce_kernel, (unsigned)blocks, 256, 0, rs, a.ws, g->D, g->M, g->N, g->ldd, splits,
                                                          g->out_fp32, g->accumulate);

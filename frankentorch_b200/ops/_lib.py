@@ -160,6 +160,7 @@ def load(build_if_missing: bool = True):
         "ftk_present_rgba8": [vp, vp, i, i, ll, i, vp],
         "ftk_im2col_1d": [vp, vp, i, i, i, i, i, i, vp],
         "ftk_wait_probe": [vp, i, ll, vp, vp],
+        "ftk_stream_order": [vp, vp],
     }
     # descriptors packed by GEMM_DESC / ATTN_DESC (a second function object per entry: argument types are per object)
     for name, sym in (("gemm_packed", "ftk_gemm_bf16"), ("attn_fwd_packed", "ftk_attn_fwd"),

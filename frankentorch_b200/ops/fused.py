@@ -41,8 +41,9 @@ class SideWork:
         self.tape, self.device = tape, device
         self.on = SideWork.enabled and device.type == "cuda"
         self._marks = []
-        self._held = []            # partial tiles of split products, read on the side stream until the join
+        self._held = []            # scratch and operands of the side stream's kernels, until the join
         self._saved_fn = None
+        self.main = self.side = 0  # raw handles
 
     @classmethod
     def stream_for(cls, device: torch.device) -> torch.cuda.Stream:
@@ -53,11 +54,13 @@ class SideWork:
 
     def __enter__(self):
         if self.on:
-            self.main = torch.cuda.current_stream(self.device)
-            self.side = SideWork.stream_for(self.device)
-            ev = torch.cuda.Event()
-            ev.record(self.main)
-            self.side.wait_event(ev)
+            dev = self.device.index
+            if dev is not None and dev != K._get_device():
+                self.on = False    # the kernels go to the current device's stream: there is nothing to overlap with
+                return self
+            self.main = K._stream()
+            self.side = SideWork.stream_for(self.device).cuda_stream
+            K.stream_order(self.main, self.side)
             self._saved_fn = self.tape.leaf_grad_written_fn
             if self._saved_fn is not None:
                 self.tape.leaf_grad_written_fn = self._marks.append      # held back until the join
@@ -65,9 +68,7 @@ class SideWork:
 
     def __exit__(self, *exc):
         if self.on:
-            ev = torch.cuda.Event()
-            ev.record(self.side)
-            self.main.wait_event(ev)
+            K.stream_order(self.side, self.main)
             self._held.clear()
             self.tape.leaf_grad_written_fn = self._saved_fn
             if self._saved_fn is not None and exc[0] is None:
@@ -75,18 +76,22 @@ class SideWork:
                     self._saved_fn(nid)
         return False
 
+    def sees_main(self) -> None:
+        """The side stream waits for what the main stream holds now."""
+        if self.on:
+            K.stream_order(self.main, self.side)
+
     def wgrad(self, dy2d, x2d, out=None, accumulate=False):
         """Weight gradient GEMM on the main stream; its split-K reduction (if any) on the side stream."""
         if not self.on:
             return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate)
-        return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate, reduce_stream=self.side.cuda_stream,
-                              keep=self._held)
+        return K.linear_wgrad(dy2d, x2d, out=out, accumulate=accumulate, reduce_stream=self.side, keep=self._held)
 
     def colsum(self, dy2d, out=None, accumulate=False):
         if not self.on:
             return K.colsum(dy2d, out=out, accumulate=accumulate)
-        with torch.cuda.stream(self.side):
-            return K.colsum(dy2d, out=out, accumulate=accumulate)
+        self._held.append(dy2d)
+        return K.colsum(dy2d, out=out, accumulate=accumulate, stream=self.side, keep=self._held)
 
 
 class WgradQueue:
@@ -206,7 +211,7 @@ def linear(tape: TensorTape, x: int, w: int, b: Optional[int] = None, *, act: Op
     epi = {None: K.EPI_NONE, "gelu_tanh": K.EPI_GELU_TANH, "gelu_erf": K.EPI_GELU_ERF, "relu": K.EPI_RELU}[act]
     depi = {None: K.EPI_NONE, "gelu_tanh": K.EPI_MUL_DGELU_TANH, "gelu_erf": K.EPI_MUL_DGELU_ERF,
             "relu": K.EPI_MUL_DRELU}[act]
-    aux = torch.empty((x2.shape[0], wv.shape[0]), dtype=torch.bfloat16, device=xv.device) if act else None
+    aux = xv.new_empty((x2.shape[0], wv.shape[0]), dtype=torch.bfloat16) if act else None
     r2 = _rows(rv) if rv is not None else None
     y = K.linear_fwd(x2, wv, bv, epi=epi, resid=r2, aux=aux)
     if xv.dim() != 2:
@@ -250,7 +255,7 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
     r2 = _rows(rv)
     epi = {"gelu_tanh": K.EPI_GELU_TANH, "gelu_erf": K.EPI_GELU_ERF, "relu": K.EPI_RELU}[act]
     depi = {"gelu_tanh": K.EPI_MUL_DGELU_TANH, "gelu_erf": K.EPI_MUL_DGELU_ERF, "relu": K.EPI_MUL_DRELU}[act]
-    u = torch.empty((x2.shape[0], w1v.shape[0]), dtype=torch.bfloat16, device=xv.device)
+    u = xv.new_empty((x2.shape[0], w1v.shape[0]), dtype=torch.bfloat16)
     h = K.linear_fwd(x2, w1v, b1v, epi=epi, aux=u)
     y = _as(K.linear_fwd(h, w2v, b2v, resid=r2), rv)
 
@@ -260,11 +265,7 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
             db2 = _bgrad_into(targets, 4, g2, side)
             dw2 = _wgrad_into(targets, 3, g2, h, side)
             du = K.linear_dgrad(g2, w2v, epi=depi, resid=u)      # (dY @ w2) * act'(U)
-            # du is produced on the main stream: the side stream must see it before it sums its columns
-            if side.on:
-                ev = torch.cuda.Event()
-                ev.record(side.main)
-                side.side.wait_event(ev)
+            side.sees_main()         # du is produced on the main stream, its columns are summed on the side stream
             db1 = _bgrad_into(targets, 2, du, side)
             dw1 = _wgrad_into(targets, 1, du, x2, side)
             dx = _as(K.linear_dgrad(du, w1v), xv)
@@ -327,12 +328,13 @@ def attention_packed(tape: TensorTape, qkv: int, n_heads: int, *, causal: bool =
     B, S, d3 = qv.shape
     d = d3 // 3
     hd = d // n_heads
-    q, k, v = (qv[:, :, i * d:(i + 1) * d].view(B, S, n_heads, hd) for i in range(3))
+    split = lambda t: (t if d3 == 3 * d else t[:, :, :3 * d]).view(B, S, 3, n_heads, hd).unbind(2)      # noqa: E731
+    q, k, v = split(qv)
     o, lse = K.attention_fwd(q, k, v, causal=causal, scale=scale)
 
     def vjp(go, targets):
         dqkv = torch.empty_like(qv)
-        dq, dk, dv = (dqkv[:, :, i * d:(i + 1) * d].view(B, S, n_heads, hd) for i in range(3))
+        dq, dk, dv = split(dqkv)
         K.attention_bwd(q, k, v, o, lse, go.reshape(B, S, n_heads, hd), causal=causal, scale=scale,
                         dq=dq, dk=dk, dv=dv)
         return [dqkv]

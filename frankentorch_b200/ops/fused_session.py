@@ -77,7 +77,7 @@ class FusedSession:
     def _check_mm(self, a: torch.Tensor, k: int, n: int, bias: Optional[torch.Tensor]) -> None:
         if a.dim() != 2 or a.shape[1] != k:
             raise FusedKernelError(f"matmul_bias: a is {tuple(a.shape)}, the weight is [{k}, {n}]")
-        if bias is not None and tuple(bias.shape) != (n,):
+        if bias is not None and bias.shape != (n,):
             raise FusedKernelError(f"matmul_bias: bias is {tuple(bias.shape)}, expected ({n},)")
 
     def matmul_bias(self, a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -92,7 +92,7 @@ class FusedSession:
         """The same over a resident weight: no per-call layout work.  ``gelu`` and ``resid`` fold the activation
         and the residual add into the GEMM epilogue (the reference launches them as separate kernels)."""
         self._check_mm(a, w.rows, w.cols, bias)
-        if resid is not None and tuple(resid.shape) != (a.shape[0], w.cols):
+        if resid is not None and resid.shape != (a.shape[0], w.cols):
             raise FusedKernelError(f"matmul_bias_w16: resid is {tuple(resid.shape)}")
         return self.K.gemm(a, w.data, bias=bias, resid=resid, epi=self.K.EPI_GELU_TANH if gelu else self.K.EPI_NONE)
 

@@ -125,7 +125,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     their output rows are left as they were (expert batches with capacity padding).
     """
     _bf16(a, "a"), _bf16(b, "b")
-    if a.dim() != 2 or b.dim() != 2 or a.stride(1) != 1 or b.stride(1) != 1:
+    sa, sb = a.stride(), b.stride()
+    if len(sa) != 2 or len(sb) != 2 or sa[1] != 1 or sb[1] != 1:
         raise KernelError("gemm operands must be 2-D with unit inner stride")
     M, K = a.shape
     if a_mn:
@@ -136,10 +137,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if K != Kb:
         raise KernelError(f"gemm K mismatch: {K} vs {Kb}")
     if out is None:
-        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    ldd, out_inner = out.stride() if out.dim() == 2 else (0, 0)
-    if out.shape != (M, N) or out_inner != 1:
-        raise KernelError("gemm output must be [M, N] with unit inner stride")
+        out = a.new_empty((M, N), dtype=out_dtype)
+        ldd = N
+    else:
+        ldd, out_inner = out.stride() if out.dim() == 2 else (0, 0)
+        if out.shape != (M, N) or out_inner != 1:
+            raise KernelError("gemm output must be [M, N] with unit inner stride")
+    out_t = out.dtype
     resid_ptr = ldr = aux_ptr = 0
     if resid is not None:
         _bf16(resid, "resid")
@@ -149,7 +153,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if aux.stride(0) != ldd:
             raise KernelError("aux must share the row stride of the output")
         aux_ptr = aux.data_ptr()
-    if out.dtype not in (torch.float32, torch.bfloat16):
+    if out_t is not torch.float32 and out_t is not torch.bfloat16:
         raise KernelError("gemm output must be bf16 or fp32")
     seg_ptr = 0
     if seg_counts is not None:
@@ -159,42 +163,41 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             raise KernelError("seg_counts needs one entry per segment of rows of a row-major A operand")
         seg_ptr = seg_counts.data_ptr()
     lib = _lib.load()
-    ws, ws_ptr, ws_bytes = None, 0, 0
-
-    def pack() -> bytes:
-        return _lib.GEMM_DESC.pack(
-            M, N, K, 1, 1, int(a_mn), int(b_mn), a.data_ptr(), a.stride(0), 0, 0, b.data_ptr(), b.stride(0), 0, 0,
+    # the descriptor's fields in front of the workspace and behind it
+    head = (M, N, K, 1, 1, int(a_mn), int(b_mn), a.data_ptr(), sa[0], 0, 0, b.data_ptr(), sb[0], 0, 0,
             out.data_ptr(), ldd, 0, 0, 0 if bias is None else bias.data_ptr(), resid_ptr, ldr, 0, 0, aux_ptr, float(alpha),
-            int(epi), 1 if out.dtype == torch.float32 else 0, int(accumulate), int(force_bn), int(max_ctas), ws_ptr,
-            ws_bytes, int(split_k), reduce_stream or 0, seg_ptr, int(seg_rows) if seg_ptr else 0)
-
-    def plan():
-        bn, sp = C.c_int(0), C.c_int(1)
-        rc = lib.ftk_gemm_plan(C.byref(FtkGemmDesc.from_buffer_copy(pack())), C.byref(bn), C.byref(sp))
-        return rc, bn.value, sp.value
+            int(epi), 1 if out_t is torch.float32 else 0, int(accumulate), int(force_bn), int(max_ctas))
+    tail = (int(split_k), reduce_stream or 0, seg_ptr, int(seg_rows) if seg_ptr else 0)
+    ws, ws_ptr, ws_bytes = None, 0, 0
     if split_k != 1 and K > SPLIT_ABOVE_K and bias is None and resid is None and aux is None and epi == EPI_NONE and \
             seg_counts is None:
         # Partial tiles go to scratch of this call alone, in the order of the launching stream: products of other
-        # streams, threads and captured graphs are never written over.
-        ws_ptr, ws_bytes = 256, GEMM_WORKSPACE_BYTES      # a stand-in: the plan looks at the size
-        rc, _, sp = plan()
-        ws_ptr = ws_bytes = 0
+        # streams, threads and captured graphs are never written over.  (256 stands for the scratch: the plan looks at the size.)
+        rc, _, sp = _gemm_plan(lib, _lib.GEMM_DESC.pack(*head, 256, GEMM_WORKSPACE_BYTES, *tail))
         if rc == 0 and sp > 1:
             ws = torch.empty(sp * M * N, dtype=torch.float32, device=a.device)
             ws_ptr, ws_bytes = ws.data_ptr(), sp * M * N * 4
+    desc = _lib.GEMM_DESC.pack(*head, ws_ptr, ws_bytes, *tail)
     what = "ftk_gemm_bf16"
     if _TRACE is not None:          # name the tile the planner picks for this problem
-        rc, bn, sp = plan()
+        rc, bn, sp = _gemm_plan(lib, desc)
         if rc == 0:
             what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn - 256, sp)) if bn > 256 else \
                 ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn, sp))
-    _chk(lib.gemm_packed(pack(), _stream()), what)
+    _chk(lib.gemm_packed(desc, _stream()), what)
     if reduce_stream is not None and ws is not None:
         if keep is not None:
             keep.append(ws)
         else:
             ws.record_stream(torch.cuda.ExternalStream(reduce_stream, device=a.device))
     return out
+
+
+def _gemm_plan(lib, desc: bytes) -> Tuple[int, int, int]:
+    """(status, tile code, splits) that the planner picks for a packed descriptor."""
+    bn, sp = C.c_int(0), C.c_int(1)
+    rc = lib.ftk_gemm_plan(C.byref(FtkGemmDesc.from_buffer_copy(desc)), C.byref(bn), C.byref(sp))
+    return rc, bn.value, sp.value
 
 
 def gemm_grouped(problems, *, a_mn: bool = True, b_mn: bool = True, max_ctas: int = 0) -> None:
@@ -273,26 +276,25 @@ def linear_wgrad(dy, x, *, out=None, accumulate=False, reduce_stream=None, keep=
 def _attn_desc(q, k, v, o, lse, causal, scale, d_o=0, delta=0, dq=0, dk=0, dv=0) -> bytes:
     # q/k/v/o: views of shape [B, S, H, hd] (any strides with unit inner stride)
     shape = q.shape
-    B, S, H, hd = shape
-    ptrs, strides = [], []
+    strides = []
     for name, t in (("q", q), ("k", k), ("v", v), ("o", o)):
         _bf16(t, name)
-        bs, ss, hs, inner = t.stride() if t.dim() == 4 else (0, 0, 0, 0)
-        if t.shape != shape or inner != 1:
+        st = t.stride()
+        if t.shape != shape or len(st) != 4 or st[3] != 1:
             raise KernelError(f"attention operand {name} must be [B,S,H,hd] with unit inner stride")
-        ptrs.append(t.data_ptr())
-        strides += (bs, ss, hs)
+        strides.append(st[:3])
+    B, S, H, hd = shape
     return _lib.ATTN_DESC.pack(B, H, S, hd, int(causal), float(scale if scale is not None else 1.0 / math.sqrt(hd)),
-                               ptrs[0], ptrs[1], ptrs[2], *strides[:9], ptrs[3], *strides[9:], lse.data_ptr(), d_o, delta,
-                               dq, dk, dv)
+                               q.data_ptr(), k.data_ptr(), v.data_ptr(), *strides[0], *strides[1], *strides[2],
+                               o.data_ptr(), *strides[3], lse.data_ptr(), d_o, delta, dq, dk, dv)
 
 
 def attention_fwd(q, k, v, *, causal=True, scale=None, out=None):
     """Flash attention forward.  q/k/v: ``[B, S, H, hd]`` bf16 views.  Returns ``(o, lse)``."""
     B, S, H, hd = q.shape
     if out is None:
-        out = torch.empty((B, S, H, hd), dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
+        out = q.new_empty((B, S, H, hd), dtype=torch.bfloat16)
+    lse = q.new_empty((B, H, S), dtype=torch.float32)
     d = _attn_desc(q, k, v, out, lse, causal, scale)
     _chk(_lib.load().attn_fwd_packed(d, _stream()), "ftk_attn_fwd")
     return out, lse
@@ -307,7 +309,7 @@ def attention_bwd(q, k, v, o, lse, d_o, *, causal=True, scale=None, dq=None, dk=
     for name, t, ref in (("dq", dq, q), ("dk", dk, k), ("dv", dv, v), ("d_o", d_o, o)):
         if t.stride() != ref.stride():
             raise KernelError(f"{name} must share the strides of its primal")
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
+    delta = q.new_empty((B, H, S), dtype=torch.float32)
     d = _attn_desc(q, k, v, o, lse, causal, scale, d_o.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(),
                    dv.data_ptr())
     _chk(_lib.load().attn_bwd_packed(d, _stream()), "ftk_attn_bwd")
@@ -319,8 +321,7 @@ def layernorm_fwd(x, gamma, beta, eps=1e-5, resid=None, out=None):
     """Returns ``(y, mean, rstd, x_sum)``; ``x_sum`` is ``x + resid`` when ``resid`` is given."""
     rows, cols = x.shape
     y = torch.empty_like(x) if out is None else out
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+    mean, rstd = x.new_empty(rows, dtype=torch.float32), x.new_empty(rows, dtype=torch.float32)
     xs = torch.empty_like(x) if resid is not None else None
     _chk(_lib.load().ftk_layernorm_fwd(x.data_ptr(), _ptr(resid), _ptr(xs), gamma.data_ptr(),
                                        _ptr(beta), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
@@ -334,11 +335,10 @@ def layernorm_bwd(dy, x, gamma, mean, rstd, *, dx_add=None, dgamma=None, dbeta=N
     lib = _lib.load()
     dx = torch.empty_like(x) if out is None else out
     if dgamma is None:
-        dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
-        dbeta = torch.empty(cols, dtype=torch.float32, device=x.device)
+        dgamma, dbeta = x.new_empty(cols, dtype=torch.float32), x.new_empty(cols, dtype=torch.float32)
         accumulate = False
     nblk = lib.ftk_layernorm_bwd_blocks(rows)
-    partial = torch.empty(2 * nblk * cols, dtype=torch.float32, device=x.device)
+    partial = x.new_empty(2 * nblk * cols, dtype=torch.float32)
     _chk(lib.ftk_layernorm_bwd(dy.data_ptr(), x.data_ptr(), gamma.data_ptr(), mean.data_ptr(),
                                rstd.data_ptr(), _ptr(dx_add), dx.data_ptr(), dgamma.data_ptr(),
                                dbeta.data_ptr(), partial.data_ptr(), rows, cols, int(accumulate),
@@ -349,7 +349,7 @@ def layernorm_bwd(dy, x, gamma, mean, rstd, *, dx_add=None, dgamma=None, dbeta=N
 def rmsnorm_fwd(x, gamma, eps=1e-6):
     rows, cols = x.shape
     y = torch.empty_like(x)
-    rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
+    rstd = x.new_empty(rows, dtype=torch.float32)
     _chk(_lib.load().ftk_rmsnorm_fwd(x.data_ptr(), gamma.data_ptr(), y.data_ptr(), rstd.data_ptr(),
                                      rows, cols, float(eps), _stream()), "ftk_rmsnorm_fwd")
     return y, rstd
@@ -360,10 +360,10 @@ def rmsnorm_bwd(dy, x, gamma, rstd, *, dgamma=None, accumulate=False):
     lib = _lib.load()
     dx = torch.empty_like(x)
     if dgamma is None:
-        dgamma = torch.empty(cols, dtype=torch.float32, device=x.device)
+        dgamma = x.new_empty(cols, dtype=torch.float32)
         accumulate = False
     nblk = lib.ftk_layernorm_bwd_blocks(rows)
-    partial = torch.empty(nblk * cols, dtype=torch.float32, device=x.device)
+    partial = x.new_empty(nblk * cols, dtype=torch.float32)
     _chk(lib.ftk_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), gamma.data_ptr(), rstd.data_ptr(),
                              dx.data_ptr(), dgamma.data_ptr(), partial.data_ptr(), rows, cols,
                              int(accumulate), _stream()), "ftk_rmsnorm_bwd")
@@ -472,17 +472,30 @@ def dropout(x, p, seed, offset=0):
     return y
 
 
-def colsum(x, out=None, accumulate=False):
-    """fp32 column sums of a bf16 ``[rows, cols]`` matrix (bias gradient), fixed order."""
+def colsum(x, out=None, accumulate=False, *, stream: Optional[int] = None, keep: Optional[list] = None):
+    """fp32 column sums of a bf16 ``[rows, cols]`` matrix (bias gradient), fixed order.
+
+    ``stream`` (a raw stream handle) launches there instead of on the current stream.  The scratch belongs to the current
+    stream all the same and goes to ``keep``, which the caller drops behind its join of that stream; so does an ``out`` that is
+    allocated here."""
     rows, cols = x.shape
     lib = _lib.load()
     if out is None:
-        out = torch.empty(cols, dtype=torch.float32, device=x.device)
+        out = x.new_empty(cols, dtype=torch.float32)
         accumulate = False
-    partial = torch.empty(lib.ftk_colsum_blocks(rows) * cols, dtype=torch.float32, device=x.device)
+    partial = x.new_empty(lib.ftk_colsum_blocks(rows) * cols, dtype=torch.float32)
+    if keep is not None:
+        keep += (partial, out)
     _chk(lib.ftk_colsum_bf16(x.data_ptr(), out.data_ptr(), partial.data_ptr(), rows, cols, x.stride(0),
-                             int(accumulate), _stream()), "ftk_colsum_bf16")
+                             int(accumulate), _stream() if stream is None else stream), "ftk_colsum_bf16")
     return out
+
+
+def stream_order(first: int, then: int) -> None:
+    """Work queued on the raw stream ``then`` from here on waits for what ``first`` holds now (current device)."""
+    rc = _lib.load().ftk_stream_order(first, then)
+    if rc != 0:
+        raise KernelError(f"ftk_stream_order: returned {rc}")
 
 
 # --------------------------------------------------------------------------------------- embedding
