@@ -72,7 +72,7 @@ int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits);
 // Work queued on stream `then` from here on waits for what stream `first` holds now (both of the current device).
 int ftk_stream_order(void* first, void* then);
 // `n` (1..8) products with one K and one pair of operand layouts, fp32 outputs (store or accumulate), no other
-// epilogue, as one persistent launch of 256 x 192 CTA-pair tiles: the weight gradients of a transformer block fill the
+// epilogue, as one persistent launch of 256 x 192 or 256 x 384 CTA-pair tiles: the weight gradients of a transformer block fill the
 // GPU together where each alone would need split-K and a reduction kernel.
 int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream);
 int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n);      // the CTAs it takes (<= max_ctas).  No launch.

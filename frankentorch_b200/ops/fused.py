@@ -98,8 +98,8 @@ class WgradQueue:
     """Weight gradients of consecutive backward rules, collected and launched together.
 
     A weight gradient ``dW = dy^T x`` of a transformer block has 24 - 96 output tiles: alone it needs split-K
-    and a reduction kernel to occupy 148 SMs.  The four of a block together are two full waves of 256 x 192 tiles
-    on 74 CTA pairs (``K.gemm_grouped``), each output element reduced over the tokens by one pair in order.  A rule hands
+    and a reduction kernel to occupy 148 SMs.  The four of a block together fill one wave of 256 x 384 tiles or two of
+    256 x 192 on 74 CTA pairs (``K.gemm_grouped``), each output element reduced over the tokens by one pair in order.  A rule hands
     its weight gradient to the queue instead of launching it; the queue launches when it holds enough tiles
     (or eight problems) and when the backward pass ends (``TensorTape.backward`` calls :meth:`flush`).  The
     operands stay referenced until then; nothing in a backward pass writes them in place.  The observer of
