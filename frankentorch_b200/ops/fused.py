@@ -26,10 +26,11 @@ class SideWork:
     """Small memory-bound kernels of a backward rule (bias column sums, split-K reductions) run on a
     second stream next to the rule's GEMMs and are joined before the rule returns.
 
-    Entering makes the side stream wait for everything the main stream holds (the incoming gradient
-    is complete); leaving makes the main stream wait for the side stream, and only then tells the
-    tape's observer which parameter gradients were written (a data-parallel bucket must not start
-    before the split-K reduction that finishes its last gradient).  Nothing about the arithmetic
+    Each launch on the side stream is ordered behind everything the main stream holds at that point
+    (operands are complete, and scratch that was just taken from the main stream's pool is no longer in
+    use there); leaving makes the main stream wait for the side stream if anything was launched on it,
+    and only then tells the tape's observer which parameter gradients were written (a data-parallel
+    bucket must not start before the split-K reduction that finishes its last gradient).  Nothing about the arithmetic
     changes: the same kernels see the same data.  Works eagerly and under CUDA-graph capture (the
     fork and the join are captured as parallel branches).  ``FT_SIDE_STREAM=0`` keeps everything on
     one stream."""
@@ -41,7 +42,7 @@ class SideWork:
         self.tape, self.device = tape, device
         self.on = SideWork.enabled and device.type == "cuda"
         self._marks = []
-        self._held = []            # scratch and operands of the side stream's kernels, until the join
+        self._held = []            # scratch and operands of the side stream's kernels, until the join; empty: nothing to join
         self._saved_fn = None
         self.main = self.side = 0  # raw handles
 
@@ -60,7 +61,6 @@ class SideWork:
                 return self
             self.main = K._stream()
             self.side = SideWork.stream_for(self.device).cuda_stream
-            K.stream_order(self.main, self.side)
             self._saved_fn = self.tape.leaf_grad_written_fn
             if self._saved_fn is not None:
                 self.tape.leaf_grad_written_fn = self._marks.append      # held back until the join
@@ -68,18 +68,14 @@ class SideWork:
 
     def __exit__(self, *exc):
         if self.on:
-            K.stream_order(self.side, self.main)
-            self._held.clear()
+            if self._held:
+                K.stream_order(self.side, self.main)
+                self._held.clear()
             self.tape.leaf_grad_written_fn = self._saved_fn
             if self._saved_fn is not None and exc[0] is None:
                 for nid in self._marks:
                     self._saved_fn(nid)
         return False
-
-    def sees_main(self) -> None:
-        """The side stream waits for what the main stream holds now."""
-        if self.on:
-            K.stream_order(self.main, self.side)
 
     def wgrad(self, dy2d, x2d, out=None, accumulate=False):
         """Weight gradient GEMM on the main stream; its split-K reduction (if any) on the side stream."""
@@ -90,7 +86,6 @@ class SideWork:
     def colsum(self, dy2d, out=None, accumulate=False):
         if not self.on:
             return K.colsum(dy2d, out=out, accumulate=accumulate)
-        self._held.append(dy2d)
         return K.colsum(dy2d, out=out, accumulate=accumulate, stream=self.side, keep=self._held)
 
 
@@ -265,7 +260,6 @@ def mlp_up_down(tape: TensorTape, x: int, w1: int, b1: int, w2: int, b2: int, re
             db2 = _bgrad_into(targets, 4, g2, side)
             dw2 = _wgrad_into(targets, 3, g2, h, side)
             du = K.linear_dgrad(g2, w2v, epi=depi, resid=u)      # (dY @ w2) * act'(U)
-            side.sees_main()         # du is produced on the main stream, its columns are summed on the side stream
             db1 = _bgrad_into(targets, 2, du, side)
             dw1 = _wgrad_into(targets, 1, du, x2, side)
             dx = _as(K.linear_dgrad(du, w1v), xv)

@@ -184,12 +184,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if rc == 0:
             what = ("ftk::gemm2_bf16_sm100<256x%d,cta_group2,splitK=%d>" % (bn - 256, sp)) if bn > 256 else \
                 ("ftk::gemm_bf16_sm100<128x%d,splitK=%d>" % (bn, sp))
+    if ws is not None and reduce_stream is not None and keep is not None:
+        keep.append(ws)
     _chk(lib.gemm_packed(desc, _stream()), what)
-    if reduce_stream is not None and ws is not None:
-        if keep is not None:
-            keep.append(ws)
-        else:
-            ws.record_stream(torch.cuda.ExternalStream(reduce_stream, device=a.device))
+    if ws is not None and reduce_stream is not None and keep is None:
+        ws.record_stream(torch.cuda.ExternalStream(reduce_stream, device=a.device))
     return out
 
 
@@ -475,19 +474,25 @@ def dropout(x, p, seed, offset=0):
 def colsum(x, out=None, accumulate=False, *, stream: Optional[int] = None, keep: Optional[list] = None):
     """fp32 column sums of a bf16 ``[rows, cols]`` matrix (bias gradient), fixed order.
 
-    ``stream`` (a raw stream handle) launches there instead of on the current stream.  The scratch belongs to the current
-    stream all the same and goes to ``keep``, which the caller drops behind its join of that stream; so does an ``out`` that is
-    allocated here."""
+    ``stream`` (a raw stream handle) launches there instead of on the current stream, behind everything that the current
+    stream holds.  The scratch and an ``out`` that is allocated here come from the current stream's pool all the same; they go
+    to ``keep`` with ``x``, and the caller drops them behind its join of ``stream``."""
     rows, cols = x.shape
     lib = _lib.load()
     if out is None:
         out = x.new_empty(cols, dtype=torch.float32)
         accumulate = False
     partial = x.new_empty(lib.ftk_colsum_blocks(rows) * cols, dtype=torch.float32)
-    if keep is not None:
-        keep += (partial, out)
+    if stream is None:
+        stream = _stream()
+    else:
+        if keep is not None:
+            keep += (x, partial, out)
+        # Behind the allocations and directly ahead of the launch: a block of the current stream's pool may have been freed a
+        # moment ago, by another thread too, while a kernel of the current stream still reads or writes it.
+        stream_order(_stream(), stream)
     _chk(lib.ftk_colsum_bf16(x.data_ptr(), out.data_ptr(), partial.data_ptr(), rows, cols, x.stride(0),
-                             int(accumulate), _stream() if stream is None else stream), "ftk_colsum_bf16")
+                             int(accumulate), stream), "ftk_colsum_bf16")
     return out
 
 
