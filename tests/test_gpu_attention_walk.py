@@ -95,3 +95,25 @@ def test_backward_of_short_items(cuda_device, B, S, H, hd, causal):
     for got, ref in zip(view(first), _reference(q, k, v, go, causal)[1:]):
         assert got.isfinite().all()
         assert float((got.double() - ref).norm() / ref.norm()) < 1e-2      # as above
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,S,H,strides", [
+    (1, 200, 3, lambda S, H, hd: (S * H * hd + 1, H * hd, hd, 1)),      # one sequence of a buffer with an odd row
+    (1, 1, 5, lambda S, H, hd: (3, 7, hd, 1)),                          # one token: neither stride is stepped over
+    (1, 70, 1, lambda S, H, hd: (5, hd, 3, 1)),                         # one head
+    (1, 1, 1, lambda S, H, hd: (1, 1, 1, 1)),
+    (2, 130, 1, lambda S, H, hd: (S * hd, hd, 1, 1)),
+    (3, 1, 2, lambda S, H, hd: (2 * hd, 1, hd, 1)),
+])
+def test_output_strides_of_extents_of_one(cuda_device, B, S, H, strides, hd):
+    """A stride that nothing steps over may be anything, also one that is no multiple of 16 bytes."""
+    from frankentorch_b200.ops import kernels as K
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    q, k, v = (torch.randn(B, S, H, hd, generator=g, device=cuda_device).to(torch.bfloat16) for _ in range(3))
+    ref, ref_lse = K.attention_fwd(q, k, v, causal=True)
+    store = torch.full((B * S * H * hd + 64,), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    out, lse = K.attention_fwd(q, k, v, causal=True, out=store.as_strided((B, S, H, hd), strides(S, H, hd)))
+    K.check_status()
+    assert torch.equal(out, ref) and torch.equal(lse, ref_lse)
+    assert bool((store[B * S * H * hd:] == 7.0).all())
