@@ -69,6 +69,8 @@ int ftk_gemm_bf16(const FtkGemmDesc* g, void* stream);
 // Which kernel ftk_gemm_bf16 would launch: *bn = 128 / 192 / 256 (one CTA per 128 x bn tile) or 384 to 512
 // (CTA-pair kernel, tiles of 256 x (bn - 256), cta_group::2); *splits = split-K factor.  No launch.
 int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits);
+// Row blocks of 256 that its CTA-pair kernel walks as one group (all of them: m fastest), 0 for a single-CTA tile.  No launch.
+int ftk_gemm_walk(const FtkGemmDesc* g);
 // Work queued on stream `then` from here on waits for what stream `first` holds now (both of the current device).
 int ftk_stream_order(void* first, void* then);
 // `n` (1..8) products with one K and one pair of operand layouts, fp32 outputs (store or accumulate), no other

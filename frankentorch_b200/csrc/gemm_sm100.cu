@@ -158,16 +158,26 @@ static void set_divisors(GemmArgs& a, int bm, int bn) {
 // row blocks of A against one or two column blocks of B, and an A that is larger than what L2 keeps is read again for every
 // few columns: from memory, which costs time and, where the power limit sets the clock, the clock of the tensor pipe.  In
 // groups, the tiles in flight are a patch of the output and A is read once (B again for each group, but from L2 if it fits).
-// us in a loop at the power limit, m fastest / groups of 4 / of 8: 8192 x 2048 x 8192 240 / 218 / 216, 16384 x 2048 x 4096
-// 274 / 201 / 200, 16384 x 8192 x 4096 1040 / 839 / 819, 50304 x 768 x 8192 (weight gradient of a GPT-2 head) 620 / 499 / 519,
-// 50304 x 1024 x 4096 445 / 291 / 334.  An A of up to half of L2 stays there as it is and B streams past it once: 4096 x 4096 x
-// 4096 108 / 113 / 111, and 8192 x 50304 x 768, whose B is the larger operand, 535 / 585 / 549.
+// us, m fastest / groups of 4 / of 8, in bursts shorter than the power limit needs to act (in loops of 8 ms and more it lowers the
+// clock until all walks are within 4 % of each other): 8192 x 2048 x 8192 194 / 187 / 188, 16384 x 4096 x 4096 403 / 343 / 347,
+// 32768 x 8192 x 4096 1819 / 1523 / 1504, 65536 x 4096 x 1024 457 / 351 / 349; a weight gradient of a GPT-2 head, 50304 x 768 x 8192,
+// 465 / 411 (groups of 4).  An A of up to half of L2 stays there as it is and B streams past it once: 4096 x 4096 x 4096 108 / 113 /
+// 111 and 8192 x 50304 x 768, whose B is the larger operand, 535 / 585 / 549 (both in a loop).
+// A B beyond L2 comes from memory once per group, so there are half as many, of 16: m fastest / groups of 8 / of 16
+// 8192 x 50304 x 8192 5337 / 5587 / 5148, 8192 x 24576 x 8192 2515 / 2529 / 2376, 16384 x 32768 x 4096 3512 / 3322 / 2932,
+// 16384 x 12288 x 8192 (192 MB) 2722 / 2548 / 2393.  With fewer than 32 row blocks three or more column blocks are in flight
+// anyway, and a B of several times L2 is not worth reading again: 6144 x 50304 x 8192 3781 / 4064 / 3882, 6144 x 32768 x 8192
+// 2405 / 2506 / 2447, 4096 x 24576 x 16384 2442 / 2553.
+static uint32_t pair_group(long long M, long long N, long long K, uint32_t tm, uint32_t tn) {
+  const long long a = 2 * M * K, b = 2 * N * K, MB = 1ll << 20;
+  if (a <= 64 * MB || (tm < 32 && b > 320 * MB)) return tm;
+  const uint32_t gm = b > 128 * MB ? 16 : (tn < 16 ? 4 : 8);
+  return gm < tm ? gm : tm;
+}
+
 static void set_pair_groups(GemmArgs& a) {
   const uint32_t tm = a.by_tiles_m.d, tn = a.by_tiles_mn.d / tm;
-  uint32_t gm = tm;
-  if (2ll * a.M * a.K > (64ll << 20)) gm = tn < 16 ? 4 : 8;
-  if (gm > tm) gm = tm;
-  const uint32_t last = tm % gm ? tm % gm : gm;
+  const uint32_t gm = pair_group(a.M, a.N, a.K, tm, tn), last = tm % gm ? tm % gm : gm;
   a.by_group = FastDiv(gm * tn);
   a.by_gm = FastDiv(gm);
   a.by_gm_last = FastDiv(last);
@@ -552,6 +562,15 @@ extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
 extern "C" int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits) {
   if (!bn || !splits) return -2;
   return plan_gemm(g, bn, splits);
+}
+
+// Row blocks of 256 that the pair kernel would walk as one group for this problem (all of them: m fastest), 0 for a single-CTA
+// tile.  Launches nothing.
+extern "C" int ftk_gemm_walk(const FtkGemmDesc* g) {
+  int bn = 0, splits = 1;
+  const int rc = plan_gemm(g, &bn, &splits);
+  if (rc || bn <= 256) return rc;
+  return (int)pair_group(g->M, g->N, g->K, (uint32_t)((g->M + 255) / 256), (uint32_t)((g->N + bn - 257) / (bn - 256)));
 }
 
 // (one event per device and thread, re-recorded per call: another thread's record between this one's record and wait would

@@ -60,6 +60,22 @@ def test_widths_that_fill_the_last_wave():
     assert _plan(8192, 2304, 768)[:2] == (0, 512) and _plan(8192, 3072, 768)[:2] == (0, 448)
 
 
+@pytest.mark.parametrize("M,N,K,rows", [
+    (4096, 8192, 8192, 16),        # A is half of L2: m fastest over its 16 row blocks
+    (8192, 2048, 8192, 4), (16384, 8192, 4096, 8), (8192, 8192, 8192, 8),      # B within L2: it is read again from there
+    (8192, 8448, 8192, 16), (16384, 32768, 4096, 16), (8192, 50304, 8192, 16),      # B beyond L2: fewer passes over it
+    (6144, 12288, 8192, 16), (6144, 50304, 8192, 24), (4096, 24576, 16384, 16),      # several times L2, few row blocks: one pass
+])
+def test_row_block_groups_follow_both_operands(M, N, K, rows):
+    """A B beyond L2 is read from memory again for every group: groups of 8 took 8 % longer than none for 6144 x 50304 x 8192, 5 % for
+    8192 x 50304 x 8192."""
+    for b_mn in (0, 1):
+        assert _plan(M, N, K, b_mn=b_mn)[:2] == (0, 512)
+        assert _lib.load().ftk_gemm_walk(C.byref(_desc(M, N, K, b_mn=b_mn))) == rows
+    assert _lib.load().ftk_gemm_walk(C.byref(_desc(64, N, K))) == 0
+    assert _lib.load().ftk_gemm_walk(C.byref(_desc(0, N, K))) == -2
+
+
 def test_wide_tiles_of_a_group():
     """256 x 384 tiles where they fill the pairs and the reduction is long: the weight gradients of a block of 768 are 72 of them
     (144 CTAs) over 8192 rows, and 144 narrow ones on all CTAs over 512."""

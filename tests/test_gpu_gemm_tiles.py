@@ -241,3 +241,12 @@ def test_widths_of_an_odd_number_of_chunks_other_forms(cuda_device, bn):
     test_rows_without_aligned_segments(cuda_device, bn=bn, N=37, ldd=37, off=0)
     test_bf16_accumulation_and_residual_rows(cuda_device, bn=bn, kind="bias_gelu", ldr=73)
     test_row_block_groups(cuda_device, bn=bn, M=7 * 256, N=8 * 256 + 136, K=24576, splits=1)
+
+
+@pytest.mark.parametrize("bn", [256 + 160, 256 + 256])
+@pytest.mark.parametrize("M,N,K", [
+    (17 * 256 + 8, 8200, 8200),       # groups of sixteen for a B beyond L2, a last group of two
+    (22 * 256 + 136, 4352, 6144),     # groups of eight, a last group of seven
+])
+def test_row_block_groups_of_a_large_b(cuda_device, bn, M, N, K):
+    test_row_block_groups(cuda_device, bn=bn, M=M, N=N, K=K, splits=1)
