@@ -95,7 +95,7 @@ struct DkvCfg {
 // One persistent CTA per SM walks (key block, head, batch) items; every ring and every barrier runs on across items, so the
 // loads and the first score products of an item are issued under the last block and the output of the one before.  With one
 // CTA per item, set-up, first loads and output were ~15000 cycles per item against 1800 per block.
-template <int HD>
+template <int HD, bool LATE>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -402,8 +402,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     kb * AT_T + qd * 32, h, b, p.S);
       }
     };
-    // head_dim 64: an item's output leaves behind the first block of the next item, so the exponentials wait neither for its last
-    // products nor for the drain (between two items' blocks went ~3300 cycles, 800 of them for the products and 2100 for the
+    // LATE (head_dim 64): an item's output leaves behind the first block of the next item, so the exponentials wait neither for its
+    // last products nor for the drain (between two items' blocks went ~3300 cycles, 800 of them for the products and 2100 for the
     // output, where a block takes 1830: B8 S1024 H12 causal, five items a CTA, 45.7 -> 39.7 us).  head_dim 128: it is staged in
     // the dS^T tile and leaves at once (B4 S2048 H16 149 -> 142 us by the TMA stores alone).
     int late_kb = -1, late_b = 0, late_h = 0;
@@ -461,7 +461,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(pt_ready);      // one arrival per warp
-          if (late_kb >= 0) {                        // (acc_done of its last block was waited for above)
+          if (LATE && late_kb >= 0) {                // (acc_done of its last block was waited for above)
             drain(late_kb, late_b, late_h);
             late_kb = -1;
           }
@@ -500,7 +500,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         blk ^= 1u;
       }
       if (!ok) break;
-      if (C::TS) {
+      if (LATE) {
         late_kb = kb;
         late_b = b;
         late_h = h;
@@ -509,7 +509,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       drain(kb, b, h);
     }
-    if (ok && late_kb >= 0 && mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) drain(late_kb, late_b, late_h);
+    if (LATE && ok && late_kb >= 0 && mbar_wait_warp(acc_done, blk ^ 1u, ctx, FT_ERR_WAIT_TMEM_FULL)) drain(late_kb, late_b, late_h);
     if (lane == 0) bulk_wait_read_all();
   }
 
@@ -545,17 +545,17 @@ struct DqCfg {
   static_assert(SMEM <= 232448, "shared memory");
 };
 
-// Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.  Between two items: the Q and
-// dO tiles go back to the loader with the last score products, delta of the next item is made under the last dQ product, and
-// the output leaves through the K tile of the last block, which the loader gets back when it has left.  (Staged in the Q tile, with
-// one such buffer for head_dim 128, an item waited ~2500 cycles for its tiles and made delta behind them: B4 S2048 H16 causal
-// 111 -> 101 us, B8 S1024 H12 head size 64 43.2 -> 40.6 us.)
+// Persistent like the dK / dV kernel.  dS goes to the tensor core through tensor memory, two buffers.  Between two items (MANY: some
+// CTA has a second one): the Q and dO tiles go back to the loader with the last score products, delta of the next item is made
+// under the last dQ product, and the output leaves through the K tile of the last block, which the loader gets back when it has
+// left.  (Staged in the Q tile, with one such buffer for head_dim 128, an item waited ~2500 cycles for its tiles and made delta
+// behind them: B4 S2048 H16 causal 111 -> 101 us, B8 S1024 H12 head size 64 43.2 -> 40.6 us.)
 //
 // It also makes delta = rowsum(dO o O), which the dK / dV kernel behind it reads: dO is in shared memory here anyway and the
-// item's share of O is fetched one item ahead, so the sums run under the item's first score products.  (A kernel of its own
+// item's share of O is fetched one item ahead.  (A kernel of its own
 // in front of both read dO once more and stood on the path of the whole backward: B8 S1024 H12 head size 64 causal 75.1 -> 72.5 us,
 // B4 S2048 H16 head size 128 252 -> 246 us, B4 S128 H2 11.7 -> 10.4 us.)
-template <int HD>
+template <int HD, bool MANY>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -818,8 +818,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int qb = query_block(item), hb = item - (nkv_all - 1 - qb) * n_hb, b = p.by_h.div(hb), h = hb - b * p.H;
       const int q0 = qb * AT_T, grow = q0 + row, nkv = key_blocks(qb);
       const f32x2 nl = pk2(-lse_n, -lse_n);
-      item = walk.next();
-      fetch_rows(item);
+      item = MANY ? walk.next() : -1;
+      if (MANY) fetch_rows(item);
       if (!mbar_wait_warp(d_ready, it_ph, ctx, FT_ERR_WAIT_WARPS)) { ok = false; break; }
       const float dl_row = -s_delta[it_ph * AT_T + row];
       it_ph ^= 1u;
@@ -860,11 +860,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (lane == 0) mbar_arrive(&ds_ready[rd.s]);      // one arrival per warp
         rd.step();
         blk ^= 1u;
-        if (j == 0) output_left();
+        if (MANY && j == 0) output_left();
         if (j + 1 < nkv) rk.step();
       }
       // under the last product: delta of the next item (whose tiles were loaded under the last block)
-      if (ok && item >= 0) ok = make_delta(item, it_ph);
+      if (MANY && ok && item >= 0) ok = make_delta(item, it_ph);
       // the buffer of the last block is the one before rd
       if (!ok || !mbar_wait_warp(&acc_done[rd.s ^ 1], rd.s == 0 ? rd.ph ^ 1u : rd.ph, ctx, FT_ERR_WAIT_TMEM_FULL)) {
         ok = false;
@@ -913,16 +913,28 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   if (!p.status) return -6;
   static bool attr = false;
   if (!attr) {
-    if ((rc = set_smem(attn_bwd_dkv_kernel<HD>, DkvCfg<HD>::SMEM))) return rc;
-    if ((rc = set_smem(attn_bwd_dq_kernel<HD>, DqCfg<HD>::SMEM))) return rc;
+    if ((rc = set_smem(attn_bwd_dkv_kernel<HD, false>, DkvCfg<HD>::SMEM))) return rc;
+    if ((rc = set_smem(attn_bwd_dkv_kernel<HD, HD == 64>, DkvCfg<HD>::SMEM))) return rc;
+    if ((rc = set_smem(attn_bwd_dq_kernel<HD, true>, DqCfg<HD>::SMEM))) return rc;
+    if ((rc = set_smem(attn_bwd_dq_kernel<HD, false>, DqCfg<HD>::SMEM))) return rc;
     attr = true;
   }
   const long long nrows = (long long)a->B * a->S * a->H;
   if (nrows > 0x7fffffffll) return -2;
   unsigned grid = 0;
   if ((rc = set_items(p, a, AT_T, &grid))) return rc;
-  launch_pdl(attn_bwd_dq_kernel<HD>, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, tdq, p);      // writes delta
-  launch_pdl(attn_bwd_dkv_kernel<HD>, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, out, p);
+  // An item that ends under the next one costs its kernel's block loop registers: about 70 cycles of 1830 a block.  So where no CTA
+  // has a second item both kernels take the form without, and dK / dV ends an item at once also where 1100 cycles saved per item
+  // boundary are less than that (blocks per item: half of them under a causal mask).  us, always under the next / by this rule:
+  // B1 S4096 H4 causal 62.9 / 60.7, B1 S1024 H12 21.7 / 20.6, B8 S763 H3 20.1 / 19.1 (one item a CTA); B2 S1024 H12 causal 23.5 / 23.1,
+  // B1 S4096 H6 causal 65.3 / 64.3; ended at once / by this rule: B8 S256 H12 15.8 / 15.0, B4 S1024 H12 37.2 / 36.3.
+  const long long items = p.n_tiles, nb = (a->S + AT_T - 1) / AT_T;
+  const bool many = items > (long long)grid;
+  const bool late = HD == 64 && 32 * (items - (long long)grid) > items * (a->causal ? nb + 1 : 2 * nb);
+  auto dq = many ? attn_bwd_dq_kernel<HD, true> : attn_bwd_dq_kernel<HD, false>;
+  auto dkv = late ? attn_bwd_dkv_kernel<HD, HD == 64> : attn_bwd_dkv_kernel<HD, false>;
+  launch_pdl(dq, grid, BW_THREADS, DqCfg<HD>::SMEM, s, tq, tk, tv, tdo, tdq, p);      // writes delta
+  launch_pdl(dkv, grid, BW_THREADS, DkvCfg<HD>::SMEM, s, tq, tk, tv, tdo, out, p);
   return (int)cudaGetLastError();
 }
 

@@ -117,3 +117,16 @@ def test_output_strides_of_extents_of_one(cuda_device, B, S, H, strides, hd):
     K.check_status()
     assert torch.equal(out, ref) and torch.equal(lse, ref_lse)
     assert bool((store[B * S * H * hd:] == 7.0).all())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,S,H,causal", [
+    (4, 100, 37, True),        # 148 items: one for each CTA
+    (1, 64, 149, False),       # one item more, of one block
+    (1, 1920, 10, True),       # 150 items of up to fifteen blocks: a second item is seldom
+    (1, 2100, 12, False),      # 204 items of seventeen blocks: outputs leave at the end of their item
+    (2, 700, 31, True),        # 372 items of up to six blocks: under the next one
+])
+def test_forms_of_the_backward(cuda_device, B, S, H, causal, hd):
+    """Which form of the kernels runs follows from the number of items and of blocks; values as in the walk over items."""
+    test_walk_over_items(cuda_device, B=B, S=S, H=H, hd=hd, causal=causal)
