@@ -78,6 +78,7 @@ int ftk_stream_order(void* first, void* then);
 // GPU together where each alone would need split-K and a reduction kernel.
 int ftk_gemm_group_bf16(const FtkGemmDesc* descs, int n, void* stream);
 int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n);      // the CTAs it takes (<= max_ctas).  No launch.
+int ftk_gemm_group_width(const FtkGemmDesc* descs, int n);     // columns of its tiles, 0: the products in turn on one CTA.  No launch.
 
 // ---- GEMM fused with a collective over NVLink peer memory --------------------------------
 // One kernel: `comm_ctas` CTAs move shards / reduce partials while the rest run the GEMM.

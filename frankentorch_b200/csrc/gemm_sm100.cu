@@ -557,6 +557,13 @@ extern "C" int ftk_gemm_group_ctas(const FtkGemmDesc* descs, int n) {
   return plan_group(descs, n).ctas;
 }
 
+// Columns of its tiles: 192 or 384, or 0 where one CTA is all that max_ctas allows and the products run in turn.  Launches nothing.
+extern "C" int ftk_gemm_group_width(const FtkGemmDesc* descs, int n) {
+  if (!descs || n < 1 || n > GG_MAX) return -2;
+  const GroupPlan plan = plan_group(descs, n);
+  return plan.ctas < 2 ? 0 : plan.bn;
+}
+
 // Which kernel ftk_gemm_bf16 would launch for this problem: *bn = 128 / 192 / 256 (single-CTA tile 128 x bn) or
 // 384 to 512 in steps of 32 (CTA-pair kernel, tiles of 256 x (bn - 256)); *splits = split-K factor.  Launches nothing.
 extern "C" int ftk_gemm_plan(const FtkGemmDesc* g, int* bn, int* splits) {

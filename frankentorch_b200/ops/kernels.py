@@ -226,8 +226,12 @@ def gemm_grouped(problems, *, a_mn: bool = True, b_mn: bool = True, max_ctas: in
         g.B, g.ldb = b.data_ptr(), b.stride(0)
         g.D, g.ldd = out.data_ptr(), out.stride(0)
         g.alpha, g.out_fp32, g.accumulate, g.max_ctas = 1.0, 1, int(bool(accumulate)), int(max_ctas)
-    _chk(_lib.load().ftk_gemm_group_bf16(arr, n, _stream()),
-         "ftk::gemm_group_bf16_sm100<cta_group2,problems=%d>" % n)
+    lib, what = _lib.load(), "ftk_gemm_group_bf16"
+    if _TRACE is not None:          # name the tile the planner picks for these problems
+        w = lib.ftk_gemm_group_width(arr, n)
+        what = ("ftk::gemm_group_bf16_sm100<256x%d,cta_group2,problems=%d>" % (w, n)) if w else \
+            "ftk::gemm_bf16_sm100<128x192,problems=%d>" % n
+    _chk(lib.ftk_gemm_group_bf16(arr, n, _stream()), what)
 
 
 # Most bytes of partial tiles that the tile planner may spend on one product, and the reduction length up to which it never

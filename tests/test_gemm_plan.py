@@ -87,6 +87,34 @@ def test_wide_tiles_of_a_group():
         assert fn(arr, 4) == ctas
 
 
+def test_the_width_of_a_group_is_reported(monkeypatch):
+    """The trace of a grouped launch names the tile that the planner picks."""
+    import torch
+    from frankentorch_b200.ops import kernels as K
+    lib = _lib.load()
+
+    class Library:
+        def ftk_gemm_group_bf16(self, arr, n, stream):
+            return 0
+
+        def ftk_gemm_group_width(self, arr, n):
+            return lib.ftk_gemm_group_width(arr, n)
+
+    monkeypatch.setattr(K, "_bf16", lambda t, name: None)
+    monkeypatch.setattr(K, "_stream", lambda: 0)
+    monkeypatch.setattr(_lib, "load", lambda *a, **k: Library())
+    names = []
+    for rows, ctas in ((8192, 148), (512, 148), (8192, 1)):
+        probs = [(torch.empty(rows, m, dtype=torch.bfloat16), torch.empty(rows, n, dtype=torch.bfloat16), torch.empty(m, n), False)
+                 for m, n in ((2304, 768), (768, 768), (3072, 768), (768, 3072))]
+        K.trace_begin()
+        K.gemm_grouped(probs, max_ctas=ctas)
+        names += K.trace_end()
+    assert names == ["ftk::gemm_group_bf16_sm100<256x384,cta_group2,problems=4>",
+                     "ftk::gemm_group_bf16_sm100<256x192,cta_group2,problems=4>", "ftk::gemm_bf16_sm100<128x192,problems=4>"]
+    assert lib.ftk_gemm_group_width(None, 1) == -2
+
+
 @pytest.mark.gpu
 def test_a_group_on_one_cta(cuda_device):
     import torch

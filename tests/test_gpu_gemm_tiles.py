@@ -250,3 +250,33 @@ def test_widths_of_an_odd_number_of_chunks_other_forms(cuda_device, bn):
 ])
 def test_row_block_groups_of_a_large_b(cuda_device, bn, M, N, K):
     test_row_block_groups(cuda_device, bn=bn, M=M, N=N, K=K, splits=1)
+
+
+@pytest.mark.parametrize("mn", [True, False])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("pad", [4, 1])
+@pytest.mark.parametrize("K,ctas,width", [(4104, 4, 384), (4104, 0, 192), (136, 2, 192), (8200, 2, 384)])
+def test_both_widths_of_grouped_tiles(cuda_device, K, ctas, width, pad, accumulate, mn):
+    """The width that the case is meant for runs, and nothing is written beside the outputs, nor is anything of them left out."""
+    from frankentorch_b200.ops import kernels as k
+    probs, refs, stores = [], [], []
+    for i, (M, N) in enumerate([(264, 384), (520, 760), (256, 392), (304, 376)]):
+        a, b = _rand((K, M), 50 + i, cuda_device), _rand((K, N), 60 + i, cuda_device, K ** -0.5)
+        ref = a.double().t() @ b.double()
+        if not mn:
+            a, b = a.t().contiguous(), b.t().contiguous()
+        store = torch.full((M + 1, N + pad), 0.25, device=cuda_device)
+        if not accumulate:
+            store[:M, :N] = float("nan")
+        probs.append((a, b, store[:M, :N], accumulate))
+        refs.append(ref + 0.25 if accumulate else ref)
+        stores.append(store)
+    k.trace_begin()
+    k.gemm_grouped(probs, a_mn=mn, b_mn=mn, max_ctas=ctas)
+    assert k.trace_end() == ["ftk::gemm_group_bf16_sm100<256x%d,cta_group2,problems=4>" % width]
+    k.check_status()
+    for store, ref in zip(stores, refs):
+        M, N = ref.shape
+        assert bool((store[M:] == 0.25).all()) and bool((store[:, N:] == 0.25).all())
+        # fp32 sums of K products whose squares add up to about one
+        assert float((store[:M, :N].double() - ref).abs().max()) <= K * 2.0 ** -24 + 2.0 ** -20 * float(ref.abs().max())
