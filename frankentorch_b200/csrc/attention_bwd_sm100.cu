@@ -908,7 +908,7 @@ static int attn_bwd_launch(const FtkAttnDesc* a, cudaStream_t s) {
   if ((rc = make_map(&tdq, a->dq, a, a->q_bs, a->q_ss, a->q_hs, 32, 32))) return rc;
   if ((rc = make_map(&out.m[1], a->dk, a, a->k_bs, a->k_ss, a->k_hs, 32, 32))) return rc;
   if ((rc = make_map(&out.m[0], a->dv, a, a->v_bs, a->v_ss, a->v_hs, 32, 32))) return rc;
-  AttnArgs p;
+  AttnArgs p{};
   fill_args(p, a);
   if (!p.status) return -6;
   static bool attr = false;

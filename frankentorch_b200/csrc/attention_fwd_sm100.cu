@@ -464,7 +464,7 @@ static int attn_fwd2_launch(const FtkAttnDesc* a, cudaStream_t s) {
   if ((rc = make_map(&tv, a->v, a, a->v_bs, a->v_ss, a->v_hs))) return rc;
   // (the stride of an extent of one is never stepped over and may be anything)
   if ((rc = make_map(&to, a->o, a, a->B > 1 ? a->o_bs : 0, a->S > 1 ? a->o_ss : a->hd, a->H > 1 ? a->o_hs : 0, 64, 32))) return rc;
-  AttnArgs p;
+  AttnArgs p{};
   fill_args(p, a);
   if (!p.status) return -6;
   static bool attr = false;

@@ -20,12 +20,13 @@ struct AttnArgs {
   int causal;
   float sl2;    // scale * log2(e)
   float scale;
-  __nv_bfloat16* o;
+  const __nv_bfloat16* o;      // read by the dQ kernel (outputs leave through tensor maps)
   long long o_bs, o_ss, o_hs;
   float* lse;
   float* delta;             // written by the dQ kernel, read by the dK / dV kernel
-  __nv_bfloat16 *dq, *dk, *dv;
-  long long dq_bs, dq_ss, dq_hs, dk_bs, dk_ss, dk_hs, dv_bs, dv_ss, dv_hs;
+  // Nothing reads these 96 bytes.  Without them the compiler allocates the registers of the backward loops of head size 64 another
+  // way (dK / dV spills 8 bytes, dQ takes 83 instead of 85): B1 S4096 H6 causal 65.4 -> 67.5 us, B8 S256 H12 causal 14.9 -> 14.5.
+  long long unused[12];
   int* status;
   int n_tiles;             // work items of the persistent kernels: blocks of rows x heads x batch
   FastDiv by_hb, by_h;     // / (H * B), / H
@@ -155,15 +156,9 @@ static inline void fill_args(AttnArgs& p, const FtkAttnDesc* a) {
   p.B = a->B; p.H = a->H; p.S = a->S; p.causal = a->causal;
   p.scale = a->scale;
   p.sl2 = a->scale * 1.4426950408889634f;
-  p.o = reinterpret_cast<__nv_bfloat16*>(a->o);
+  p.o = reinterpret_cast<const __nv_bfloat16*>(a->o);
   p.o_bs = a->o_bs; p.o_ss = a->o_ss; p.o_hs = a->o_hs;
   p.lse = a->lse; p.delta = a->delta;
-  p.dq = reinterpret_cast<__nv_bfloat16*>(a->dq);
-  p.dk = reinterpret_cast<__nv_bfloat16*>(a->dk);
-  p.dv = reinterpret_cast<__nv_bfloat16*>(a->dv);
-  p.dq_bs = a->q_bs; p.dq_ss = a->q_ss; p.dq_hs = a->q_hs;
-  p.dk_bs = a->k_bs; p.dk_ss = a->k_ss; p.dk_hs = a->k_hs;
-  p.dv_bs = a->v_bs; p.dv_ss = a->v_ss; p.dv_hs = a->v_hs;
   p.status = ftk_status_word();
 }
 
