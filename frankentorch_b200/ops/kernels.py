@@ -480,23 +480,27 @@ def colsum(x, out=None, accumulate=False, *, stream: Optional[int] = None, keep:
 
     ``stream`` (a raw stream handle) launches there instead of on the current stream, behind everything that the current
     stream holds.  The scratch and an ``out`` that is allocated here come from the current stream's pool all the same; they go
-    to ``keep`` with ``x``, and the caller drops them behind its join of ``stream``."""
+    to ``keep`` with ``x``, and the caller drops them behind its join of ``stream``.  Without ``keep`` the allocator holds their
+    memory back until ``stream`` is done with it."""
     rows, cols = x.shape
     lib = _lib.load()
     if out is None:
         out = x.new_empty(cols, dtype=torch.float32)
         accumulate = False
     partial = x.new_empty(lib.ftk_colsum_blocks(rows) * cols, dtype=torch.float32)
-    if stream is None:
-        stream = _stream()
-    else:
+    aside = stream is not None
+    if aside:
         if keep is not None:
             keep += (x, partial, out)
         # Behind the allocations and directly ahead of the launch: a block of the current stream's pool may have been freed a
         # moment ago, by another thread too, while a kernel of the current stream still reads or writes it.
         stream_order(_stream(), stream)
     _chk(lib.ftk_colsum_bf16(x.data_ptr(), out.data_ptr(), partial.data_ptr(), rows, cols, x.stride(0),
-                             int(accumulate), stream), "ftk_colsum_bf16")
+                             int(accumulate), stream if aside else _stream()), "ftk_colsum_bf16")
+    if aside and keep is None:
+        other = torch.cuda.ExternalStream(stream, device=x.device)
+        for t in (x, partial, out):
+            t.record_stream(other)
     return out
 
 

@@ -118,6 +118,19 @@ def test_kernels_of_another_device_keep_to_one_stream(fake, monkeypatch):
     assert [e for e in fake.events if e[0] != "take"] == [("sum", MAIN)]
 
 
+def test_column_sums_aside_without_a_list(fake, monkeypatch):
+    """A caller that keeps nothing: the memory of operand, scratch and result is held back until the other stream is done with it."""
+    recorded = []
+    monkeypatch.setattr(torch.cuda, "ExternalStream", lambda handle, device=None: handle)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, s: recorded.append((t.numel(), s)), raising=False)
+    dy = torch.zeros(16, 8, dtype=torch.bfloat16)
+    out = K.colsum(dy, stream=SIDE)
+    assert sorted(recorded) == [(out.numel(), SIDE), (2 * 8, SIDE), (dy.numel(), SIDE)]
+    K.colsum(dy)
+    K.colsum(dy, stream=SIDE, keep=[])
+    assert len(recorded) == 3
+
+
 # ------------------------------------------------------------------------------------------------ the rules on a GPU
 NAMES = ("x", "w0", "b0", "w1", "b1", "w2", "b2")
 
@@ -188,3 +201,21 @@ def test_two_threads_on_one_stream(cuda_device, monkeypatch, bound):
     [t.join() for t in ts]
     K.check_status()
     assert not errors and bad == [0, 0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kept", [True, False])
+def test_column_sums_on_another_stream(cuda_device, kept):
+    side = torch.cuda.Stream(cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(11)
+    for rows, cols in ((4096, 3072), (300, 136), (1, 8)):
+        x = torch.randn(rows, cols, generator=g, device=cuda_device).to(torch.bfloat16)
+        ref = K.colsum(x)
+        for _ in range(20):
+            keep = [] if kept else None
+            got = K.colsum(x.clone(), stream=side.cuda_stream, keep=keep)
+            junk = [torch.full((n,), 7.0, device=cuda_device) for n in (cols, 2 * cols, 64 * cols, rows * cols // 2 + 1)]
+            torch.cuda.current_stream().wait_stream(side)
+            assert torch.equal(got, ref)
+            del keep, junk
+    K.check_status()
