@@ -417,9 +417,9 @@ static int plan_gemm(const FtkGemmDesc* g, int* bn_out, int* splits_out) {
   for (int bi = 0; bi < 8; ++bi) {
     if (bn_opts[bi] > 256 && (sms < 2 || g->M < 256 || g->seg_counts)) continue;
     if (g->force_bn && bn_opts[bi] != g->force_bn) continue;
-    // 160 and 224 columns fill the last wave of forward products (1500 x 3840 x 1280 in 144 tiles of 160 14.0 us, 120 of 192
-    // 15.0; 1500 x 5120 x 1280 in 138 of 224 17.3, 120 of 256 19.0).  A half of 80 or 112 columns of a B given [K, N] loads 128
-    // all the same, and nothing is gained (17.2 and 17.5, 21.7 and 20.5).
+    // 160 and 224 columns fill the last wave of forward products: with bias, in a captured loop with the operands in L2, 1500 x 3840 x
+    // 1280 in 144 tiles of 160 12.6 us, 120 of 192 13.5; 1500 x 5120 x 1280 in 138 of 224 15.2, 120 of 256 16.6.  A half of 80 or 112
+    // columns of a B given [K, N] loads 128 all the same, and nothing is gained: in a sequence of calls 17.2 and 17.5, 21.7 and 20.5.
     if ((bn_opts[bi] == 416 || bn_opts[bi] == 480) && g->b_mn && !g->force_bn) continue;
     for (int si = 0; si < 8; ++si) {
       const int s = s_opts[si];
